@@ -36,6 +36,11 @@ constexpr int TILE = 32;
 #define BK_EPS ((double)1e-15f)
 #define BK_ZERO_THRESHOLD ((double)1e-35f)
 
+// Grow rounds (bk_rounds.cuh).
+constexpr int kMaxRoundW = 16;        // leaves expanded per round at most
+constexpr int kMaxRoundOut = 32;      // expanded leaves that wait for their split at most
+constexpr int kMaxRoundLeaves = 512;  // leaves a decision keeps in shared memory
+
 struct DevFeature {
   int32_t num_bin, missing, default_bin, mfb;
   int32_t offset;  // 1 when the most frequent bin is 0 (its bin is not in the histogram slice)
@@ -101,6 +106,13 @@ struct Params {
   int32_t n_icons;     // interaction constraints: how many feature sets, of `path_words` words each
   int32_t path_words;  // words of a feature bitset: ceil(F / 32)
   const uint32_t* icons;  // [n_icons][path_words] inner-feature bitsets
+  // grow rounds (bk_rounds.cuh)
+  int32_t round_w, round_out;  // leaves expanded per round at most; expanded leaves not yet split at most
+  int32_t max_exp;             // expansions of one tree at most: num_leaves - 1 + round_out
+  int32_t n_groups;            // feature groups of a round's search, one candidate each
+  int32_t n_numeric, unit_penalty;  // numerical features (first in `order`); every feature's penalty is 1
+  const int32_t* order;        // [F] inner features: the numerical ones, then the categorical ones
+  int32_t cand_rows;           // rows of Job::cand and Job::splittable: 1 + 2 max_exp nodes
 };
 
 // Per-leaf constants of one searched leaf (FindBestThreshold's preamble, feature_histogram.rs:
@@ -110,7 +122,10 @@ struct LeafConst {
   int64_t first_x, brk_x;  // quantized path: validity thresholds on the accumulated hessian
   float mgs_up, mgs_dn;    // min_gain_shift rounded up / down to fp32
   float gsf, hsf, l2f;     // fp32 copies of the gradient / hessian scales and lambda_l2
-  float _pad;
+  // the warp search's bounds (bk_search_warp.cuh): hs2 = h + 2 lambda_l2, the error bound's factor
+  // and constant (bk1 < 0: the leaf is outside its range), min_gain_shift - s0 rounded up / down
+  float hs2, bk1, bk0, d_up, d_dn;
+  int32_t go;              // 0: the leaf is not searched (grow rounds: 1 the left child, 2 the right child)
   double gs, hs;           // quantized path: the gradient / hessian scales
   LeafSum ls;              // the leaf's sums (its LeafSplits), as leaf_sum[leaf] holds them
 };
@@ -140,6 +155,7 @@ struct JobState {
   uint32_t col_rng;
   int32_t bytree_on;
   double bynode_fraction;
+  int32_t fin_q, _pad;  // grow rounds: which copy of the rounds' state the tree ended in
   uint32_t mt[624];
 };
 
@@ -179,6 +195,7 @@ struct Job {
   int64_t* part_cnt;   // [part_grid] partition block counts (scratch)
   double* red;         // reduction partials (scratch)
   int64_t* ired;       // integer reduction partials (scratch)
+  uint8_t* rounds;     // the grow rounds' state (RoundView in bk_rounds.cuh)
 };
 
 // The jobs of one grow-loop launch, passed by value: the kernel parameters sit in the constant
@@ -203,13 +220,11 @@ inline void for_job_groups(const Job* h_jobs, int num_jobs, F f) {
   }
 }
 
-// The bin bitsets of categorical candidates, stored after the [L][F] candidates in the same
+// The bin bitsets of categorical candidates, stored after the candidates in the same
 // allocation (8 words per (leaf, feature); written only by categorical searches).
-__host__ __device__ __forceinline__ size_t cand_cat_words(int num_leaves, int F) {
-  return (size_t)num_leaves * (size_t)F * 8;
-}
+__host__ __device__ __forceinline__ size_t cand_cat_words(int rows, int F) { return (size_t)rows * (size_t)F * 8; }
 __device__ __forceinline__ uint32_t* cand_cat_bits(const Job& J, const Params& p, int32_t leaf, int32_t f) {
-  return reinterpret_cast<uint32_t*>(J.cand + (size_t)p.num_leaves * p.F) + ((size_t)leaf * p.F + f) * 8;
+  return reinterpret_cast<uint32_t*>(J.cand + (size_t)p.cand_rows * p.F) + ((size_t)leaf * p.F + f) * 8;
 }
 
 // The features on the path to `leaf` (SerialTreeLearner::branch_features, serial.rs:233-234) as a
@@ -249,6 +264,18 @@ size_t hist_smem_bytes(const Params& p, int threads, bool quant, bool wide);
 
 // The bookkeeping of the last split of a tree partitioned in one pass (counter pair `par`).
 void launch_apply_split(const Job* h_jobs, int num_jobs, const Params& p, int par, cudaStream_t s);
+// A grow round's three launches (bk_rounds.cuh), q the round's parity, and the tree's finish: leaf
+// arrays and records from the committed splits (jobs that are not done are left alone).
+void launch_hist_round(const Job* h_jobs, int num_jobs, const Params& p, const uint8_t* bins_rt,
+                       const uint8_t* bins_tm, const HistLaunch& hl, int q, cudaStream_t s);
+void launch_search_round(const Job* h_jobs, int num_jobs, const Params& p, const DevFeature* feats, int q,
+                         cudaStream_t s);
+void launch_partition_round(const Job* h_jobs, int num_jobs, const Params& p, const uint8_t* bins_cm,
+                            const DevFeature* feats, int q, cudaStream_t s);
+void launch_rounds_finish(const Job* h_jobs, int num_jobs, const Params& p, cudaStream_t s);
+size_t rounds_state_bytes(int num_leaves, int max_exp, int F);
+// Feature groups of a round's search for this configuration (Params::n_groups).
+int rounds_groups(const Params& p);
 // clear_par >= 0: the launch zeroes that single-pass partition counter pair first. decide: its
 // last CTA decides and records the split (else the single-pass partition decides it).
 void launch_search(const Job* h_jobs, int num_jobs, const Params& p, const DevFeature* feats, int clear_par,
@@ -270,8 +297,11 @@ void launch_root_sums(const Job* d_jobs, int num_jobs, const Params& p, int exac
 void launch_renew(const Job* d_jobs, int num_jobs, const Params& p, cudaStream_t s);
 void launch_add_score(const Job* d_jobs, int num_jobs, const Params& p, const double* leaf_vals, double* score,
                       cudaStream_t s);
-void launch_add_score_own(const Job* d_jobs, int num_jobs, const Params& p, double rate, double* score,
+// need_stop: nothing is added unless every job's tree is finished (JobState::stop)
+void launch_add_score_own(const Job* d_jobs, int num_jobs, const Params& p, double rate, double* score, int need_stop,
                           cudaStream_t s);
+// Zeroes the first `bytes` bytes (a multiple of 16) of every job's histogram pool.
+void launch_zero_pool(void* pool, size_t bytes_per_job, size_t bytes, int num_jobs, cudaStream_t s);
 void launch_row_leaf(const Job* d_jobs, int num_jobs, const Params& p, int32_t* out, cudaStream_t s);
 void launch_mt_seed(const Job* d_jobs, int num_jobs, uint32_t seed, cudaStream_t s);
 constexpr int kRootGrid = 256;
@@ -292,6 +322,7 @@ cudaError_t objective_gradients(int kind, const double* score, const float* labe
                                 const ObjectiveWeights& ow, float* g, float* h, int32_t* bad_label, cudaStream_t s);
 cudaError_t objective_loss(int kind, const double* score, const float* label, int64_t n, int K, double* partial,
                            int grid, int32_t* bad_label, cudaStream_t s);
-void launch_tree_begin(const Job* d_jobs, int num_jobs, const Params& p, cudaStream_t s);
+// rounds: the tree grows in rounds (bk_rounds.cuh), else one split at a time
+void launch_tree_begin(const Job* d_jobs, int num_jobs, const Params& p, bool rounds, cudaStream_t s);
 
 }  // namespace bk

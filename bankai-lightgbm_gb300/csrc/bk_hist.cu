@@ -389,7 +389,8 @@ __device__ __forceinline__ void hist_int_loop(const Params& p, const Range& R, c
 template <bool WIDE, bool NIBBLE>
 __device__ __forceinline__ void hist_int_rows(const Job& J, const Params& p, const Range& R, const TileGeom& geo,
                                               const uint8_t* __restrict__ bins_rt, const uint8_t* __restrict__ bins_tm,
-                                              int flush_rounds, int direct_rows, bool in_cluster, unsigned char* smem) {
+                                              int flush_rounds, int direct_rows, bool in_cluster, unsigned char* smem,
+                                              bool more = false) {
   const int tile = blockIdx.y;
   const int Bt = geo.bins;
   const IntHist<WIDE> H{smem, Bt};
@@ -416,6 +417,11 @@ __device__ __forceinline__ void hist_int_rows(const Job& J, const Params& p, con
       const uint32_t s = H.hot()[gi];
       gg += hot_g(s);
       hh += (int32_t)(s & 0xffffu);
+    }
+    if (more) {  // the CTA's next rows belong to another leaf
+      H.cold_g()[gi] = 0;
+      H.cold_h()[e] = 0;
+      if (!WIDE) H.hot()[gi] = 0u;
     }
     if (gg | hh) {
       int64_t pk = (int64_t)gg * 4294967296LL + (int64_t)hh;
@@ -502,6 +508,116 @@ __global__ void __launch_bounds__(1024, 1)
   }
 }
 
+// ---- grow rounds (bk_rounds.cuh): the smaller children of up to kMaxRoundW expansions ----
+// The children's rows, one after the other, are cut into gridDim.x equal intervals (at least
+// hist_min_rows rows each), so every CTA of a tile takes the same number of rows whatever the
+// leaves' sizes; a CTA whose interval crosses from one leaf into the next flushes and clears its
+// shared histogram there. round_cut() starts every leaf at an interval of its own where that costs
+// little (small rounds): a second leaf costs its CTA a pass of its own.
+struct RoundRows {
+  int64_t off[kMaxRoundW];  // where expansion e's rows start among all
+  int32_t begin[kMaxRoundW], count[kMaxRoundW], buf[kMaxRoundW], slot[kMaxRoundW];
+  int32_t n, root;
+  RoundCut cut;
+};
+
+// Every thread calls it, between the launch's wait and its rows; ends with a barrier. The search
+// constants of expansion e are computed by the last two warps of one CTA per expansion, spread over
+// the grid from its end (whose CTAs are the ones without rows when there are few), before the rows
+// of those warps.
+__device__ __forceinline__ void round_rows(const Job& J, const Params& p, int q, RoundRows* s) {
+  const RoundView v = round_view(J, p);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  if (warp == 0) {
+    const int n_cur = __ldcg(&v.hdr[q].n_cur);
+    int32_t rows = 0;
+    if (lane < kMaxRoundW) {  // loaded with the count (stale past it), not after it
+      const RoundExp c = v.cur[q * kMaxRoundW + lane];
+      const int32_t L = (int32_t)__ldcg(v.pcnt + ((size_t)q * kMaxRoundW + lane) * 2);
+      const HistPart h = round_hist_part(p, c, L);
+      if (lane < n_cur) {
+        rows = h.go ? h.count : 0;
+        s->begin[lane] = h.begin;
+        s->count[lane] = rows;
+        s->buf[lane] = h.buf;
+        s->slot[lane] = h.slot;
+        if (lane == 0) s->root = c.x < 0;
+      }
+    }
+    int64_t off;
+    const RoundCut cut = round_cut(rows, n_cur, (int)gridDim.x, p.hist_min_rows, 32, 2048, lane, &off);
+    if (lane < n_cur) s->off[lane] = off;
+    if (lane == 0) {
+      s->n = n_cur;
+      s->cut = cut;
+    }
+  } else if (warp >= nwarps - 2) {
+    const int cta = (int)(gridDim.x - 1 - blockIdx.x) * (int)gridDim.y + (int)blockIdx.y;  // from the grid's end
+    const int ctas = (int)(gridDim.x * gridDim.y);
+    if (cta < kMaxRoundW) {
+      const int n_cur = __ldcg(&v.hdr[q].n_cur);
+      for (int e = cta; e < n_cur; e += ctas) {
+        const RoundExp c = v.cur[q * kMaxRoundW + e];
+        const int32_t L = (int32_t)__ldcg(v.pcnt + ((size_t)q * kMaxRoundW + e) * 2);
+        round_leaf_constants(J, p, c, L, e, warp - (nwarps - 2), lane);
+      }
+    }
+  }
+}
+
+// The part of this CTA's interval that lies in expansion e: false when it has no row of it. `last`:
+// no later leaf has rows in the interval.
+__device__ __forceinline__ bool round_segment(const Job& J, const Params& p, const RoundRows& s, int e, Range* r,
+                                              bool* single, bool* last) {
+  const int64_t q0 = (int64_t)blockIdx.x * s.cut.per, q1 = q0 + s.cut.per;
+  const int64_t off = s.off[e];
+  const int64_t a = max(q0, off), b = min(q1, off + s.count[e]);
+  if (a >= b) return false;
+  r->r0 = a - off;
+  r->r1 = b - off;
+  r->count = s.count[e];
+  r->idx = leaf_idx(J, s.buf[e]) + s.begin[e];
+  r->direct = r->count == p.n;  // all rows in order: the index buffer is the identity
+  r->pk_row = s.root != 0;      // the root: no leaf-ordered copy yet
+  r->pk = r->pk_row ? J.packed : (J.pk0 ? leaf_pk(J, s.buf[e]) + s.begin[e] : nullptr);
+  r->slot = s.slot[e];
+  *last = s.cut.apart || b == q1 || e == s.n - 1;
+  *single = *last && a == q0;
+  return true;
+}
+
+template <bool WIDE>
+__global__ void __launch_bounds__(1024, 1)
+    k_hist_int_round(const JobTable jobs, Params p, const uint8_t* __restrict__ bins_rt,
+                     const uint8_t* __restrict__ bins_tm, int flush_rounds, int direct_rows, int q) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ RoundRows rows;
+  const TileGeom geo = p.tiles[blockIdx.y];  // static: loaded while the previous kernel finishes
+  {
+    uint4* z = reinterpret_cast<uint4*>(smem);
+    const int n16 = (WIDE ? 2 : 3) * geo.bins * TILE / 4;
+    for (int e = threadIdx.x; e < n16; e += blockDim.x) z[e] = make_uint4(0, 0, 0, 0);
+  }
+  griddep_wait();
+  griddep_launch();
+  const Job& J = jobs.job[blockIdx.z];
+  round_rows(J, p, q, &rows);
+  __syncthreads();
+  for (int e = 0; e < rows.n; ++e) {
+    Range R;
+    bool single, last;
+    if (!round_segment(J, p, rows, e, &R, &single, &last)) continue;
+    // a CTA that adds straight to the pool slot stages its rows over the shared histogram, so it
+    // takes rows of one leaf only
+    const int direct = single ? direct_rows : -1;
+    if (geo.nibble)
+      hist_int_rows<WIDE, true>(J, p, R, geo, bins_rt, bins_tm, flush_rounds, direct, false, smem, !last);
+    else
+      hist_int_rows<WIDE, false>(J, p, R, geo, bins_rt, bins_tm, flush_rounds, direct, false, smem, !last);
+    if (last) break;
+  }
+}
+
 // Adds one row's gradient (and hessian) to the fp32 (hi, lo) pairs of bin `e`: hi takes the
 // value by atomicAdd, which returns the previous sum, and lo the exact rounding error of that
 // addition (TwoSum); with a constant hessian the hessian slot counts rows.
@@ -568,7 +684,8 @@ __device__ __forceinline__ void add_own_row_float(float* ghi, float* glo, float*
 template <bool CONST_HESS, bool NIBBLE>
 __device__ __forceinline__ void hist_float_rows(const Job& J, const Params& p, const Range& R, const TileGeom& geo,
                                                 const uint8_t* __restrict__ bins_rt,
-                                                const uint8_t* __restrict__ bins_tm, unsigned char* smem) {
+                                                const uint8_t* __restrict__ bins_tm, unsigned char* smem,
+                                                bool more = false) {
   const int tile = blockIdx.y;
   const int B = geo.bins;
   const bool half = geo.width == 16;  // one 16-byte run per row
@@ -630,6 +747,39 @@ __device__ __forceinline__ void hist_float_rows(const Job& J, const Params& p, c
       atomicAdd(&slot[e].x, gs);
       atomicAdd(&slot[e].y, hs);
     }
+    if (more) {  // the CTA's next rows belong to another leaf
+      ghi[e] = glo[e] = hhi[e] = 0.f;
+      if (!CONST_HESS) hlo[e] = 0.f;
+    }
+  }
+}
+
+template <bool CONST_HESS>
+__global__ void __launch_bounds__(1024, 1)
+    k_hist_float_round(const JobTable jobs, Params p, const uint8_t* __restrict__ bins_rt,
+                       const uint8_t* __restrict__ bins_tm, int q) {
+  extern __shared__ __align__(16) unsigned char smem[];
+  __shared__ RoundRows rows;
+  const TileGeom geo = p.tiles[blockIdx.y];  // static: loaded while the previous kernel finishes
+  {
+    uint4* z = reinterpret_cast<uint4*>(smem);
+    const int n16 = (CONST_HESS ? 3 : 4) * geo.bins * TILE / 4;
+    for (int e = threadIdx.x; e < n16; e += blockDim.x) z[e] = make_uint4(0, 0, 0, 0);
+  }
+  griddep_wait();
+  griddep_launch();
+  const Job& J = jobs.job[blockIdx.z];
+  round_rows(J, p, q, &rows);
+  __syncthreads();
+  for (int e = 0; e < rows.n; ++e) {
+    Range R;
+    bool single, last;
+    if (!round_segment(J, p, rows, e, &R, &single, &last)) continue;
+    if (geo.nibble)
+      hist_float_rows<CONST_HESS, true>(J, p, R, geo, bins_rt, bins_tm, smem, !last);
+    else
+      hist_float_rows<CONST_HESS, false>(J, p, R, geo, bins_rt, bins_tm, smem, !last);
+    if (last) break;
   }
 }
 
@@ -690,6 +840,25 @@ void launch_hist(const Job* h_jobs, int num_jobs, const Params& p, const uint8_t
   });
 }
 
+void launch_hist_round(const Job* h_jobs, int num_jobs, const Params& p, const uint8_t* bins_rt,
+                       const uint8_t* bins_tm, const HistLaunch& hl, int q, cudaStream_t s) {
+  for_job_groups(h_jobs, num_jobs, [&](const JobTable& t, int nz) {
+    const dim3 grid(hl.blocks_per_tile, p.T, nz), block(hl.threads);
+    if (p.quant) {
+      if (hl.flush_rounds > 0)
+        (void)launch_kernel(k_hist_int_round<false>, grid, block, hl.smem, s, p.pdl, t, p, bins_rt, bins_tm,
+                            hl.flush_rounds, hl.direct_rows, q);
+      else
+        (void)launch_kernel(k_hist_int_round<true>, grid, block, hl.smem, s, p.pdl, t, p, bins_rt, bins_tm, 1,
+                            hl.direct_rows, q);
+    } else if (p.const_hess) {
+      (void)launch_kernel(k_hist_float_round<true>, grid, block, hl.smem, s, p.pdl, t, p, bins_rt, bins_tm, q);
+    } else {
+      (void)launch_kernel(k_hist_float_round<false>, grid, block, hl.smem, s, p.pdl, t, p, bins_rt, bins_tm, q);
+    }
+  });
+}
+
 cudaError_t hist_set_smem_attrs(size_t smem) {
   // The attribute belongs to the kernel on the current device: remember the largest value set on
   // each device and only ever raise it, so learners created earlier with larger tiles keep working.
@@ -707,6 +876,13 @@ cudaError_t hist_set_smem_attrs(size_t smem) {
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_hist_int<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_hist_float<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_hist_float<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_hist_int_round<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_hist_int_round<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_hist_float_round<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_hist_float_round<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
   if (e == cudaSuccess) current[dev] = smem;
   return e;
 }

@@ -7,6 +7,7 @@
 #include "bk_common.cuh"
 #include "bk_grow.cuh"
 #include "bk_math.cuh"
+#include "bk_rounds.cuh"
 
 namespace bk {
 
@@ -75,9 +76,10 @@ __device__ __forceinline__ double parent_output_of(const Params& p, bool root, c
 }
 
 // One warp: the constants of side `side` (0 = smaller leaf, 1 = larger leaf) of the coming search,
-// for a leaf with sums `ls` (`root`: the tree's only leaf).
+// for a leaf with sums `ls` (`root`: the tree's only leaf). In a grow round `side` is 2 e + side for
+// expansion e, and `go` says which child of the leaf it is.
 __device__ __forceinline__ void compute_leaf_const_ls(const Job& J, const Params& p, const JobState* st, int side,
-                                                      const LeafSum& ls, bool root, int lane) {
+                                                      const LeafSum& ls, bool root, int lane, int32_t go = 1) {
   LeafConst c;
   c.first_x = c.brk_x = 0;
   if (p.quant) {
@@ -95,10 +97,26 @@ __device__ __forceinline__ void compute_leaf_const_ls(const Job& J, const Params
   c.mgs = leaf_gain(p, c.sum_g, c.sum_h, ls.num_data, c.parent) + p.min_gain;
   c.mgs_up = __double2float_ru(c.mgs);
   c.mgs_dn = __double2float_rd(c.mgs);
+  {
+    // without lambda_l2, s0 is the leaf's own gain (up to its rounding, which the bounds allow for)
+    const double h2 = c.sum_h + 2.0 * p.l2;
+    const double s0 = p.l2 == 0.0 ? c.mgs - p.min_gain : c.sum_g * c.sum_g / h2;
+    const double d = p.l2 == 0.0 ? p.min_gain : c.mgs - s0;
+    c.hs2 = (float)h2;
+    const float ymin = (float)(p.min_hess + p.l2), s0f = (float)s0, arel = 4e-15f + 1.01e-15f / ymin;
+    c.bk1 = 44.0f * 5.9604645e-08f + arel;
+    c.bk0 = s0f * arel + 1e-24f;
+    if (!(ymin >= 1e-6f) || !(c.hs2 <= 1e10f) || !(s0f < 1e30f) ||
+        (p.quant && (ls.int_sum & 0xffffffffLL) >= 0x80000000LL))
+      c.bk1 = -1.f;
+    const bool ok = !isnan(c.mgs) && !isnan(d);  // else every threshold is evaluated
+    c.d_up = ok ? __double2float_ru(d) : CUDART_INF_F;
+    c.d_dn = ok ? __double2float_rd(d) : -CUDART_INF_F;
+  }
   c.gsf = (float)st->gscale;
   c.hsf = (float)st->hscale;
   c.l2f = (float)p.l2;
-  c._pad = 0.f;
+  c.go = go;
   c.gs = st->gscale;
   c.hs = st->hscale;
   c.ls = ls;
@@ -241,6 +259,35 @@ __device__ __forceinline__ void hist_apply_split(const Job& J, const Params& p, 
   LeafSum small, large;
   split_children(info, o, &small, &large);
   compute_leaf_const_ls(J, p, st, warp, warp ? large : small, false, lane);
+}
+
+// One warp (side 0, then side 1): the search constants of expansion e's smaller / larger child, from
+// the expanded leaf's candidate record and the partition's row counts, and (side 0) the counts of
+// the histogram's work. Children that are not searched only get go = 0.
+__device__ __forceinline__ void round_leaf_constants(const Job& J, const Params& p, const RoundExp& c, int32_t L, int e,
+                                                     int side, int lane) {
+  JobState* st = J.st;
+  const HistPart h = round_hist_part(p, c, L);
+  if (side == 0 && lane == 0 && h.go) {
+    unsigned long long* rows = reinterpret_cast<unsigned long long*>(h.count == p.n ? &st->hist_rows_direct
+                                                                                    : &st->hist_rows_gather);
+    atomicAdd(rows, (unsigned long long)h.count);
+    atomicAdd(reinterpret_cast<unsigned long long*>(&st->hist_builds), 1ull);
+  }
+  if (!h.go || (c.x < 0 && side == 1)) {
+    if (lane == 0) J.lconst[2 * e + side].go = 0;
+    return;
+  }
+  if (c.x < 0) {
+    compute_leaf_const_ls(J, p, st, 2 * e, J.leaf_sum[0], true, lane);
+    return;
+  }
+  const Cand& info = J.cand[(size_t)c.node * p.F + c.inner];
+  const int32_t R = c.count - L;
+  const bool left = (side == 0) == h.left_smaller;
+  const LeafSum ls = left ? LeafSum{info.lsg, info.lsh, info.left_output, info.lint, L, 0}
+                          : LeafSum{info.rsg, info.rsh, info.right_output, info.rint, R, 0};
+  compute_leaf_const_ls(J, p, st, 2 * e + side, ls, false, lane, left ? 1 : 2);
 }
 
 }  // namespace bk

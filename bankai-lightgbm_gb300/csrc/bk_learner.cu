@@ -158,7 +158,7 @@ struct bk_learner {
   float* d_g = nullptr;
   float* d_h = nullptr;
   int32_t* d_rows = nullptr;
-  size_t pool_bytes_per_job = 0;
+  size_t pool_bytes_per_job = 0, slot_bytes = 0;
   void* d_pool = nullptr;
   std::vector<void*> allocs;
   // host staging
@@ -174,13 +174,15 @@ struct bk_learner {
   std::vector<int32_t> h_tree;
   // graph
   cudaGraphExec_t graph_exec = nullptr;
+  cudaGraphExec_t graph_more = nullptr;  // grow rounds: further rounds of a tree that the first graph did not finish
   uint64_t graph_gen = 0;  // bumped whenever the captured kernels' parameters change
 
   // The captured grow loop no longer matches the learner's parameters: captured anew when next
   // needed (here and in every learner group that holds this learner).
   void drop_graph() {
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
-    graph_exec = nullptr;
+    if (graph_more) cudaGraphExecDestroy(graph_more);
+    graph_exec = graph_more = nullptr;
     ++graph_gen;
   }
   // timing
@@ -198,6 +200,7 @@ struct bk_learner {
 
   ~bk_learner() {
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
+    if (graph_more) cudaGraphExecDestroy(graph_more);
     for (void* a : allocs) cudaFree(a);
     if (h_records) cudaFreeHost(h_records);
     if (h_leaf_values) cudaFreeHost(h_leaf_values);
@@ -267,12 +270,37 @@ struct bk_learner {
     record_hist_event(4 * it + 3);
   }
 
+  // Grow rounds (bk_rounds.cuh) in the graph form, unless something goes by the splits' order (the
+  // by-node sampler's stream, per-split phase timing, the renewal's row order) or by one leaf at a
+  // time (thread-block clusters over a leaf's histogram CTAs), or the leaves do not fit the decision.
+  bool rounds() const {
+    return loop_mode == 1 && !timing && !p.bynode && !(p.quant && p.renew) && hl.cluster == 1 && p.max_exp > 0;
+  }
+  // Rounds captured with the tree: doubling up to round_w leaves, then round_w splits a round, and a
+  // few more for the trees whose best leaves come one after the other; even, as the rounds' two
+  // copies of the state alternate. A tree that needs more gets them from graph_more.
+  int first_rounds() const {
+    int r = (p.num_leaves - 1 + p.round_w - 1) / p.round_w + 3;
+    for (int w = 1; w < p.round_w; w *= 2) ++r;
+    return std::min(r + (r & 1), p.num_leaves + (p.num_leaves & 1));
+  }
+  void run_rounds(int n) {
+    for (int r = 0; r < n; ++r) {
+      launch_hist_round(jobs.data(), K, p, d_bins_rt, d_bins_tm, hl, r & 1, stream);
+      launch_search_round(jobs.data(), K, p, d_feat, r & 1, stream);
+      launch_partition_round(jobs.data(), K, p, d_bins_cm, d_feat, r & 1, stream);
+    }
+    launch_rounds_finish(jobs.data(), K, p, stream);
+  }
+
   void tree_prologue() {
     launch_init_rows(d_jobs, K, p, d_rows, stream);
     if (p.quant) launch_discretize(d_jobs, K, p, d_noise_g, d_noise_h, stream);
     launch_root_sums(d_jobs, K, p, exact_quant_root, stream);
-    CK(cudaMemsetAsync(d_pool, 0, pool_bytes_per_job * K, stream));
-    launch_tree_begin(d_jobs, K, p, stream);
+    // histograms are added up in zeroed slots: one per split
+    launch_zero_pool(d_pool, pool_bytes_per_job, slot_bytes * (size_t)(rounds() ? 1 + p.max_exp : p.num_leaves), K,
+                     stream);
+    launch_tree_begin(d_jobs, K, p, rounds(), stream);
   }
 
   void tree_epilogue() {
@@ -280,18 +308,29 @@ struct bk_learner {
     if (p.quant && p.renew) launch_renew(d_jobs, K, p, stream);
   }
 
-  void run_graph() {
-    if (!graph_exec) {
+  // Everything of an iteration's trees on the stream: the prologue and the grow loop (in rounds: the
+  // first rounds).
+  void issue_trees() {
+    tree_prologue();
+    if (rounds()) {
+      run_rounds(first_rounds());
+      return;
+    }
+    for (int it = 0; it < p.num_leaves - 1; ++it) {
+      step_a(it);
+      step_b(it);
+    }
+    tree_epilogue();
+  }
+
+  template <typename Issue>
+  void launch_captured(cudaGraphExec_t& exec, Issue issue) {
+    if (!exec) {
       cudaGraph_t g = nullptr;
       CK(cudaStreamBeginCapture(stream, cudaStreamCaptureModeThreadLocal));
       capturing = true;
       try {
-        tree_prologue();
-        for (int it = 0; it < p.num_leaves - 1; ++it) {
-          step_a(it);
-          step_b(it);
-        }
-        tree_epilogue();
+        issue();
       } catch (...) {
         capturing = false;
         cudaStreamEndCapture(stream, &g);
@@ -300,10 +339,29 @@ struct bk_learner {
       }
       capturing = false;
       CK(cudaStreamEndCapture(stream, &g));
-      CK(cudaGraphInstantiate(&graph_exec, g, 0));
-      CK(cudaGraphDestroy(g));
+      cudaError_t e = cudaGraphInstantiate(&exec, g, 0);
+      cudaGraphDestroy(g);
+      if (e != cudaSuccess) exec = nullptr;
+      CK(e);
     }
-    CK(cudaGraphLaunch(graph_exec, stream));
+    CK(cudaGraphLaunch(exec, stream));
+  }
+
+  void run_graph() {
+    launch_captured(graph_exec, [&] { issue_trees(); });
+  }
+
+  // After the job states have been read back: whether every job's tree is finished. A tree grown one
+  // split at a time always is.
+  bool trees_done() const {
+    if (!rounds()) return true;
+    for (int j = 0; j < K; ++j)
+      if (!h_state[j].stop) return false;
+    return true;
+  }
+  // Further rounds for trees that are not (every round takes at least one split).
+  void run_more_rounds() {
+    launch_captured(graph_more, [&] { run_rounds(std::max(4, first_rounds() / 4 * 2)); });
   }
 
   void run_stepwise() {
@@ -339,6 +397,17 @@ const char* bk_last_error(void) { return g_last_error.c_str(); }
 }  // extern "C"
 
 namespace {
+
+// How many leaves a grow round expands: an eighth of the tree's leaves (4 to 16). Rounds per tree on
+// a 255-leaf tree of the L2 workload, one split at a time 254: 4 leaves 66, 8 36, 16 22; on its
+// 63-leaf tree 4 18, 8 12, 16 12; on its 31-leaf tree 2 16, 4 10, 8 9. More leaves a round than that
+// only add expansions that are never split.
+void rounds_shape(Params& p) {
+  p.round_w = std::min(kMaxRoundW, std::max(4, (p.num_leaves + 7) / 8));
+  p.round_out = std::min(kMaxRoundOut, 2 * p.round_w);
+  p.max_exp = p.num_leaves <= kMaxRoundLeaves ? p.num_leaves - 1 + p.round_out : 0;
+  p.cand_rows = std::max(p.num_leaves, 1 + 2 * p.max_exp);
+}
 
 int learner_create(const bk_feature* features, int32_t num_features, const uint8_t* bins, int64_t num_data,
                    const bk_config* c, int32_t num_jobs, bk_learner** out, bool device_bins) {
@@ -402,6 +471,7 @@ int learner_create(const bk_feature* features, int32_t num_features, const uint8
     p.bynode = 0;
     p.n_icons = 0;
     p.path_words = (num_features + 31) / 32;
+    rounds_shape(p);
     p.icons = nullptr;
     L->K = num_jobs;
     int maxb = 0;
@@ -445,6 +515,17 @@ int learner_create(const bk_feature* features, int32_t num_features, const uint8
     p.search_narrow = 1;
     for (const DevFeature& d : L->h_feat)
       if (d.cat || d.len > 63) p.search_narrow = 0;
+    // a grow round's search takes the numerical features in groups, then the categorical ones
+    std::vector<int32_t> order;
+    p.unit_penalty = 1;
+    for (int pass = 0; pass < 2; ++pass) {
+      for (int f = 0; f < num_features; ++f)
+        if (L->h_feat[f].cat == pass) order.push_back(f);
+      if (pass == 0) p.n_numeric = (int)order.size();
+    }
+    for (const DevFeature& d : L->h_feat)
+      if (d.penalty != 1.0) p.unit_penalty = 0;
+    p.n_groups = rounds_groups(p);
     // the feature tiles' stored-bin layouts: 16-byte runs of 4-bit bins for tiles whose features
     // all have at most 16 group bins, 8-bit runs otherwise (16 bytes for a last tile of at most
     // 16 features, else 32); each tile's shared histogram holds its largest feature's group bins
@@ -511,6 +592,9 @@ int learner_create(const bk_feature* features, int32_t num_features, const uint8
         return -1;
       }
     }
+    int32_t* d_order = L->dalloc<int32_t>(num_features);
+    CK(cudaMemcpy(d_order, order.data(), sizeof(int32_t) * num_features, cudaMemcpyHostToDevice));
+    p.order = d_order;
     TileGeom* d_tiles = L->dalloc<TileGeom>(p.T);
     CK(cudaMemcpy(d_tiles, L->h_tiles.data(), sizeof(TileGeom) * p.T, cudaMemcpyHostToDevice));
     p.tiles = d_tiles;
@@ -543,7 +627,9 @@ int learner_create(const bk_feature* features, int32_t num_features, const uint8
     L->d_g = L->dalloc<float>(n * K);
     L->d_h = L->dalloc<float>(n * K);
     L->d_rows = L->dalloc<int32_t>(n);
-    L->pool_bytes_per_job = (size_t)Lv * p.T * p.B * TILE * (quant ? sizeof(int64_t) : sizeof(double2));
+    // one histogram slot per leaf; in grow rounds one for the root and two for every expansion
+    L->slot_bytes = (size_t)p.T * p.B * TILE * (quant ? sizeof(int64_t) : sizeof(double2));
+    L->pool_bytes_per_job = (size_t)std::max(Lv, 1 + 2 * p.max_exp) * L->slot_bytes;
     L->d_pool = L->dalloc<uint8_t>(L->pool_bytes_per_job * K);
     JobState* d_states = L->dalloc<JobState>(K);
     CK(cudaMemset(d_states, 0, sizeof(JobState) * K));
@@ -571,14 +657,14 @@ int learner_create(const bk_feature* features, int32_t num_features, const uint8
       J.bgain = L->dalloc<double>(Lv);
       J.bfeat = L->dalloc<int32_t>(Lv);
       // the candidates, then the categorical candidates' bin bitsets
-      J.cand = L->dalloc<Cand>((size_t)Lv * F + (cand_cat_words(Lv, F) * sizeof(uint32_t) + sizeof(Cand) - 1) /
-                                                     sizeof(Cand));
-      J.cgain = L->dalloc<double>(2 * (size_t)F);
+      J.cand = L->dalloc<Cand>((size_t)p.cand_rows * F +
+                               (cand_cat_words(p.cand_rows, F) * sizeof(uint32_t) + sizeof(Cand) - 1) / sizeof(Cand));
+      J.cgain = L->dalloc<double>(2 * (size_t)p.round_w * F);
       J.csplit = L->dalloc<uint8_t>(2 * (size_t)F);
-      J.cthr = L->dalloc<uint32_t>(2 * (size_t)F);
+      J.cthr = L->dalloc<uint32_t>(2 * (size_t)p.round_w * F);
       J.bsplit = L->dalloc<int64_t>(Lv);
-      J.lconst = L->dalloc<LeafConst>(2);
-      J.splittable = L->dalloc<uint8_t>((size_t)Lv * F);
+      J.lconst = L->dalloc<LeafConst>(2 * (size_t)p.round_w);
+      J.splittable = L->dalloc<uint8_t>((size_t)p.cand_rows * F);
       // used, the two by-node masks, the sample scratch, then every leaf's path bitset
       J.used = L->dalloc<uint8_t>(4 * (size_t)F + sizeof(uint32_t) * (size_t)Lv * p.path_words);
       CK(cudaMemset(J.used, 1, 4 * (size_t)F));
@@ -592,6 +678,11 @@ int learner_create(const bk_feature* features, int32_t num_features, const uint8
       J.red = L->dalloc<double>(2 * kRootGrid);
       J.ired = L->dalloc<int64_t>(2 * kRootGrid);
       CK(cudaMemset(J.records, 0, sizeof(bk_split) * Lv));
+      if (p.max_exp > 0) {
+        const size_t bytes = rounds_state_bytes(Lv, p.max_exp, F);
+        J.rounds = L->dalloc<uint8_t>(bytes);
+        CK(cudaMemset(J.rounds, 0, bytes));
+      }
     }
     L->d_jobs = L->dalloc<Job>(K);
     CK(cudaMemcpy(L->d_jobs, L->jobs.data(), sizeof(Job) * K, cudaMemcpyHostToDevice));
@@ -638,6 +729,8 @@ namespace {
 // the grow loop of every job, optionally the score update with the new trees (shrunk on the
 // device), and the copies of the split records, leaf values and job states into pinned host
 // buffers. Returns false with the error set on invalid arguments; CUDA errors throw.
+void enqueue_results(bk_learner* L, double shrinkage, double* score);
+
 bool train_enqueue(bk_learner* L, const float* gradients, const float* hessians, int32_t on_device,
                    const int32_t* rows, int64_t num_rows, double shrinkage, double* score) {
   const Params& p = L->p;
@@ -673,11 +766,22 @@ bool train_enqueue(bk_learner* L, const float* gradients, const float* hessians,
   }
   if (L->loop_mode == 1) L->run_graph();
   else L->run_stepwise();
+  enqueue_results(L, shrinkage, score);
+  CK(cudaEventRecord(L->ev_end, L->stream));
+  return true;
+}
+
+// What follows the trees on the learner's stream: the score update (if any), and the copies of the
+// results into pinned host buffers. Trees that need more rounds leave the score alone; the same is
+// issued again behind their further rounds.
+void enqueue_results(bk_learner* L, double shrinkage, double* score) {
+  const Params& p = L->p;
+  const int Lv = p.num_leaves;
   if (score) {
-    launch_add_score_own(L->d_jobs, L->K, p, shrinkage, score, L->stream);
+    launch_add_score_own(L->d_jobs, L->K, p, shrinkage, score, L->rounds() ? 1 : 0, L->stream);
     CK(cudaGetLastError());
   }
-  for (size_t j = 0; j < K; ++j) {
+  for (size_t j = 0; j < (size_t)L->K; ++j) {
     const Job& J = L->jobs[j];
     CK(cudaMemcpyAsync(L->h_records + j * Lv, J.records, sizeof(bk_split) * (Lv - 1), cudaMemcpyDeviceToHost,
                        L->stream));
@@ -687,9 +791,26 @@ bool train_enqueue(bk_learner* L, const float* gradients, const float* hessians,
   }
   // labels the objective kernels rejected since the previous train call
   CK(cudaMemcpyAsync(L->h_bad_label, L->d_bad_label, sizeof(int32_t), cudaMemcpyDeviceToHost, L->stream));
-  CK(cudaMemsetAsync(L->d_bad_label, 0, sizeof(int32_t), L->stream));
-  CK(cudaEventRecord(L->ev_end, L->stream));
-  return true;
+}
+
+// With the learners' streams waited for: the further rounds of those whose trees are not finished,
+// all of them queued before any is waited for. scores: per learner, or null.
+void finish_trees(bk_learner* const* learners, size_t count, double shrinkage, double* const* scores) {
+  std::vector<bk_learner*> open;
+  for (int k = 0;; ++k) {
+    open.clear();
+    for (size_t i = 0; i < count; ++i) {
+      bk_learner* L = learners[i];
+      if (L->trees_done()) continue;
+      if (k > L->p.num_leaves) throw CudaError{"the grow rounds did not finish a tree"};
+      L->run_more_rounds();
+      enqueue_results(L, shrinkage, scores ? scores[i] : nullptr);
+      CK(cudaEventRecord(L->ev_end, L->stream));
+      open.push_back(L);
+    }
+    if (open.empty()) return;
+    for (bk_learner* L : open) CK(cudaStreamSynchronize(L->stream));
+  }
 }
 
 // After train_finish: a multiclass label outside [0, K) met by bk_learner_objective_gradients
@@ -701,16 +822,14 @@ bool labels_ok(bk_learner* L) {
   return false;
 }
 
-// The synchronous half: waits for the learner's stream, reads the timings and fills the outputs.
+// The synchronous half, with the learner's stream waited for and its trees finished: reads the
+// timings and fills the outputs.
 void train_finish(bk_learner* L, bk_split* splits, double* leaf_values, double* root_outputs,
                   int32_t* num_leaves_out, bool timed = true) {
   const Params& p = L->p;
   const size_t K = (size_t)L->K;
   const int Lv = p.num_leaves;
-  if (timed) {
-    CK(cudaStreamSynchronize(L->stream));
-    CK(cudaGetLastError());
-  }
+  if (*L->h_bad_label != 0) CK(cudaMemsetAsync(L->d_bad_label, 0, sizeof(int32_t), L->stream));
   float ms = 0.f;
   if (timed) CK(cudaEventElapsedTime(&ms, L->ev_start, L->ev_end));
   L->last_total_ms = ms;
@@ -763,6 +882,9 @@ int bk_learner_train(bk_learner* L, const float* gradients, const float* hessian
   }
   try {
     if (!train_enqueue(L, gradients, hessians, on_device, rows, num_rows, 0.0, nullptr)) return -1;
+    CK(cudaStreamSynchronize(L->stream));
+    CK(cudaGetLastError());
+    finish_trees(&L, 1, 0.0, nullptr);
     train_finish(L, splits, leaf_values, root_outputs, num_leaves_out);
     if (!labels_ok(L)) return -1;
   } catch (const CudaError& e) {
@@ -828,6 +950,9 @@ int bk_learner_autotune(bk_learner* L, const float* gradients, const float* hess
       for (int r = 0; r <= trials; ++r) {
         CK(cudaMemcpyAsync(L->jobs[0].st, saved, state_bytes, cudaMemcpyDeviceToDevice, L->stream));
         if (!train_enqueue(L, L->d_g, L->d_h, 1, nullptr, 0, 0.0, nullptr)) throw CudaError{g_last_error};
+        CK(cudaStreamSynchronize(L->stream));
+        CK(cudaGetLastError());
+        finish_trees(&L, 1, 0.0, nullptr);
         train_finish(L, nullptr, nullptr, nullptr, nullptr);
         if (r > 0) t.push_back(L->last_total_ms);
       }
@@ -931,6 +1056,9 @@ int bk_learners_train_batch(bk_learner* const* learners, int32_t count, const fl
         set_error("bk_learners_train_batch: %s", msg.c_str());
         return -1;
       }
+    for (int32_t k = 0; k < count; ++k) CK(cudaStreamSynchronize(learners[k]->stream));
+    CK(cudaGetLastError());
+    finish_trees(learners, (size_t)count, shrinkage, scores);
     for (i = 0; i < count; ++i)
       train_finish(learners[i], splits ? splits[i] : nullptr, leaf_values ? leaf_values[i] : nullptr,
                    root_outputs ? root_outputs[i] : nullptr, num_leaves_out ? num_leaves_out[i] : nullptr);
@@ -960,7 +1088,6 @@ namespace {
 void group_enqueue(bk_learner* L, const float* gradients, const float* hessians, double shrinkage, double* score) {
   const Params& p = L->p;
   const size_t n = (size_t)p.n, K = (size_t)L->K;
-  const int Lv = p.num_leaves;
   if (gradients != L->d_g)
     CK(cudaMemcpyAsync(L->d_g, gradients, n * K * sizeof(float), cudaMemcpyDeviceToDevice, L->stream));
   if (hessians != L->d_h)
@@ -974,27 +1101,9 @@ void group_enqueue(bk_learner* L, const float* gradients, const float* hessians,
                        cudaMemcpyHostToDevice, L->stream));
   }
   L->capturing = true;
-  L->tree_prologue();
-  for (int it = 0; it < Lv - 1; ++it) {
-    L->step_a(it);
-    L->step_b(it);
-  }
-  L->tree_epilogue();
+  L->issue_trees();
   L->capturing = false;
-  if (score) {
-    launch_add_score_own(L->d_jobs, L->K, p, shrinkage, score, L->stream);
-    CK(cudaGetLastError());
-  }
-  for (size_t j = 0; j < K; ++j) {
-    const Job& J = L->jobs[j];
-    CK(cudaMemcpyAsync(L->h_records + j * Lv, J.records, sizeof(bk_split) * (Lv - 1), cudaMemcpyDeviceToHost,
-                       L->stream));
-    CK(cudaMemcpyAsync(L->h_leaf_values + j * Lv, J.leaf_value, sizeof(double) * Lv, cudaMemcpyDeviceToHost,
-                       L->stream));
-    CK(cudaMemcpyAsync(&L->h_state[j], J.st, offsetof(JobState, mt), cudaMemcpyDeviceToHost, L->stream));
-  }
-  CK(cudaMemcpyAsync(L->h_bad_label, L->d_bad_label, sizeof(int32_t), cudaMemcpyDeviceToHost, L->stream));
-  CK(cudaMemsetAsync(L->d_bad_label, 0, sizeof(int32_t), L->stream));
+  enqueue_results(L, shrinkage, score);
 }
 
 }  // namespace
@@ -1145,6 +1254,7 @@ int bk_learner_group_train(bk_learner_group* G, const float* const* gradients, c
     CK(cudaGraphLaunch(G->exec, G->stream));
     CK(cudaStreamSynchronize(G->stream));
     CK(cudaGetLastError());
+    finish_trees(G->learners.data(), count, shrinkage, scores);
     for (i = 0; i < count; ++i)
       train_finish(G->learners[i], splits ? splits[i] : nullptr, leaf_values ? leaf_values[i] : nullptr,
                    root_outputs ? root_outputs[i] : nullptr, num_leaves_out ? num_leaves_out[i] : nullptr, false);

@@ -13,6 +13,7 @@
 #include "bk_decide.cuh"
 #include "bk_grow.cuh"
 #include "bk_launch.cuh"
+#include "bk_rounds.cuh"
 
 namespace bk {
 
@@ -260,6 +261,87 @@ __global__ void __launch_bounds__(kThreads) k_part_scatter(const JobTable jobs, 
   if (threadIdx.x == 0) J.st->part_done = 0u;
 }
 
+// Rows [r0, r1) of a single-pass partition, tile by tile: the counters `left` / `right` hand out the
+// slots from the front and from the back of the range.
+__device__ __forceinline__ void onepass_rows(const PartRange& R, bool quant, const uint8_t* lut, int64_t* left,
+                                             int64_t* right, int32_t (*s_pre)[kThreads / 32], int32_t* s_tile_left,
+                                             int64_t* s_off) {
+  unsigned long long* cnt_left = reinterpret_cast<unsigned long long*>(left);
+  unsigned long long* cnt_right = reinterpret_cast<unsigned long long*>(right);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const unsigned lanes_below = (1u << lane) - 1u;
+  // A tile's element j = k * kThreads + threadIdx.x (item k of this thread): every load and store
+  // instruction covers 32 consecutive elements. Rows keep the tile's element order on both sides.
+  for (int64_t base = R.r0; base < R.r1; base += kThreads * kItems) {
+    int32_t rows[kItems];
+    uint32_t flags = 0;
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+      const int64_t e = base + k * kThreads + threadIdx.x;
+      rows[k] = e < R.r1 ? __ldg(R.src + e) : -1;
+    }
+    int32_t pkv[kItems];
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+      const int64_t e = base + k * kThreads + threadIdx.x;
+      pkv[k] = (quant && rows[k] >= 0) ? part_pk(R, e, rows[k]) : 0;
+    }
+#pragma unroll
+    for (int k = 0; k < kItems; ++k)
+      if (rows[k] >= 0 && lut[__ldg(R.col + rows[k])]) flags |= 1u << k;
+    // left rows before each element of the tile, in element order: within the warp's 32 elements
+    // of item k by ballot, across (item, warp) groups by one scan of kItems * warps counts
+    int32_t in_warp[kItems];
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+      const unsigned b = __ballot_sync(FULL, (flags >> k) & 1u);
+      in_warp[k] = __popc(b & lanes_below);
+      if (lane == 0) s_pre[k][warp] = __popc(b);
+    }
+    __syncthreads();
+    if (warp == 0) {
+      // kItems * warps = 64 group counts in element order (item-major), two per lane
+      constexpr int kGroups = kItems * (kThreads / 32);
+      static_assert(kGroups == 64, "two groups per lane");
+      int32_t* flat = &s_pre[0][0];
+      const int32_t c0 = flat[2 * lane], c1 = flat[2 * lane + 1];
+      int32_t x = c0 + c1;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int32_t y = __shfl_up_sync(FULL, x, o);
+        if (lane >= o) x += y;
+      }
+      const int32_t excl = x - (c0 + c1);
+      __syncwarp();
+      flat[2 * lane] = excl;
+      flat[2 * lane + 1] = excl + c0;
+      if (lane == 31) *s_tile_left = x;
+    }
+    __syncthreads();
+    const int32_t tile_left = *s_tile_left;
+    const int32_t n = (int32_t)min((int64_t)kThreads * kItems, R.r1 - base);
+    if (threadIdx.x == 0) {
+      s_off[0] = (int64_t)atomicAdd(cnt_left, (unsigned long long)tile_left);
+      s_off[1] = (int64_t)atomicAdd(cnt_right, (unsigned long long)(n - tile_left));
+    }
+    __syncthreads();
+    // left rows fill [lo, lo + tile_left); right rows fill the tile's slots ending at count - ro
+    const int64_t lo = s_off[0];
+    const int64_t ro = R.count - s_off[1] - (n - tile_left);
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+      const int32_t j = k * kThreads + (int32_t)threadIdx.x;
+      if (j < n) {
+        const int32_t left_before = s_pre[k][warp] + in_warp[k];
+        const int64_t slot = ((flags >> k) & 1u) ? lo + left_before : ro + (j - left_before);
+        R.dst[slot] = rows[k];
+        if (quant) R.pk_dst[slot] = (int16_t)pkv[k];
+      }
+    }
+    __syncthreads();  // s_pre and s_off are rewritten by the next tile
+  }
+}
+
 // Single-pass partition, for when the order of a child's rows inside its range cannot change any
 // result (no leaf renewal: integer histograms, the score update and the row -> leaf map do not
 // depend on it). Each 2048-row tile claims the slots of its left rows from the front of the
@@ -308,85 +390,94 @@ __global__ void __launch_bounds__(kThreads) k_part_onepass(const JobTable jobs, 
   if (prefetched) build_route_of(J, p, dec, route_feature(s_route[dec.inner]), lut);
   else build_route(J, p, dec, feats, lut);
   __syncthreads();
-  unsigned long long* cnt_left = reinterpret_cast<unsigned long long*>(&st->pcnt[par][0]);
-  unsigned long long* cnt_right = reinterpret_cast<unsigned long long*>(&st->pcnt[par][1]);
   __shared__ int32_t s_pre[kItems][kThreads / 32];  // left rows before each (item, warp) group
   __shared__ int32_t s_tile_left;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned lanes_below = (1u << lane) - 1u;
-  // A tile's element j = k * kThreads + threadIdx.x (item k of this thread): every load and store
-  // instruction covers 32 consecutive elements. Rows keep the tile's element order on both sides.
-  for (int64_t base = R.r0; base < R.r1; base += kThreads * kItems) {
-    int32_t rows[kItems];
-    uint32_t flags = 0;
-#pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-      const int64_t e = base + k * kThreads + threadIdx.x;
-      rows[k] = e < R.r1 ? __ldg(R.src + e) : -1;
+  onepass_rows(R, p.quant != 0, lut, &st->pcnt[par][0], &st->pcnt[par][1], s_pre, &s_tile_left, s_off);
+}
+
+// The partition of a grow round (bk_rounds.cuh): every CTA takes the round's decision, then moves its
+// share of the chosen leaves' rows in one pass (round_cut: equal intervals of whole 256-row blocks); a
+// CTA whose interval crosses into the next leaf builds that leaf's route table there.
+__global__ void __launch_bounds__(kThreads) k_part_round(const JobTable jobs, Params p,
+                                                         const uint8_t* __restrict__ bins_cm,
+                                                         const DevFeature* __restrict__ feats, int q) {
+  __shared__ uint8_t lut[256];
+  __shared__ int64_t s_off[2];
+  __shared__ int32_t s_pre[kItems][kThreads / 32];
+  __shared__ int32_t s_tile_left;
+  __shared__ RoundSmem rs;
+  const Job& J = jobs.job[blockIdx.z];
+  decide_round_load(J, p, q, rs);
+  __syncthreads();
+  decide_round_open(rs);
+  griddep_wait();
+  // the next histogram launch may be scheduled now: its CTAs zero their shared histograms while
+  // this partition runs
+  griddep_launch();
+  if (rs.hdr.stop) {  // the tree is finished: only keep the other copy of the state saying so
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+      RoundHdr* h = round_view(J, p).hdr + (q ^ 1);
+      h->stop = 1;
+      h->n_cur = 0;
     }
-    int32_t pkv[kItems];
-#pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-      const int64_t e = base + k * kThreads + threadIdx.x;
-      pkv[k] = (p.quant && rows[k] >= 0) ? part_pk(R, e, rows[k]) : 0;
+    return;
+  }
+  decide_round_fold(J, p, rs);
+  __syncthreads();
+  if (threadIdx.x < 32) decide_round_commit(J, p, blockIdx.x == 0, rs);
+  __syncthreads();
+  decide_round_choose(J, p, q, blockIdx.x == 0, rs);
+  if (blockIdx.x == 0) decide_round_store(J, p, q, rs);
+  const int n = rs.hdr.n_cur;
+  if (n == 0) return;
+  if (threadIdx.x < 32) {
+    const int lane = threadIdx.x;
+    int64_t off;
+    const RoundCut cut = round_cut(lane < n ? rs.nxt[lane].count : 0, n, (int)gridDim.x, kThreads, kThreads,
+                                   4 * kThreads, lane, &off);
+    if (lane < n) rs.off[lane] = off;
+    if (lane == 0) rs.cut = cut;
+  }
+  __syncthreads();
+  const int64_t q0 = (int64_t)blockIdx.x * rs.cut.per, q1 = q0 + rs.cut.per;
+  int64_t* pcnt = reinterpret_cast<int64_t*>(round_view(J, p).pcnt) + (size_t)(q ^ 1) * 2 * kMaxRoundW;
+  for (int e = 0; e < n; ++e) {
+    const RoundExp& c = rs.nxt[e];
+    const int64_t off = rs.off[e];
+    const int64_t a = max(q0, off), b = min(q1, off + c.count);
+    if (a < b) {
+      Decision d;
+      d.leaf = c.node;
+      d.inner = c.inner;
+      d.thr = c.thr;
+      PartRange R;
+      const int buf = c.depth_buf & 1;
+      R.begin = c.begin;
+      R.count = c.count;
+      R.r0 = a - off;
+      R.r1 = b - off;
+      R.src = leaf_idx(J, buf) + R.begin;
+      R.dst = leaf_idx_w(J, 1 - buf) + R.begin;
+      R.col = bins_cm + (size_t)d.inner * (size_t)p.n;
+      R.pk_row = c.node == 0;  // the root: no leaf-ordered copy yet
+      R.pk_src = p.quant ? (R.pk_row ? J.packed : leaf_pk(J, buf) + R.begin) : nullptr;
+      R.pk_dst = p.quant ? leaf_pk(J, 1 - buf) + R.begin : nullptr;
+      build_route(J, p, d, feats, lut);
+      __syncthreads();
+      onepass_rows(R, p.quant != 0, lut, pcnt + 2 * e, pcnt + 2 * e + 1, s_pre, &s_tile_left, s_off);
+      if (rs.cut.apart) break;
     }
-#pragma unroll
-    for (int k = 0; k < kItems; ++k)
-      if (rows[k] >= 0 && lut[__ldg(R.col + rows[k])]) flags |= 1u << k;
-    // left rows before each element of the tile, in element order: within the warp's 32 elements
-    // of item k by ballot, across (item, warp) groups by one scan of kItems * warps counts
-    int32_t in_warp[kItems];
-#pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-      const unsigned b = __ballot_sync(FULL, (flags >> k) & 1u);
-      in_warp[k] = __popc(b & lanes_below);
-      if (lane == 0) s_pre[k][warp] = __popc(b);
-    }
-    __syncthreads();
-    if (warp == 0) {
-      // kItems * warps = 64 group counts in element order (item-major), two per lane
-      constexpr int kGroups = kItems * (kThreads / 32);
-      static_assert(kGroups == 64, "two groups per lane");
-      int32_t* flat = &s_pre[0][0];
-      const int32_t c0 = flat[2 * lane], c1 = flat[2 * lane + 1];
-      int32_t x = c0 + c1;
-#pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int32_t y = __shfl_up_sync(FULL, x, o);
-        if (lane >= o) x += y;
-      }
-      const int32_t excl = x - (c0 + c1);
-      __syncwarp();
-      flat[2 * lane] = excl;
-      flat[2 * lane + 1] = excl + c0;
-      if (lane == 31) s_tile_left = x;
-    }
-    __syncthreads();
-    const int32_t tile_left = s_tile_left;
-    const int32_t n = (int32_t)min((int64_t)kThreads * kItems, R.r1 - base);
-    if (threadIdx.x == 0) {
-      s_off[0] = (int64_t)atomicAdd(cnt_left, (unsigned long long)tile_left);
-      s_off[1] = (int64_t)atomicAdd(cnt_right, (unsigned long long)(n - tile_left));
-    }
-    __syncthreads();
-    // left rows fill [lo, lo + tile_left); right rows fill the tile's slots ending at count - ro
-    const int64_t lo = s_off[0];
-    const int64_t ro = R.count - s_off[1] - (n - tile_left);
-#pragma unroll
-    for (int k = 0; k < kItems; ++k) {
-      const int32_t j = k * kThreads + (int32_t)threadIdx.x;
-      if (j < n) {
-        const int32_t left_before = s_pre[k][warp] + in_warp[k];
-        const int64_t slot = ((flags >> k) & 1u) ? lo + left_before : ro + (j - left_before);
-        R.dst[slot] = rows[k];
-        if (p.quant) R.pk_dst[slot] = (int16_t)pkv[k];
-      }
-    }
-    __syncthreads();  // s_pre and s_off are rewritten by the next tile
   }
 }
 
 }  // namespace
+
+void launch_partition_round(const Job* h_jobs, int num_jobs, const Params& p, const uint8_t* bins_cm,
+                            const DevFeature* feats, int q, cudaStream_t s) {
+  for_job_groups(h_jobs, num_jobs, [&](const JobTable& t, int nz) {
+    (void)launch_kernel(k_part_round, dim3(p.part_grid, 1, nz), dim3(kThreads), 0, s, p.pdl, t, p, bins_cm, feats, q);
+  });
+}
 
 void launch_partition(const Job* h_jobs, int num_jobs, const Params& p, const uint8_t* bins_cm,
                       const DevFeature* feats, bool stable, int par, bool decide, cudaStream_t s) {

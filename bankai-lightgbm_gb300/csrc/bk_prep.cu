@@ -309,9 +309,12 @@ __global__ void k_add_score(const Job* __restrict__ jobs, Params p, const double
 // The same update with the tree's own leaf outputs from the device, shrunk as Tree::apply_shrinkage
 // does (tree.rs:446-463): score += round_to_zero(leaf_value * rate). A one-leaf tree adds nothing
 // (train.rs:776-795 turns it into a constant tree instead).
-__global__ void k_add_score_own(const Job* __restrict__ jobs, Params p, double rate, double* __restrict__ score) {
+__global__ void k_add_score_own(const Job* __restrict__ jobs, Params p, double rate, double* __restrict__ score,
+                                int need_stop) {
   const Job& J = jobs[blockIdx.z];
   const int32_t leaf = blockIdx.y;
+  for (int j = 0; need_stop && j < (int)gridDim.z; ++j)
+    if (!jobs[j].st->stop) return;  // the trees need more rounds: the update comes after those
   if (leaf >= J.st->tree_leaves || J.st->tree_leaves <= 1) return;
   double v = __dmul_rn(J.leaf_value[leaf], rate);
   if (v >= -BK_ZERO_THRESHOLD && v <= BK_ZERO_THRESHOLD) v = 0.0;
@@ -320,6 +323,12 @@ __global__ void k_add_score_own(const Job* __restrict__ jobs, Params p, double r
   double* sc = score + (size_t)blockIdx.z * p.n;
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < cnt; k += (int64_t)gridDim.x * blockDim.x)
     sc[idx[k]] += v;
+}
+
+__global__ void k_zero_pool(uint4* __restrict__ pool, size_t per_job, size_t n) {
+  uint4* z = pool + (size_t)blockIdx.z * per_job;
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x)
+    z[i] = make_uint4(0, 0, 0, 0);
 }
 
 __global__ void k_row_leaf(const Job* __restrict__ jobs, Params p, int32_t* __restrict__ out) {
@@ -366,9 +375,13 @@ void launch_add_score(const Job* d_jobs, int num_jobs, const Params& p, const do
   k_add_score<<<dim3(8, p.num_leaves, num_jobs), 256, 0, s>>>(d_jobs, p, leaf_vals, score);
 }
 
-void launch_add_score_own(const Job* d_jobs, int num_jobs, const Params& p, double rate, double* score,
+void launch_add_score_own(const Job* d_jobs, int num_jobs, const Params& p, double rate, double* score, int need_stop,
                           cudaStream_t s) {
-  k_add_score_own<<<dim3(8, p.num_leaves, num_jobs), 256, 0, s>>>(d_jobs, p, rate, score);
+  k_add_score_own<<<dim3(8, p.num_leaves, num_jobs), 256, 0, s>>>(d_jobs, p, rate, score, need_stop);
+}
+
+void launch_zero_pool(void* pool, size_t bytes_per_job, size_t bytes, int num_jobs, cudaStream_t s) {
+  k_zero_pool<<<dim3(1024, 1, num_jobs), 256, 0, s>>>(reinterpret_cast<uint4*>(pool), bytes_per_job / 16, bytes / 16);
 }
 
 void launch_row_leaf(const Job* d_jobs, int num_jobs, const Params& p, int32_t* out, cudaStream_t s) {

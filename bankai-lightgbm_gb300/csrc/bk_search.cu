@@ -33,6 +33,8 @@
 #include "bk_launch.cuh"
 #include "bk_leaf.cuh"
 #include "bk_math.cuh"
+#include "bk_search.cuh"
+#include "bk_search_warp.cuh"
 
 namespace bk {
 
@@ -41,45 +43,6 @@ namespace {
 constexpr int kSearchThreads = kDecideThreads;  // one thread per local bin
 constexpr int kSearchWarps = kSearchThreads / 32;
 
-template <typename T>
-__device__ __forceinline__ T warp_incl_scan(T v, int lane) {
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    T u = __shfl_up_sync(FULL, v, o);
-    if (lane >= o) v += u;
-  }
-  return v;
-}
-
-// Inclusive scan towards lower lanes: lane l gets the sum over lanes l .. 31.
-template <typename T>
-__device__ __forceinline__ T warp_incl_scan_down(T v, int lane) {
-#pragma unroll
-  for (int o = 1; o < 32; o <<= 1) {
-    T u = __shfl_down_sync(FULL, v, o);
-    if (lane + o < 32) v += u;
-  }
-  return v;
-}
-
-template <typename T>
-__device__ __forceinline__ T warp_sum(T v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(FULL, v, o);
-  return v;
-}
-
-
-__device__ __forceinline__ int64_t unpack_g(int64_t pk) { return pk >> 32; }
-__device__ __forceinline__ int64_t unpack_h(int64_t pk) { return pk & 0xffffffffLL; }
-
-// Order-preserving integer keys of non-NaN floats and doubles (negative zero counts as zero),
-// computed with integer operations only.
-__device__ __forceinline__ int32_t float_key(float x) {
-  int32_t b = __float_as_int(x);
-  if (b == (int32_t)0x80000000) b = 0;
-  return b ^ ((b >> 31) & 0x7fffffff);
-}
 // ---- fp32 prefilter of the plain split gain (no L1 / max_delta_step / path_smooth) ----
 // The reference evaluates gl^2/(hl+l2) + gr^2/(hr+l2) in f64 for every threshold. Each candidate is
 // first evaluated in fp32 together with a rigorous bound E on |fp32 - f64| (u = 2^-24): the
@@ -142,7 +105,11 @@ __device__ __forceinline__ double int_split_gain(const Params& p, int64_t lg, in
 struct SearchIn {
   LeafConst C;
   LeafSum S0;
-  int32_t sslot, lslot;
+  // pool slots: the smaller leaf's, the one the larger leaf's histogram goes to, and its parent's
+  // (the same slot when one leaf is split at a time)
+  int32_t sslot, lslot, pslot;
+  int32_t group; // a grow round's search: the feature group of the candidate, else -1
+  int32_t crow;  // row of the compact candidate copies: the side, or 2 e + side in a grow round
   // the integer search's two pool entries of this thread (IntPool), loaded from the slots known
   // before the wait; valid when those slots are the state's
   int64_t sv, lv;
@@ -150,12 +117,12 @@ struct SearchIn {
 };
 
 // The pool entries thread t of an integer search scans: the smaller leaf's bin t + 1 of feature
-// f (none at the most-frequent bin, which the fix rewrites) and, on side 1, the larger leaf's.
+// f (none at the most-frequent bin, which the fix rewrites) and, on side 1, its parent's.
 struct IntPool {
   int64_t sv, lv;
 };
 __device__ __forceinline__ IntPool int_pool(const Job& J, const Params& p, const DevFeature& m, int side, int32_t f,
-                                            int32_t sslot, int32_t lslot) {
+                                            int32_t sslot, int32_t pslot) {
   const int t = threadIdx.x;
   const size_t slot_stride = (size_t)p.T * p.B * TILE;
   const size_t feat_off = (size_t)(f / TILE) * p.B * TILE + (f % TILE) + (size_t)(t + 1) * TILE;
@@ -164,44 +131,8 @@ __device__ __forceinline__ IntPool int_pool(const Job& J, const Params& p, const
   const bool in = t < m.len;
   IntPool r;
   r.sv = (in && !(fix && t == m.mfb)) ? pool[(size_t)sslot * slot_stride + feat_off] : 0;
-  r.lv = (side && in) ? pool[(size_t)lslot * slot_stride + feat_off] : 0;
+  r.lv = (side && in) ? pool[(size_t)pslot * slot_stride + feat_off] : 0;
   return r;
-}
-
-__device__ void cand_reset(Cand* c, int32_t real, int32_t inner) {
-  c->gain = -CUDART_INF;
-  c->left_output = c->right_output = 0.0;
-  c->lsg = c->lsh = c->rsg = c->rsh = 0.0;
-  c->lint = c->rint = 0;
-  c->feature = real;
-  c->inner = inner;
-  c->threshold = 0;
-  c->left_count = c->right_count = 0;
-  c->default_left = 1;
-  c->splittable = 0;
-  c->categorical = 0;
-}
-
-// Direction geometry of FindBestThreshold[Int] (feature_histogram.rs:219-357, :673-830): direction
-// 0 is the reverse scan (right side accumulates, default left, positions t = tf_r down to 1 - off),
-// direction 1 the forward scan (left side accumulates, positions t = -1 or 0 up to t_end).
-struct ScanGeom {
-  bool two, skip, fwd_rest;
-  int off, tf_r, t_end;
-};
-
-__device__ __forceinline__ ScanGeom scan_geom(const DevFeature& m) {
-  ScanGeom G;
-  G.two = m.num_bin > 2 && m.missing != 0;
-  G.skip = G.two && m.missing == 1;
-  const bool na = G.two && m.missing == 2;
-  G.off = m.offset;
-  G.tf_r = m.num_bin - 1 - G.off - (na ? 1 : 0);
-  G.t_end = m.num_bin - 2 - G.off;
-  // with NaN missing and the most-frequent bin 0, the forward scan's left side starts as
-  // everything outside the slice, at position t = -1 (held by the last thread)
-  G.fwd_rest = na && G.off == 1;
-  return G;
 }
 
 // Scan order: the reverse scan visits higher bins first, the forward scan lower bins first.
@@ -273,69 +204,11 @@ __device__ __forceinline__ Eval eval_float(const Params& p, int d, double ag, do
   return v;
 }
 
-// One quarter of a queued position's evaluation, as one lane computes it (plain gains: no L1,
-// max_delta_step or path_smooth). Role 0 / 1: the left / right leaf gain (simd.rs:6-8,
-// feature_histogram.rs:148-176: left + right = the split gain, in that order); role 2 / 3: the
-// left / right output (feature_histogram.rs:79-104) with the side's SplitInfo sums and count
-// (feature_histogram.rs:240-357, :700-830). Both are one division, num / (den + lambda_l2), so all
-// four lanes run the same instructions: gain = g^2 / (h + l2), output = -g / (h + l2).
-struct SidePart {
-  double val;     // the leaf gain (roles 0, 1) or the output (roles 2, 3)
-  double sg, sh;  // the side's sums as the SplitInfo stores them (roles 2, 3)
-  int32_t n;      // the side's count (roles 2, 3)
-};
-
-// Role `role` of an integer threshold with left sums (lg, lh): the hessian gets kEpsilon added for
-// the gain (feature_histogram.rs:878-925), the output and the SplitInfo use the plain sums, the
-// counts are round_int(hess * cnt_factor) — exactly as int_split_gain and eval_int compute them.
-__device__ __forceinline__ SidePart int_side(const Params& p, int64_t lg, int64_t lh, int64_t tg, int64_t th,
-                                             double gs, double hs, double cnt_factor, int role) {
-  const bool right = (role & 1) != 0, gain = role < 2;
-  const int64_t sg = right ? tg - lg : lg, sh = right ? th - lh : lh;
-  const double dg = (double)(int32_t)sg * gs, dh = (double)(uint32_t)sh * hs;
-  SidePart r;
-  r.n = round_int((double)(uint32_t)sh * cnt_factor);
-  const double sq = dg * dg;
-  const double he = dh + BK_EPS;
-  const double num = gain ? sq : -dg;
-  const double den = (gain ? he : dh) + p.l2;
-  r.val = num / den;
-  r.sg = dg;
-  r.sh = dh;
-  return r;
-}
-
-// Role `role` of a float threshold of direction d with accumulated sums (ag, ah, c): the gain
-// takes the sums split_gains gets (the reverse scan's right side is the accumulated one), the
-// output and the SplitInfo the right side from the left sums, as eval_float computes them.
-__device__ __forceinline__ SidePart float_side(const Params& p, int d, double ag, double ah, int32_t c, double sum_g,
-                                               double sum_h, int32_t num_data, int role) {
-  const bool right = (role & 1) != 0, gain = role < 2;
-  const double slg = d == 0 ? sum_g - ag : ag, slh = d == 0 ? sum_h - ah : ah;
-  const int32_t lc = d == 0 ? num_data - c : c;
-  // the gain's sums: the accumulated side as accumulated, the other as total minus it
-  const double gg = !right ? slg : (d == 0 ? ag : sum_g - ag);
-  const double gh = !right ? slh : (d == 0 ? ah : sum_h - ah);
-  // the SplitInfo's sums: the right side from the left sums
-  const double og = !right ? slg : sum_g - slg, oh = !right ? slh : sum_h - slh;
-  SidePart r;
-  r.n = !right ? lc : num_data - lc;
-  const double sq = gg * gg;
-  const double num = gain ? sq : -og;
-  const double den = (gain ? gh : oh) + p.l2;
-  r.val = num / den;
-  r.sg = og;
-  r.sh = oh - BK_EPS;
-  return r;
-}
-
 // One direction's stop / prefilter summary of a warp (published before one barrier).
 struct WarpFilt {
   int32_t lb;      // the warp's first `break` position in scan order (kNoneLo / kNoneHi: none)
   int32_t mb, ma;  // best certified fp32 lower-bound key of positions before lb / of all positions
 };
-
-constexpr int kNoneLo = -0x7fffffff, kNoneHi = 0x7fffffff;
 
 // A position queued for its f64 gain (PLAIN gains): evaluated by warp 0.
 struct QEnt {
@@ -500,14 +373,6 @@ __device__ __forceinline__ void resolve_dir(const SearchSmemT<NW>& sm, int d, bo
   *M = m;
 }
 
-// !(gain <= mgs) without an f64 comparison.
-__device__ __forceinline__ bool gain_passes(double gain, double mgs) {
-  return dnan(gain) || dnan(mgs) || dkey(gain) > dkey(mgs);
-}
-__device__ __forceinline__ bool is_neg_inf(double x) {
-  return (unsigned long long)__double_as_longlong(x) == 0xfff0000000000000ULL;
-}
-
 // Appends this thread's entry (when `push`) to direction d's queue, one shared atomic per warp.
 template <int NW>
 __device__ __forceinline__ void queue_push(SearchSmemT<NW>& sm, int d, bool push, const QEnt& e, int lane) {
@@ -617,12 +482,31 @@ __device__ __forceinline__ void eval_queues(SearchSmemT<NW>& sm, int warp, int l
   }
 }
 
-__device__ __forceinline__ void store_cand(const Job& J, const Params& p, int side, int32_t leaf, int32_t f,
+// A grow round's candidate of feature group `g` (its node's record is in J.cand already) and the
+// node's splittable flag of feature f.
+__device__ __forceinline__ void store_round_cand(const Job& J, const Params& p, int crow, int g, int32_t node, int32_t f,
+                                                 const Cand& c) {
+  RoundCand r;
+  r.key = dnan(c.gain) ? kNoKey : dkey(c.gain);
+  r.pk = ((uint32_t)f << 9) | ((uint32_t)(c.default_left != 0) << 8) | c.threshold;
+  r.real = c.feature;
+  round_view(J, p).cand[(size_t)crow * p.n_groups + g] = r;
+  J.splittable[(size_t)node * p.F + f] = (uint8_t)c.splittable;
+}
+
+// `row`: the leaf (or, in a grow round, the node) the candidate belongs to; `crow`: its place among
+// the search's compact copies. In a grow round the node's splittable flag is written here; otherwise
+// the split decision writes it to the leaf's slot.
+__device__ __forceinline__ void store_cand(const Job& J, const Params& p, const SearchIn& si, int32_t row, int32_t f,
                                            const Cand& c) {
-  J.cand[(size_t)leaf * p.F + f] = c;
-  J.cgain[side * p.F + f] = c.gain;
-  J.csplit[side * p.F + f] = (uint8_t)c.splittable;
-  J.cthr[side * p.F + f] = c.threshold | ((uint32_t)(c.default_left != 0) << 31);
+  J.cand[(size_t)row * p.F + f] = c;
+  if (si.group >= 0) {
+    store_round_cand(J, p, si.crow, si.group, row, f, c);
+    return;
+  }
+  J.cgain[(size_t)si.crow * p.F + f] = c.gain;
+  J.cthr[(size_t)si.crow * p.F + f] = c.threshold | ((uint32_t)(c.default_left != 0) << 31);
+  J.csplit[(size_t)si.crow * p.F + f] = (uint8_t)c.splittable;
 }
 
 // The combination of the directions (feature_histogram.rs:240-357, :700-830): the reverse scan
@@ -630,8 +514,8 @@ __device__ __forceinline__ void store_cand(const Job& J, const Params& p, int si
 // SplitInfo (`eval_of(best, direction)`), the penalty and the feature's candidate record. Warp 0,
 // every lane with the same values.
 template <typename EvalOf>
-__device__ __forceinline__ void finish_cand(const Job& J, const Params& p, const DevFeature& m, int side, int32_t leaf,
-                                            int32_t f, const ScanGeom& G, double mgs, const DirBest (&r)[2],
+__device__ __forceinline__ void finish_cand(const Job& J, const Params& p, const DevFeature& m, const SearchIn& si,
+                                            int32_t leaf, int32_t f, const ScanGeom& G, double mgs, const DirBest (&r)[2],
                                             const int (&rs)[2], int lane, EvalOf eval_of) {
   const int nd = G.two ? 2 : 1;
   int sp = 0, ch = -1;
@@ -674,7 +558,7 @@ __device__ __forceinline__ void finish_cand(const Job& J, const Params& p, const
   c.gain *= m.penalty;
   c.splittable = sp;
   c.missing = m.missing;
-  if (lane == 0) store_cand(J, p, side, leaf, f, c);
+  if (lane == 0) store_cand(J, p, si, leaf, f, c);
 }
 
 // FindBestThresholdInt for one (leaf, feature): feature_histogram.rs:673-830, scans :839-1142.
@@ -695,7 +579,7 @@ __device__ void search_int(const Job& J, const Params& p, const SearchIn& si, co
   const bool fix = m.mfb > 0;  // offset 0: the slice holds every bin and the most frequent one is empty
   const bool in = t < m.len;
   // the smaller leaf's most-frequent entry is rewritten by its side-0 CTA; side 1 never reads it
-  const IntPool pv = si.pre ? IntPool{si.sv, si.lv} : int_pool(J, p, m, side, f, si.sslot, si.lslot);
+  const IntPool pv = si.pre ? IntPool{si.sv, si.lv} : int_pool(J, p, m, side, f, si.sslot, si.pslot);
   const int64_t sv = pv.sv, lv = pv.lv;
   const ScanGeom G = scan_geom(m);
   if (t < 2) sm.qn[t] = 0;
@@ -820,7 +704,7 @@ __device__ void search_int(const Job& J, const Params& p, const SearchIn& si, co
     combine_best(sm, lane, r, rs);
   }
   // FindBestThresholdInt's combination of the directions (feature_histogram.rs:700-830)
-  finish_cand(J, p, m, side, leaf, f, G, C.mgs, r, rs, lane, [&](const DirBest& b, int d) {
+  finish_cand(J, p, m, si, leaf, f, G, C.mgs, r, rs, lane, [&](const DirBest& b, int d) {
     (void)d;
     if (PLAIN) {  // evaluated with the gain
       Eval v = b.ev;
@@ -852,7 +736,7 @@ __device__ void search_float(const Job& J, const Params& p, const SearchIn& si, 
   const bool fix = m.mfb > 0;
   const bool in = t < m.len;
   double2 sv = (in && !(fix && t == m.mfb)) ? hs[(size_t)(t + 1) * TILE] : zero;
-  const double2 lv = (side && in) ? hl[(size_t)(t + 1) * TILE] : zero;
+  const double2 lv = (side && in) ? pool[(size_t)si.pslot * slot_stride + feat_off + (size_t)(t + 1) * TILE] : zero;
   const ScanGeom G = scan_geom(m);
   if (t < 2) sm.qn[t] = 0;
   const double sum_g = C.sum_g, sum_h = C.sum_h;
@@ -1045,7 +929,7 @@ __device__ void search_float(const Job& J, const Params& p, const SearchIn& si, 
     combine_best(sm, lane, r, rs);
   }
   // FindBestThreshold's combination of the directions (feature_histogram.rs:240-357)
-  finish_cand(J, p, m, side, leaf, f, G, C.mgs, r, rs, lane, [&](const DirBest& b, int d) {
+  finish_cand(J, p, m, si, leaf, f, G, C.mgs, r, rs, lane, [&](const DirBest& b, int d) {
     if (PLAIN) return b.ev;  // evaluated with the gain
     return eval_float(p, d, __longlong_as_double(b.a), __longlong_as_double(b.b), b.c, sum_g, sum_h, num_data,
                       C.parent, b.ev.gain, lane);
@@ -1139,7 +1023,7 @@ __device__ void search_cat(const Job& J, const Params& p, const SearchIn& si, co
     int64_t* hs = pool + (size_t)si.sslot * slot_stride + feat_off;
     int64_t* hl = pool + (size_t)(side ? si.lslot : si.sslot) * slot_stride + feat_off;
     const int64_t sv = (in && !(fix && t == m.mfb)) ? hs[(size_t)(t + 1) * TILE] : 0;
-    const int64_t lv = (side && in) ? hl[(size_t)(t + 1) * TILE] : 0;
+    const int64_t lv = (side && in) ? pool[(size_t)si.pslot * slot_stride + feat_off + (size_t)(t + 1) * TILE] : 0;
     int64_t v = side ? lv - sv : sv;
     if (fix) {
       const int64_t a = warp_sum(sv);
@@ -1164,7 +1048,7 @@ __device__ void search_cat(const Job& J, const Params& p, const SearchIn& si, co
     double2* hl = pool + (size_t)(side ? si.lslot : si.sslot) * slot_stride + feat_off;
     const double2 zero = make_double2(0.0, 0.0);
     double2 sv = (in && !(fix && t == m.mfb)) ? hs[(size_t)(t + 1) * TILE] : zero;
-    const double2 lv = (side && in) ? hl[(size_t)(t + 1) * TILE] : zero;
+    const double2 lv = (side && in) ? pool[(size_t)si.pslot * slot_stride + feat_off + (size_t)(t + 1) * TILE] : zero;
     if (fix) {
       const double ag = warp_sum(sv.x), ah = warp_sum(sv.y);
       if (lane == 0) {
@@ -1409,7 +1293,7 @@ __device__ void search_cat(const Job& J, const Params& p, const SearchIn& si, co
   c.gain *= m.penalty;
   c.splittable = sp;
   c.missing = m.missing;
-  if (lane == 0) store_cand(J, p, side, leaf, f, c);
+  if (lane == 0) store_cand(J, p, si, leaf, f, c);
   if (lane < 8) cand_cat_bits(J, p, leaf, f)[lane] = word;
 }
 
@@ -1460,7 +1344,9 @@ __global__ void __launch_bounds__(32 * NW) k_search(const JobTable jobs, Params 
   const uint8_t used = J.used[f];
   SearchIn si;
   si.sslot = st->smaller_slot;
-  si.lslot = st->larger_slot;
+  si.lslot = si.pslot = st->larger_slot;
+  si.group = -1;
+  si.crow = side;
   si.C = J.lconst[side];
   si.S0 = side ? J.lconst[0].ls : si.C.ls;
   si.pre = false;
@@ -1501,6 +1387,241 @@ __global__ void __launch_bounds__(32 * NW) k_search(const JobTable jobs, Params 
   if (threadIdx.x == 0) st->search_done = 0u;
 }
 
+// The search of a grow round (bk_rounds.cuh): blockIdx.x = 2 * feature group + side, blockIdx.y = the
+// expansion. The larger child's histogram goes to a slot of its own, with everything of the
+// parent's that the search does not derive (bin 0, features that are not searched) copied. The
+// expansion and, on the quantized path, the parent's bins are read while the histogram launch
+// finishes: both were written before it.
+// WARP: groups of kWarpFeatures numerical features, a warp each (bk_search_warp.cuh), then one
+// categorical feature per CTA; otherwise one feature per CTA in the form of k_search.
+struct RoundSearch {
+  const RoundHdr* hdr;
+  RoundExp c;
+  int32_t stop;
+  bool active;
+};
+
+__device__ __forceinline__ RoundSearch round_search_load(const Job& J, const Params& p, int q, int e) {
+  const RoundView v = round_view(J, p);
+  RoundSearch r;
+  r.hdr = v.hdr + q;
+  const int32_t n_cur = __ldcg(&r.hdr->n_cur);
+  r.stop = __ldcg(&r.hdr->stop);
+  r.active = e < n_cur;
+  r.c.x = -1;
+  r.c.node = r.c.slot = r.c.sslot = r.c.lslot = 0;
+  if (r.active) r.c = v.cur[q * kMaxRoundW + e];
+  return r;
+}
+
+// Whether feature f is searched for the expansion's children.
+__device__ __forceinline__ bool round_used(const Job& J, const Params& p, const RoundExp& c, int f) {
+  return J.tree_mask[f] && (c.x < 0 || __ldcg(&J.splittable[(size_t)c.node * p.F + f]));
+}
+
+// After the wait, first thing: the row counters of the expansions that this round's partition is
+// given (their last reader, the histogram launch of the round before, has finished).
+__device__ __forceinline__ void round_clear_counters(const Job& J, const Params& p, const RoundSearch& r, int q) {
+  if (!r.stop && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x < 2 * kMaxRoundW)
+    round_view(J, p).pcnt[(size_t)(q ^ 1) * 2 * kMaxRoundW + threadIdx.x] = 0;
+}
+
+// One feature on the whole CTA (k_search's forms).
+template <bool PLAIN, bool QUANT, int NW>
+__device__ __forceinline__ void round_search_cta(const Job& J, const Params& p, const RoundExp& c, const DevFeature& m,
+                                                 int f, int g, int e, int side, bool used, SearchSmemT<NW>& sm) {
+  using V = typename std::conditional<QUANT, int64_t, double2>::type;
+  const int t = (int)threadIdx.x;
+  SearchIn si;
+  si.group = g;
+  si.crow = 2 * e + side;
+  si.C = J.lconst[si.crow];
+  si.S0 = side ? J.lconst[2 * e].ls : si.C.ls;
+  if (!si.C.go) return;  // not searched (uniform over the expansion's side): no candidates
+  const int32_t node = c.x < 0 ? 0 : 2 * c.x + si.C.go;
+  si.sslot = c.x < 0 ? c.slot : c.sslot;
+  si.lslot = c.lslot;
+  si.pslot = c.slot;
+  si.pre = false;
+  si.sv = si.lv = 0;
+  const size_t slot_stride = (size_t)p.T * p.B * TILE;
+  const size_t feat_off = (size_t)(f / TILE) * p.B * TILE + (f % TILE);
+  V* pool = reinterpret_cast<V*>(J.pool);
+  if (side) {  // the slot entries the search does not write
+    const V* parent = pool + (size_t)c.slot * slot_stride + feat_off;
+    V* larger = pool + (size_t)c.lslot * slot_stride + feat_off;
+    if (t == 0) larger[0] = parent[0];
+    if (!used)
+      for (int b = t + 1; b < m.gbins; b += 32 * NW) larger[(size_t)b * TILE] = parent[(size_t)b * TILE];
+  }
+  if (!used) {  // uniform over the CTA
+    if (t == 0) {
+      round_view(J, p).cand[(size_t)si.crow * p.n_groups + g] = RoundCand{kNoKey, 0u, 0x7fffffff};
+      J.splittable[(size_t)node * p.F + f] = 0;
+    }
+    return;
+  }
+  if constexpr (NW == kSearchWarps) {
+    if (m.cat) {
+      search_cat<QUANT>(J, p, si, m, side, f, node, sm);
+      return;
+    }
+  }
+  if constexpr (QUANT) search_int<PLAIN>(J, p, si, m, side, f, node, sm);
+  else search_float<PLAIN>(J, p, si, m, side, f, node, sm);
+}
+
+template <bool PLAIN, bool QUANT, int NW>
+__global__ void __launch_bounds__(32 * NW) k_search_round(const JobTable jobs, Params p,
+                                                          const DevFeature* __restrict__ feats, int q) {
+  __shared__ SearchSmemT<NW> sm;
+  const int side = (int)(blockIdx.x & 1u), e = (int)blockIdx.y, f = (int)(blockIdx.x >> 1);
+  const DevFeature m = feats[f];  // static: loaded while the histogram launch finishes
+  const Job& J = jobs.job[blockIdx.z];
+  const RoundSearch r = round_search_load(J, p, q, e);
+  const bool used = r.active && round_used(J, p, r.c, f);
+  griddep_wait();
+  // the partition may be scheduled now: its CTAs read the round's state while this search runs
+  griddep_launch();
+  round_clear_counters(J, p, r, q);
+  if (r.active) round_search_cta<PLAIN, QUANT, NW>(J, p, r.c, m, f, f, e, side, used, sm);
+}
+
+// CAT: the learner has categorical features (their search's registers and code stay out otherwise).
+template <bool CAT>
+__global__ void __launch_bounds__(32 * kWarpFeatures, 3)
+    k_search_round_warp(const JobTable jobs, Params p, const DevFeature* __restrict__ feats, int q) {
+  union Smem {
+    WarpSearchSmem w;
+    typename std::conditional<CAT, SearchSmem, int>::type c;
+    __device__ Smem() {}
+  };
+  __shared__ Smem sm;
+  const int side = (int)(blockIdx.x & 1u), e = (int)blockIdx.y, g = (int)(blockIdx.x >> 1);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int n_num_groups = (p.n_numeric + kWarpFeatures - 1) / kWarpFeatures;
+  const bool numeric = !CAT || g < n_num_groups;
+  // the warp's feature (the CTA's, for a categorical one)
+  const int oi = numeric ? g * kWarpFeatures + warp : p.n_numeric + (g - n_num_groups);
+  const int f = (!numeric || oi < p.n_numeric) ? p.order[oi] : -1;
+  DevFeature m{};
+  if (f >= 0) m = feats[f];  // static: loaded while the histogram launch finishes
+  // the group's bins are moved with thread = (bin t0 + 32 i, feature fj of the group): eight adjacent
+  // features' bins are 64 consecutive bytes of the pool
+  const int j = threadIdx.x & (kWarpFeatures - 1), t0 = (int)threadIdx.x / kWarpFeatures;
+  const int oj = g * kWarpFeatures + j;
+  const int fj = (numeric && oj < p.n_numeric) ? p.order[oj] : -1;
+  int lenj = 0, mfbj = -1;
+  if (fj >= 0) {
+    lenj = feats[fj].len;
+    mfbj = feats[fj].mfb > 0 ? feats[fj].mfb : -1;
+  }
+  const Job& J = jobs.job[blockIdx.z];
+  const RoundSearch r = round_search_load(J, p, q, e);
+  const RoundExp c = r.c;
+  const bool used = r.active && f >= 0 && round_used(J, p, c, f);
+  const size_t slot_stride = (size_t)p.T * p.B * TILE;
+  int64_t* pool = reinterpret_cast<int64_t*>(J.pool);
+  const size_t offj = fj >= 0 ? (size_t)(fj / TILE) * p.B * TILE + (fj % TILE) + TILE : 0;  // its bin 1
+  int64_t lv[8], lv0 = 0;
+  bool usedj = false;
+  if (r.active && side && c.x >= 0 && fj >= 0) {
+    const int64_t* parent = pool + (size_t)c.slot * slot_stride + offj;
+    usedj = round_used(J, p, c, fj);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int t = t0 + 32 * i;
+      lv[i] = t < lenj ? parent[(size_t)t * TILE] : 0;
+    }
+    if (t0 == 0) lv0 = parent[-TILE];
+  }
+  griddep_wait();
+  // the partition may be scheduled now: its CTAs read the round's state while this search runs
+  griddep_launch();
+  round_clear_counters(J, p, r, q);
+  if (!r.active) return;
+  if constexpr (CAT) {
+    if (!numeric) {
+      round_search_cta<true, true, kSearchWarps>(J, p, c, m, f, g, e, side, used, sm.c);
+      return;
+    }
+  }
+  const int crow = 2 * e + side;
+  const LeafConst& C = J.lconst[crow];
+  if (!C.go) return;  // uniform over the CTA
+  const int32_t node = c.x < 0 ? 0 : 2 * c.x + C.go;
+  if (fj >= 0) {
+    // the larger leaf: parent minus smaller, bin 0 and the features that are not searched copied
+    // (their most frequent bin is fixed below)
+    const int64_t* hs = pool + (size_t)(c.x < 0 ? c.slot : c.sslot) * slot_stride + offj;
+    int64_t* hl = pool + (size_t)c.lslot * slot_stride + offj;
+    if (side && t0 == 0) hl[-TILE] = lv0;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int t = t0 + 32 * i;
+      int64_t v = 0;
+      if (t < lenj) {
+        if (side && !usedj) {
+          hl[(size_t)t * TILE] = lv[i];
+        } else if (t != mfbj) {
+          v = hs[(size_t)t * TILE];
+          if (side) {
+            v = lv[i] - v;
+            hl[(size_t)t * TILE] = v;
+          }
+        }
+      }
+      sm.w.w[j].e[slice_at(t)] = v;
+    }
+  }
+  __syncthreads();
+  int64_t* own = pool + (size_t)(side ? c.lslot : (c.x < 0 ? c.slot : c.sslot)) * slot_stride +
+                 (f >= 0 ? (size_t)(f / TILE) * p.B * TILE + (f % TILE) : 0);
+  const ScanGeom G = scan_geom(m);
+  WarpSlice& ws = sm.w.w[warp];
+  WarpSearch sr;
+  const int nb = m.len > 63 ? 8 : 2;
+  int32_t M = float_key(-CUDART_INF_F);
+  if (used) M = sr.bounds(m, G, C, own, ws, nb, lane);
+  if (lane == 0) sm.w.m[warp] = M;
+  __syncthreads();
+  if (p.unit_penalty) {
+#pragma unroll
+    for (int w = 0; w < kWarpFeatures; ++w) M = max(M, sm.w.m[w]);
+  }
+  long long key = kNoKey;
+  Cand cd;
+  if (used) {
+    ExactBest r2[2];
+    sr.queue(C, M, ws, nb, lane);
+    int split = sr.certain;
+    exact_batches(p, ws, sr.n, sr.T, sr.base_f, C, lane, r2);
+    split |= r2[0].split | (G.two ? r2[1].split : 0);
+    cd = warp_cand(m, G, f, C, r2, split);
+    key = dnan(cd.gain) ? kNoKey : dkey(cd.gain);
+  }
+  if (lane == 0) {
+    sm.w.key[warp] = key;
+    sm.w.real[warp] = f >= 0 ? m.real : 0x7fffffff;
+    if (f >= 0) J.splittable[(size_t)node * p.F + f] = used ? (uint8_t)cd.splittable : (uint8_t)0;
+  }
+  __syncthreads();
+  // the group's candidate: the highest gain, then the smaller real feature
+  int best = 0;
+#pragma unroll
+  for (int w = 1; w < kWarpFeatures; ++w)
+    if (sm.w.key[w] > sm.w.key[best] || (sm.w.key[w] == sm.w.key[best] && sm.w.real[w] < sm.w.real[best])) best = w;
+  if (warp != best || lane != 0) return;
+  RoundCand rc{kNoKey, 0u, 0x7fffffff};
+  if (key != kNoKey) {
+    J.cand[(size_t)node * p.F + f] = cd;
+    rc.key = key;
+    rc.pk = ((uint32_t)f << 9) | ((uint32_t)(cd.default_left != 0) << 8) | cd.threshold;
+    rc.real = cd.feature;
+  }
+  round_view(J, p).cand[(size_t)crow * p.n_groups + g] = rc;
+}
+
 // The bookkeeping of a tree's last split when it was partitioned in one pass (no histogram launch
 // follows it to apply it).
 __global__ void __launch_bounds__(32) k_apply_split(const JobTable jobs, Params p, int par) {
@@ -1511,9 +1632,105 @@ __global__ void __launch_bounds__(32) k_apply_split(const JobTable jobs, Params 
   post_split_writes(J, p, o, (int)threadIdx.x);
 }
 
+// The rounds' state at the root of a tree: one leaf, the root the first round's only expansion.
+__device__ __forceinline__ void rounds_begin(const Job& J, const Params& p) {
+  const RoundView v = round_view(J, p);
+  const int t = threadIdx.x;
+  if (t < 2 * 2 * kMaxRoundW) v.pcnt[t] = 0;
+  if (t == 0) {
+    const int32_t count = (int32_t)J.st->root_count;
+    RoundHdr h{};
+    h.leaves = 1;
+    h.last_x = -1;
+    v.hdr[1] = h;
+    h.n_cur = 1;
+    v.hdr[0] = h;
+    LeafEnt e{};
+    e.key = dkey(-CUDART_INF);
+    e.pay = (long long)-1 * 4294967296LL;
+    e.feat = -1;
+    e.out = -1;
+    e.count = count;
+    v.leaf[0] = e;
+    RoundExp c{};
+    c.x = -1;
+    c.out = -1;
+    c.count = count;
+    v.cur[0] = c;
+  }
+}
+
+// The finished tree: leaf arrays from the final leaves, split records from the committed splits
+// (the arguments of Tree::split_numerical / split_categorical, serial.rs:1685-1876).
+__global__ void __launch_bounds__(256) k_rounds_finish(const JobTable jobs, Params p) {
+  const Job& J = jobs.job[blockIdx.z];
+  const JobState* st = J.st;
+  if (!st->stop) return;
+  const RoundView v = round_view(J, p);
+  const int32_t leaves = st->tree_leaves;
+  const RoundHdr h = v.hdr[st->fin_q];  // the copy of the state that the last decision wrote
+  const LeafEnt* ent = v.leaf + (size_t)st->fin_q * p.num_leaves;
+  const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
+  // the tree's last split, when it was taken before its rows were partitioned
+  const int32_t last_L = h.last_x >= 0 ? (int32_t)v.pcnt[(size_t)h.last_par * 2 * kMaxRoundW] : 0;
+  if (i < leaves) {
+    const LeafEnt e = ent[i];
+    int32_t begin = e.begin, count = e.count, slot = e.slot;
+    if (h.last_x >= 0 && e.node > 2 * h.last_x) {  // one of its children (no later nodes exist)
+      const bool left = e.node == 1 + 2 * h.last_x;
+      const int32_t R = count - last_L, pslot = ent[v.commit[leaves - 2].leaf].slot;
+      const bool go = !(p.max_depth > 0 && (e.depth_buf >> 1) >= p.max_depth) &&
+                      !(R < p.min_data * 2 && last_L < p.min_data * 2);
+      slot = !go ? (left ? pslot : -1) : (left == (last_L < R) ? round_sslot(h.last_x) : pslot);
+      begin = left ? begin : begin + last_L;
+      count = left ? last_L : R;
+    }
+    J.leaf_begin[i] = begin;
+    J.leaf_count[i] = count;
+    J.leaf_buf[i] = e.depth_buf & 1;
+    J.leaf_slot[i] = slot;
+    J.leaf_depth[i] = e.depth_buf >> 1;
+    if (e.node > 0) {  // a tree of one leaf keeps the root's output
+      const int2 xi = v.xinfo[(e.node - 1) >> 1];
+      const Cand& info = J.cand[(size_t)xi.x * p.F + xi.y];
+      const double o = (e.node & 1) ? info.left_output : info.right_output;
+      J.leaf_value[i] = isnan(o) ? 0.0 : o;
+    }
+  }
+  if (i < leaves - 1) {
+    const Commit c = v.commit[i];
+    const int2 xi = v.xinfo[c.x];
+    const Cand info = J.cand[(size_t)xi.x * p.F + xi.y];
+    const int32_t L = c.L >= 0 ? c.L : last_L;
+    int32_t count = c.count;
+    bk_split& r = J.records[i];
+    r.leaf = c.leaf;
+    r.right_leaf = i + 1;
+    r.inner_feature = info.inner;
+    r.real_feature = info.feature;
+    r.threshold = info.threshold;
+    r.default_left = info.default_left;
+    r.missing_type = info.missing;
+    r.left_count = L;
+    r.right_count = count - L;
+    r.left_output = info.left_output;
+    r.right_output = info.right_output;
+    r.left_sum_gradient = info.lsg;
+    r.left_sum_hessian = info.lsh;
+    r.right_sum_gradient = info.rsg;
+    r.right_sum_hessian = info.rsh;
+    r.gain = info.gain;
+    r.left_int_sum = info.lint;
+    r.right_int_sum = info.rint;
+    r.categorical = info.categorical;
+    r._pad = 0;
+    for (int w = 0; w < 8; ++w) r.cat_bins[w] = info.categorical ? cand_cat_bits(J, p, xi.x, xi.y)[w] : 0u;
+  }
+}
+
 // Root of a tree (serial.rs:658-776 after the root sums, then :580-586 and the first
 // BeforeFindBestSplit). leaf_sum[0] and root_count are already set.
-__global__ void __launch_bounds__(256) k_tree_begin(const Job* __restrict__ jobs, Params p) {
+__global__ void __launch_bounds__(256) k_tree_begin(const Job* __restrict__ jobs, Params p, int rounds) {
   const Job& J = jobs[blockIdx.z];
   JobState* st = J.st;
   for (int i = threadIdx.x; i < p.num_leaves; i += blockDim.x) {
@@ -1545,8 +1762,9 @@ __global__ void __launch_bounds__(256) k_tree_begin(const Job* __restrict__ jobs
       J.leaf_value[0] = st->root_output;
     }
     __syncwarp();
-    before_find_best_split(J, p, st, 0, -1, lane);
+    if (!rounds) before_find_best_split(J, p, st, 0, -1, lane);
   }
+  if (rounds) rounds_begin(J, p);
 }
 
 }  // namespace
@@ -1583,8 +1801,44 @@ void launch_apply_split(const Job* h_jobs, int num_jobs, const Params& p, int pa
   });
 }
 
-void launch_tree_begin(const Job* d_jobs, int num_jobs, const Params& p, cudaStream_t s) {
-  k_tree_begin<<<dim3(1, 1, num_jobs), 256, 0, s>>>(d_jobs, p);
+// The warp form takes the quantized, plain searches; the others keep a CTA per feature.
+static bool search_round_warp(const Params& p) { return p.quant && !p.use_l1 && !p.use_max && !p.use_smooth; }
+
+int rounds_groups(const Params& p) {
+  if (!search_round_warp(p)) return p.F;
+  return (p.n_numeric + kWarpFeatures - 1) / kWarpFeatures + (p.F - p.n_numeric);
+}
+
+void launch_search_round(const Job* h_jobs, int num_jobs, const Params& p, const DevFeature* feats, int q,
+                         cudaStream_t s) {
+  const bool plain = !p.use_l1 && !p.use_max && !p.use_smooth;
+  const bool narrow = plain && p.search_narrow;  // as in launch_search
+  for_job_groups(h_jobs, num_jobs, [&](const JobTable& t, int nz) {
+    const dim3 grid((unsigned)(2 * p.n_groups), p.round_w, nz);
+    auto go = [&](auto kern, int threads) {
+      (void)launch_kernel(kern, grid, dim3(threads), 0, s, p.pdl, t, p, feats, q);
+    };
+    if (search_round_warp(p) && p.n_numeric < p.F) go(k_search_round_warp<true>, 32 * kWarpFeatures);
+    else if (search_round_warp(p)) go(k_search_round_warp<false>, 32 * kWarpFeatures);
+    else if (p.quant) go(k_search_round<false, true, 8>, kSearchThreads);
+    else if (narrow) go(k_search_round<true, false, 2>, 64);
+    else if (plain) go(k_search_round<true, false, 8>, kSearchThreads);
+    else go(k_search_round<false, false, 8>, kSearchThreads);
+  });
+}
+
+void launch_tree_begin(const Job* d_jobs, int num_jobs, const Params& p, bool rounds, cudaStream_t s) {
+  k_tree_begin<<<dim3(1, 1, num_jobs), 256, 0, s>>>(d_jobs, p, rounds ? 1 : 0);
+}
+
+void launch_rounds_finish(const Job* h_jobs, int num_jobs, const Params& p, cudaStream_t s) {
+  for_job_groups(h_jobs, num_jobs, [&](const JobTable& t, int nz) {
+    k_rounds_finish<<<dim3((p.num_leaves + 255) / 256, 1, nz), 256, 0, s>>>(t, p);
+  });
+}
+
+size_t rounds_state_bytes(int num_leaves, int max_exp, int F) {
+  return round_view(nullptr, num_leaves, max_exp, F).bytes;
 }
 
 }  // namespace bk
