@@ -290,9 +290,13 @@ void launch_partition(const Job* h_jobs, int num_jobs, const Params& p, const ui
 cudaError_t hist_set_smem_attrs(size_t smem);
 
 // bk_prep.cu
-void launch_init_rows(const Job* d_jobs, int num_jobs, const Params& p, const int32_t* rows, cudaStream_t s);
+// bagged_only: the identity of an unbagged root is not written
+void launch_init_rows(const Job* d_jobs, int num_jobs, const Params& p, const int32_t* rows, bool bagged_only,
+                      cudaStream_t s);
+// noise_gf / noise_hf: the noise rounded to fp32 (launch_noise_f32)
 void launch_discretize(const Job* d_jobs, int num_jobs, const Params& p, const double* noise_g, const double* noise_h,
-                       cudaStream_t s);
+                       const float* noise_gf, const float* noise_hf, cudaStream_t s);
+void launch_noise_f32(const double* a, float* b, int64_t n, cudaStream_t s);
 void launch_root_sums(const Job* d_jobs, int num_jobs, const Params& p, int exact_quant_root, cudaStream_t s);
 void launch_renew(const Job* d_jobs, int num_jobs, const Params& p, cudaStream_t s);
 void launch_add_score(const Job* d_jobs, int num_jobs, const Params& p, const double* leaf_vals, double* score,
@@ -304,7 +308,7 @@ void launch_add_score_own(const Job* d_jobs, int num_jobs, const Params& p, doub
 void launch_zero_pool(void* pool, size_t bytes_per_job, size_t bytes, int num_jobs, cudaStream_t s);
 void launch_row_leaf(const Job* d_jobs, int num_jobs, const Params& p, int32_t* out, cudaStream_t s);
 void launch_mt_seed(const Job* d_jobs, int num_jobs, uint32_t seed, cudaStream_t s);
-constexpr int kRootGrid = 256;
+constexpr int kRootGrid = 1216;  // CTAs of the root sums and the discretization: eight per SM
 
 // bk_predict.cu
 cudaError_t predict_tree(const DevFeature* feats, int32_t num_leaves, const int32_t* d_tree, const double* d_leaf_value,

@@ -152,6 +152,7 @@ struct bk_learner {
   std::vector<TileGeom> h_tiles;
   double* d_noise_g = nullptr;
   double* d_noise_h = nullptr;
+  float *d_noise_gf = nullptr, *d_noise_hf = nullptr;  // the same in fp32
   // jobs
   std::vector<Job> jobs;
   Job* d_jobs = nullptr;
@@ -294,8 +295,8 @@ struct bk_learner {
   }
 
   void tree_prologue() {
-    launch_init_rows(d_jobs, K, p, d_rows, stream);
-    if (p.quant) launch_discretize(d_jobs, K, p, d_noise_g, d_noise_h, stream);
+    launch_init_rows(d_jobs, K, p, d_rows, rounds(), stream);
+    if (p.quant) launch_discretize(d_jobs, K, p, d_noise_g, d_noise_h, d_noise_gf, d_noise_hf, stream);
     launch_root_sums(d_jobs, K, p, exact_quant_root, stream);
     // histograms are added up in zeroed slots: one per split
     launch_zero_pool(d_pool, pool_bytes_per_job, slot_bytes * (size_t)(rounds() ? 1 + p.max_exp : p.num_leaves), K,
@@ -622,6 +623,10 @@ int learner_create(const bk_feature* features, int32_t num_features, const uint8
       L->d_noise_h = L->dalloc<double>(n);
       CK(cudaMemcpy(L->d_noise_g, ng.data(), n * sizeof(double), cudaMemcpyHostToDevice));
       CK(cudaMemcpy(L->d_noise_h, nh.data(), n * sizeof(double), cudaMemcpyHostToDevice));
+      L->d_noise_gf = L->dalloc<float>(n);
+      L->d_noise_hf = L->dalloc<float>(n);
+      launch_noise_f32(L->d_noise_g, L->d_noise_gf, num_data, L->stream);
+      launch_noise_f32(L->d_noise_h, L->d_noise_hf, num_data, L->stream);
     }
     const int Lv = p.num_leaves, F = num_features, K = num_jobs;
     L->d_g = L->dalloc<float>(n * K);

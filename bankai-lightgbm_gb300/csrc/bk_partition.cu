@@ -32,6 +32,7 @@ struct PartRange {
   const int16_t* pk_src;
   int16_t* pk_dst;
   bool pk_row;
+  bool all;  // every row in order: the row of position e is e
 };
 
 __device__ __forceinline__ int32_t part_pk(const PartRange& R, int64_t e, int32_t row) {
@@ -63,6 +64,7 @@ __device__ __forceinline__ void part_range(const Job& J, const Params& p, const 
   r->src = leaf_idx(J, buf) + r->begin;
   r->dst = leaf_idx_w(J, 1 - buf) + r->begin;
   r->col = bins_cm + (size_t)d.inner * (size_t)p.n;
+  r->all = false;
   r->pk_row = d.new_leaf == 1;  // the root (one leaf when decided): no leaf-ordered copy yet
   r->pk_src = p.quant ? (r->pk_row ? J.packed : leaf_pk(J, buf) + r->begin) : nullptr;
   r->pk_dst = p.quant ? leaf_pk(J, 1 - buf) + r->begin : nullptr;
@@ -278,7 +280,7 @@ __device__ __forceinline__ void onepass_rows(const PartRange& R, bool quant, con
 #pragma unroll
     for (int k = 0; k < kItems; ++k) {
       const int64_t e = base + k * kThreads + threadIdx.x;
-      rows[k] = e < R.r1 ? __ldg(R.src + e) : -1;
+      rows[k] = e < R.r1 ? (R.all ? (int32_t)e : __ldg(R.src + e)) : -1;
     }
     int32_t pkv[kItems];
 #pragma unroll
@@ -460,6 +462,7 @@ __global__ void __launch_bounds__(kThreads) k_part_round(const JobTable jobs, Pa
       R.dst = leaf_idx_w(J, 1 - buf) + R.begin;
       R.col = bins_cm + (size_t)d.inner * (size_t)p.n;
       R.pk_row = c.node == 0;  // the root: no leaf-ordered copy yet
+      R.all = c.node == 0 && c.count == p.n;  // an unbagged root: the identity
       R.pk_src = p.quant ? (R.pk_row ? J.packed : leaf_pk(J, buf) + R.begin) : nullptr;
       R.pk_dst = p.quant ? leaf_pk(J, 1 - buf) + R.begin : nullptr;
       build_route(J, p, d, feats, lut);

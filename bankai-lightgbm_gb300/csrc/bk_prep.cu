@@ -9,6 +9,8 @@
 //   - score update and leaf lookup over the final partition (serial.rs:1974-1990).
 #include <math_constants.h>
 
+#include <algorithm>
+
 #include "bk_math.cuh"
 
 namespace bk {
@@ -17,9 +19,12 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 
-__global__ void k_init_rows(const Job* __restrict__ jobs, Params p, const int32_t* __restrict__ rows) {
+// The root's row indices. Without bagging they are the identity, which the grow rounds (and every
+// reader of a leaf of all rows) derive instead of reading: `bagged_only` skips those 4 bytes a row.
+__global__ void k_init_rows(const Job* __restrict__ jobs, Params p, const int32_t* __restrict__ rows, int bagged_only) {
   const Job& J = jobs[blockIdx.z];
   const int64_t cnt = J.st->root_count;
+  if (bagged_only && !J.st->use_rows) return;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cnt; i += (int64_t)gridDim.x * blockDim.x)
     J.idx0[i] = J.st->use_rows ? rows[i] : (int32_t)i;
 }
@@ -77,17 +82,29 @@ __global__ void k_disc_reset(const Job* __restrict__ jobs) {
   s->red_flags = 0u;
 }
 
-// max |g| and max h over all rows (order-free), and the refused cases (mod.rs:134-155).
-__global__ void k_disc_reduce(const Job* __restrict__ jobs, Params p) {
+// max |g| and max h over all rows (order-free), and the refused cases (mod.rs:134-155). HBM-bound:
+// 16-byte loads, four rows a thread and step (10M rows: 28 -> 22 us).
+__global__ void __launch_bounds__(256) k_disc_reduce(const Job* __restrict__ jobs, Params p) {
   const Job& J = jobs[blockIdx.z];
   float mg = 0.f, mh = 0.f;
   uint32_t bad = 0;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.n; i += (int64_t)gridDim.x * blockDim.x) {
-    float g = J.g[i], h = J.h[i];
+  auto take = [&](float g, float h) {
     if (!isfinite(g) || !isfinite(h) || h < 0.f) bad = 1u;
     mg = fmaxf(mg, fabsf(g));
     mh = fmaxf(mh, h);
+  };
+  const int64_t step = (int64_t)gridDim.x * blockDim.x, t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  // a job's rows start at a multiple of n floats: 16-byte loads where that is aligned
+  const bool vec = ((reinterpret_cast<uintptr_t>(J.g) | reinterpret_cast<uintptr_t>(J.h)) & 15u) == 0u;
+  const int64_t n4 = vec ? p.n / 4 : 0;
+  for (int64_t i = t; i < n4; i += step) {
+    const float4 g = reinterpret_cast<const float4*>(J.g)[i], h = reinterpret_cast<const float4*>(J.h)[i];
+    take(g.x, h.x);
+    take(g.y, h.y);
+    take(g.z, h.z);
+    take(g.w, h.w);
   }
+  for (int64_t i = 4 * n4 + t; i < p.n; i += step) take(J.g[i], J.h[i]);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     mg = fmaxf(mg, __shfl_xor_sync(FULL, mg, o));
@@ -102,11 +119,11 @@ __global__ void k_disc_reduce(const Job* __restrict__ jobs, Params p) {
   }
 }
 
-// One thread for all jobs, in job order: the K class trees of an iteration share one
-// discretizer, so their rotation offsets are consecutive draws of one engine (held by job 0).
-__global__ void k_disc_setup(const Job* __restrict__ jobs, int num_jobs, Params p) {
-  JobState* eng = jobs[0].st;
-  for (int j = 0; j < num_jobs; ++j) {
+// The scales of every job on a thread each; then one thread in job order: the K class trees of an
+// iteration share one discretizer, so their rotation offsets are consecutive draws of one engine
+// (held by job 0).
+__global__ void __launch_bounds__(32) k_disc_setup(const Job* __restrict__ jobs, int num_jobs, Params p) {
+  for (int j = threadIdx.x; j < num_jobs; j += 32) {
     JobState* s = jobs[j].st;
     float max_g = __uint_as_float(s->red_maxg), max_h = __uint_as_float(s->red_maxh);
     bool ok = s->red_flags == 0u && max_g != 0.f && (p.const_hess || max_h != 0.f);
@@ -116,8 +133,12 @@ __global__ void k_disc_setup(const Job* __restrict__ jobs, int num_jobs, Params 
     s->hscale = p.const_hess ? (double)max_h : (double)max_h / (double)p.quant_bins;
     s->inv_g = 1.0 / s->gscale;
     s->inv_h = 1.0 / s->hscale;
-    if (p.stochastic) s->start_pos = mt_uniform_int_inclusive(eng, (uint32_t)p.n);
   }
+  __syncwarp();
+  if (threadIdx.x != 0 || !p.stochastic) return;
+  JobState* eng = jobs[0].st;
+  for (int j = 0; j < num_jobs; ++j)
+    if (jobs[j].st->disc_ok) jobs[j].st->start_pos = mt_uniform_int_inclusive(eng, (uint32_t)p.n);
 }
 
 __device__ __forceinline__ int32_t sat_i8(double v) {  // Rust `f64 as i8`
@@ -127,31 +148,88 @@ __device__ __forceinline__ int32_t sat_i8(double v) {  // Rust `f64 as i8`
   return (int32_t)trunc(v);
 }
 
-__global__ void k_discretize(const Job* __restrict__ jobs, Params p, const double* __restrict__ noise_g,
-                             const double* __restrict__ noise_h) {
+// trunc(v * scale + noise) saturated to int8, as f64 arithmetic gives it. f64 costs 64 cycles of a
+// scheduler's pipe per warp instruction on this part, so the value is computed in fp32 first: its
+// error is at most 4u (|x| + 1) (u = 2^-24: the scale's and the noise's rounding, the product, the
+// sum), so a result further than twice that from every whole number truncates to the same one; the
+// others (about one row in 400,000) are evaluated in f64.
+__device__ __forceinline__ int32_t disc_value(float v, float scale_f, float noise_f, double scale, const double* noise,
+                                              double off, bool fused) {
+  const float x = fmaf(v, scale_f, v >= 0.f ? noise_f : -noise_f);
+  const float w = rintf(x);
+  if (fabsf(x - w) > 8.0f * 5.9604645e-08f * (fabsf(x) + 1.0f) && fabsf(x) < 126.0f) return (int32_t)x;
+  const double nv = noise ? *noise : off, dv = (double)v;
+  return sat_i8(madd(dv, scale, dv >= 0.0 ? nv : -nv, fused));
+}
+
+// Four rows a thread; also the root's integer sums when the root is all rows (k_root_partial then has
+// nothing to do). HBM-bound: 4 bytes each of gradient (hessian), fp32 noise, 2 of result a row (10M
+// rows, constant hessian: 181 -> 25 us; with hessians 336 -> 44; the f64 form was bound by the f64 pipe).
+__global__ void __launch_bounds__(256) k_discretize(const Job* __restrict__ jobs, Params p,
+                                                    const double* __restrict__ noise_g,
+                                                    const double* __restrict__ noise_h,
+                                                    const float* __restrict__ noise_gf,
+                                                    const float* __restrict__ noise_hf) {
+  __shared__ long long sg_s[8], sh_s[8];
   const Job& J = jobs[blockIdx.z];
   const JobState* s = J.st;
   if (!s->disc_ok) return;
   const double ig = s->inv_g, ih = s->inv_h;
+  const float igf = (float)ig, ihf = (float)ih;
   const bool fused = p.fused != 0;
-  const int64_t start = s->start_pos;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < p.n; i += (int64_t)gridDim.x * blockDim.x) {
-    double gv = (double)J.g[i];
-    int32_t gi, hi;
+  const uint32_t n = (uint32_t)p.n, start = s->start_pos;
+  long long sg = 0, sh = 0;
+  auto one = [&](uint32_t i, float g, float h) -> uint32_t {
+    uint32_t pos = i + start;  // both at most n < 2^31
+    if (pos >= n) pos -= n;
+    int32_t gi, hi = 1;
     if (p.stochastic) {
-      int64_t pos = i + start;
-      if (pos >= p.n) pos -= p.n;
-      double noise = noise_g[pos];
-      double sn = gv >= 0.0 ? noise : -noise;
-      gi = sat_i8(madd(gv, ig, sn, fused));
-      hi = p.const_hess ? 1 : sat_i8(madd((double)J.h[i], ih, noise_h[pos], fused));
+      gi = disc_value(g, igf, noise_gf[pos], ig, noise_g + pos, 0.0, fused);
+      if (!p.const_hess) hi = disc_value(h, ihf, noise_hf[pos], ih, noise_h + pos, 0.0, fused);
     } else {
-      double off = gv >= 0.0 ? 0.5 : -0.5;
-      gi = sat_i8(madd(gv, ig, off, fused));
-      hi = p.const_hess ? 1 : sat_i8(madd((double)J.h[i], ih, 0.5, fused));
+      gi = disc_value(g, igf, 0.5f, ig, nullptr, 0.5, fused);
+      if (!p.const_hess) hi = disc_value(h, ihf, 0.5f, ih, nullptr, 0.5, fused);
     }
-    J.packed[i] = (int16_t)((gi * 256) | (hi & 0xff));
+    sg += gi;
+    sh += hi & 0xff;
+    return (uint32_t)((gi * 256) | (hi & 0xff)) & 0xffffu;
+  };
+  const uint32_t step = gridDim.x * blockDim.x, t = blockIdx.x * blockDim.x + threadIdx.x;
+  const bool vec = (((reinterpret_cast<uintptr_t>(J.g) | reinterpret_cast<uintptr_t>(J.h)) & 15u) |
+                    (reinterpret_cast<uintptr_t>(J.packed) & 7u)) == 0u;
+  const uint32_t n4 = vec ? n / 4u : 0u;
+  for (uint32_t k = t; k < n4; k += step) {
+    const float4 g = reinterpret_cast<const float4*>(J.g)[k];
+    const float4 h = p.const_hess ? make_float4(0.f, 0.f, 0.f, 0.f) : reinterpret_cast<const float4*>(J.h)[k];
+    const uint32_t a = one(4u * k, g.x, h.x), b = one(4u * k + 1u, g.y, h.y);
+    const uint32_t c = one(4u * k + 2u, g.z, h.z), d = one(4u * k + 3u, g.w, h.w);
+    reinterpret_cast<uint2*>(J.packed)[k] = make_uint2(a | (b << 16), c | (d << 16));
   }
+  for (uint32_t i = 4u * n4 + t; i < n; i += step) J.packed[i] = (int16_t)one(i, J.g[i], p.const_hess ? 0.f : J.h[i]);
+  if (s->use_rows) return;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    sg += __shfl_xor_sync(FULL, sg, o);
+    sh += __shfl_xor_sync(FULL, sh, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    sg_s[threadIdx.x >> 5] = sg;
+    sh_s[threadIdx.x >> 5] = sh;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int w = 1; w < 8; ++w) {
+      sg += sg_s[w];
+      sh += sh_s[w];
+    }
+    J.ired[2 * blockIdx.x] = sg;
+    J.ired[2 * blockIdx.x + 1] = sh;
+  }
+}
+
+__global__ void k_noise_f32(const double* __restrict__ a, float* __restrict__ b, int64_t n) {
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
+    b[i] = (float)a[i];
 }
 
 // ---- root sums ----
@@ -165,10 +243,12 @@ __global__ void __launch_bounds__(256) k_root_partial(const Job* __restrict__ jo
   __shared__ long long ig_s[8], ih_s[8];
   const Job& J = jobs[blockIdx.z];
   const int64_t cnt = J.st->root_count;
+  const bool bagged = J.st->use_rows != 0;
+  if (p.quant && !bagged && J.st->disc_ok) return;  // the discretization has left its sums
   double sg = 0.0, sh = 0.0;
   long long ig = 0, ih = 0;
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < cnt; k += (int64_t)gridDim.x * blockDim.x) {
-    int64_t i = J.idx0[k];
+    const int64_t i = bagged ? J.idx0[k] : k;
     if (p.quant) {
       int32_t pk = J.packed[i];
       ig += (int8_t)(pk >> 8);
@@ -209,18 +289,36 @@ __global__ void __launch_bounds__(256) k_root_partial(const Job* __restrict__ jo
   }
 }
 
-__global__ void k_root_finish(const Job* __restrict__ jobs, Params p, int exact_quant_root) {
+// One warp: the partials, lane l taking CTAs l, l + 32, ... and a tree over the lanes (one lane over
+// all of them took 45 us: a chain of f64 additions).
+__global__ void __launch_bounds__(32) k_root_finish(const Job* __restrict__ jobs, Params p, int exact_quant_root) {
   const Job& J = jobs[blockIdx.z];
   JobState* s = J.st;
   const int lane = threadIdx.x;
   double sg = 0.0, sh = 0.0;
   int64_t ig = 0, ih = 0;
-  if (lane == 0) {
-    for (int b = 0; b < kRootGrid; ++b) {
-      sg += J.red[2 * b];
-      sh += J.red[2 * b + 1];
-      ig += J.ired[2 * b];
-      ih += J.ired[2 * b + 1];
+  static_assert(kRootGrid % 32 == 0, "whole rounds of the warp");
+  if (p.quant) {
+#pragma unroll 4
+    for (int b = 0; b < kRootGrid; b += 32) {
+      ig += J.ired[2 * (b + lane)];
+      ih += J.ired[2 * (b + lane) + 1];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      ig += __shfl_xor_sync(FULL, ig, o);
+      ih += __shfl_xor_sync(FULL, ih, o);
+    }
+  } else {
+#pragma unroll 4
+    for (int b = 0; b < kRootGrid; b += 32) {
+      sg += J.red[2 * (b + lane)];
+      sh += J.red[2 * (b + lane) + 1];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      sg += __shfl_xor_sync(FULL, sg, o);
+      sh += __shfl_xor_sync(FULL, sh, o);
     }
   }
   if (p.quant && !exact_quant_root) {
@@ -231,7 +329,7 @@ __global__ void k_root_finish(const Job* __restrict__ jobs, Params p, int exact_
       int64_t k = base + lane;
       int32_t gi = 0, hi = 0;
       if (k < cnt) {
-        int32_t pk = J.packed[J.idx0[k]];
+        int32_t pk = J.packed[s->use_rows ? J.idx0[k] : (int32_t)k];
         gi = (int8_t)(pk >> 8);
         hi = pk & 0xff;
       }
@@ -270,12 +368,13 @@ __global__ void __launch_bounds__(32) k_renew(const Job* __restrict__ jobs, Para
   const int lane = threadIdx.x;
   const int64_t begin = J.leaf_begin[leaf], cnt = J.leaf_count[leaf];
   const int32_t* idx = leaf_idx(J, J.leaf_buf[leaf]) + begin;
+  const bool all = cnt == p.n;  // every row, in order
   double s1 = 0.0, s2 = 0.0;
   for (int64_t base = 0; base < cnt; base += 32) {
     int64_t k = base + lane;
     float gv = 0.f, hv = 0.f;
     if (k < cnt) {
-      int32_t r = idx[k];
+      int32_t r = all ? (int32_t)k : idx[k];
       gv = J.g[r];
       hv = J.h[r];
     }
@@ -293,36 +392,99 @@ __global__ void __launch_bounds__(32) k_renew(const Job* __restrict__ jobs, Para
 }
 
 // ---- score update / leaf lookup over the final partition ----
-__global__ void k_add_score(const Job* __restrict__ jobs, Params p, const double* __restrict__ vals,
-                            double* __restrict__ score) {
+// The leaves' row ranges tile the positions 0 .. root count of the index buffers, so every CTA takes
+// the same number of positions (`per`), whatever the leaves' sizes: it lists the leaves that overlap
+// them (one thread per leaf), then walks those parts, four positions a thread in flight. (A grid over
+// leaves left the chip to the largest ones: the score update of ten 63-leaf trees on 2M rows took 515
+// us, now 132.) Bound by the scattered 8-byte updates: 10M rows, whose score outgrows L2, 167 us.
+constexpr int kLeafParts = 256;  // leaves looked at per pass
+
+// Calls f(leaf, rows[4]) for this CTA's rows (-1: none). All 256 threads call it.
+template <typename F>
+__device__ __forceinline__ void for_leaf_rows(const Job& J, const Params& p, int per, F f) {
+  __shared__ int32_t s_leaf[kLeafParts], s_n;
+  const int32_t leaves = J.st->tree_leaves;
+  const int64_t q0 = (int64_t)blockIdx.x * per, q1 = q0 + per;
+  for (int32_t l0 = 0; l0 < leaves; l0 += kLeafParts) {
+    if (threadIdx.x == 0) s_n = 0;
+    __syncthreads();
+    const int32_t l = l0 + (int32_t)threadIdx.x;
+    static_assert(kLeafParts == 256, "one leaf per thread");
+    if (l < leaves) {
+      const int64_t b = J.leaf_begin[l], c = J.leaf_count[l];
+      if (b < q1 && b + c > q0) s_leaf[atomicAdd(&s_n, 1)] = l;
+    }
+    __syncthreads();
+    for (int k = 0; k < s_n; ++k) {
+      const int32_t leaf = s_leaf[k];
+      const int64_t b = J.leaf_begin[leaf], c = J.leaf_count[leaf];
+      const int32_t* idx = leaf_idx(J, J.leaf_buf[leaf]);
+      const bool all = c == p.n;  // every row, in order
+      const int64_t e0 = max(b, q0), e1 = min(b + c, q1);
+      for (int64_t i = e0 + threadIdx.x; i < e1; i += 4 * 256) {
+        int32_t row[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) row[u] = i + u * 256 < e1 ? (all ? (int32_t)(i + u * 256) : idx[i + u * 256]) : -1;
+        f(leaf, row);
+      }
+    }
+    __syncthreads();
+  }
+}
+
+__device__ __forceinline__ void add_rows(double* __restrict__ sc, const int32_t (&row)[4], double v) {
+  double x[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) x[u] = row[u] >= 0 ? sc[row[u]] : 0.0;
+#pragma unroll
+  for (int u = 0; u < 4; ++u)
+    if (row[u] >= 0) sc[row[u]] = x[u] + v;
+}
+
+__global__ void __launch_bounds__(256) k_add_score(const Job* __restrict__ jobs, Params p, int per,
+                                                   const double* __restrict__ vals, double* __restrict__ score) {
   const Job& J = jobs[blockIdx.z];
-  const int32_t leaf = blockIdx.y;
-  if (leaf >= J.st->tree_leaves || J.st->tree_leaves <= 1) return;
-  const double v = vals[(size_t)blockIdx.z * p.num_leaves + leaf];
-  const int64_t begin = J.leaf_begin[leaf], cnt = J.leaf_count[leaf];
-  const int32_t* idx = leaf_idx(J, J.leaf_buf[leaf]) + begin;
+  if (J.st->tree_leaves <= 1) return;
+  const double* v = vals + (size_t)blockIdx.z * p.num_leaves;
   double* sc = score + (size_t)blockIdx.z * p.n;
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < cnt; k += (int64_t)gridDim.x * blockDim.x)
-    sc[idx[k]] += v;
+  for_leaf_rows(J, p, per, [&](int32_t leaf, const int32_t (&row)[4]) { add_rows(sc, row, v[leaf]); });
 }
 
 // The same update with the tree's own leaf outputs from the device, shrunk as Tree::apply_shrinkage
 // does (tree.rs:446-463): score += round_to_zero(leaf_value * rate). A one-leaf tree adds nothing
 // (train.rs:776-795 turns it into a constant tree instead).
-__global__ void k_add_score_own(const Job* __restrict__ jobs, Params p, double rate, double* __restrict__ score,
-                                int need_stop) {
+__global__ void __launch_bounds__(256) k_add_score_own(const Job* __restrict__ jobs, Params p, int per, double rate,
+                                                       double* __restrict__ score, int need_stop) {
   const Job& J = jobs[blockIdx.z];
-  const int32_t leaf = blockIdx.y;
   for (int j = 0; need_stop && j < (int)gridDim.z; ++j)
     if (!jobs[j].st->stop) return;  // the trees need more rounds: the update comes after those
-  if (leaf >= J.st->tree_leaves || J.st->tree_leaves <= 1) return;
-  double v = __dmul_rn(J.leaf_value[leaf], rate);
-  if (v >= -BK_ZERO_THRESHOLD && v <= BK_ZERO_THRESHOLD) v = 0.0;
-  const int64_t begin = J.leaf_begin[leaf], cnt = J.leaf_count[leaf];
-  const int32_t* idx = leaf_idx(J, J.leaf_buf[leaf]) + begin;
+  if (J.st->tree_leaves <= 1) return;
   double* sc = score + (size_t)blockIdx.z * p.n;
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < cnt; k += (int64_t)gridDim.x * blockDim.x)
-    sc[idx[k]] += v;
+  for_leaf_rows(J, p, per, [&](int32_t leaf, const int32_t (&row)[4]) {
+    double v = __dmul_rn(J.leaf_value[leaf], rate);
+    if (v >= -BK_ZERO_THRESHOLD && v <= BK_ZERO_THRESHOLD) v = 0.0;
+    add_rows(sc, row, v);
+  });
+}
+
+__global__ void __launch_bounds__(256) k_row_leaf(const Job* __restrict__ jobs, Params p, int per,
+                                                  int32_t* __restrict__ out) {
+  const Job& J = jobs[blockIdx.z];
+  int32_t* o = out + (size_t)blockIdx.z * p.n;
+  for_leaf_rows(J, p, per, [&](int32_t leaf, const int32_t (&row)[4]) {
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (row[u] >= 0) o[row[u]] = leaf;
+  });
+}
+
+// Positions per CTA: about eight CTAs per SM, 256 to 4096.
+static int leaf_rows_per(const Params& p) {
+  const int64_t per = ceil_div64(ceil_div64(p.n, 1216), 256) * 256;
+  return (int)std::min<int64_t>(std::max<int64_t>(per, 256), 4096);
+}
+static dim3 leaf_rows_grid(const Params& p, int num_jobs) {
+  return dim3((unsigned)ceil_div64(p.n, leaf_rows_per(p)), 1, num_jobs);
 }
 
 __global__ void k_zero_pool(uint4* __restrict__ pool, size_t per_job, size_t n) {
@@ -331,21 +493,11 @@ __global__ void k_zero_pool(uint4* __restrict__ pool, size_t per_job, size_t n) 
     z[i] = make_uint4(0, 0, 0, 0);
 }
 
-__global__ void k_row_leaf(const Job* __restrict__ jobs, Params p, int32_t* __restrict__ out) {
-  const Job& J = jobs[blockIdx.z];
-  const int32_t leaf = blockIdx.y;
-  if (leaf >= J.st->tree_leaves) return;
-  const int64_t begin = J.leaf_begin[leaf], cnt = J.leaf_count[leaf];
-  const int32_t* idx = leaf_idx(J, J.leaf_buf[leaf]) + begin;
-  int32_t* o = out + (size_t)blockIdx.z * p.n;
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < cnt; k += (int64_t)gridDim.x * blockDim.x)
-    o[idx[k]] = leaf;
-}
-
 }  // namespace
 
-void launch_init_rows(const Job* d_jobs, int num_jobs, const Params& p, const int32_t* rows, cudaStream_t s) {
-  k_init_rows<<<dim3(1024, 1, num_jobs), 256, 0, s>>>(d_jobs, p, rows);
+void launch_init_rows(const Job* d_jobs, int num_jobs, const Params& p, const int32_t* rows, bool bagged_only,
+                      cudaStream_t s) {
+  k_init_rows<<<dim3(1024, 1, num_jobs), 256, 0, s>>>(d_jobs, p, rows, bagged_only ? 1 : 0);
 }
 
 void launch_mt_seed(const Job* d_jobs, int num_jobs, uint32_t seed, cudaStream_t s) {
@@ -353,12 +505,15 @@ void launch_mt_seed(const Job* d_jobs, int num_jobs, uint32_t seed, cudaStream_t
   k_mt_seed<<<1, 1, 0, s>>>(d_jobs, seed);
 }
 
+void launch_noise_f32(const double* a, float* b, int64_t n, cudaStream_t s) { k_noise_f32<<<1024, 256, 0, s>>>(a, b, n); }
+
 void launch_discretize(const Job* d_jobs, int num_jobs, const Params& p, const double* noise_g, const double* noise_h,
-                       cudaStream_t s) {
+                       const float* noise_gf, const float* noise_hf, cudaStream_t s) {
   k_disc_reset<<<dim3(1, 1, num_jobs), 1, 0, s>>>(d_jobs);
-  k_disc_reduce<<<dim3(512, 1, num_jobs), 256, 0, s>>>(d_jobs, p);
-  k_disc_setup<<<1, 1, 0, s>>>(d_jobs, num_jobs, p);
-  k_discretize<<<dim3(1024, 1, num_jobs), 256, 0, s>>>(d_jobs, p, noise_g, noise_h);
+  const unsigned grid = (unsigned)std::min<int64_t>(ceil_div64(p.n, 1024), 1216);
+  k_disc_reduce<<<dim3(grid, 1, num_jobs), 256, 0, s>>>(d_jobs, p);
+  k_disc_setup<<<1, 32, 0, s>>>(d_jobs, num_jobs, p);
+  k_discretize<<<dim3(kRootGrid, 1, num_jobs), 256, 0, s>>>(d_jobs, p, noise_g, noise_h, noise_gf, noise_hf);
 }
 
 void launch_root_sums(const Job* d_jobs, int num_jobs, const Params& p, int exact_quant_root, cudaStream_t s) {
@@ -372,12 +527,12 @@ void launch_renew(const Job* d_jobs, int num_jobs, const Params& p, cudaStream_t
 
 void launch_add_score(const Job* d_jobs, int num_jobs, const Params& p, const double* leaf_vals, double* score,
                       cudaStream_t s) {
-  k_add_score<<<dim3(8, p.num_leaves, num_jobs), 256, 0, s>>>(d_jobs, p, leaf_vals, score);
+  k_add_score<<<leaf_rows_grid(p, num_jobs), 256, 0, s>>>(d_jobs, p, leaf_rows_per(p), leaf_vals, score);
 }
 
 void launch_add_score_own(const Job* d_jobs, int num_jobs, const Params& p, double rate, double* score, int need_stop,
                           cudaStream_t s) {
-  k_add_score_own<<<dim3(8, p.num_leaves, num_jobs), 256, 0, s>>>(d_jobs, p, rate, score, need_stop);
+  k_add_score_own<<<leaf_rows_grid(p, num_jobs), 256, 0, s>>>(d_jobs, p, leaf_rows_per(p), rate, score, need_stop);
 }
 
 void launch_zero_pool(void* pool, size_t bytes_per_job, size_t bytes, int num_jobs, cudaStream_t s) {
@@ -385,7 +540,7 @@ void launch_zero_pool(void* pool, size_t bytes_per_job, size_t bytes, int num_jo
 }
 
 void launch_row_leaf(const Job* d_jobs, int num_jobs, const Params& p, int32_t* out, cudaStream_t s) {
-  k_row_leaf<<<dim3(8, p.num_leaves, num_jobs), 256, 0, s>>>(d_jobs, p, out);
+  k_row_leaf<<<leaf_rows_grid(p, num_jobs), 256, 0, s>>>(d_jobs, p, leaf_rows_per(p), out);
 }
 
 }  // namespace bk
