@@ -17,47 +17,108 @@
 // host turns into an error (a label is never used as an index without this check).
 #include <math_constants.h>
 
+#include <cmath>
+
 #include "bk_common.cuh"
+#include "bk_pair.cuh"
 
 namespace bk {
 
 namespace {
 
-__global__ void k_grad_l2(const double* __restrict__ score, const float* __restrict__ label, int64_t n,
-                          const float* __restrict__ w, float* __restrict__ g, float* __restrict__ h) {
+// The gradients end as fp32, so they are computed as fp32 pairs and, where a pair's error could move
+// the rounding, in f64 (bk_pair.cuh): the same fp32 numbers without the f64 pipe. `rel` is the bound on
+// a pair's relative error, plus what the f64 evaluation itself rounds away. Measured, 10M rows: L2 60
+// -> 48 us (HBM), binary 637 -> 89 us; softmax of ten classes on 2M rows 1277 -> 282 us (issue).
+__host__ __device__ constexpr float kTwo(int e) { return e >= 0 ? (float)(1ull << e) : 1.0f / (float)(1ull << -e); }
+
+__global__ void __launch_bounds__(256) k_grad_l2(const double* __restrict__ score, const float* __restrict__ label,
+                                                 int64_t n, const float* __restrict__ w, float* __restrict__ g,
+                                                 float* __restrict__ h) {
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    const float d = (float)(score[i] - (double)label[i]);
+    const double s = score[i];
+    const float l = label[i];
+    bool ok;
+    const Pair sp = pair_of(s, &ok);
+    Pair d = two_sum(sp.hi, -l);
+    d = quick_two_sum(d.hi, __fadd_rn(d.lo, sp.lo));
+    const float rel = __fdividef(__fmul_rn(kTwo(-46), fabsf(sp.hi)), fabsf(d.hi)) + kTwo(-50);
+    float v;
+    if (!pair_round(d, rel, &v) || !ok) v = (float)(s - (double)l);
     if (w) {
       const float wi = w[i];
-      g[i] = __fmul_rn(d, wi);
+      g[i] = __fmul_rn(v, wi);
       h[i] = wi;
     } else {
-      g[i] = d;
+      g[i] = v;
       h[i] = 1.0f;
     }
   }
 }
 
-__global__ void k_grad_binary(const double* __restrict__ score, const float* __restrict__ label, int64_t n,
-                              double sigmoid, const float* __restrict__ w, double lw_neg, double lw_pos,
-                              float* __restrict__ g, float* __restrict__ h) {
+// The reference's arithmetic of one binary row in f64.
+__device__ __noinline__ float2 binary_row(double score, bool pos, double sigmoid, double lw, const float* wi) {
+  const double lab = pos ? 1.0 : -1.0;
+  const double t = -lab * sigmoid;
+  const double e = exp(lab * sigmoid * score);
+  const double response = t / (1.0 + e);
+  const double ar = fabs(response);
+  const double q = ar * (sigmoid - ar);
+  if (wi) return make_float2((float)(response * lw * (double)*wi), (float)(q * lw * (double)*wi));
+  return make_float2((float)(response * lw), (float)(q * lw));
+}
+
+__global__ void __launch_bounds__(256) k_grad_binary(const double* __restrict__ score, const float* __restrict__ label,
+                                                     int64_t n, double sigmoid, const float* __restrict__ w,
+                                                     double lw_neg, double lw_pos, const ExpTable T,
+                                                     float* __restrict__ g, float* __restrict__ h) {
+  __shared__ ExpTable st;
+  if (threadIdx.x < 32) {
+    st.hi[threadIdx.x] = T.hi[threadIdx.x];
+    st.lo[threadIdx.x] = T.lo[threadIdx.x];
+  }
+  __syncthreads();
+  bool ok_s, ok_n, ok_p;
+  const Pair sg = pair_of(sigmoid, &ok_s), ln = pair_of(lw_neg, &ok_n), lp = pair_of(lw_pos, &ok_p);
+  const bool unit = lw_neg == 1.0 && lw_pos == 1.0, one = sigmoid == 1.0;
+  const bool ok_c = ok_s && ok_n && ok_p;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const double s = score[i];
     const bool pos = label[i] > 0.0f;
-    double lab = pos ? 1.0 : -1.0;
-    const double lw = pos ? lw_pos : lw_neg;
-    double t = -lab * sigmoid;
-    double e = exp(lab * sigmoid * score[i]);
-    double response = t / (1.0 + e);
-    double ar = fabs(response);
-    double q = ar * (sigmoid - ar);
-    if (w) {
-      const double wi = (double)w[i];
-      g[i] = (float)(response * lw * wi);
-      h[i] = (float)(q * lw * wi);
-    } else {
-      g[i] = (float)(response * lw);
-      h[i] = (float)(q * lw);
+    bool ok;
+    Pair z = pair_of(one ? s : sigmoid * s, &ok);
+    if (!pos) z = pair_neg(z);
+    ok = ok && ok_c && fabsf(z.hi) <= 60.0f;
+    float gv = 0.f, hv = 0.f;
+    if (ok) {
+      // response = -label s / (1 + e), hessian |response| (s - |response|) = s^2 e / (1 + e)^2
+      const Pair e = pair_exp(z, st);
+      const Pair d = e.hi > 1.0f ? pair_add(e, Pair{1.f, 0.f}) : pair_add(Pair{1.f, 0.f}, e);
+      Pair r = pair_div(sg, d);
+      const Pair c = pair_mul(r, e);  // s - |response|
+      Pair q = pair_mul(r, c);
+      const float rel_h = kTwo(-39) + __fdividef(__fmul_rn(kTwo(-50), sg.hi), c.hi);
+      if (!unit) {
+        const Pair lw = pos ? lp : ln;
+        r = pair_mul(r, lw);
+        q = pair_mul(q, lw);
+      }
+      if (w) {
+        const Pair wi{w[i], 0.f};
+        r = pair_mul(r, wi);
+        q = pair_mul(q, wi);
+      }
+      const bool a = pair_round(r, kTwo(-40), &gv), b = pair_round(q, rel_h, &hv);
+      ok = a && b;
+      if (pos) gv = -gv;
     }
+    if (!ok) {
+      const float2 v = binary_row(s, pos, sigmoid, pos ? lw_pos : lw_neg, w ? w + i : nullptr);
+      gv = v.x;
+      hv = v.y;
+    }
+    g[i] = gv;
+    h[i] = hv;
   }
 }
 
@@ -68,30 +129,106 @@ __device__ __forceinline__ int class_of(float lf, int K, int32_t* bad_label) {
   return -1;
 }
 
-__global__ void k_grad_softmax(const double* __restrict__ score, const float* __restrict__ label, int64_t n, int K,
-                               const float* __restrict__ w, float* __restrict__ g, float* __restrict__ h,
-                               int32_t* __restrict__ bad_label) {
+// The reference's arithmetic of one softmax row in f64.
+__device__ __noinline__ void softmax_row(const double* __restrict__ score, int64_t n, int64_t i, int K, int lab,
+                                         const float* __restrict__ w, float* __restrict__ g, float* __restrict__ h) {
   const double factor = (double)K / ((double)K - 1.0);
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    double rec[32];
-    double wmax = score[i];
-    for (int k = 1; k < K; ++k) wmax = fmax(score[(size_t)k * n + i], wmax);
-    double wsum = 0.0;
-    for (int k = 0; k < K; ++k) {
-      rec[k] = exp(score[(size_t)k * n + i] - wmax);
-      wsum += rec[k];
-    }
-    const int lab = class_of(label[i], K, bad_label);
-    const double wi = w ? (double)w[i] : 1.0;
-    for (int k = 0; k < K; ++k) {
-      double p = rec[k] / wsum;
-      double gi = lab == k ? p - 1.0 : p;
-      double hi = factor * p;
-      hi = hi * (1.0 - p);
-      g[(size_t)k * n + i] = (float)(w ? gi * wi : gi);
-      h[(size_t)k * n + i] = (float)(w ? hi * wi : hi);
-    }
+  double rec[32];
+  double wmax = score[i];
+  for (int k = 1; k < K; ++k) wmax = fmax(score[(size_t)k * n + i], wmax);
+  double wsum = 0.0;
+  for (int k = 0; k < K; ++k) {
+    rec[k] = exp(score[(size_t)k * n + i] - wmax);
+    wsum += rec[k];
   }
+  const double wi = w ? (double)w[i] : 1.0;
+  for (int k = 0; k < K; ++k) {
+    double p = rec[k] / wsum;
+    double gi = lab == k ? p - 1.0 : p;
+    double hi = factor * p;
+    hi = hi * (1.0 - p);
+    g[(size_t)k * n + i] = (float)(w ? gi * wi : gi);
+    h[(size_t)k * n + i] = (float)(w ? hi * wi : hi);
+  }
+}
+
+// The classes' exponentials of a thread's row stay in shared memory ([K][128] pairs) between the sum
+// and the gradients. Scores up to 64 in magnitude take pairs.
+constexpr int kSoftmaxThreads = 128;
+__global__ void __launch_bounds__(kSoftmaxThreads)
+    k_grad_softmax(const double* __restrict__ score, const float* __restrict__ label, int64_t n, int K,
+                   const float* __restrict__ w, const ExpTable T, float* __restrict__ g, float* __restrict__ h,
+                   int32_t* __restrict__ bad_label) {
+  extern __shared__ float2 s_e[];
+  __shared__ ExpTable st;
+  if (threadIdx.x < 32) {
+    st.hi[threadIdx.x] = T.hi[threadIdx.x];
+    st.lo[threadIdx.x] = T.lo[threadIdx.x];
+  }
+  __syncthreads();
+  bool ok_f;
+  const Pair factor = pair_of((double)K / ((double)K - 1.0), &ok_f);
+  float2* mine = s_e + threadIdx.x;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    const int lab = class_of(label[i], K, bad_label);
+    // the scores as pairs; their maximum (pairs compare like the scores up to 2^-53, which the bound allows)
+    bool ok = ok_f;
+    Pair top{-CUDART_INF_F, 0.f};
+    for (int k = 0; k < K; ++k) {
+      bool o;
+      const Pair x = pair_of(score[(size_t)k * n + i], &o);
+      ok = ok && o && fabsf(x.hi) <= 64.0f;
+      mine[k * kSoftmaxThreads] = make_float2(x.hi, x.lo);
+      if (x.hi > top.hi || (x.hi == top.hi && x.lo > top.lo)) top = x;
+    }
+    Pair sum{0.f, 0.f}, others{0.f, 0.f};
+    top = pair_neg(top);
+    for (int k = 0; ok && k < K; ++k) {
+      const float2 x = mine[k * kSoftmaxThreads];
+      const Pair z = pair_add(Pair{x.x, x.y}, top);
+      ok = z.hi >= -60.0f;
+      const Pair e = ok ? pair_exp(z, st) : Pair{0.f, 0.f};
+      sum = pair_add(sum, e);
+      if (k != lab) others = pair_add(others, e);
+      mine[k * kSoftmaxThreads] = make_float2(e.hi, e.lo);
+    }
+    const Pair wi{w ? w[i] : 1.0f, 0.f};
+    for (int k = 0; ok && k < K; ++k) {
+      const float2 x = mine[k * kSoftmaxThreads];
+      const Pair e{x.x, x.y};
+      const Pair p = pair_div(e, sum);
+      const Pair rest = k == lab ? others : pair_add(sum, pair_neg(e));
+      const Pair np = pair_div(rest, sum);  // 1 - p
+      const float inv = __fdividef(1.0f, np.hi);
+      Pair gp = k == lab ? np : p, hp = pair_mul(pair_mul(factor, p), np);
+      const float rel_g = kTwo(-38) + (k == lab ? __fmul_rn(kTwo(-51), inv) : 0.f);
+      const float rel_h = kTwo(-37) + __fmul_rn(k == lab ? kTwo(-51) : kTwo(-40), inv);
+      if (w) {
+        gp = pair_mul(gp, wi);
+        hp = pair_mul(hp, wi);
+      }
+      float gv, hv;
+      const bool a = pair_round(gp, rel_g, &gv), b = pair_round(hp, rel_h, &hv);
+      ok = a && b;
+      if (k == lab) gv = -gv;
+      if (ok) {
+        g[(size_t)k * n + i] = gv;
+        h[(size_t)k * n + i] = hv;
+      }
+    }
+    if (!ok) softmax_row(score, n, i, K, lab, w, g, h);
+  }
+}
+
+// 2^(j / 32), from the host's f64 exp2.
+ExpTable exp_table() {
+  ExpTable t;
+  for (int j = 0; j < 32; ++j) {
+    const double v = std::exp2((double)j / 32.0);
+    t.hi[j] = (float)v;
+    t.lo[j] = (float)(v - (double)t.hi[j]);
+  }
+  return t;
 }
 
 // Per-CTA partial losses (mean squared error / log loss / multiclass log loss).
@@ -130,11 +267,14 @@ __global__ void k_loss(int kind, const double* __restrict__ score, const float* 
 
 cudaError_t objective_gradients(int kind, const double* score, const float* label, int64_t n, int K, double sigmoid,
                                 const ObjectiveWeights& ow, float* g, float* h, int32_t* bad_label, cudaStream_t s) {
-  const int grid = 1024, threads = 256;
+  const int grid = 1216, threads = 256;  // eight CTAs per SM
+  static const ExpTable table = exp_table();
   if (kind == 0) k_grad_l2<<<grid, threads, 0, s>>>(score, label, n, ow.row, g, h);
   else if (kind == 1)
-    k_grad_binary<<<grid, threads, 0, s>>>(score, label, n, sigmoid, ow.row, ow.label_neg, ow.label_pos, g, h);
-  else k_grad_softmax<<<grid, threads, 0, s>>>(score, label, n, K, ow.row, g, h, bad_label);
+    k_grad_binary<<<grid, threads, 0, s>>>(score, label, n, sigmoid, ow.row, ow.label_neg, ow.label_pos, table, g, h);
+  else
+    k_grad_softmax<<<grid, kSoftmaxThreads, (size_t)K * kSoftmaxThreads * sizeof(float2), s>>>(
+        score, label, n, K, ow.row, table, g, h, bad_label);
   return cudaGetLastError();
 }
 
