@@ -111,6 +111,8 @@ struct Params {
   int32_t max_exp;             // expansions of one tree at most: num_leaves - 1 + round_out
   int32_t n_groups;            // feature groups of a round's search, one candidate each
   int32_t n_numeric, unit_penalty;  // numerical features (first in `order`); every feature's penalty is 1
+  int32_t cta_full, cta_extra, cta_last;  // histogram CTAs of a round (hist_split_ctas)
+  int32_t hot_shift;           // quantized histograms' 32-bit hot counters hold (grad << hot_shift) + hess
   const int32_t* order;        // [F] inner features: the numerical ones, then the categorical ones
   int32_t cand_rows;           // rows of Job::cand and Job::splittable: 1 + 2 max_exp nodes
 };
@@ -138,7 +140,7 @@ struct JobState {
   int32_t split_inner, new_leaf, use_rows;
   uint32_t split_thr;  // threshold of the chosen split | default_left << 31
   int64_t root_count, total_left;
-  int64_t pcnt[2][2];  // single-pass partition: rows placed from the front / back, per split parity
+  int64_t pcnt[2][2];  // single-pass partition, per split parity: rows placed from the front (low half) and back (high)
   int64_t hist_begin, hist_count;  // the smaller leaf's row range and index buffer, for the histogram
   int32_t hist_buf, split_buf;
   int64_t split_begin, split_count;  // the chosen leaf's row range and index buffer, for the partition
@@ -249,6 +251,7 @@ struct HistLaunch {
   int flush_rounds;  // quantized: rounds of 32*warps rows between 16-bit -> 32-bit flushes (0: wide)
   int direct_rows;   // quantized: a CTA with at most this many rows adds each (row, feature) to the
                      // pool slot with a global atomic instead of through a shared histogram
+  int round_ctas = 1;  // grow rounds: CTAs over all tiles
   int cluster = 1;   // quantized: CTAs of a tile per thread-block cluster, which add up their shared
                      // histograms through distributed shared memory before one flush (1: none)
 };
@@ -261,6 +264,8 @@ cudaError_t check_bins_device(const uint8_t* bins, int64_t n, int32_t F, const D
 void launch_hist(const Job* h_jobs, int num_jobs, const Params& p, const uint8_t* bins_rt, const uint8_t* bins_tm,
                  const HistLaunch& hl, int post, int par, cudaStream_t s);
 size_t hist_smem_bytes(const Params& p, int threads, bool quant, bool wide);
+// Splits `total` histogram CTAs (at least one per tile) over the tiles by what their rows cost.
+void hist_split_ctas(Params& p, int total);
 
 // The bookkeeping of the last split of a tree partitioned in one pass (counter pair `par`).
 void launch_apply_split(const Job* h_jobs, int num_jobs, const Params& p, int par, cudaStream_t s);

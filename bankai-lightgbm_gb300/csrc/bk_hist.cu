@@ -56,6 +56,7 @@ struct Range {
   const int16_t* pk;  // packed values: by row for the root, else in leaf order
   int32_t slot;       // the pool slot the histogram goes to
   bool direct, pk_row;
+  int hot_shift;      // Params::hot_shift
 };
 
 // The smaller leaf's rows for this CTA: 1 with rows, 2 without rows for this CTA (r->slot set),
@@ -72,7 +73,7 @@ __device__ __forceinline__ int cta_range(const Job& J, const Params& p, int bloc
   int64_t begin, count;
   int32_t buf;
   if (post) {
-    const SplitOutcome o = split_outcome(p, st, __ldcg(&st->pcnt[par][0]));
+    const SplitOutcome o = split_outcome(p, st, __ldcg(&st->pcnt[par][0]) & 0xffffffffLL);
     if (stop) return 0;
     hist_apply_split(J, p, o);
     if (!o.go) return 0;
@@ -107,6 +108,7 @@ __device__ __forceinline__ int cta_range(const Job& J, const Params& p, int bloc
   r->idx = leaf_idx(J, buf) + begin;
   r->direct = (count == p.n);  // all rows in order: the index buffer is the identity
   r->pk = r->pk_row ? J.packed : (J.pk0 ? leaf_pk(J, buf) + begin : nullptr);
+  r->hot_shift = p.hot_shift;
   return 1;
 }
 
@@ -118,6 +120,14 @@ struct RoundLoad {
   uint4 a, b;
   int32_t v;
 };
+
+// A tile of 17 to 32 features takes 32 steps, one per feature. One of at most 16 takes `steps` = 16, 8
+// or 4 (the least that covers its features): the 32 columns of the shared histogram then hold
+// 32 / steps copies of its features, feature f in columns f, f + steps, ..., and the lanes with the
+// same high bits share a copy. At step k lane l adds to column k ^ l either way. Features past the
+// tile's last one (padding, bin 0) add to columns of their own, which the flush skips: that is cheaper
+// than a test per step (4M rows: 20 features 86 -> 47 us, 4 features 55 -> 37 us).
+__device__ __forceinline__ int tile_steps(int nf) { return nf > 16 ? 32 : (nf > 8 ? 16 : (nf > 4 ? 8 : 4)); }
 
 // Positions are 32-bit: a leaf has fewer than 2^31 rows, and a lookahead position past the
 // leaf's end stays below 2^32. `swap` (0 or 1) exchanges the two 16-byte halves of a 32-byte run
@@ -140,13 +150,14 @@ __device__ __forceinline__ RoundLoad load_round_int(const uint8_t* tb, uint32_t 
     int32_t pk = R.pk[R.pk_row ? (uint32_t)row : i];
     int32_t gi = (int32_t)(int8_t)(pk >> 8);
     int32_t hi = pk & 0xff;
-    L.v = wide ? ((gi & 0xffff) | (hi << 16)) : gi * 65536 + hi;
+    L.v = wide ? ((gi & 0xffff) | (hi << 16)) : (int32_t)(((uint32_t)gi << R.hot_shift) + (uint32_t)hi);
   }
   return L;
 }
 
-// The gradient half of a 16:16 hot counter (grad * 65536 + hess, hess in [0, 65536)).
-__device__ __forceinline__ int32_t hot_g(uint32_t s) { return ((int32_t)s - (int32_t)(s & 0xffffu)) >> 16; }
+// The two halves of a hot counter, (grad << shift) + hess with hess in [0, 2^shift).
+__device__ __forceinline__ int32_t hot_h(uint32_t s, int shift) { return (int32_t)(s & ((1u << shift) - 1u)); }
+__device__ __forceinline__ int32_t hot_g(uint32_t s, int shift) { return ((int32_t)s - hot_h(s, shift)) >> shift; }
 
 // Lane f's stored bin of staged row j: byte f of the row's 32-byte run, or the nibble f of its
 // 16-byte run (low nibble for even f).
@@ -158,9 +169,9 @@ __device__ __forceinline__ uint32_t staged_bin(const uint8_t* sb, int j, int lan
 
 // The (grad << 32) + hess pool value of a row's packed statistics as the kernel carries them.
 template <bool WIDE>
-__device__ __forceinline__ unsigned long long pool_value(int32_t v) {
-  const int32_t g = WIDE ? (int32_t)(int16_t)(v & 0xffff) : hot_g((uint32_t)v);
-  const int32_t h = WIDE ? (v >> 16) : (v & 0xffff);
+__device__ __forceinline__ unsigned long long pool_value(int32_t v, int shift) {
+  const int32_t g = WIDE ? (int32_t)(int16_t)(v & 0xffff) : hot_g((uint32_t)v, shift);
+  const int32_t h = WIDE ? (v >> 16) : hot_h((uint32_t)v, shift);
   return (unsigned long long)((int64_t)g * 4294967296LL + (int64_t)h);
 }
 
@@ -186,9 +197,10 @@ __device__ __forceinline__ void add_wide(const IntHist<true>& H, uint32_t bin, i
   atomicAdd(&H.cold_h()[bin * TILE + f], v >> 16);
 }
 
-// Adds a row's packed value to the hot counter at byte offset (bin << 8) | 4 f.
-__device__ __forceinline__ void add_hot(unsigned char* base, uint32_t off, int32_t v) {
-  atomicAdd(reinterpret_cast<uint32_t*>(base + off), (uint32_t)v);
+// Adds a row's packed value to the hot counter at shared address `at` (the histogram's start plus
+// (bin << 8) | 4 f).
+__device__ __forceinline__ void add_hot(uint32_t at, int32_t v) {
+  asm volatile("red.shared.add.u32 [%0], %1;" ::"r"(at), "r"(v) : "memory");
 }
 
 // w[i] <- w[i ^ (q & (2 TOP - 1))] (N a power of two, TOP <= N / 2): one select per word and bit.
@@ -205,94 +217,104 @@ __device__ __forceinline__ void xor_permute(uint32_t (&w)[N], uint32_t q) {
   }
 }
 
-// Every lane adds its own row (its run and packed value as loaded) to the shared histogram, one
-// feature per step: at step k lane l takes feature k ^ l, so the 32 lanes of each atomic hit 32
-// different features — 32 different banks, whatever their bins — and no row is staged through
-// shared memory or broadcast. The run's words are first permuted by the lane's high feature bits
-// (a word index that varies by lane cannot be a register index) and, for 8-bit bins, the bytes of
-// each word by its low bits, so step k finds its bin at a fixed position: one byte permute gives
-// bin << 8, and one logic op adds the feature's offset 4 (k ^ l) to make the hot counter's byte
-// offset. A 16-byte run of 8-bit bins (at most 16 features) takes feature (k ^ l) & 15 at step
-// k < 16 (lanes l and l ^ 16 share a column). Features at or past nf, the tile's feature count,
-// get nothing. A lane without a row carries zeros. The full 8-bit run arrives with its halves
-// already exchanged for lanes 16-31 (bit 2 of the word permutation).
+// The bins of a lane's row as counter offsets, for 8-bit bins. At step k lane l takes feature
+// (k ^ l) mod steps and adds to column k ^ l, so the 32 lanes of each atomic hit 32 different columns,
+// 32 different banks, whatever their bins; no row is staged through shared memory or broadcast. The
+// run's words are permuted by the lane's high feature bits (a word index that varies by lane cannot be
+// a register index); within a word, step j takes byte j ^ (l & 3). One byte permute then makes the hot
+// counter's byte offset (bin << 8) | 4 column: byte 1 from the run's word, byte 0 from a word of the
+// four columns' offsets (all below 128, so their sign fills bytes 2 and 3 with zeros); `sel[j]`
+// selects the bytes of step j. The loop is bound by the ALU pipe, so one instruction per step instead
+// of two (and none to permute the bytes) is what counts: 4M rows x 96 features 123 -> 107 us.
+struct ColumnPerm {
+  uint32_t sel[4], col0, base;  // base: the histogram's shared address
+  __device__ __forceinline__ ColumnPerm(uint32_t lane, const unsigned char* smem) {
+    base = (uint32_t)__cvta_generic_to_shared(smem);
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+      const uint32_t b = j ^ (lane & 3u);
+      sel[j] = (b << 4) | (4u + b) | ((12u + b) << 8) | ((12u + b) << 12);
+    }
+    // byte b: 4 times the column of byte b of the first word after the permutation
+    col0 = (lane & ~3u) * 0x04040404u + 0x0c080400u;
+  }
+};
+__device__ __forceinline__ uint32_t prmt(uint32_t a, uint32_t b, uint32_t sel) {
+  uint32_t r;
+  asm("prmt.b32 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(sel));
+  return r;
+}
+
+template <bool WIDE, int W>
+__device__ __forceinline__ void add_words8(const IntHist<WIDE>& H, const uint32_t (&w)[W], int32_t v, const ColumnPerm& cp) {
+#pragma unroll
+  for (int i = 0; i < W; ++i) {
+    const uint32_t col = cp.col0 ^ ((uint32_t)i * 0x10101010u);
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t off = prmt(w[i], col, cp.sel[j]);
+      if constexpr (WIDE) add_wide(H, off >> 8, v, (off & 255u) >> 2);
+      else add_hot(cp.base + off, v);
+    }
+  }
+}
+
+// 4-bit bins: feature f at bits 4 (f & 7) of word f >> 3
+template <bool WIDE, int W>
+__device__ __forceinline__ void add_words4(const IntHist<WIDE>& H, const uint32_t (&w)[W], int32_t v, uint32_t lane,
+                                           int steps, uint32_t base) {
+#pragma unroll
+  for (int k = 0; k < 8 * W; ++k) {
+    if (W == 1 && k >= steps) break;  // four or eight steps
+    const uint32_t f = (uint32_t)k ^ lane;
+    const uint32_t bin = (w[k >> 3] >> ((((uint32_t)k ^ lane) & (steps == 4 ? 3u : 7u)) << 2)) & 15u;
+    if constexpr (WIDE) add_wide(H, bin, v, f);
+    else add_hot(base + ((bin << 8) | (f << 2)), v);
+  }
+}
+
 template <bool WIDE, bool NIBBLE>
-__device__ __forceinline__ void add_own_row(const IntHist<WIDE>& H, const RoundLoad& L, uint32_t lane, bool half,
-                                            uint32_t nf) {
+__device__ __forceinline__ void add_own_row(const IntHist<WIDE>& H, const RoundLoad& L, uint32_t lane, int steps,
+                                            const ColumnPerm& cp) {
   const int32_t v = L.v;
   if (NIBBLE) {
-    // 32 features in four words, feature f at bits 4 (f & 7) of word f >> 3
-    uint32_t w[4] = {L.a.x, L.a.y, L.a.z, L.a.w};
-    xor_permute<4>(w, (lane >> 3) & 3u);
-#pragma unroll
-    for (int k = 0; k < 32; ++k) {
-      const uint32_t f = (uint32_t)k ^ lane;
-      const uint32_t bin = (w[k >> 3] >> ((((uint32_t)k & 7u) ^ (lane & 7u)) << 2)) & 15u;
-      if (f < nf) {
-        if constexpr (WIDE) add_wide(H, bin, v, f);
-        else add_hot(H.base, (bin << 8) | (f << 2), v);
-      }
+    if (steps == 32) {
+      uint32_t w[4] = {L.a.x, L.a.y, L.a.z, L.a.w};
+      xor_permute<4>(w, (lane >> 3) & 3u);
+      add_words4<WIDE, 4>(H, w, v, lane, 32, cp.base);
+    } else if (steps == 16) {
+      uint32_t w[2] = {L.a.x, L.a.y};
+      xor_permute<2>(w, (lane >> 3) & 1u);
+      add_words4<WIDE, 2>(H, w, v, lane, 16, cp.base);
+    } else {
+      uint32_t w[1] = {L.a.x};
+      add_words4<WIDE, 1>(H, w, v, lane, steps, cp.base);
     }
     return;
   }
-  // byte i of each word <- byte i ^ (lane & 3)
-  const uint32_t bsel = 0x3210u ^ ((lane & 3u) * 0x1111u);
-  if (half) {
-    // at most 16 features in four words, feature f in byte f & 3 of word f >> 2
+  if (steps == 32) {
+    // 32 features in eight words, feature f in byte f & 3 of word f >> 2; the full run arrives with its
+    // halves already exchanged for lanes 16-31 (bit 2 of the word permutation)
+    uint32_t w[8] = {L.a.x, L.a.y, L.a.z, L.a.w, L.b.x, L.b.y, L.b.z, L.b.w};
+    xor_permute<8, 2>(w, lane >> 2);
+    add_words8<WIDE, 8>(H, w, v, cp);
+  } else if (steps == 16) {
     uint32_t w[4] = {L.a.x, L.a.y, L.a.z, L.a.w};
     xor_permute<4>(w, (lane >> 2) & 3u);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) w[i] = __byte_perm(w[i], 0u, bsel);
-    const uint32_t l4 = (lane & 15u) << 2;
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const uint32_t f = ((uint32_t)k ^ lane) & 15u;
-      if (f < nf) {
-        if constexpr (WIDE) {
-          add_wide(H, __byte_perm(w[k >> 2], 0u, 0x4440u | (uint32_t)(k & 3)), v, f);
-        } else {
-          const uint32_t b8 = __byte_perm(w[k >> 2], 0u, 0x4404u | ((uint32_t)(k & 3) << 4));
-          add_hot(H.base, b8 | (l4 ^ ((uint32_t)k << 2)), v);
-        }
-      }
-    }
-    return;
-  }
-  // 32 features in eight words, feature f in byte f & 3 of word f >> 2
-  uint32_t w[8] = {L.a.x, L.a.y, L.a.z, L.a.w, L.b.x, L.b.y, L.b.z, L.b.w};
-  xor_permute<8, 2>(w, lane >> 2);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) w[i] = __byte_perm(w[i], 0u, bsel);
-  const uint32_t l4 = lane << 2;
-  if (nf >= 32u) {
-#pragma unroll
-    for (int k = 0; k < 32; ++k) {
-      if constexpr (WIDE) {
-        add_wide(H, __byte_perm(w[k >> 2], 0u, 0x4440u | (uint32_t)(k & 3)), v, (uint32_t)k ^ lane);
-      } else {
-        const uint32_t b8 = __byte_perm(w[k >> 2], 0u, 0x4404u | ((uint32_t)(k & 3) << 4));
-        add_hot(H.base, b8 | (l4 ^ ((uint32_t)k << 2)), v);
-      }
-    }
+    add_words8<WIDE, 4>(H, w, v, cp);
+  } else if (steps == 8) {
+    uint32_t w[2] = {L.a.x, L.a.y};
+    xor_permute<2>(w, (lane >> 2) & 1u);
+    add_words8<WIDE, 2>(H, w, v, cp);
   } else {
-#pragma unroll
-    for (int k = 0; k < 32; ++k) {
-      const uint32_t f = (uint32_t)k ^ lane;
-      if (f < nf) {
-        if constexpr (WIDE) {
-          add_wide(H, __byte_perm(w[k >> 2], 0u, 0x4440u | (uint32_t)(k & 3)), v, f);
-        } else {
-          const uint32_t b8 = __byte_perm(w[k >> 2], 0u, 0x4404u | ((uint32_t)(k & 3) << 4));
-          add_hot(H.base, b8 | (l4 ^ ((uint32_t)k << 2)), v);
-        }
-      }
-    }
+    uint32_t w[1] = {L.a.x};
+    add_words8<WIDE, 1>(H, w, v, cp);
   }
 }
 
 // Folds the hot counters into the cold ones and clears them. Every thread of the CTA calls it
 // between barriers.
-__device__ __forceinline__ void fold_hot(const IntHist<false>& H) {
+__device__ __forceinline__ void fold_hot(const IntHist<false>& H, int shift) {
   uint4* row4 = reinterpret_cast<uint4*>(H.base);   // 16 per bin: 8 hot, then 8 cold gradient
   int4* h4 = reinterpret_cast<int4*>(H.cold_h());  // 8 per bin
   for (int e = threadIdx.x; e < H.Bt * (TILE / 4); e += blockDim.x) {
@@ -302,14 +324,14 @@ __device__ __forceinline__ void fold_hot(const IntHist<false>& H) {
     if (s.x | s.y | s.z | s.w) {
       int4* gp = reinterpret_cast<int4*>(hp + 8);
       int4 g = *gp, h = h4[e];
-      g.x += hot_g(s.x);
-      g.y += hot_g(s.y);
-      g.z += hot_g(s.z);
-      g.w += hot_g(s.w);
-      h.x += (int32_t)(s.x & 0xffffu);
-      h.y += (int32_t)(s.y & 0xffffu);
-      h.z += (int32_t)(s.z & 0xffffu);
-      h.w += (int32_t)(s.w & 0xffffu);
+      g.x += hot_g(s.x, shift);
+      g.y += hot_g(s.y, shift);
+      g.z += hot_g(s.z, shift);
+      g.w += hot_g(s.w, shift);
+      h.x += hot_h(s.x, shift);
+      h.y += hot_h(s.y, shift);
+      h.z += hot_h(s.z, shift);
+      h.w += hot_h(s.w, shift);
       *gp = g;
       h4[e] = h;
       *hp = make_uint4(0, 0, 0, 0);
@@ -317,81 +339,92 @@ __device__ __forceinline__ void fold_hot(const IntHist<false>& H) {
   }
 }
 
-// The row loop of one integer-histogram CTA: with DIRECT every (row, feature) goes to the pool
-// slot by a global atomic, otherwise to the CTA's shared histogram (the hot counters folded into
-// the cold ones every `flush_rounds` rounds, before either half can overflow; the last round's
-// are folded by the flush).
-template <bool WIDE, bool NIBBLE, bool DIRECT>
-__device__ __forceinline__ void hist_int_loop(const Params& p, const Range& R, const TileGeom& geo, const uint8_t* tb,
-                                              size_t rs, int flush_rounds, unsigned long long* slot,
-                                              unsigned char* smem) {
-  const int tile = blockIdx.y;
+// The row loop of an integer-histogram CTA that adds to its shared histogram (the hot counters folded
+// into the cold ones every `flush_rounds` rounds, before either half can overflow; the last round's
+// are folded by the flush). Software pipeline: the next round's runs and the round after's row indices
+// are in flight while this round is added up; two rounds per iteration, so the buffers change roles
+// without moves.
+template <bool WIDE, bool NIBBLE>
+__device__ __forceinline__ void hist_int_loop(const Params& p, const Range& R, const TileGeom& geo, int tile,
+                                              const uint8_t* tb, size_t rs, int flush_rounds, unsigned char* smem) {
   const int Bt = geo.bins;
   const bool half = geo.width == 16;  // one 16-byte run per row
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   const IntHist<WIDE> H{smem, Bt};
-  uint4* my_stage = reinterpret_cast<uint4*>(smem) + warp * 64;
-  int32_t* my_v = reinterpret_cast<int32_t*>(reinterpret_cast<uint4*>(smem) + nwarps * 64) + warp * 32;
-  const uint8_t* sb = reinterpret_cast<const uint8_t*>(my_stage);
-  // lanes / features past the last feature of the last tile (padding) add nothing
-  const uint32_t tile_feats = (uint32_t)min(TILE, p.F - tile * TILE);
-  const bool feat_lane = (uint32_t)lane < tile_feats;
+  const int steps = tile_steps(min(TILE, p.F - tile * TILE));
+  const ColumnPerm cp((uint32_t)lane, smem);
   const uint32_t r0 = (uint32_t)R.r0, r1 = (uint32_t)R.r1;
   const uint32_t per_round = (uint32_t)(TILE * nwarps);
   const uint32_t rounds = (r1 - r0 + per_round - 1u) / per_round;
   const uint32_t rs32 = (uint32_t)rs;
   // the full 8-bit path loads lanes 16-31's runs with their halves exchanged
-  const uint32_t swap = (!DIRECT && !NIBBLE && !half) ? ((uint32_t)lane >> 4) & 1u : 0u;
-  // software pipeline: the next round's runs and the round after's row indices are in flight
-  // while this round is added up; `pos` is this lane's row position in the current round
-  uint32_t pos = r0 + (uint32_t)(warp * TILE + lane);
-  RoundLoad cur = load_round_int(tb, rs32, R, pos, round_row32(R, pos, r1), WIDE, half, swap);
+  const uint32_t swap = (!NIBBLE && !half) ? ((uint32_t)lane >> 4) & 1u : 0u;
+  uint32_t pos = r0 + (uint32_t)(warp * TILE + lane);  // this lane's row position in the current round
+  RoundLoad a = load_round_int(tb, rs32, R, pos, round_row32(R, pos, r1), WIDE, half, swap), b;
   int32_t row_nxt = round_row32(R, pos + per_round, r1);
   int until_flush = flush_rounds;
-  for (uint32_t rd = 0; rd < rounds; ++rd, pos += per_round) {
+  uint32_t left = rounds;
+  auto step = [&](RoundLoad& cur, RoundLoad& nxt) {
     const int32_t row_nn = round_row32(R, pos + 2u * per_round, r1);
-    RoundLoad nxt = load_round_int(tb, rs32, R, pos + per_round, row_nxt, WIDE, half, swap);
+    nxt = load_round_int(tb, rs32, R, pos + per_round, row_nxt, WIDE, half, swap);
     row_nxt = row_nn;
-    const uint32_t base = pos - (uint32_t)lane;  // the warp's first row position of the round
-    if (base < r1) {
-      if (DIRECT) {
-        // global atomics: the round's rows are staged so that each atomic covers one row's 32
-        // features, 32 consecutive pool entries
-        my_stage[lane * 2] = cur.a;
-        if (!half) my_stage[lane * 2 + 1] = cur.b;
-        my_v[lane] = cur.v;
-        __syncwarp();
-        const int jn = (int)min(32u, r1 - base);  // warp-uniform
-        for (int j = 0; j < jn; ++j) {
-          const uint32_t b0 = staged_bin<NIBBLE>(sb, j, lane);
-          const int32_t v0 = my_v[j];
-          if (feat_lane) atomicAdd(slot + b0 * TILE + lane, pool_value<WIDE>(v0));
-        }
-        __syncwarp();
-      } else {
-        add_own_row<WIDE, NIBBLE>(H, cur, (uint32_t)lane, half, tile_feats);
-      }
-    }
-    cur = nxt;
-    if constexpr (!WIDE && !DIRECT) {
-      if (--until_flush == 0 && rd + 1 < rounds) {
+    if (pos - (uint32_t)lane < r1) add_own_row<WIDE, NIBBLE>(H, cur, (uint32_t)lane, steps, cp);
+    pos += per_round;
+    --left;
+    if constexpr (!WIDE) {
+      if (--until_flush == 0 && left != 0u) {
         until_flush = flush_rounds;
         __syncthreads();
-        fold_hot(H);
+        fold_hot(H, p.hot_shift);
         __syncthreads();
       }
     }
+  };
+  while (left > 1u) {
+    step(a, b);
+    step(b, a);
+  }
+  if (left) step(a, b);
+}
+
+// The row loop of a CTA with few rows: every (row, feature) goes to the pool slot by a global atomic.
+// The round's rows are staged so that each atomic covers one row's 32 features, 32 consecutive pool
+// entries.
+template <bool WIDE, bool NIBBLE>
+__device__ __forceinline__ void hist_int_direct(const Params& p, const Range& R, const TileGeom& geo, int tile,
+                                                const uint8_t* tb, size_t rs, unsigned long long* slot, unsigned char* smem) {
+  const bool half = geo.width == 16;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
+  uint4* my_stage = reinterpret_cast<uint4*>(smem) + warp * 64;
+  int32_t* my_v = reinterpret_cast<int32_t*>(reinterpret_cast<uint4*>(smem) + nwarps * 64) + warp * 32;
+  const uint8_t* sb = reinterpret_cast<const uint8_t*>(my_stage);
+  // lanes past the last feature of the last tile (padding) add nothing
+  const bool feat_lane = lane < p.F - tile * TILE;
+  const uint32_t r1 = (uint32_t)R.r1, per_round = (uint32_t)(TILE * nwarps);
+  for (uint32_t base = (uint32_t)R.r0 + (uint32_t)(warp * TILE); base < r1; base += per_round) {
+    const uint32_t pos = base + (uint32_t)lane;
+    const RoundLoad cur = load_round_int(tb, (uint32_t)rs, R, pos, round_row32(R, pos, r1), WIDE, half, 0u);
+    my_stage[lane * 2] = cur.a;
+    if (!half) my_stage[lane * 2 + 1] = cur.b;
+    my_v[lane] = cur.v;
+    __syncwarp();
+    const int jn = (int)min(32u, r1 - base);  // warp-uniform
+    for (int j = 0; j < jn; ++j) {
+      const uint32_t b0 = staged_bin<NIBBLE>(sb, j, lane);
+      const int32_t v0 = my_v[j];
+      if (feat_lane) atomicAdd(slot + b0 * TILE + lane, pool_value<WIDE>(v0, p.hot_shift));
+    }
+    __syncwarp();
   }
 }
 
 // The rows and flush of one integer-histogram CTA, its range known (NIBBLE: the tile holds
 // 4-bit bins).
 template <bool WIDE, bool NIBBLE>
-__device__ __forceinline__ void hist_int_rows(const Job& J, const Params& p, const Range& R, const TileGeom& geo,
+__device__ __forceinline__ void hist_int_rows(const Job& J, const Params& p, const Range& R, const TileGeom& geo, int tile,
                                               const uint8_t* __restrict__ bins_rt, const uint8_t* __restrict__ bins_tm,
                                               int flush_rounds, int direct_rows, bool in_cluster, unsigned char* smem,
                                               bool more = false) {
-  const int tile = blockIdx.y;
   const int Bt = geo.bins;
   const IntHist<WIDE> H{smem, Bt};
   unsigned long long* slot = reinterpret_cast<unsigned long long*>(J.pool) +
@@ -404,26 +437,33 @@ __device__ __forceinline__ void hist_int_rows(const Job& J, const Params& p, con
   const uint8_t* tb = dense ? bins_tm + geo.tm_off : bins_rt + geo.rt_off;
   const size_t rs = dense ? (size_t)tile_width(geo) : (size_t)p.rt_stride;
   if (direct) {
-    hist_int_loop<WIDE, NIBBLE, true>(p, R, geo, tb, rs, flush_rounds, slot, smem);
+    hist_int_direct<WIDE, NIBBLE>(p, R, geo, tile, tb, rs, slot, smem);
     return;
   }
-  hist_int_loop<WIDE, NIBBLE, false>(p, R, geo, tb, rs, flush_rounds, slot, smem);
+  hist_int_loop<WIDE, NIBBLE>(p, R, geo, tile, tb, rs, flush_rounds, smem);
   if (in_cluster) return;  // a cluster flushes its CTAs' histograms together
   __syncthreads();
+  const int nf = min(TILE, p.F - tile * TILE), steps = tile_steps(nf);
   for (int e = threadIdx.x; e < Bt * TILE; e += blockDim.x) {
-    const int gi = (e >> 5) * IntHist<WIDE>::GS + (e & (TILE - 1));  // (bin, feature) in the row layout
+    const int bin = e >> 5, col = e & (TILE - 1);
+    const int gi = bin * IntHist<WIDE>::GS + col;  // (bin, column) in the row layout
     int32_t gg = H.cold_g()[gi], hh = H.cold_h()[e];
     if (!WIDE) {
       const uint32_t s = H.hot()[gi];
-      gg += hot_g(s);
-      hh += (int32_t)(s & 0xffffu);
+      gg += hot_g(s, p.hot_shift);
+      hh += hot_h(s, p.hot_shift);
     }
     if (more) {  // the CTA's next rows belong to another leaf
       H.cold_g()[gi] = 0;
       H.cold_h()[e] = 0;
       if (!WIDE) H.hot()[gi] = 0u;
     }
-    if (gg | hh) {
+    // the feature's copies sit in the warp's lanes
+    for (int o = steps; o < TILE; o <<= 1) {
+      gg += __shfl_xor_sync(0xffffffffu, gg, o);
+      hh += __shfl_xor_sync(0xffffffffu, hh, o);
+    }
+    if ((gg | hh) && col < nf) {
       int64_t pk = (int64_t)gg * 4294967296LL + (int64_t)hh;
       atomicAdd(slot + e, (unsigned long long)pk);
     }
@@ -442,9 +482,10 @@ __device__ __forceinline__ void hist_cluster_flush(const Params& p, const TileGe
                                                    uint32_t ncta, unsigned char* smem) {
   const int Bt = geo.bins;
   const IntHist<WIDE> H{smem, Bt};
+  const int nf = min(TILE, p.F - (int)blockIdx.y * TILE), steps = tile_steps(nf);
   const int n4 = Bt * TILE / 4;  // int4 groups of the tile's bins: a multiple of 64 (Bt a multiple of 8)
   __syncthreads();
-  if constexpr (!WIDE) fold_hot(H);
+  if constexpr (!WIDE) fold_hot(H, p.hot_shift);
   cluster_sync_all();
   const uint32_t rank = cluster_ctarank();
   const int per = n4 / (int)ncta;
@@ -465,9 +506,11 @@ __device__ __forceinline__ void hist_cluster_flush(const Params& p, const TileGe
     }
     const int32_t gg[4] = {g.x, g.y, g.z, g.w}, hh[4] = {h.x, h.y, h.z, h.w};
 #pragma unroll
-    for (int k = 0; k < 4; ++k)
-      if (gg[k] | hh[k])
-        atomicAdd(slot + 4 * e + k, (unsigned long long)((int64_t)gg[k] * 4294967296LL + (int64_t)hh[k]));
+    for (int k = 0; k < 4; ++k) {
+      const int f = (4 * (e & 7) + k) & (steps - 1);  // a column holds a copy of feature column mod steps
+      if ((gg[k] | hh[k]) && f < nf)
+        atomicAdd(slot + (e >> 3) * TILE + f, (unsigned long long)((int64_t)gg[k] * 4294967296LL + (int64_t)hh[k]));
+    }
   }
   cluster_sync_all();
 }
@@ -497,9 +540,9 @@ __global__ void __launch_bounds__(1024, 1)
   if (rc == 0 || (rc == 2 && ncta == 1)) return;
   if (rc == 1) {
     if (geo.nibble)
-      hist_int_rows<WIDE, true>(J, p, R, geo, bins_rt, bins_tm, flush_rounds, direct_rows, ncta > 1, smem);
+      hist_int_rows<WIDE, true>(J, p, R, geo, blockIdx.y, bins_rt, bins_tm, flush_rounds, direct_rows, ncta > 1, smem);
     else
-      hist_int_rows<WIDE, false>(J, p, R, geo, bins_rt, bins_tm, flush_rounds, direct_rows, ncta > 1, smem);
+      hist_int_rows<WIDE, false>(J, p, R, geo, blockIdx.y, bins_rt, bins_tm, flush_rounds, direct_rows, ncta > 1, smem);
   }
   if (ncta > 1) {
     unsigned long long* slot = reinterpret_cast<unsigned long long*>(J.pool) +
@@ -509,7 +552,7 @@ __global__ void __launch_bounds__(1024, 1)
 }
 
 // ---- grow rounds (bk_rounds.cuh): the smaller children of up to kMaxRoundW expansions ----
-// The children's rows, one after the other, are cut into gridDim.x equal intervals (at least
+// The children's rows, one after the other, are cut into an interval for each CTA of a tile (at least
 // hist_min_rows rows each), so every CTA of a tile takes the same number of rows whatever the
 // leaves' sizes; a CTA whose interval crosses from one leaf into the next flushes and clears its
 // shared histogram there. round_cut() starts every leaf at an interval of its own where that costs
@@ -521,11 +564,21 @@ struct RoundRows {
   RoundCut cut;
 };
 
+// A CTA's tile, its place among the tile's CTAs and their number (hist_split_ctas): the first
+// cta_extra full tiles have cta_full + 1 CTAs, the others cta_full; a narrow last tile has cta_last.
+__device__ __forceinline__ int3 round_cta(const Params& p) {
+  const int b = (int)blockIdx.x, c1 = p.cta_full + 1, full = p.T - (p.cta_last ? 1 : 0);
+  const int n1 = p.cta_extra * c1, n2 = n1 + (full - p.cta_extra) * p.cta_full;
+  if (b < n1) return make_int3(b / c1, b % c1, c1);
+  if (b < n2) return make_int3(p.cta_extra + (b - n1) / p.cta_full, (b - n1) % p.cta_full, p.cta_full);
+  return make_int3(full, b - n2, p.cta_last);
+}
+
 // Every thread calls it, between the launch's wait and its rows; ends with a barrier. The search
 // constants of expansion e are computed by the last two warps of one CTA per expansion, spread over
 // the grid from its end (whose CTAs are the ones without rows when there are few), before the rows
 // of those warps.
-__device__ __forceinline__ void round_rows(const Job& J, const Params& p, int q, RoundRows* s) {
+__device__ __forceinline__ void round_rows(const Job& J, const Params& p, int q, int ctas, RoundRows* s) {
   const RoundView v = round_view(J, p);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
   if (warp == 0) {
@@ -545,18 +598,17 @@ __device__ __forceinline__ void round_rows(const Job& J, const Params& p, int q,
       }
     }
     int64_t off;
-    const RoundCut cut = round_cut(rows, n_cur, (int)gridDim.x, p.hist_min_rows, 32, 2048, lane, &off);
+    const RoundCut cut = round_cut(rows, n_cur, ctas, p.hist_min_rows, 32, 2048, lane, &off);
     if (lane < n_cur) s->off[lane] = off;
     if (lane == 0) {
       s->n = n_cur;
       s->cut = cut;
     }
   } else if (warp >= nwarps - 2) {
-    const int cta = (int)(gridDim.x - 1 - blockIdx.x) * (int)gridDim.y + (int)blockIdx.y;  // from the grid's end
-    const int ctas = (int)(gridDim.x * gridDim.y);
-    if (cta < kMaxRoundW) {
+    const int from_end = (int)(gridDim.x - 1 - blockIdx.x);
+    if (from_end < kMaxRoundW) {
       const int n_cur = __ldcg(&v.hdr[q].n_cur);
-      for (int e = cta; e < n_cur; e += ctas) {
+      for (int e = from_end; e < n_cur; e += (int)gridDim.x) {
         const RoundExp c = v.cur[q * kMaxRoundW + e];
         const int32_t L = (int32_t)__ldcg(v.pcnt + ((size_t)q * kMaxRoundW + e) * 2);
         round_leaf_constants(J, p, c, L, e, warp - (nwarps - 2), lane);
@@ -567,9 +619,9 @@ __device__ __forceinline__ void round_rows(const Job& J, const Params& p, int q,
 
 // The part of this CTA's interval that lies in expansion e: false when it has no row of it. `last`:
 // no later leaf has rows in the interval.
-__device__ __forceinline__ bool round_segment(const Job& J, const Params& p, const RoundRows& s, int e, Range* r,
-                                              bool* single, bool* last) {
-  const int64_t q0 = (int64_t)blockIdx.x * s.cut.per, q1 = q0 + s.cut.per;
+__device__ __forceinline__ bool round_segment(const Job& J, const Params& p, const RoundRows& s, int cta, int e,
+                                              Range* r, bool* single, bool* last) {
+  const int64_t q0 = (int64_t)cta * s.cut.per, q1 = q0 + s.cut.per;
   const int64_t off = s.off[e];
   const int64_t a = max(q0, off), b = min(q1, off + s.count[e]);
   if (a >= b) return false;
@@ -581,6 +633,7 @@ __device__ __forceinline__ bool round_segment(const Job& J, const Params& p, con
   r->pk_row = s.root != 0;      // the root: no leaf-ordered copy yet
   r->pk = r->pk_row ? J.packed : (J.pk0 ? leaf_pk(J, s.buf[e]) + s.begin[e] : nullptr);
   r->slot = s.slot[e];
+  r->hot_shift = p.hot_shift;
   *last = s.cut.apart || b == q1 || e == s.n - 1;
   *single = *last && a == q0;
   return true;
@@ -592,7 +645,8 @@ __global__ void __launch_bounds__(1024, 1)
                      const uint8_t* __restrict__ bins_tm, int flush_rounds, int direct_rows, int q) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ RoundRows rows;
-  const TileGeom geo = p.tiles[blockIdx.y];  // static: loaded while the previous kernel finishes
+  const int3 m = round_cta(p);
+  const TileGeom geo = p.tiles[m.x];  // static: loaded while the previous kernel finishes
   {
     uint4* z = reinterpret_cast<uint4*>(smem);
     const int n16 = (WIDE ? 2 : 3) * geo.bins * TILE / 4;
@@ -601,19 +655,19 @@ __global__ void __launch_bounds__(1024, 1)
   griddep_wait();
   griddep_launch();
   const Job& J = jobs.job[blockIdx.z];
-  round_rows(J, p, q, &rows);
+  round_rows(J, p, q, m.z, &rows);
   __syncthreads();
   for (int e = 0; e < rows.n; ++e) {
     Range R;
     bool single, last;
-    if (!round_segment(J, p, rows, e, &R, &single, &last)) continue;
+    if (!round_segment(J, p, rows, m.y, e, &R, &single, &last)) continue;
     // a CTA that adds straight to the pool slot stages its rows over the shared histogram, so it
     // takes rows of one leaf only
     const int direct = single ? direct_rows : -1;
     if (geo.nibble)
-      hist_int_rows<WIDE, true>(J, p, R, geo, bins_rt, bins_tm, flush_rounds, direct, false, smem, !last);
+      hist_int_rows<WIDE, true>(J, p, R, geo, m.x, bins_rt, bins_tm, flush_rounds, direct, false, smem, !last);
     else
-      hist_int_rows<WIDE, false>(J, p, R, geo, bins_rt, bins_tm, flush_rounds, direct, false, smem, !last);
+      hist_int_rows<WIDE, false>(J, p, R, geo, m.x, bins_rt, bins_tm, flush_rounds, direct, false, smem, !last);
     if (last) break;
   }
 }
@@ -639,54 +693,65 @@ __device__ __forceinline__ void add_float(float* ghi, float* glo, float* hhi, fl
 // step k (32 different banks per atomic), from its run permuted once per row so that each step's
 // bin sits at a fixed position. The full 8-bit run arrives with its halves already exchanged for
 // lanes 16-31.
+template <bool CONST_HESS, int W>
+__device__ __forceinline__ void add_words8_float(float* ghi, float* glo, float* hhi, float* hlo, const uint32_t (&w)[W],
+                                                 float2 v, uint32_t lane) {
+#pragma unroll
+  for (int k = 0; k < 4 * W; ++k)
+    add_float<CONST_HESS>(ghi, glo, hhi, hlo,
+                          __byte_perm(w[k >> 2], 0u, 0x4440u | (uint32_t)(k & 3)) * TILE + ((uint32_t)k ^ lane), v);
+}
+
 template <bool CONST_HESS, bool NIBBLE>
 __device__ __forceinline__ void add_own_row_float(float* ghi, float* glo, float* hhi, float* hlo, const uint4& a,
-                                                  const uint4& b, float2 v, uint32_t lane, bool half, uint32_t nf) {
+                                                  const uint4& b, float2 v, uint32_t lane, int steps) {
   if (NIBBLE) {
+    // feature f at bits 4 (f & 7) of word f >> 3
     uint32_t w[4] = {a.x, a.y, a.z, a.w};
-    xor_permute<4>(w, (lane >> 3) & 3u);
+    if (steps == 32) xor_permute<4>(w, (lane >> 3) & 3u);
+    else if (steps == 16 && (lane & 8u)) w[0] = a.y, w[1] = a.x;
+    const uint32_t m = steps == 4 ? 3u : 7u;
 #pragma unroll
     for (int k = 0; k < 32; ++k) {
+      if (k >= steps) break;
       const uint32_t f = (uint32_t)k ^ lane;
-      const uint32_t bin = (w[k >> 3] >> ((((uint32_t)k & 7u) ^ (lane & 7u)) << 2)) & 15u;
-      if (f < nf) add_float<CONST_HESS>(ghi, glo, hhi, hlo, bin * TILE + f, v);
+      const uint32_t bin = (w[k >> 3] >> ((f & m) << 2)) & 15u;
+      add_float<CONST_HESS>(ghi, glo, hhi, hlo, bin * TILE + f, v);
     }
     return;
   }
   const uint32_t bsel = 0x3210u ^ ((lane & 3u) * 0x1111u);  // byte i of each word <- byte i ^ (lane & 3)
-  if (half) {
+  if (steps == 32) {
+    uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+    xor_permute<8, 2>(w, lane >> 2);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) w[i] = __byte_perm(w[i], 0u, bsel);
+    add_words8_float<CONST_HESS, 8>(ghi, glo, hhi, hlo, w, v, lane);
+  } else if (steps == 16) {
     uint32_t w[4] = {a.x, a.y, a.z, a.w};
     xor_permute<4>(w, (lane >> 2) & 3u);
 #pragma unroll
     for (int i = 0; i < 4; ++i) w[i] = __byte_perm(w[i], 0u, bsel);
-#pragma unroll
-    for (int k = 0; k < 16; ++k) {
-      const uint32_t f = ((uint32_t)k ^ lane) & 15u;
-      const uint32_t bin = __byte_perm(w[k >> 2], 0u, 0x4440u | (uint32_t)(k & 3));
-      if (f < nf) add_float<CONST_HESS>(ghi, glo, hhi, hlo, bin * TILE + f, v);
-    }
-    return;
-  }
-  uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-  xor_permute<8, 2>(w, lane >> 2);
-#pragma unroll
-  for (int i = 0; i < 8; ++i) w[i] = __byte_perm(w[i], 0u, bsel);
-#pragma unroll
-  for (int k = 0; k < 32; ++k) {
-    const uint32_t f = (uint32_t)k ^ lane;
-    const uint32_t bin = __byte_perm(w[k >> 2], 0u, 0x4440u | (uint32_t)(k & 3));
-    if (f < nf) add_float<CONST_HESS>(ghi, glo, hhi, hlo, bin * TILE + f, v);
+    add_words8_float<CONST_HESS, 4>(ghi, glo, hhi, hlo, w, v, lane);
+  } else if (steps == 8) {
+    uint32_t w[2] = {a.x, a.y};
+    xor_permute<2>(w, (lane >> 2) & 1u);
+    w[0] = __byte_perm(w[0], 0u, bsel);
+    w[1] = __byte_perm(w[1], 0u, bsel);
+    add_words8_float<CONST_HESS, 2>(ghi, glo, hhi, hlo, w, v, lane);
+  } else {
+    uint32_t w[1] = {__byte_perm(a.x, 0u, bsel)};
+    add_words8_float<CONST_HESS, 1>(ghi, glo, hhi, hlo, w, v, lane);
   }
 }
 
 // The rows and flush of one float-histogram CTA, its range known (NIBBLE: the tile holds 4-bit
 // bins).
 template <bool CONST_HESS, bool NIBBLE>
-__device__ __forceinline__ void hist_float_rows(const Job& J, const Params& p, const Range& R, const TileGeom& geo,
+__device__ __forceinline__ void hist_float_rows(const Job& J, const Params& p, const Range& R, const TileGeom& geo, int tile,
                                                 const uint8_t* __restrict__ bins_rt,
                                                 const uint8_t* __restrict__ bins_tm, unsigned char* smem,
                                                 bool more = false) {
-  const int tile = blockIdx.y;
   const int B = geo.bins;
   const bool half = geo.width == 16;  // one 16-byte run per row
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarps = blockDim.x >> 5;
@@ -700,7 +765,7 @@ __device__ __forceinline__ void hist_float_rows(const Job& J, const Params& p, c
   const bool dense = R.count * 4 >= p.n;
   const uint8_t* tb = dense ? bins_tm + geo.tm_off : bins_rt + geo.rt_off;
   const uint32_t rs = dense ? (uint32_t)tile_width(geo) : (uint32_t)p.rt_stride;
-  const uint32_t tile_feats = (uint32_t)min(TILE, p.F - tile * TILE);
+  const int nf = min(TILE, p.F - tile * TILE), steps = tile_steps(nf);
   const float* G = J.g;
   const float* H = J.h;
   const uint32_t r0 = (uint32_t)R.r0, r1 = (uint32_t)R.r1;
@@ -731,7 +796,7 @@ __device__ __forceinline__ void hist_float_rows(const Job& J, const Params& p, c
     float2 nv;
     load(row_nxt, na, nb, nv);
     row_nxt = row_nn;
-    if (pos < r1) add_own_row_float<CONST_HESS, NIBBLE>(ghi, glo, hhi, hlo, ca, cb, cv, (uint32_t)lane, half, tile_feats);
+    if (pos < r1) add_own_row_float<CONST_HESS, NIBBLE>(ghi, glo, hhi, hlo, ca, cb, cv, (uint32_t)lane, steps);
     ca = na;
     cb = nb;
     cv = nv;
@@ -743,7 +808,12 @@ __device__ __forceinline__ void hist_float_rows(const Job& J, const Params& p, c
     double gs = (double)ghi[e] + (double)glo[e];
     double hs = CONST_HESS ? (double)hcnt[e] * h0 : (double)hhi[e] + (double)hlo[e];
     bool touched = CONST_HESS ? hcnt[e] != 0u : (ghi[e] != 0.f || glo[e] != 0.f || hhi[e] != 0.f || hlo[e] != 0.f);
-    if (touched) {
+    for (int o = steps; o < TILE; o <<= 1) {  // the feature's copies sit in the warp's lanes
+      gs += __shfl_xor_sync(0xffffffffu, gs, o);
+      hs += __shfl_xor_sync(0xffffffffu, hs, o);
+      touched = __shfl_xor_sync(0xffffffffu, (int)touched, o) || touched;
+    }
+    if (touched && (e & (TILE - 1)) < nf) {
       atomicAdd(&slot[e].x, gs);
       atomicAdd(&slot[e].y, hs);
     }
@@ -760,7 +830,8 @@ __global__ void __launch_bounds__(1024, 1)
                        const uint8_t* __restrict__ bins_tm, int q) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ RoundRows rows;
-  const TileGeom geo = p.tiles[blockIdx.y];  // static: loaded while the previous kernel finishes
+  const int3 m = round_cta(p);
+  const TileGeom geo = p.tiles[m.x];  // static: loaded while the previous kernel finishes
   {
     uint4* z = reinterpret_cast<uint4*>(smem);
     const int n16 = (CONST_HESS ? 3 : 4) * geo.bins * TILE / 4;
@@ -769,16 +840,16 @@ __global__ void __launch_bounds__(1024, 1)
   griddep_wait();
   griddep_launch();
   const Job& J = jobs.job[blockIdx.z];
-  round_rows(J, p, q, &rows);
+  round_rows(J, p, q, m.z, &rows);
   __syncthreads();
   for (int e = 0; e < rows.n; ++e) {
     Range R;
     bool single, last;
-    if (!round_segment(J, p, rows, e, &R, &single, &last)) continue;
+    if (!round_segment(J, p, rows, m.y, e, &R, &single, &last)) continue;
     if (geo.nibble)
-      hist_float_rows<CONST_HESS, true>(J, p, R, geo, bins_rt, bins_tm, smem, !last);
+      hist_float_rows<CONST_HESS, true>(J, p, R, geo, m.x, bins_rt, bins_tm, smem, !last);
     else
-      hist_float_rows<CONST_HESS, false>(J, p, R, geo, bins_rt, bins_tm, smem, !last);
+      hist_float_rows<CONST_HESS, false>(J, p, R, geo, m.x, bins_rt, bins_tm, smem, !last);
     if (last) break;
   }
 }
@@ -802,9 +873,9 @@ __global__ void __launch_bounds__(1024, 1)
   Range R;
   if (cta_range(J, p, blocks_per_tile, post, par, &R) != 1) return;
   if (geo.nibble)
-    hist_float_rows<CONST_HESS, true>(J, p, R, geo, bins_rt, bins_tm, smem);
+    hist_float_rows<CONST_HESS, true>(J, p, R, geo, blockIdx.y, bins_rt, bins_tm, smem);
   else
-    hist_float_rows<CONST_HESS, false>(J, p, R, geo, bins_rt, bins_tm, smem);
+    hist_float_rows<CONST_HESS, false>(J, p, R, geo, blockIdx.y, bins_rt, bins_tm, smem);
 }
 
 }  // namespace
@@ -815,8 +886,7 @@ size_t hist_smem_bytes(const Params& p, int threads, bool quant, bool wide) {
   size_t bins = (size_t)p.B * TILE;
   // the integer kernel's direct CTAs stage their rows over the (unused) shared histogram
   if (quant) return std::max((wide ? 0 : bins * 4) + bins * 8, stage + warps * 32 * 4);
-  if (p.const_hess) return bins * 12;
-  return bins * 16;
+  return bins * (p.const_hess ? 12 : 16);
 }
 
 void launch_hist(const Job* h_jobs, int num_jobs, const Params& p, const uint8_t* bins_rt, const uint8_t* bins_tm,
@@ -843,7 +913,7 @@ void launch_hist(const Job* h_jobs, int num_jobs, const Params& p, const uint8_t
 void launch_hist_round(const Job* h_jobs, int num_jobs, const Params& p, const uint8_t* bins_rt,
                        const uint8_t* bins_tm, const HistLaunch& hl, int q, cudaStream_t s) {
   for_job_groups(h_jobs, num_jobs, [&](const JobTable& t, int nz) {
-    const dim3 grid(hl.blocks_per_tile, p.T, nz), block(hl.threads);
+    const dim3 grid(hl.round_ctas, 1, nz), block(hl.threads);
     if (p.quant) {
       if (hl.flush_rounds > 0)
         (void)launch_kernel(k_hist_int_round<false>, grid, block, hl.smem, s, p.pdl, t, p, bins_rt, bins_tm,
@@ -857,6 +927,17 @@ void launch_hist_round(const Job* h_jobs, int num_jobs, const Params& p, const u
       (void)launch_kernel(k_hist_float_round<false>, grid, block, hl.smem, s, p.pdl, t, p, bins_rt, bins_tm, q);
     }
   });
+}
+
+void hist_split_ctas(Params& p, int total) {
+  // a row costs a narrow tile's CTA about three quarters of what it costs a full one's (4M rows: 29
+  // against 39 us above the launch's fixed part)
+  const bool narrow = p.F % TILE != 0 && p.F % TILE <= 16;
+  const int full = p.T - (narrow ? 1 : 0);
+  total = std::max(total, p.T);
+  p.cta_last = !narrow ? 0 : (full == 0 ? total : std::max(1, std::min(total - full, (int)(total * 0.75 / (full + 0.75)))));
+  p.cta_full = full ? (total - p.cta_last) / full : 0;
+  p.cta_extra = full ? (total - p.cta_last) % full : 0;
 }
 
 cudaError_t hist_set_smem_attrs(size_t smem) {

@@ -213,6 +213,15 @@ struct bk_learner {
     if (stream) cudaStreamDestroy(stream);
   }
 
+  // The launch shape to start from: one wave of histogram CTAs (one per SM) and two partition CTAs per
+  // SM, shared by the jobs of a launch. A CTA's fixed work (its prologue, its flush, the decision)
+  // outweighs the rows it gets once the jobs' CTAs queue up: ten class trees of 2M x 64 rows took 4.79
+  // ms an iteration with a full wave for each job, 4.07 with one for all.
+  std::array<int, 5> default_shape() const {
+    const int share = std::min(K, kJobsPerLaunch);
+    return {256, std::max(1, num_sms / (p.T * share)), std::max(1, 2 * num_sms / share), 0, 1};
+  }
+
   // The launch shape of the grow-loop kernels, clamped to what the dataset's rows can fill: a
   // leaf never has more rows than the dataset, so CTAs past n / min_rows would never get rows.
   // Results do not depend on it (integer histograms are exact; the float path changes only its
@@ -230,6 +239,12 @@ struct bk_learner {
       hl.blocks_per_tile = std::max(hl.cluster, hl.blocks_per_tile / hl.cluster * hl.cluster);
     }
     p.part_grid = (int)std::max<int64_t>(1, std::min<int64_t>(std::min(part_grid, kMaxPartGrid), (n + 255) / 256));
+    // grow rounds split the same number of histogram CTAs unevenly; a full wave takes every SM
+    const int sms = num_sms / std::min(K, kJobsPerLaunch), per_wave = std::max(1, sms / p.T);
+    const int total = hl.blocks_per_tile % per_wave == 0 && p.T < sms ? hl.blocks_per_tile / per_wave * sms
+                                                                      : hl.blocks_per_tile * p.T;
+    hist_split_ctas(p, total);
+    hl.round_ctas = std::max(total, p.T);
     drop_graph();
   }
 
@@ -554,12 +569,23 @@ int learner_create(const bk_feature* features, int32_t num_features, const uint8
     // tiles, each taking at least 256 rows; two partition CTAs per SM; no more CTAs than the
     // dataset's rows can fill; no direct-atomic CTAs (bk_learner_autotune may change all four)
     L->hl.threads = 1024;
-    L->set_launch_shape(256, L->num_sms / p.T, 2 * L->num_sms, 0, 1);
+    {
+      const std::array<int, 5> d = L->default_shape();
+      L->set_launch_shape(d[0], d[1], d[2], d[3], d[4]);
+    }
     bool wide = false;
     if (quant) {
       int max_h = p.const_hess ? 1 : p.quant_bins;
       int max_g = p.quant_bins / 2 + 1;
-      int flush_rows = std::min(65535 / max_h, 32767 / max_g);
+      // the hot counters' split that lets the most rows in before either half can overflow
+      int flush_rows = 0;
+      for (int s = 8; s <= 23; ++s) {
+        const int rows = std::min(((1 << s) - 1) / max_h, ((1 << (31 - s)) - 1) / max_g);
+        if (rows > flush_rows) {
+          flush_rows = rows;
+          p.hot_shift = s;
+        }
+      }
       int per_round = 32 * (L->hl.threads / 32);
       L->hl.flush_rounds = flush_rows / per_round;
       wide = L->hl.flush_rounds == 0;
@@ -929,7 +955,6 @@ int bk_learner_autotune(bk_learner* L, const float* gradients, const float* hess
       return 0;
     }
   }
-  const int sms = L->num_sms, T = L->p.T;
   const int saved_mode = L->loop_mode;
   JobState* saved = nullptr;
   const size_t state_bytes = sizeof(JobState) * (size_t)L->K;
@@ -967,7 +992,7 @@ int bk_learner_autotune(bk_learner* L, const float* gradients, const float* hess
     };
     // coordinate descent from the default shape: rows per histogram CTA, histogram CTAs per
     // feature tile, partition CTAs
-    std::array<int, 5> best = {256, sms / T, 2 * sms, 0, 1};
+    std::array<int, 5> best = L->default_shape();
     double best_ms = measure(best).second;
     auto consider = [&](std::array<int, 5> c) {
       auto r = measure(c);
@@ -979,8 +1004,9 @@ int bk_learner_autotune(bk_learner* L, const float* gradients, const float* hess
     // rows per histogram CTA: small values spread small leaves over more SMs; large ones give
     // mid-size leaves fewer CTAs, so fewer shared histograms to flush into the pool slot
     for (int mr : {64, 128, 512, 1024, 2048, 4096, 8192, 16384}) consider({mr, best[1], best[2], best[3], best[4]});
-    for (int ct : {2 * sms / T, sms / (2 * T)}) consider({best[0], ct, best[2], best[3], best[4]});
-    for (int pg : {sms, 4 * sms}) consider({best[0], best[1], pg, best[3], best[4]});
+    const std::array<int, 5> first = L->default_shape();
+    for (int ct : {2 * first[1], std::max(1, first[1] / 2)}) consider({best[0], ct, best[2], best[3], best[4]});
+    for (int pg : {std::max(1, first[2] / 2), 2 * first[2]}) consider({best[0], best[1], pg, best[3], best[4]});
     if (L->p.quant) {
       // the global-atomic variant of the quantized histogram for CTAs with few rows
       for (int dr : {128, 256, 512, 1024, 2048}) consider({best[0], best[1], best[2], dr, best[4]});

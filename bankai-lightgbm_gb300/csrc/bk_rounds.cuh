@@ -87,7 +87,7 @@ struct RoundView {
   RoundHdr* hdr;     // [2]
   RoundExp* cur;     // [2][kMaxRoundW]
   OutEnt* out;       // [2][kMaxRoundOut]
-  long long* pcnt;   // [2][kMaxRoundW][2] rows the partition placed from the front / back
+  long long* pcnt;   // [2][kMaxRoundW][2] rows the partition placed from the front (low half) and the back (high)
   LeafEnt* leaf;     // [2][num_leaves]
   Commit* commit;    // [num_leaves]
   int2* xinfo;       // [max_exp] node and inner feature of every expansion

@@ -1628,7 +1628,7 @@ __global__ void __launch_bounds__(32) k_apply_split(const JobTable jobs, Params 
   const Job& J = jobs.job[blockIdx.z];
   JobState* st = J.st;
   if (st->stop) return;
-  const SplitOutcome o = split_outcome(p, st, __ldcg(&st->pcnt[par][0]));
+  const SplitOutcome o = split_outcome(p, st, __ldcg(&st->pcnt[par][0]) & 0xffffffffLL);
   post_split_writes(J, p, o, (int)threadIdx.x);
 }
 
@@ -1672,7 +1672,7 @@ __global__ void __launch_bounds__(256) k_rounds_finish(const JobTable jobs, Para
   const LeafEnt* ent = v.leaf + (size_t)st->fin_q * p.num_leaves;
   const int i = (int)(blockIdx.x * blockDim.x + threadIdx.x);
   // the tree's last split, when it was taken before its rows were partitioned
-  const int32_t last_L = h.last_x >= 0 ? (int32_t)v.pcnt[(size_t)h.last_par * 2 * kMaxRoundW] : 0;
+  const int32_t last_L = h.last_x >= 0 ? (int32_t)(v.pcnt[(size_t)h.last_par * 2 * kMaxRoundW] & 0xffffffffLL) : 0;
   if (i < leaves) {
     const LeafEnt e = ent[i];
     int32_t begin = e.begin, count = e.count, slot = e.slot;
