@@ -112,6 +112,7 @@ struct Params {
   int32_t n_groups;            // feature groups of a round's search, one candidate each
   int32_t n_numeric, unit_penalty;  // numerical features (first in `order`); every feature's penalty is 1
   int32_t cta_full, cta_extra, cta_last;  // histogram CTAs of a round (hist_split_ctas)
+  int32_t fix_bits;            // float histograms: bits of a fixed-point value (the sum of n of them fits 95 bits and a sign)
   int32_t hot_shift;           // quantized histograms' 32-bit hot counters hold (grad << hot_shift) + hess
   const int32_t* order;        // [F] inner features: the numerical ones, then the categorical ones
   int32_t cand_rows;           // rows of Job::cand and Job::splittable: 1 + 2 max_exp nodes
@@ -157,7 +158,8 @@ struct JobState {
   uint32_t col_rng;
   int32_t bytree_on;
   double bynode_fraction;
-  int32_t fin_q, _pad;  // grow rounds: which copy of the rounds' state the tree ended in
+  int32_t fin_q;    // grow rounds: which copy of the rounds' state the tree ended in
+  int32_t fix_ok;   // float path: the tree's histograms use fixed-point sums (red_maxg / red_maxh: largest exponents)
   uint32_t mt[624];
 };
 

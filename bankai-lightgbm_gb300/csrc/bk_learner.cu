@@ -573,6 +573,9 @@ int learner_create(const bk_feature* features, int32_t num_features, const uint8
       const std::array<int, 5> d = L->default_shape();
       L->set_launch_shape(d[0], d[1], d[2], d[3], d[4]);
     }
+    // a sum of n values below 2^fix_bits stays below 2^94
+    p.fix_bits = 94;
+    while (p.fix_bits > 24 && (num_data >> (94 - p.fix_bits)) != 0) --p.fix_bits;
     bool wide = false;
     if (quant) {
       int max_h = p.const_hess ? 1 : p.quant_bins;

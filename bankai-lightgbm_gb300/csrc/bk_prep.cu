@@ -238,6 +238,21 @@ __global__ void k_noise_f32(const double* __restrict__ a, float* __restrict__ b,
 // scale whenever every partial sum is exactly representable (power-of-two bin counts and fewer
 // than 2^29 units), which is then bit-identical to the reference's sequential sum; otherwise a
 // single warp sums sequentially in row order like the reference.
+// The float path also finds the largest and the smallest non-zero magnitude of the gradients and
+// hessians (their bits, max << 32 | min), for the histograms' unit.
+__device__ __forceinline__ int64_t join_range(int64_t a, int64_t b) {
+  const uint32_t lo = min((uint32_t)a, (uint32_t)b), hi = max((uint32_t)(a >> 32), (uint32_t)(b >> 32));
+  return (int64_t)(((uint64_t)hi << 32) | lo);
+}
+
+// Whether every value of the range is a 24-bit multiple of a unit below 2^bits of them, and its
+// largest biased exponent.
+__device__ __forceinline__ bool fixed_fits(int64_t range, int bits, uint32_t* emax) {
+  const uint32_t hi = (uint32_t)(range >> 32), lo = min((uint32_t)range, hi);
+  *emax = max(hi >> 23, 1u);
+  return hi < 0x7f800000u && (int)*emax - (int)max(lo >> 23, 1u) <= bits - 24;
+}
+
 __global__ void __launch_bounds__(256) k_root_partial(const Job* __restrict__ jobs, Params p) {
   __shared__ double sg_s[8], sh_s[8];
   __shared__ long long ig_s[8], ih_s[8];
@@ -247,6 +262,13 @@ __global__ void __launch_bounds__(256) k_root_partial(const Job* __restrict__ jo
   if (p.quant && !bagged && J.st->disc_ok) return;  // the discretization has left its sums
   double sg = 0.0, sh = 0.0;
   long long ig = 0, ih = 0;
+  // float path: the largest and the smallest non-zero magnitude's bits
+  uint32_t max_g = 0, min_g = 0x7fffffffu, max_h = 0, min_h = 0x7fffffffu;
+  auto range = [](float v, uint32_t& hi, uint32_t& lo) {
+    const uint32_t a = __float_as_uint(v) & 0x7fffffffu;
+    hi = max(hi, a);
+    if (a) lo = min(lo, a);
+  };
   for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < cnt; k += (int64_t)gridDim.x * blockDim.x) {
     const int64_t i = bagged ? J.idx0[k] : k;
     if (p.quant) {
@@ -254,8 +276,11 @@ __global__ void __launch_bounds__(256) k_root_partial(const Job* __restrict__ jo
       ig += (int8_t)(pk >> 8);
       ih += pk & 0xff;
     } else {
-      sg += (double)J.g[i];
-      sh += (double)J.h[i];
+      const float g = J.g[i], h = J.h[i];
+      sg += (double)g;
+      sh += (double)h;
+      range(g, max_g, min_g);
+      range(h, max_h, min_h);
     }
   }
 #pragma unroll
@@ -264,8 +289,18 @@ __global__ void __launch_bounds__(256) k_root_partial(const Job* __restrict__ jo
     sh += __shfl_xor_sync(FULL, sh, o);
     ig += __shfl_xor_sync(FULL, ig, o);
     ih += __shfl_xor_sync(FULL, ih, o);
+    if (!p.quant) {
+      max_g = max(max_g, __shfl_xor_sync(FULL, max_g, o));
+      min_g = min(min_g, __shfl_xor_sync(FULL, min_g, o));
+      max_h = max(max_h, __shfl_xor_sync(FULL, max_h, o));
+      min_h = min(min_h, __shfl_xor_sync(FULL, min_h, o));
+    }
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (!p.quant) {
+    ig = (long long)(((unsigned long long)max_g << 32) | min_g);
+    ih = (long long)(((unsigned long long)max_h << 32) | min_h);
+  }
   if (lane == 0) {
     sg_s[warp] = sg;
     sh_s[warp] = sh;
@@ -279,8 +314,13 @@ __global__ void __launch_bounds__(256) k_root_partial(const Job* __restrict__ jo
     for (int w = 0; w < 8; ++w) {
       a += sg_s[w];
       b += sh_s[w];
-      c += ig_s[w];
-      d += ih_s[w];
+      if (p.quant) {
+        c += ig_s[w];
+        d += ih_s[w];
+      } else {
+        c = join_range(w ? c : ig_s[w], ig_s[w]);
+        d = join_range(w ? d : ih_s[w], ih_s[w]);
+      }
     }
     J.red[2 * blockIdx.x] = a;
     J.red[2 * blockIdx.x + 1] = b;
@@ -314,11 +354,20 @@ __global__ void __launch_bounds__(32) k_root_finish(const Job* __restrict__ jobs
     for (int b = 0; b < kRootGrid; b += 32) {
       sg += J.red[2 * (b + lane)];
       sh += J.red[2 * (b + lane) + 1];
+      ig = join_range(b ? ig : J.ired[2 * lane], J.ired[2 * (b + lane)]);
+      ih = join_range(b ? ih : J.ired[2 * lane + 1], J.ired[2 * (b + lane) + 1]);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       sg += __shfl_xor_sync(FULL, sg, o);
       sh += __shfl_xor_sync(FULL, sh, o);
+      ig = join_range(ig, __shfl_xor_sync(FULL, ig, o));
+      ih = join_range(ih, __shfl_xor_sync(FULL, ih, o));
+    }
+    if (lane == 0) {
+      const bool g_ok = fixed_fits(ig, p.fix_bits, &s->red_maxg);
+      const bool h_ok = fixed_fits(ih, p.fix_bits, &s->red_maxh);
+      s->fix_ok = g_ok && h_ok ? 1 : 0;
     }
   }
   if (p.quant && !exact_quant_root) {
