@@ -318,6 +318,14 @@ void launch_mt_seed(const Job* d_jobs, int num_jobs, uint32_t seed, cudaStream_t
 constexpr int kRootGrid = 1216;  // CTAs of the root sums and the discretization: eight per SM
 
 // bk_predict.cu
+// Packs a validated tree for predict_staged into `out` (52 bytes per leaf + 16 at most) and returns the
+// bytes, or 0 when the tree does not fit that form. column_of: scratch for every feature.
+size_t predict_pack(const DevFeature* h_feat, int32_t num_leaves, const int32_t* left, const int32_t* right,
+                    const int32_t* feature, const uint32_t* threshold, const int8_t* type, const uint32_t* cat_bins,
+                    const double* leaf_value, const uint8_t* bins, int64_t m, int32_t* column_of, unsigned char* out,
+                    int32_t* num_columns);
+cudaError_t predict_staged(int32_t F, int32_t num_leaves, int32_t num_columns, const unsigned char* d_packed,
+                           const uint8_t* bins, int64_t m, double* score, cudaStream_t s);
 cudaError_t predict_tree(const DevFeature* feats, int32_t num_leaves, const int32_t* d_tree, const double* d_leaf_value,
                          const uint8_t* bins, int64_t m, double* score, cudaStream_t s);
 

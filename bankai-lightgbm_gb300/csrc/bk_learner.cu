@@ -170,9 +170,10 @@ struct bk_learner {
   ObjectiveWeights obj_w;          // row / label weights of the device objectives (caller-owned rows)
   int32_t* h_bad_label = nullptr;  // pinned copy, read by the train call that follows the gradients
   double* d_leaf_vals_in = nullptr;
-  int32_t* d_tree = nullptr;     // one tree's node arrays for prediction (13 x (num_leaves - 1))
+  int32_t* d_tree = nullptr;     // one tree's node arrays for prediction (13 x (num_leaves - 1), or packed)
   double* d_tree_values = nullptr;
-  std::vector<int32_t> h_tree;
+  std::vector<int32_t> h_tree, h_column;
+  std::vector<unsigned char> h_packed;
   // graph
   cudaGraphExec_t graph_exec = nullptr;
   cudaGraphExec_t graph_more = nullptr;  // grow rounds: further rounds of a tree that the first graph did not finish
@@ -729,7 +730,9 @@ int learner_create(const bk_feature* features, int32_t num_features, const uint8
     L->d_bad_label = L->dalloc<int32_t>(1);
     CK(cudaMemset(L->d_bad_label, 0, sizeof(int32_t)));
     L->d_leaf_vals_in = L->dalloc<double>((size_t)Lv * K);
-    L->d_tree = L->dalloc<int32_t>(13 * (size_t)Lv);
+    L->d_tree = L->dalloc<int32_t>(13 * (size_t)Lv + 4);
+    L->h_packed.resize(52 * (size_t)Lv + 16);
+    L->h_column.resize((size_t)p.F);
     L->d_tree_values = L->dalloc<double>(Lv);
     CK(cudaEventCreate(&L->ev_start));
     CK(cudaEventCreate(&L->ev_end));
@@ -1801,6 +1804,24 @@ int bk_learner_predict_add(bk_learner* L, int32_t num_leaves, const int32_t* lef
     if (!cat && threshold_in_bin[i] >= (uint32_t)L->h_feat[split_feature_inner[i]].num_bin) {
       set_error("bk_learner_predict_add: node %d splits an unknown feature or bin", i);
       return -1;
+    }
+  }
+  if (num_rows > 0) {
+    // the packed form: one copy of the tree, and columns staged in shared memory
+    int32_t ncols = 0;
+    const size_t bytes = predict_pack(L->h_feat.data(), num_leaves, left_child, right_child, split_feature_inner,
+                                      threshold_in_bin, decision_type, cat_bins, leaf_value, bins, num_rows,
+                                      L->h_column.data(), L->h_packed.data(), &ncols);
+    if (bytes > 0) {
+      try {
+        CK(cudaMemcpyAsync(L->d_tree, L->h_packed.data(), bytes, cudaMemcpyHostToDevice, L->stream));
+        CK(predict_staged(L->p.F, num_leaves, ncols, reinterpret_cast<const unsigned char*>(L->d_tree), bins, num_rows,
+                          score, L->stream));
+        CK(cudaStreamSynchronize(L->stream));
+      } catch (const CudaError& e) {
+        return fail_cuda(e);
+      }
+      return 0;
     }
   }
   L->h_tree.assign(13 * (size_t)std::max(ni, 1), 0);

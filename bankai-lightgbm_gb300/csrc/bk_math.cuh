@@ -112,7 +112,7 @@ __device__ __forceinline__ bool better_than(double ga, int32_t fa, double gb, in
 // The route of one stored bin for a numerical split of a single-feature dense group
 // (data_partition.rs:299-410 with group_view :25-40: min_bin 1, max_bin gbins - 1,
 // use_min_bin false). 1 = left.
-__device__ __forceinline__ uint8_t route_bin(const DevFeature& m, uint32_t threshold, bool default_left, uint32_t bin) {
+__host__ __device__ __forceinline__ uint8_t route_bin(const DevFeature& m, uint32_t threshold, bool default_left, uint32_t bin) {
   const uint32_t min_bin = 1, max_bin = (uint32_t)m.gbins - 1;
   const uint32_t default_bin = (uint32_t)m.default_bin, mfb = (uint32_t)m.mfb;
   bool miss_zero = false, miss_na = false, mfb_zero = false, mfb_na = false;
