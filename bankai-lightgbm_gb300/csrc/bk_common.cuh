@@ -305,7 +305,6 @@ void launch_discretize(const Job* d_jobs, int num_jobs, const Params& p, const d
                        const float* noise_gf, const float* noise_hf, cudaStream_t s);
 void launch_noise_f32(const double* a, float* b, int64_t n, cudaStream_t s);
 void launch_root_sums(const Job* d_jobs, int num_jobs, const Params& p, int exact_quant_root, cudaStream_t s);
-void launch_renew(const Job* d_jobs, int num_jobs, const Params& p, cudaStream_t s);
 void launch_add_score(const Job* d_jobs, int num_jobs, const Params& p, const double* leaf_vals, double* score,
                       cudaStream_t s);
 // need_stop: nothing is added unless every job's tree is finished (JobState::stop)
@@ -313,9 +312,29 @@ void launch_add_score_own(const Job* d_jobs, int num_jobs, const Params& p, doub
                           cudaStream_t s);
 // Zeroes the first `bytes` bytes (a multiple of 16) of every job's histogram pool.
 void launch_zero_pool(void* pool, size_t bytes_per_job, size_t bytes, int num_jobs, cudaStream_t s);
-void launch_row_leaf(const Job* d_jobs, int num_jobs, const Params& p, int32_t* out, cudaStream_t s);
+// need_stop: only finished jobs' rows
+void launch_row_leaf(const Job* d_jobs, int num_jobs, const Params& p, int32_t* out, int need_stop, cudaStream_t s);
 void launch_mt_seed(const Job* d_jobs, int num_jobs, uint32_t seed, cudaStream_t s);
 constexpr int kRootGrid = 1216;  // CTAs of the root sums and the discretization: eight per SM
+
+// bk_renew.cu
+struct RenewBuffers {
+  void* sums = nullptr;        // the chunks' summaries of every job, `slots` per job
+  int64_t slots = 0;
+  int32_t* row_leaf = nullptr; // [jobs][n], grouping only, as the rest
+  int32_t* counts = nullptr;   // [jobs][num_leaves][CTAs]
+  int32_t* order = nullptr;    // [jobs][n]: the leaves' rows in the root's order
+};
+struct RenewSizes {
+  int64_t slots;
+  size_t sums, counts, rows;  // per job: bytes; elements; elements of row_leaf and order
+};
+RenewSizes renew_sizes(const Params& p, bool grouped);
+// After grow rounds: every finished job's rows grouped by leaf in the root's order.
+void launch_group_rows(const Job* d_jobs, int num_jobs, const Params& p, const int32_t* d_rows, const RenewBuffers& b,
+                       cudaStream_t s);
+// grouped: the rows are b.order's, and only finished jobs are renewed; else the leaves' own order
+void launch_renew(const Job* d_jobs, int num_jobs, const Params& p, const RenewBuffers& b, bool grouped, cudaStream_t s);
 
 // bk_predict.cu
 // Packs a validated tree for predict_staged into `out` (52 bytes per leaf + 16 at most) and returns the

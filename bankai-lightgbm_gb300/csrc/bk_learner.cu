@@ -159,6 +159,7 @@ struct bk_learner {
   float* d_g = nullptr;
   float* d_h = nullptr;
   int32_t* d_rows = nullptr;
+  RenewBuffers renew;
   size_t pool_bytes_per_job = 0, slot_bytes = 0;
   void* d_pool = nullptr;
   std::vector<void*> allocs;
@@ -268,7 +269,8 @@ struct bk_learner {
   // One grow-loop step (iteration `it`) of all jobs; with timing on, events split the step into
   // histogram / search / partition phases.
   // The plain form keeps the reference's stable compaction; so does leaf renewal, whose f64 sums
-  // run in leaf row order. Otherwise split `it` is partitioned in one pass, counting into the
+  // run in leaf row order (after grow rounds the rows are grouped in that order again). Otherwise
+  // split `it` is partitioned in one pass, counting into the
   // counter pair it & 1, and the histogram launch of step it + 1 applies its bookkeeping.
   bool stable_partition() const { return loop_mode == 0 || (p.quant && p.renew); }
   void step_a(int it) {
@@ -288,10 +290,10 @@ struct bk_learner {
   }
 
   // Grow rounds (bk_rounds.cuh) in the graph form, unless something goes by the splits' order (the
-  // by-node sampler's stream, per-split phase timing, the renewal's row order) or by one leaf at a
+  // by-node sampler's stream, per-split phase timing) or by one leaf at a
   // time (thread-block clusters over a leaf's histogram CTAs), or the leaves do not fit the decision.
   bool rounds() const {
-    return loop_mode == 1 && !timing && !p.bynode && !(p.quant && p.renew) && hl.cluster == 1 && p.max_exp > 0;
+    return loop_mode == 1 && !timing && !p.bynode && hl.cluster == 1 && p.max_exp > 0;
   }
   // Rounds captured with the tree: doubling up to round_w leaves, then round_w splits a round, and a
   // few more for the trees whose best leaves come one after the other; even, as the rounds' two
@@ -308,6 +310,10 @@ struct bk_learner {
       launch_partition_round(jobs.data(), K, p, d_bins_cm, d_feat, r & 1, stream);
     }
     launch_rounds_finish(jobs.data(), K, p, stream);
+    if (p.quant && p.renew) {
+      launch_group_rows(d_jobs, K, p, d_rows, renew, stream);
+      launch_renew(d_jobs, K, p, renew, true, stream);
+    }
   }
 
   void tree_prologue() {
@@ -322,7 +328,7 @@ struct bk_learner {
 
   void tree_epilogue() {
     if (!stable_partition()) launch_apply_split(jobs.data(), K, p, (p.num_leaves - 2) & 1, stream);
-    if (p.quant && p.renew) launch_renew(d_jobs, K, p, stream);
+    if (p.quant && p.renew) launch_renew(d_jobs, K, p, renew, false, stream);
   }
 
   // Everything of an iteration's trees on the stream: the prologue and the grow loop (in rounds: the
@@ -717,6 +723,16 @@ int learner_create(const bk_feature* features, int32_t num_features, const uint8
         const size_t bytes = rounds_state_bytes(Lv, p.max_exp, F);
         J.rounds = L->dalloc<uint8_t>(bytes);
         CK(cudaMemset(J.rounds, 0, bytes));
+      }
+    }
+    if (p.quant && p.renew) {
+      const RenewSizes r = renew_sizes(p, p.max_exp > 0);
+      L->renew.slots = r.slots;
+      L->renew.sums = L->dalloc<uint8_t>(r.sums * K);
+      if (p.max_exp > 0) {
+        L->renew.counts = L->dalloc<int32_t>(r.counts * K);
+        L->renew.row_leaf = L->dalloc<int32_t>(r.rows * K);
+        L->renew.order = L->dalloc<int32_t>(r.rows * K);
       }
     }
     L->d_jobs = L->dalloc<Job>(K);
@@ -1472,7 +1488,7 @@ int bk_learner_row_leaf(bk_learner* L, int32_t* out) {
     int32_t* d = nullptr;
     CK(cudaMallocAsync((void**)&d, n * K * sizeof(int32_t), L->stream));
     CK(cudaMemsetAsync(d, 0xff, n * K * sizeof(int32_t), L->stream));
-    launch_row_leaf(L->d_jobs, L->K, p, d, L->stream);
+    launch_row_leaf(L->d_jobs, L->K, p, d, 0, L->stream);
     CK(cudaMemcpyAsync(out, d, n * K * sizeof(int32_t), cudaMemcpyDeviceToHost, L->stream));
     CK(cudaFreeAsync(d, L->stream));
     CK(cudaStreamSynchronize(L->stream));

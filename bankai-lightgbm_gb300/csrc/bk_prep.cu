@@ -4,8 +4,6 @@
 //     per-tree stochastic-rounding rotation drawn on the device from a std::mt19937 state
 //     (mt19937.rs:32-128), so every draw happens exactly when the reference draws;
 //   - root leaf sums (serial.rs:705-775);
-//   - quantized leaf renewal (serial.rs:634-655), summed sequentially in leaf row order like the
-//     reference so the f64 sums round identically;
 //   - score update and leaf lookup over the final partition (serial.rs:1974-1990).
 #include <math_constants.h>
 
@@ -409,37 +407,6 @@ __global__ void __launch_bounds__(32) k_root_finish(const Job* __restrict__ jobs
   }
 }
 
-// ---- leaf renewal (quantized, quant_train_renew_leaf) ----
-__global__ void __launch_bounds__(32) k_renew(const Job* __restrict__ jobs, Params p) {
-  const Job& J = jobs[blockIdx.z];
-  const int32_t leaf = blockIdx.x;
-  if (leaf >= J.st->tree_leaves) return;
-  const int lane = threadIdx.x;
-  const int64_t begin = J.leaf_begin[leaf], cnt = J.leaf_count[leaf];
-  const int32_t* idx = leaf_idx(J, J.leaf_buf[leaf]) + begin;
-  const bool all = cnt == p.n;  // every row, in order
-  double s1 = 0.0, s2 = 0.0;
-  for (int64_t base = 0; base < cnt; base += 32) {
-    int64_t k = base + lane;
-    float gv = 0.f, hv = 0.f;
-    if (k < cnt) {
-      int32_t r = all ? (int32_t)k : idx[k];
-      gv = J.g[r];
-      hv = J.h[r];
-    }
-    int jn = (int)min((int64_t)32, cnt - base);
-    for (int j = 0; j < jn; ++j) {
-      float a = __shfl_sync(FULL, gv, j), b = __shfl_sync(FULL, hv, j);
-      s1 += (double)a;
-      s2 += (double)b;
-    }
-  }
-  if (lane == 0) {
-    double o = leaf_output(true, true, false, s1, s2, p, (int32_t)cnt, 0.0);
-    J.leaf_value[leaf] = round_to_zero(o);
-  }
-}
-
 // ---- score update / leaf lookup over the final partition ----
 // The leaves' row ranges tile the positions 0 .. root count of the index buffers, so every CTA takes
 // the same number of positions (`per`), whatever the leaves' sizes: it lists the leaves that overlap
@@ -517,8 +484,9 @@ __global__ void __launch_bounds__(256) k_add_score_own(const Job* __restrict__ j
 }
 
 __global__ void __launch_bounds__(256) k_row_leaf(const Job* __restrict__ jobs, Params p, int per,
-                                                  int32_t* __restrict__ out) {
+                                                  int32_t* __restrict__ out, int need_stop) {
   const Job& J = jobs[blockIdx.z];
+  if (need_stop && !J.st->stop) return;
   int32_t* o = out + (size_t)blockIdx.z * p.n;
   for_leaf_rows(J, p, per, [&](int32_t leaf, const int32_t (&row)[4]) {
 #pragma unroll
@@ -570,10 +538,6 @@ void launch_root_sums(const Job* d_jobs, int num_jobs, const Params& p, int exac
   k_root_finish<<<dim3(1, 1, num_jobs), 32, 0, s>>>(d_jobs, p, exact_quant_root);
 }
 
-void launch_renew(const Job* d_jobs, int num_jobs, const Params& p, cudaStream_t s) {
-  k_renew<<<dim3(p.num_leaves, 1, num_jobs), 32, 0, s>>>(d_jobs, p);
-}
-
 void launch_add_score(const Job* d_jobs, int num_jobs, const Params& p, const double* leaf_vals, double* score,
                       cudaStream_t s) {
   k_add_score<<<leaf_rows_grid(p, num_jobs), 256, 0, s>>>(d_jobs, p, leaf_rows_per(p), leaf_vals, score);
@@ -588,8 +552,8 @@ void launch_zero_pool(void* pool, size_t bytes_per_job, size_t bytes, int num_jo
   k_zero_pool<<<dim3(1024, 1, num_jobs), 256, 0, s>>>(reinterpret_cast<uint4*>(pool), bytes_per_job / 16, bytes / 16);
 }
 
-void launch_row_leaf(const Job* d_jobs, int num_jobs, const Params& p, int32_t* out, cudaStream_t s) {
-  k_row_leaf<<<leaf_rows_grid(p, num_jobs), 256, 0, s>>>(d_jobs, p, leaf_rows_per(p), out);
+void launch_row_leaf(const Job* d_jobs, int num_jobs, const Params& p, int32_t* out, int need_stop, cudaStream_t s) {
+  k_row_leaf<<<leaf_rows_grid(p, num_jobs), 256, 0, s>>>(d_jobs, p, leaf_rows_per(p), out, need_stop);
 }
 
 }  // namespace bk
