@@ -128,6 +128,7 @@ struct LeafConst {
   // the warp search's bounds (bk_search_warp.cuh): hs2 = h + 2 lambda_l2, the error bound's factor
   // and constant (bk1 < 0: the leaf is outside its range), min_gain_shift - s0 rounded up / down
   float hs2, bk1, bk0, d_up, d_dn;
+  double r2;               // float path: g / (h + 2 lambda_l2)
   int32_t go;              // 0: the leaf is not searched (grow rounds: 1 the left child, 2 the right child)
   double gs, hs;           // quantized path: the gradient / hessian scales
   LeafSum ls;              // the leaf's sums (its LeafSplits), as leaf_sum[leaf] holds them

@@ -43,6 +43,7 @@
 #include <algorithm>
 #include <mutex>
 
+#include "bk_fixed.cuh"
 #include "bk_launch.cuh"
 #include "bk_leaf.cuh"
 
@@ -692,56 +693,6 @@ struct FloatHist {
     return reinterpret_cast<uint32_t*>(base + (size_t)r * region) + ((e >> 5) * 64 + plane * 32 + (e & 31));
   }
 };
-
-// A row's value as a 96-bit two's complement multiple of the tree's unit.
-struct Fixed {
-  uint32_t lo, mid, hi;
-};
-
-// v's 24-bit mantissa shifted up by its exponent's distance from the smallest one that fits: `shift0`
-// = the shift of biased exponent 0. The tree's rule (JobState::fix_ok) makes 0 <= shift.
-__device__ __forceinline__ Fixed to_fixed(float v, int shift0) {
-  const uint32_t u = __float_as_uint(v), e = (u >> 23) & 0xffu, m = (u & 0x7fffffu) | (e ? 0x800000u : 0u);
-  const uint32_t s = m ? (uint32_t)((int)max(e, 1u) + shift0) : 0u;
-  const uint64_t x = (uint64_t)m << (s & 31u);
-  const uint32_t x0 = (uint32_t)x, x1 = (uint32_t)(x >> 32), w = s >> 5;
-  Fixed f;
-  f.lo = w == 0u ? x0 : 0u;
-  uint64_t top = w == 0u ? (uint64_t)x1 : (w == 1u ? x : x << 32);
-  if (u >> 31) {
-    f.lo = 0u - f.lo;
-    top = ~top + (f.lo == 0u ? 1u : 0u);
-  }
-  f.mid = (uint32_t)top;
-  f.hi = (uint32_t)(top >> 32);
-  return f;
-}
-
-// (hi:mid:lo) * 2^exp as a double, rounded to nearest even. In integer instructions: the f64 unit takes
-// 64 cycles of a scheduler for each conversion or addition of a warp.
-__device__ __forceinline__ double fixed_to_double(uint32_t lo, uint32_t mid, uint32_t hi, int exp) {
-  const bool neg = (hi >> 31) != 0u;
-  if (neg) {
-    lo = 0u - lo;
-    const uint64_t t = ~(((uint64_t)hi << 32) | mid) + (lo == 0u ? 1u : 0u);
-    mid = (uint32_t)t;
-    hi = (uint32_t)(t >> 32);
-  }
-  if (!(lo | mid | hi)) return 0.0;
-  if (hi == 0u) {  // two words at the top
-    hi = mid, mid = lo, lo = 0u, exp -= 32;
-    if (hi == 0u) hi = mid, mid = 0u, exp -= 32;
-  }
-  const int z = __clz((int)hi);
-  uint64_t top = ((uint64_t)__funnelshift_l(mid, hi, z) << 32) | __funnelshift_l(lo, mid, z);  // bit 63 set
-  const bool sticky = (lo << z) != 0u;
-  const uint32_t rest = (uint32_t)top & 0x7ffu;
-  top >>= 11;
-  if (rest > 0x400u || (rest == 0x400u && (sticky || (top & 1u)))) ++top;
-  // top in [2^52, 2^53], so its bit 52 adds one to the exponent field
-  const int64_t field = exp + 95 - z + 1022;
-  return __longlong_as_double((long long)(top + ((uint64_t)field << 52)) | (neg ? (long long)(1ull << 63) : 0));
-}
 
 // Adds (hi:mid) to the two words at shared address `at` (mid) and at + 128 (hi). The addition to mid
 // returns the word before it, which gives the carry: exact whatever the order of the rows.

@@ -103,6 +103,7 @@ __device__ __forceinline__ void compute_leaf_const_ls(const Job& J, const Params
     const double s0 = p.l2 == 0.0 ? c.mgs - p.min_gain : c.sum_g * c.sum_g / h2;
     const double d = p.l2 == 0.0 ? p.min_gain : c.mgs - s0;
     c.hs2 = (float)h2;
+    c.r2 = p.quant ? 0.0 : c.sum_g / h2;
     const float ymin = (float)(p.min_hess + p.l2), s0f = (float)s0, arel = 4e-15f + 1.01e-15f / ymin;
     c.bk1 = 44.0f * 5.9604645e-08f + arel;
     c.bk0 = s0f * arel + 1e-24f;

@@ -33,6 +33,7 @@
 #include "bk_launch.cuh"
 #include "bk_leaf.cuh"
 #include "bk_math.cuh"
+#include "bk_fixed.cuh"
 #include "bk_search.cuh"
 #include "bk_search_warp.cuh"
 
@@ -229,6 +230,9 @@ struct SearchSmemT {
   int32_t wc[3][NW];
   WarpFilt wf[2][NW];
   WarpFilt xf;  // the forward scan's position -1 (last thread)
+  // search_float_fixed: the warps' sums of gradients, hessians and counts, those that FixHistogram takes,
+  // the top bin's
+  Fixed fx[3][NW], ff[2][NW], top[3];
   int32_t spl[2][NW];
   DirBest wb[2][NW];
 };
@@ -936,6 +940,247 @@ __device__ void search_float(const Job& J, const Params& p, const SearchIn& si, 
   });
 }
 
+// The bounds on d (bk_search_warp.cuh: a threshold's gain minus the leaf-wide s0) of a plain float
+// threshold. With H2 = h + 2 l2 and yl, yr = hl + l2, hr + l2, d = t^2 H2 / (yl yr) where
+// t = gl - (g / H2) yl, the left gradients centred on the leaf's mean: one f64 multiply-add keeps what
+// cancels. Its f64 error is below 2^-50 (|gl| + |g / H2| yl); the fp32 rest, truncations of 2^-23
+// included, errs less than the 44 u of LeafConst::bk1.
+struct FloatLeaf {
+  float r2f;  // g / H2
+  int g_exp, h_exp;
+};
+__device__ __forceinline__ Approx bound_float(const Params& p, const Fixed& gl, const Fixed& hl, const Fixed& hr,
+                                              const FloatLeaf& K, const LeafConst& C) {
+  const double g = fixed_to_double(gl.lo, gl.mid, gl.hi, K.g_exp);
+  double yl = fixed_to_double(hl.lo, hl.mid, hl.hi, K.h_exp);
+  if (C.l2f != 0.f) yl += p.l2;  // uniform
+  const float t = double_to_float(fma(-C.r2, yl, g)), ylf = double_to_float(yl);
+  const float yrf = __fadd_rn(fixed_to_float(hr, K.h_exp), C.l2f);
+  const float q = __fdividef(C.hs2, __fmul_rn(ylf, yrf));
+  const float off = __fmul_rn(fmaf(fabsf(K.r2f), ylf, fabsf(double_to_float(g))), 1.7763568e-15f);  // 2^-49
+  Approx a;
+  a.g = __fmul_rn(__fmul_rn(t, t), q);
+  a.e = fmaf(__fmul_rn(off, fmaf(2.0f, fabsf(t), off)), q, fmaf(a.g, C.bk1, C.bk0));
+  a.uncertain = !(__fadd_rn(a.g, a.e) < 1e30f) || C.bk1 < 0.f;
+  return a;
+}
+__device__ __forceinline__ Filt filt_of_d(bool cand, const Approx& a, const LeafConst& C) {
+  Filt f;
+  f.unc = a.uncertain;
+  f.mp = cand && (a.uncertain || __fadd_rn(a.g, a.e) > C.d_dn);
+  f.lo = (cand && !a.uncertain) ? float_key(__fsub_rn(a.g, a.e)) : float_key(-CUDART_INF_F);
+  f.up = a.uncertain ? 0 : float_key(__fadd_rn(a.g, a.e));
+  return f;
+}
+
+// search_float for plain gains of a tree with fixed-point histograms (JobState::fix_ok): the same
+// candidate from exact sums. The bins' doubles are multiples of the tree's units, so one prefix scan of
+// 96-bit integers gives the sums of both directions (the reverse side is the total minus a prefix), the
+// validity tests compare integers, and only the queued positions' sums become doubles again. That leaves
+// two f64 instructions a bin for the larger child's difference, two for the count estimate and one a
+// threshold; with f64 scans, sums and fp32 conversions there were about 110 (32 leaves x 100 features
+// of 255 bins: 100 -> 37 us a round).
+template <int NW>
+__device__ void search_float_fixed(const Job& J, const Params& p, const SearchIn& si, const DevFeature& m, int side,
+                                   int32_t f, int32_t leaf, SearchSmemT<NW>& sm) {
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const LeafConst& C = si.C;
+  const LeafSum& S0 = si.S0;
+  const int32_t num_data = side ? C.ls.num_data : S0.num_data;
+  const size_t slot_stride = (size_t)p.T * p.B * TILE;
+  const size_t feat_off = (size_t)(f / TILE) * p.B * TILE + (f % TILE);
+  double2* pool = reinterpret_cast<double2*>(J.pool);
+  double2* hs = pool + (size_t)si.sslot * slot_stride + feat_off;
+  double2* hl = pool + (size_t)(side ? si.lslot : si.sslot) * slot_stride + feat_off;
+  const double2 zero = make_double2(0.0, 0.0);
+  const Fixed none{0u, 0u, 0u};
+  const bool fix = m.mfb > 0;
+  const bool in = t < m.len;
+  double2 sv = (in && !(fix && t == m.mfb)) ? hs[(size_t)(t + 1) * TILE] : zero;
+  const double2 lv = (side && in) ? pool[(size_t)si.pslot * slot_stride + feat_off + (size_t)(t + 1) * TILE] : zero;
+  const ScanGeom G = scan_geom(m);
+  FloatLeaf K;
+  K.g_exp = fixed_unit(p, J.st->red_maxg);
+  K.h_exp = fixed_unit(p, J.st->red_maxh);
+  K.r2f = double_to_float(C.r2);
+  if (t < 2) sm.qn[t] = 0;
+  const double sum_g = C.sum_g, sum_h = C.sum_h;
+  if (fix) {  // FixHistogram: the smaller leaf's most frequent bin is its total minus every other bin
+    Fixed a = double_to_fixed(sv.x, K.g_exp), b = double_to_fixed(sv.y, K.h_exp);
+#pragma unroll 1
+    for (int o = 16; o > 0; o >>= 1) {
+      a = a + shfl_xor_fixed(a, o);
+      b = b + shfl_xor_fixed(b, o);
+    }
+    if (lane == 0) {
+      sm.ff[0][warp] = a;
+      sm.ff[1][warp] = b;
+    }
+    __syncthreads();
+    if (t == m.mfb) {
+      a = double_to_fixed(S0.sg, K.g_exp);
+      b = double_to_fixed(S0.sh, K.h_exp);
+#pragma unroll 1
+      for (int i = 0; i < NW; ++i) {
+        a = a - sm.ff[0][i];
+        b = b - sm.ff[1][i];
+      }
+      sv = make_double2(fixed_to_double(a.lo, a.mid, a.hi, K.g_exp), fixed_to_double(b.lo, b.mid, b.hi, K.h_exp));
+      if (side == 0) hs[(size_t)(t + 1) * TILE] = sv;
+    }
+  }
+  const double2 v = side ? make_double2(lv.x - sv.x, lv.y - sv.y) : sv;
+  if (side && in) hl[(size_t)(t + 1) * TILE] = v;
+  const int32_t cn = in ? round_int(v.y * C.cnt_factor) : 0;
+  const bool skip_t = G.skip && t + G.off == m.default_bin, rin = t <= G.tf_r;
+  const Fixed vg = double_to_fixed(v.x, K.g_exp), vh = double_to_fixed(v.y, K.h_exp);
+  // one scan: the bins that the reverse scan accumulates, which are also those of every forward prefix
+  const bool acc = rin && !skip_t;
+  const Fixed wg = acc ? vg : none, wh = acc ? vh : none;
+  const int32_t wc = acc ? cn : 0;
+  Fixed pg = wg, ph = wh;
+  int32_t pc = wc;
+#pragma unroll 1
+  for (int o = 1; o < 32; o <<= 1) {
+    const Fixed a = shfl_up_fixed(pg, o, 32), b = shfl_up_fixed(ph, o, 32);
+    const int32_t c = __shfl_up_sync(FULL, pc, o);
+    if (lane >= o) {
+      pg = pg + a;
+      ph = ph + b;
+      pc += c;
+    }
+  }
+  if (lane == 31) {
+    sm.fx[0][warp] = pg;
+    sm.fx[1][warp] = ph;
+    sm.fx[2][warp] = Fixed{(uint32_t)pc, 0u, 0u};
+  }
+  if (G.fwd_rest && t == G.tf_r + 1) {  // the NaN bin: with the scanned ones, the whole slice
+    sm.top[0] = vg;
+    sm.top[1] = vh;
+    sm.top[2] = Fixed{(uint32_t)cn, 0u, 0u};
+  }
+  __syncthreads();
+  // lane 8 q + w: the prefix of quantity q over warps 0 .. w
+  Fixed tg, th;
+  int32_t tc;
+  {
+    const int q = lane >> 3, w = lane & 7;
+    Fixed x = (q < 3 && w < NW) ? sm.fx[q][w] : none;
+#pragma unroll 1
+    for (int o = 1; o < 8; o <<= 1) {
+      const Fixed y = shfl_up_fixed(x, o, 8);
+      if (w >= o) x = x + y;
+    }
+    tg = shfl_fixed(x, 7);
+    th = shfl_fixed(x, 15);
+    tc = (int32_t)__shfl_sync(FULL, x.lo, 23);
+    const int before = max(warp - 1, 0);
+    const Fixed a = shfl_fixed(x, before), b = shfl_fixed(x, 8 + before);
+    const int32_t c = (int32_t)__shfl_sync(FULL, x.lo, 16 + before);
+    if (warp > 0) {
+      pg = pg + a;
+      ph = ph + b;
+      pc += c;
+    }
+  }
+  // right sums of reverse position t, left sums of forward position t (and of the forward position -1,
+  // held by the last thread), the hessians without their kEpsilon
+  const Fixed lg = double_to_fixed(sum_g, K.g_exp), lh = double_to_fixed(C.ls.sh, K.h_exp);
+  const Fixed need = double_to_fixed(p.min_hess - BK_EPS, K.h_exp);
+  const Fixed rg = tg - (pg - wg), rh = th - (ph - wh);
+  const int32_t rc = tc - (pc - wc);
+  Fixed fg = pg, fh = ph, bh = none;
+  int32_t fc = pc, bc = 0;
+  const bool xpos = G.fwd_rest && t == 32 * NW - 1;
+  if (G.fwd_rest) {  // the forward scan starts with everything outside the slice
+    const Fixed bg = lg - (tg + sm.top[0]);
+    bh = lh - (th + sm.top[1]);
+    bc = num_data - (tc + (int32_t)sm.top[2].lo);
+    fg = xpos ? bg : bg + pg;
+    fh = xpos ? bh : bh + ph;
+    fc = xpos ? bc : bc + pc;
+  }
+  const bool first0 = t >= 1 - G.off && rin && !skip_t && !(rc < p.min_data || rh < need);
+  const bool brk0 = first0 && (num_data - rc < p.min_data || lh - rh < need);
+  const bool fok = !(fc < p.min_data || fh < need);
+  const bool first1 = G.two && !xpos && t <= G.t_end && !skip_t && fok;
+  const bool firstx = xpos && fok;
+  const bool brkf = num_data - fc < p.min_data || lh - fh < need;
+  const bool brk1 = first1 && brkf, brkx = firstx && brkf;
+  Filt fl[2];
+  {
+    Approx a{0.f, 0.f, true};
+    if (first0) a = bound_float(p, lg - rg, lh - rh, rh, K, C);
+    fl[0] = filt_of_d(first0, a, C);
+  }
+  publish_dir<true, NW>(sm, 0, brk0, t, fl[0], lane, warp);
+  {
+    Approx a{0.f, 0.f, true};
+    if (first1 || firstx) a = bound_float(p, fg, fh, lh - fh, K, C);
+    fl[1] = filt_of_d(first1 || firstx, a, C);
+    Filt nat = fl[1];
+    if (xpos) nat.lo = float_key(-CUDART_INF_F);
+    publish_dir<true, NW>(sm, 1, brk1, t, nat, lane, warp);
+  }
+  if (xpos) {
+    WarpFilt x;
+    x.lb = brkx ? -1 : kNoneHi;
+    x.ma = x.mb = fl[1].lo;
+    sm.xf = x;
+  }
+  __syncthreads();
+  int S[2];
+  int32_t M[2];
+  resolve_dir<true, NW>(sm, 0, false, &S[0], &M[0]);
+  resolve_dir<true, NW>(sm, 1, G.fwd_rest, &S[1], &M[1]);
+  const bool valid[2] = {first0 && t > S[0], xpos ? (firstx && S[1] != -1) : (first1 && t < S[1])};
+  // a position whose bin adds nothing repeats its scan predecessor (t + 1 reverse, t - 1 forward)
+  const bool empty = (wg.lo | wg.mid | wg.hi | wh.lo | wh.mid | wh.hi) == 0u && wc == 0;
+  const bool rep[2] = {empty && t + 1 <= G.tf_r && !(G.skip && t + 1 + G.off == m.default_bin),
+                       !xpos && empty && ((t >= 1 && !(G.skip && t - 1 + G.off == m.default_bin)) ||
+                                          (t == 0 && G.fwd_rest))};
+#pragma unroll
+  for (int d = 0; d < 2; ++d) {
+    const bool exact = valid[d] && !rep[d] && (fl[d].unc || (fl[d].mp && fl[d].up >= M[d]));
+    QEnt e{0, 0, 0, 0, 0};
+    if (exact) {  // the accumulated side (reverse: right, forward: left) in doubles
+      const Fixed ag = d == 0 ? rg : fg, ah = d == 0 ? rh : fh;
+      e.a = __double_as_longlong(fixed_to_double(ag.lo, ag.mid, ag.hi, K.g_exp));
+      e.b = __double_as_longlong(BK_EPS + fixed_to_double(ah.lo, ah.mid, ah.hi, K.h_exp));
+      e.c = d == 0 ? rc : fc;
+      e.t = (int16_t)(d == 0 || !xpos ? t : -1);
+      e.d = (int16_t)d;
+    }
+    queue_push(sm, d, exact, e, lane);
+  }
+  __syncthreads();
+  DirBest r[2];
+  int rs[2] = {0, 0};
+  eval_queues(
+      sm, warp, lane, C.mgs,
+      [&](const QEnt& e, int role) {
+        return float_side(p, e.d, __longlong_as_double(e.a), __longlong_as_double(e.b), e.c, sum_g, sum_h, num_data,
+                          role);
+      },
+      r, rs);
+  if (warp != 0) return;
+  finish_cand(J, p, m, si, leaf, f, G, C.mgs, r, rs, lane, [&](const DirBest& b, int) { return b.ev; });
+}
+
+// The float search of one (leaf, feature).
+template <bool PLAIN, int NW>
+__device__ __forceinline__ void search_float_any(const Job& J, const Params& p, const SearchIn& si, const DevFeature& m,
+                                                 int side, int32_t f, int32_t leaf, SearchSmemT<NW>& sm) {
+  if constexpr (PLAIN) {
+    if (J.st->fix_ok) {  // uniform
+      search_float_fixed<NW>(J, p, si, m, side, f, leaf, sm);
+      return;
+    }
+  }
+  search_float<PLAIN, NW>(J, p, si, m, side, f, leaf, sm);
+}
+
 // ---- categorical features (feature_histogram.rs:1328-1886) ----
 // One CTA per (leaf side, feature) as for numerical features; thread t holds slice index t. The
 // histogram slice is loaded, fixed and (larger side) derived by subtraction exactly as the
@@ -1365,11 +1610,11 @@ __global__ void __launch_bounds__(32 * NW) k_search(const JobTable jobs, Params 
       } else if (QUANT) {
         search_int<PLAIN>(J, p, si, m, side, f, leaf, sm);
       } else {
-        search_float<PLAIN>(J, p, si, m, side, f, leaf, sm);
+        search_float_any<PLAIN>(J, p, si, m, side, f, leaf, sm);
       }
     } else {
       if (QUANT) search_int<PLAIN>(J, p, si, m, side, f, leaf, sm);
-      else search_float<PLAIN>(J, p, si, m, side, f, leaf, sm);
+      else search_float_any<PLAIN>(J, p, si, m, side, f, leaf, sm);
     }
   }
   if constexpr (NW != kSearchWarps) return;  // the host gives the decision to a 256-thread launch
@@ -1468,11 +1713,11 @@ __device__ __forceinline__ void round_search_cta(const Job& J, const Params& p, 
     }
   }
   if constexpr (QUANT) search_int<PLAIN>(J, p, si, m, side, f, node, sm);
-  else search_float<PLAIN>(J, p, si, m, side, f, node, sm);
+  else search_float_any<PLAIN>(J, p, si, m, side, f, node, sm);
 }
 
-template <bool PLAIN, bool QUANT, int NW>
-__global__ void __launch_bounds__(32 * NW) k_search_round(const JobTable jobs, Params p,
+template <bool PLAIN, bool QUANT, int NW, int CTAS = 1>
+__global__ void __launch_bounds__(32 * NW, CTAS) k_search_round(const JobTable jobs, Params p,
                                                           const DevFeature* __restrict__ feats, int q) {
   __shared__ SearchSmemT<NW> sm;
   const int side = (int)(blockIdx.x & 1u), e = (int)blockIdx.y, f = (int)(blockIdx.x >> 1);
@@ -1809,6 +2054,11 @@ int rounds_groups(const Params& p) {
   return (p.n_numeric + kWarpFeatures - 1) / kWarpFeatures + (p.F - p.n_numeric);
 }
 
+// The float search's registers allow three CTAs per SM. From two waves of those on, four with some spilled
+// are faster: the rounds of 255 leaves x 100 features (3200 CTAs) 50 -> 37 us, of 63 leaves x 28
+// features (448 CTAs) 8 -> 11 us.
+constexpr int64_t kManySearches = 2 * 3 * 152;
+
 void launch_search_round(const Job* h_jobs, int num_jobs, const Params& p, const DevFeature* feats, int q,
                          cudaStream_t s) {
   const bool plain = !p.use_l1 && !p.use_max && !p.use_smooth;
@@ -1822,6 +2072,7 @@ void launch_search_round(const Job* h_jobs, int num_jobs, const Params& p, const
     else if (search_round_warp(p)) go(k_search_round_warp<false>, 32 * kWarpFeatures);
     else if (p.quant) go(k_search_round<false, true, 8>, kSearchThreads);
     else if (narrow) go(k_search_round<true, false, 2>, 64);
+    else if (plain && (int64_t)grid.x * grid.y * nz > kManySearches) go(k_search_round<true, false, 8, 4>, kSearchThreads);
     else if (plain) go(k_search_round<true, false, 8>, kSearchThreads);
     else go(k_search_round<false, false, 8>, kSearchThreads);
   });
