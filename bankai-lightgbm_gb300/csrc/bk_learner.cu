@@ -164,6 +164,10 @@ struct bk_learner {
   void* d_pool = nullptr;
   std::vector<void*> allocs;
   // host staging
+  // what a train call returns, on the device and in pinned host memory: [K][L] split records, [K][L]
+  // leaf values, the number of rejected labels
+  unsigned char *d_results = nullptr, *h_results = nullptr;
+  size_t results_bytes = 0;
   bk_split* h_records = nullptr;
   double* h_leaf_values = nullptr;
   JobState* h_state = nullptr;
@@ -205,10 +209,8 @@ struct bk_learner {
     if (graph_exec) cudaGraphExecDestroy(graph_exec);
     if (graph_more) cudaGraphExecDestroy(graph_more);
     for (void* a : allocs) cudaFree(a);
-    if (h_records) cudaFreeHost(h_records);
-    if (h_leaf_values) cudaFreeHost(h_leaf_values);
+    if (h_results) cudaFreeHost(h_results);
     if (h_state) cudaFreeHost(h_state);
-    if (h_bad_label) cudaFreeHost(h_bad_label);
     for (cudaEvent_t e : hist_events) cudaEventDestroy(e);
     if (ev_start) cudaEventDestroy(ev_start);
     if (ev_end) cudaEventDestroy(ev_end);
@@ -672,6 +674,11 @@ int learner_create(const bk_feature* features, int32_t num_features, const uint8
     L->slot_bytes = (size_t)p.T * p.B * TILE * (quant ? sizeof(int64_t) : sizeof(double2));
     L->pool_bytes_per_job = (size_t)std::max(Lv, 1 + 2 * p.max_exp) * L->slot_bytes;
     L->d_pool = L->dalloc<uint8_t>(L->pool_bytes_per_job * K);
+    static_assert(sizeof(bk_split) % sizeof(double) == 0, "the leaf values follow the records");
+    L->results_bytes = (sizeof(bk_split) + sizeof(double)) * (size_t)Lv * K + 16;
+    L->d_results = L->dalloc<unsigned char>(L->results_bytes);
+    CK(cudaMemset(L->d_results, 0, L->results_bytes));
+    L->d_bad_label = reinterpret_cast<int32_t*>(L->d_results + L->results_bytes - 16);
     JobState* d_states = L->dalloc<JobState>(K);
     CK(cudaMemset(d_states, 0, sizeof(JobState) * K));
     for (int j = 0; j < K; ++j) {  // no by-node sampling until bk_learner_set_bynode
@@ -712,13 +719,12 @@ int learner_create(const bk_feature* features, int32_t num_features, const uint8
       CK(cudaMemset(J.used + 4 * (size_t)F, 0, sizeof(uint32_t) * (size_t)Lv * p.path_words));
       J.tree_mask = L->dalloc<uint8_t>(F);
       CK(cudaMemset(J.tree_mask, 1, F));
-      J.records = L->dalloc<bk_split>(Lv);
-      J.leaf_value = L->dalloc<double>(Lv);
+      J.records = reinterpret_cast<bk_split*>(L->d_results) + (size_t)Lv * j;
+      J.leaf_value = reinterpret_cast<double*>(reinterpret_cast<bk_split*>(L->d_results) + (size_t)Lv * K) + (size_t)Lv * j;
       J.pool = reinterpret_cast<uint8_t*>(L->d_pool) + L->pool_bytes_per_job * j;
       J.part_cnt = L->dalloc<int64_t>(kMaxPartGrid);
       J.red = L->dalloc<double>(2 * kRootGrid);
       J.ired = L->dalloc<int64_t>(2 * kRootGrid);
-      CK(cudaMemset(J.records, 0, sizeof(bk_split) * Lv));
       if (p.max_exp > 0) {
         const size_t bytes = rounds_state_bytes(Lv, p.max_exp, F);
         J.rounds = L->dalloc<uint8_t>(bytes);
@@ -738,13 +744,12 @@ int learner_create(const bk_feature* features, int32_t num_features, const uint8
     L->d_jobs = L->dalloc<Job>(K);
     CK(cudaMemcpy(L->d_jobs, L->jobs.data(), sizeof(Job) * K, cudaMemcpyHostToDevice));
     if (quant && p.stochastic) launch_mt_seed(L->d_jobs, K, (uint32_t)c->seed, L->stream);
-    CK(cudaMallocHost(&L->h_records, sizeof(bk_split) * (size_t)Lv * K));
-    CK(cudaMallocHost(&L->h_leaf_values, sizeof(double) * (size_t)Lv * K));
+    CK(cudaMallocHost(&L->h_results, L->results_bytes));
+    std::memset(L->h_results, 0, L->results_bytes);
+    L->h_records = reinterpret_cast<bk_split*>(L->h_results);
+    L->h_leaf_values = reinterpret_cast<double*>(L->h_records + (size_t)Lv * K);
+    L->h_bad_label = reinterpret_cast<int32_t*>(L->h_leaf_values + (size_t)Lv * K);
     CK(cudaMallocHost(&L->h_state, sizeof(JobState) * K));
-    CK(cudaMallocHost(&L->h_bad_label, sizeof(int32_t)));
-    *L->h_bad_label = 0;
-    L->d_bad_label = L->dalloc<int32_t>(1);
-    CK(cudaMemset(L->d_bad_label, 0, sizeof(int32_t)));
     L->d_leaf_vals_in = L->dalloc<double>((size_t)Lv * K);
     L->d_tree = L->dalloc<int32_t>(13 * (size_t)Lv + 4);
     L->h_packed.resize(52 * (size_t)Lv + 16);
@@ -799,18 +804,7 @@ bool train_enqueue(bk_learner* L, const float* gradients, const float* hessians,
   if (hessians != L->d_h) CK(cudaMemcpyAsync(L->d_h, hessians, n * K * sizeof(float), kind, L->stream));
   int64_t root_count = rows ? num_rows : (int64_t)n;
   if (rows) CK(cudaMemcpyAsync(L->d_rows, rows, sizeof(int32_t) * num_rows, cudaMemcpyHostToDevice, L->stream));
-  for (size_t j = 0; j < K; ++j) {
-    L->h_state[j].use_rows = rows ? 1 : 0;
-    L->h_state[j].root_count = root_count;
-    L->h_state[j].hist_rows_direct = L->h_state[j].hist_rows_gather = L->h_state[j].hist_builds = 0;
-    JobState* st = L->jobs[j].st;
-    CK(cudaMemcpyAsync(&st->use_rows, &L->h_state[j].use_rows, sizeof(int32_t), cudaMemcpyHostToDevice,
-                       L->stream));
-    CK(cudaMemcpyAsync(&st->root_count, &L->h_state[j].root_count, sizeof(int64_t), cudaMemcpyHostToDevice,
-                       L->stream));
-    CK(cudaMemcpyAsync(&st->hist_rows_direct, &L->h_state[j].hist_rows_direct, 3 * sizeof(int64_t),
-                       cudaMemcpyHostToDevice, L->stream));
-  }
+  launch_job_begin(L->d_jobs, L->K, rows != nullptr, root_count, L->stream);
   if (L->timing && L->hist_events.size() != (size_t)(4 * (Lv - 1))) {
     for (cudaEvent_t e : L->hist_events) cudaEventDestroy(e);
     L->hist_events.assign(4 * (Lv - 1), nullptr);
@@ -829,21 +823,14 @@ bool train_enqueue(bk_learner* L, const float* gradients, const float* hessians,
 // issued again behind their further rounds.
 void enqueue_results(bk_learner* L, double shrinkage, double* score) {
   const Params& p = L->p;
-  const int Lv = p.num_leaves;
   if (score) {
     launch_add_score_own(L->d_jobs, L->K, p, shrinkage, score, L->rounds() ? 1 : 0, L->stream);
     CK(cudaGetLastError());
   }
-  for (size_t j = 0; j < (size_t)L->K; ++j) {
-    const Job& J = L->jobs[j];
-    CK(cudaMemcpyAsync(L->h_records + j * Lv, J.records, sizeof(bk_split) * (Lv - 1), cudaMemcpyDeviceToHost,
-                       L->stream));
-    CK(cudaMemcpyAsync(L->h_leaf_values + j * Lv, J.leaf_value, sizeof(double) * Lv, cudaMemcpyDeviceToHost,
-                       L->stream));
-    CK(cudaMemcpyAsync(&L->h_state[j], J.st, offsetof(JobState, mt), cudaMemcpyDeviceToHost, L->stream));
-  }
-  // labels the objective kernels rejected since the previous train call
-  CK(cudaMemcpyAsync(L->h_bad_label, L->d_bad_label, sizeof(int32_t), cudaMemcpyDeviceToHost, L->stream));
+  // every job's records and leaf values and the rejected labels in one copy, the states in another
+  CK(cudaMemcpyAsync(L->h_results, L->d_results, L->results_bytes, cudaMemcpyDeviceToHost, L->stream));
+  CK(cudaMemcpy2DAsync(L->h_state, sizeof(JobState), L->jobs[0].st, sizeof(JobState), offsetof(JobState, mt),
+                       (size_t)L->K, cudaMemcpyDeviceToHost, L->stream));
 }
 
 // With the learners' streams waited for: the further rounds of those whose trees are not finished,
@@ -1145,14 +1132,7 @@ void group_enqueue(bk_learner* L, const float* gradients, const float* hessians,
     CK(cudaMemcpyAsync(L->d_g, gradients, n * K * sizeof(float), cudaMemcpyDeviceToDevice, L->stream));
   if (hessians != L->d_h)
     CK(cudaMemcpyAsync(L->d_h, hessians, n * K * sizeof(float), cudaMemcpyDeviceToDevice, L->stream));
-  for (size_t j = 0; j < K; ++j) {
-    JobState* st = L->jobs[j].st;
-    CK(cudaMemcpyAsync(&st->use_rows, &L->h_state[j].use_rows, sizeof(int32_t), cudaMemcpyHostToDevice, L->stream));
-    CK(cudaMemcpyAsync(&st->root_count, &L->h_state[j].root_count, sizeof(int64_t), cudaMemcpyHostToDevice,
-                       L->stream));
-    CK(cudaMemcpyAsync(&st->hist_rows_direct, &L->h_state[j].hist_rows_direct, 3 * sizeof(int64_t),
-                       cudaMemcpyHostToDevice, L->stream));
-  }
+  launch_job_begin(L->d_jobs, L->K, false, p.n, L->stream);
   L->capturing = true;
   L->issue_trees();
   L->capturing = false;
@@ -1291,12 +1271,6 @@ int bk_learner_group_train(bk_learner_group* G, const float* const* gradients, c
   size_t i = 0;
   try {
     CK(cudaSetDevice(G->device));
-    for (bk_learner* L : G->learners)
-      for (int j = 0; j < L->K; ++j) {
-        L->h_state[j].use_rows = 0;
-        L->h_state[j].root_count = L->p.n;
-        L->h_state[j].hist_rows_direct = L->h_state[j].hist_rows_gather = L->h_state[j].hist_builds = 0;
-      }
     if (!G->current(gradients, hessians, shrinkage, scores)) G->capture(gradients, hessians, shrinkage, scores);
     // the iteration comes after the work already queued on every member's stream (the gradients
     // of bk_learner_objective_gradients, an earlier call)
@@ -1382,12 +1356,6 @@ int bk_learner_group_autotune(bk_learner_group* G, const float* const* gradients
     for (int pdl = 1; pdl >= 0; --pdl)
       for (int c = 0; c < 4; ++c) {
         apply(pdl, c);
-        for (bk_learner* L : G->learners)
-          for (int j = 0; j < L->K; ++j) {
-            L->h_state[j].use_rows = 0;
-            L->h_state[j].root_count = L->p.n;
-            L->h_state[j].hist_rows_direct = L->h_state[j].hist_rows_gather = L->h_state[j].hist_builds = 0;
-          }
         G->capture(gradients, hessians, 0.0, nullptr);
         std::vector<float> t;
         for (int r = 0; r <= trials; ++r) {  // one untimed iteration, then `trials` timed ones

@@ -17,6 +17,17 @@ namespace {
 
 constexpr unsigned FULL = 0xffffffffu;
 
+// What a train call sets in the job states (a launch; a copy per field and job took 3 us each).
+__global__ void __launch_bounds__(32) k_job_begin(const Job* __restrict__ jobs, int num_jobs, int use_rows,
+                                                  int64_t root_count) {
+  for (int j = threadIdx.x; j < num_jobs; j += 32) {
+    JobState* s = jobs[j].st;
+    s->use_rows = use_rows;
+    s->root_count = root_count;
+    s->hist_rows_direct = s->hist_rows_gather = s->hist_builds = 0;
+  }
+}
+
 // The root's row indices. Without bagging they are the identity, which the grow rounds (and every
 // reader of a leaf of all rows) derive instead of reading: `bagged_only` skips those 4 bytes a row.
 __global__ void k_init_rows(const Job* __restrict__ jobs, Params p, const int32_t* __restrict__ rows, int bagged_only) {
@@ -511,6 +522,10 @@ __global__ void k_zero_pool(uint4* __restrict__ pool, size_t per_job, size_t n) 
 }
 
 }  // namespace
+
+void launch_job_begin(const Job* d_jobs, int num_jobs, bool use_rows, int64_t root_count, cudaStream_t s) {
+  k_job_begin<<<1, 32, 0, s>>>(d_jobs, num_jobs, use_rows ? 1 : 0, root_count);
+}
 
 void launch_init_rows(const Job* d_jobs, int num_jobs, const Params& p, const int32_t* rows, bool bagged_only,
                       cudaStream_t s) {
