@@ -109,6 +109,7 @@ struct Params {
   // grow rounds (bk_rounds.cuh)
   int32_t round_w, round_out;  // leaves expanded per round at most; expanded leaves not yet split at most
   int32_t max_exp;             // expansions of one tree at most: num_leaves - 1 + round_out
+  int32_t search_jobs;         // jobs of a round's search launch
   int32_t n_groups;            // feature groups of a round's search, one candidate each
   int32_t n_numeric, unit_penalty;  // numerical features (first in `order`); every feature's penalty is 1
   int32_t cta_full, cta_extra, cta_last;  // histogram CTAs of a round (hist_split_ctas)

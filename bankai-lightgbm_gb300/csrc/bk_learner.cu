@@ -550,6 +550,7 @@ int learner_create(const bk_feature* features, int32_t num_features, const uint8
     }
     for (const DevFeature& d : L->h_feat)
       if (d.penalty != 1.0) p.unit_penalty = 0;
+    p.search_jobs = std::min<int32_t>(num_jobs, kJobsPerLaunch);
     p.n_groups = rounds_groups(p);
     // the feature tiles' stored-bin layouts: 16-byte runs of 4-bit bins for tiles whose features
     // all have at most 16 group bins, 8-bit runs otherwise (16 bytes for a last tile of at most

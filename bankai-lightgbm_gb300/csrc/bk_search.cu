@@ -78,15 +78,6 @@ __device__ __forceinline__ Approx approx_from(float xl, float yl, float xr, floa
   return a;
 }
 
-// The quantized sums fit in 32 bits (signed gradients, unsigned hessians), so the conversions are
-// single 32-bit ones.
-__device__ __forceinline__ Approx approx_int(int64_t lg, int64_t lh, int64_t tg, int64_t th, float gsf, float hsf,
-                                             float l2f) {
-  const int64_t rg = tg - lg, rh = th - lh;
-  return approx_from(__fmul_rn((float)(int32_t)lg, gsf), __fadd_rn(__fmul_rn((float)(uint32_t)lh, hsf), l2f),
-                     __fmul_rn((float)(int32_t)rg, gsf), __fadd_rn(__fmul_rn((float)(uint32_t)rh, hsf), l2f));
-}
-
 // GetSplitGains of one integer threshold (feature_histogram.rs:878-925: the hessians get
 // kEpsilon added, counts are round_int(hess * cnt_factor)).
 __device__ __forceinline__ double int_split_gain(const Params& p, int64_t lg, int64_t lh, int64_t tg, int64_t th,
@@ -642,9 +633,10 @@ __device__ void search_int(const Job& J, const Params& p, const SearchIn& si, co
 #pragma unroll
   for (int d = 0; d < 2; ++d) {
     const bool cand = d == 0 ? first0 : (first1 || firstx);
-    Approx a{0.f, 0.f, true};
-    if (PLAIN && cand) a = approx_int(lg[d], lh[d], tg, th, C.gsf, C.hsf, C.l2f);
-    fl[d] = filt_of(cand, a, C);
+    Bound b{-CUDART_INF_F, CUDART_INF_F};
+    if (PLAIN && cand)
+      b = bound_int(d == 0 ? l_int - right : (xpos ? base_f : left), (int32_t)tg, (int32_t)th, C, __fmul_rn(C.gsf, C.hsf));
+    fl[d] = Filt{cand && b.up > C.d_dn, false, float_key(cand ? b.lo : -CUDART_INF_F), float_key(b.up)};
   }
   publish_dir<PLAIN, NW>(sm, 0, brk0, t, fl[0], lane, warp);
   {
@@ -2046,8 +2038,15 @@ void launch_apply_split(const Job* h_jobs, int num_jobs, const Params& p, int pa
   });
 }
 
-// The warp form takes the quantized, plain searches; the others keep a CTA per feature.
-static bool search_round_warp(const Params& p) { return p.quant && !p.use_l1 && !p.use_max && !p.use_smooth; }
+// The warp form takes the quantized, plain searches of rounds that would not fit the chip at once with a
+// CTA per feature (by their registers two of 256 threads per SM); there the latter is faster, as it
+// spreads a feature's positions over eight warps: iterations with 20 features x 4 leaves a round (160
+// CTAs) take 467 us instead of 560, with 40 x 8 (640 CTAs) 926 instead of 908. With 64-thread CTAs
+// (narrow features) it gains up to 800 CTAs (50 x 8: 572 for 587 us), but costs learners that train
+// side by side more than that (twelve in a group: 2055 for 1960 us), so one line serves both.
+static bool search_round_warp(const Params& p) {
+  return p.quant && !p.use_l1 && !p.use_max && !p.use_smooth && 2 * p.F * p.round_w * p.search_jobs > 2 * 152;
+}
 
 int rounds_groups(const Params& p) {
   if (!search_round_warp(p)) return p.F;
@@ -2070,6 +2069,8 @@ void launch_search_round(const Job* h_jobs, int num_jobs, const Params& p, const
     };
     if (search_round_warp(p) && p.n_numeric < p.F) go(k_search_round_warp<true>, 32 * kWarpFeatures);
     else if (search_round_warp(p)) go(k_search_round_warp<false>, 32 * kWarpFeatures);
+    else if (p.quant && narrow) go(k_search_round<true, true, 2>, 64);
+    else if (p.quant && plain) go(k_search_round<true, true, 8>, kSearchThreads);
     else if (p.quant) go(k_search_round<false, true, 8>, kSearchThreads);
     else if (narrow) go(k_search_round<true, false, 2>, 64);
     else if (plain && (int64_t)grid.x * grid.y * nz > kManySearches) go(k_search_round<true, false, 8, 4>, kSearchThreads);
