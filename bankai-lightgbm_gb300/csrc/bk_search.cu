@@ -1238,6 +1238,68 @@ __device__ __forceinline__ int32_t cat_block_or(int32_t v, int32_t* w, int lane,
   return r;
 }
 
+// The scan of one direction on one warp (feature_histogram.rs:1666-1760): the positions whose gain is
+// needed. Sums and counts only grow along the scan, so the positions before the first that has enough
+// data on its left are skipped and the scan ends at the first whose right side has too little; between
+// them a position is taken when min_data_per_group rows have come since the last one taken. (One thread
+// walking it took 5 of a search's 28 us: a chain of f64 conversions and comparisons.)
+__device__ __forceinline__ void cat_scan_int(const Params& p, CatSmem<int64_t>& cs, int d, int32_t used_bin,
+                                             int32_t max_num_cat, int32_t num_data, int64_t thi, double hsc, int lane) {
+  int64_t g0 = 0, h0 = 0;
+  int32_t c0 = 0, taken = 0, q = 0;
+  const int32_t n = min(used_bin, max_num_cat);
+  for (int32_t i0 = 0; i0 < n; i0 += 32) {
+    const int32_t i = i0 + lane;
+    int64_t g = 0, h = 0;
+    int32_t c = 0;
+    if (i < n) {
+      const int32_t b = cs.sorted[d == 0 ? i : used_bin - 1 - i];
+      g = cs.a[b];
+      h = cs.b[b];
+      c = cs.cnt[b];
+    }
+    const int32_t own = c;
+    g = g0 + warp_incl_scan(g, lane);
+    h = h0 + warp_incl_scan(h, lane);
+    c = c0 + warp_incl_scan(c, lane);
+    const bool enough = i < n && !(c < p.min_data || (double)h * hsc < p.min_hess);
+    const int32_t rc = num_data - c;
+    const bool stop = enough && (rc < p.min_data || rc < p.min_data_per_group || (double)(thi - h) * hsc < p.min_hess);
+    const unsigned stops = __ballot_sync(FULL, stop);
+    const unsigned open = __ballot_sync(FULL, enough) & (stops ? (stops & (0u - stops)) - 1u : FULL);
+    // every open position is taken where each brings enough rows by itself
+    unsigned take = open;
+    if (__any_sync(FULL, ((open >> lane) & 1u) && own < p.min_data_per_group)) {
+      take = 0u;
+      int32_t last = taken;
+      for (unsigned left = open; left;) {
+        const unsigned ready = __ballot_sync(FULL, ((left >> lane) & 1u) && c - last >= p.min_data_per_group);
+        if (!ready) break;
+        const int k = __ffs(ready) - 1;
+        take |= 1u << k;
+        last = __shfl_sync(FULL, c, k);
+        left = k == 31 ? 0u : left & ~((2u << k) - 1u);
+      }
+    }
+    if ((take >> lane) & 1u) {
+      const int32_t at = q + __popc(take & ((1u << lane) - 1u));
+      if (at < kCatQueue) {
+        cs.qa[d][at] = g;
+        cs.qb[d][at] = h;
+        cs.qlc[d][at] = c;
+        cs.qi[d][at] = i;
+      }
+    }
+    if (take) taken = __shfl_sync(FULL, c, 31 - __clz((int)take));
+    q += __popc(take);
+    if (stops) break;
+    g0 = __shfl_sync(FULL, g, 31);
+    h0 = __shfl_sync(FULL, h, 31);
+    c0 = __shfl_sync(FULL, c, 31);
+  }
+  if (lane == 0) cs.qn[d] = min(q, kCatQueue);
+}
+
 template <bool QUANT>
 __device__ void search_cat(const Job& J, const Params& p, const SearchIn& si, const DevFeature& m, int side,
                            int32_t f, int32_t leaf, SearchSmem& sm) {
@@ -1392,7 +1454,8 @@ __device__ void search_cat(const Job& J, const Params& p, const SearchIn& si, co
     if (elig) {
       const long long kt = cs.key[t];
       int32_t rank = 0;
-      for (int u = 0; u < kSearchThreads; ++u) {
+#pragma unroll 4
+      for (int u = 0; u < m.len; ++u) {  // no category past the slice is eligible
         const long long ku = cs.key[u];
         rank += (ku != kNoKey && (ku < kt || (ku == kt && u < t))) ? 1 : 0;
       }
@@ -1401,39 +1464,32 @@ __device__ void search_cat(const Job& J, const Params& p, const SearchIn& si, co
     pl.l2 = p.l2 + p.cat_l2;
     __syncthreads();
     const int32_t max_num_cat = min(p.max_cat_threshold, (used_bin + 1) / 2);
-    // -- the sequential scans, one thread per direction (warp 0 ascending, warp 1 descending) --
-    if ((t == 0 || t == 32) && used_bin > 0) {
+    // -- the sequential scans: one warp per direction (warp 0 ascending, warp 1 descending), integer
+    //    sums by prefix scans; f64 sums one thread per direction, in order --
+    if constexpr (QUANT) {
+      if (warp < 2) cat_scan_int(p, cs, warp, used_bin, max_num_cat, num_data, thi, hsc, lane);
+    } else if ((t == 0 || t == 32) && used_bin > 0) {
       const int d = t == 0 ? 0 : 1;
       const int dir = d == 0 ? 1 : -1;
       int32_t pos = d == 0 ? 0 : used_bin - 1, cnt_group = 0, left_cnt = 0, q = 0;
       double lg = 0.0, lh = BK_EPS;
-      int64_t lig = 0, lih = 0;
       for (int32_t i = 0; i < used_bin && i < max_num_cat; ++i) {
         const int32_t c = cs.sorted[pos];
         pos += dir;
         const int32_t cnt = cs.cnt[c];
         left_cnt += cnt;
         cnt_group += cnt;
-        double lhv;
-        if (QUANT) {
-          lig += (int64_t)cs.a[c];
-          lih += (int64_t)cs.b[c];
-          lhv = (double)lih * hsc;
-        } else {
-          lg += (double)cs.a[c];
-          lh += (double)cs.b[c];
-          lhv = lh;
-        }
-        if (left_cnt < p.min_data || lhv < p.min_hess) continue;
+        lg += (double)cs.a[c];
+        lh += (double)cs.b[c];
+        if (left_cnt < p.min_data || lh < p.min_hess) continue;
         const int32_t right_cnt = num_data - left_cnt;
         if (right_cnt < p.min_data || right_cnt < p.min_data_per_group) break;
-        const double rhv = QUANT ? (double)(thi - lih) * hsc : sum_h - lh;
-        if (rhv < p.min_hess) break;
+        if (sum_h - lh < p.min_hess) break;
         if (cnt_group < p.min_data_per_group) continue;
         cnt_group = 0;
         if (q < kCatQueue) {
-          cs.qa[d][q] = QUANT ? (V)lig : (V)lg;
-          cs.qb[d][q] = QUANT ? (V)lih : (V)lh;
+          cs.qa[d][q] = (V)lg;
+          cs.qb[d][q] = (V)lh;
           cs.qlc[d][q] = left_cnt;
           cs.qi[d][q] = i;
           ++q;
@@ -1520,10 +1576,14 @@ __device__ void search_cat(const Job& J, const Params& p, const SearchIn& si, co
       const uint32_t b = (uint32_t)(best_i + m.offset);
       if ((int)(b >> 5) == lane) word |= 1u << (b & 31);
     } else {
-      for (int32_t i = 0; i <= best_i; ++i) {
-        const int32_t pos = best_dir == 0 ? i : used_bin - 1 - i;
-        const uint32_t b = (uint32_t)(cs.sorted[pos] + m.offset);
-        if ((int)(b >> 5) == lane) word |= 1u << (b & 31);
+      for (int32_t i0 = 0; i0 <= best_i; i0 += 32) {  // 32 categories at a time
+        const int32_t i = i0 + lane, pos = best_dir == 0 ? i : used_bin - 1 - i;
+        const uint32_t b = i <= best_i ? (uint32_t)(cs.sorted[pos] + m.offset) : 0xffffffffu;
+#pragma unroll
+        for (uint32_t w = 0; w < 8; ++w) {
+          const uint32_t bits = __reduce_or_sync(FULL, (b >> 5) == w ? 1u << (b & 31u) : 0u);
+          if ((int)w == lane) word |= bits;
+        }
       }
     }
   }
