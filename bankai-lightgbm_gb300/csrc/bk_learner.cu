@@ -260,6 +260,7 @@ struct bk_learner {
     out[4] = hl.cluster;
   }
 
+  int spare_rounds = 0;  // rounds captured beyond first_rounds()
   bool capturing = false;
   void record_hist_event(int i) {
     if (!timing || (size_t)i >= hist_events.size()) return;
@@ -338,7 +339,7 @@ struct bk_learner {
   void issue_trees() {
     tree_prologue();
     if (rounds()) {
-      run_rounds(first_rounds());
+      run_rounds(first_rounds() + spare_rounds);
       return;
     }
     for (int it = 0; it < p.num_leaves - 1; ++it) {
@@ -1134,8 +1135,13 @@ void group_enqueue(bk_learner* L, const float* gradients, const float* hessians,
   if (hessians != L->d_h)
     CK(cudaMemcpyAsync(L->d_h, hessians, n * K * sizeof(float), cudaMemcpyDeviceToDevice, L->stream));
   launch_job_begin(L->d_jobs, L->K, false, p.n, L->stream);
+  // Side by side, a round without work costs little, while learners that need more rounds get them only
+  // after the slowest one's first: twelve jobs took 1959 us an iteration without spare rounds, 1858 with
+  // four. A learner by itself pays 9 us for each.
   L->capturing = true;
+  L->spare_rounds = 4;
   L->issue_trees();
+  L->spare_rounds = 0;
   L->capturing = false;
   enqueue_results(L, shrinkage, score);
 }
@@ -1189,7 +1195,10 @@ struct bk_learner_group {
         CK(cudaStreamWaitEvent(stream, joins[i], 0));
       }
     } catch (...) {
-      for (bk_learner* L : learners) L->capturing = false;
+      for (bk_learner* L : learners) {
+        L->capturing = false;
+        L->spare_rounds = 0;
+      }
       cudaStreamEndCapture(stream, &graph);
       if (graph) cudaGraphDestroy(graph);
       throw;
