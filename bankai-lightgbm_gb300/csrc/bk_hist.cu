@@ -1,7 +1,7 @@
 // ConstructHistograms for the smaller leaf (serial.rs:891-1164), GB300 form.
 //
-// Grid: (blocks_per_tile, T, jobs). Each CTA owns one 32-feature tile and one contiguous chunk
-// of the leaf's rows. A warp takes 32 rows at a time: every lane fetches its row's run of the
+// Grid: (blocks_per_tile, T, jobs), or the CTAs of a grow round split over the tiles. Each CTA owns one
+// 32-feature tile and one contiguous chunk of the leaf's rows (in a round: of the leaves' rows). A warp takes 32 rows at a time: every lane fetches its row's run of the
 // tile (32 bytes of 8-bit bins, or 16 bytes of 4-bit bins) with 128-bit loads. The CTA-private
 // shared histogram keeps feature f's counters of every bin in bank f. Every lane adds its own
 // row feature by feature, lane l taking feature k ^ l at step k: the 32 lanes of each shared
@@ -19,7 +19,7 @@
 // same slot.
 //
 // Quantized path: the packed int8 gradient / uint8 hessian of a row is added as one 32-bit
-// value (grad << 16) + hess into a 16:16 "hot" histogram, which is folded into 32-bit
+// value (grad << shift) + hess into a "hot" histogram, which is folded into 32-bit
 // grad/hess "cold" counters before either half can overflow, and finally into the int64
 // (grad << 32) + hess pool slot. Integer sums are exact, so the result equals the reference's
 // sequential i64 histogram bit for bit.
@@ -30,13 +30,13 @@
 // slot receives each CTA's sum, rounded to a double, via f64 global atomics. A shared-memory integer
 // atomic costs 1.2 cycles of the SM a warp (1.7 with its old value), an fp32 one is a compare-and-swap
 // loop of 6.3, so the two top words cost 2.9 against a pair's 12.6 (the low word is zero for
-// all but the smallest values, and a warp whose rows have none skips it): 4M rows x 100
-// features, constant hessian: 6203 -> 1746 us of histograms in a 255-leaf tree, 250 of them the root's. When the exponents span too much
-// (or a value is not finite) the tree uses fp32 (hi, lo) pairs instead: hi is updated with atomicAdd,
-// which returns the previous value, and the exact rounding error of that addition (Knuth's TwoSum on
-// old and addend) is added to lo, which carries a sum to about 2^-48 of its rows' magnitudes. With a
-// constant hessian the hessian slot counts rows and is scaled by hessians[0] at the flush
-// (serial.rs:980-988), which is exact.
+// all but the smallest values, and a warp whose rows have none skips it): 4M rows x 100 features,
+// constant hessian: 6203 -> 1746 us of histograms in a 255-leaf tree, 250 of them the root's. When the
+// exponents span too much (or a value is not finite) the tree uses fp32 (hi, lo) pairs instead: hi is
+// updated with atomicAdd, which returns the previous value, and the exact rounding error of that addition
+// (Knuth's TwoSum on old and addend) is added to lo, which carries a sum to about 2^-48 of its rows'
+// magnitudes. With a constant hessian the hessian slot counts rows and is scaled by hessians[0] at the
+// flush (serial.rs:980-988), which is exact.
 //
 // The last CTA of tile 0 also computes the per-leaf constants of the search that follows
 // (bk_leaf.cuh) before its own rows.

@@ -1,8 +1,8 @@
 // DataPartition::Split (data_partition.rs:124-174), GB300 form: a stable partition of the
 // split leaf's row-index range into the left rows (kept in leaf order) followed by the right
-// rows (kept in leaf order), written into the other index buffer. When the rows' order inside a
-// child cannot change any result (no leaf renewal), the batched grow loop uses a single-pass
-// form instead (k_part_onepass, below).
+// rows (kept in leaf order), written into the other index buffer. The batched grow loop uses a
+// single-pass form instead, which keeps no order (k_part_onepass, k_part_round, below): only leaf
+// renewal depends on it, and after grow rounds it groups the rows in order again.
 //
 // The reference routes each row through SplitRule::route_bin; here every CTA evaluates that rule
 // once per stored bin into a 256-entry shared route table, so routing a row is one byte read of

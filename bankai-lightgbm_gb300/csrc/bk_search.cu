@@ -14,8 +14,9 @@
 //
 // The quantized path scans the packed (grad << 32) + hess sums with one block prefix scan; the
 // reverse scan's sums are the total minus the prefix, exact in integers, so its candidates are
-// bit-identical to the reference's. The float path scans f64 prefix and suffix sums (associated
-// differently from the sequential scan, about 1e-16 relative).
+// bit-identical to the reference's. The float path scans exact 96-bit integers (search_float_fixed); trees
+// without fixed-point histograms, and gains with L1 / max_delta_step / path_smooth, scan f64 prefix and
+// suffix sums (associated differently from the sequential scan, about 1e-16 relative).
 //
 // f64 is slow on this part, so it stays off the common path: the leaf constants the scans share
 // come precomputed from the histogram launch (bk_leaf.cuh), plain gains are filtered in fp32 with

@@ -9,7 +9,7 @@ A step is one boosting iteration: L2 gradients on the device, one tree (histogra
 search, partition, bookkeeping), and the score update. Two forms of the learner are timed:
   * quantized+batched: int8 discretized gradients, exact integer histograms, and the whole
     grow loop of an iteration replayed as one CUDA graph  -> the reported `value`;
-  * plain: fp32 compensated histograms with f64 gains and one host round trip per split.
+  * plain: fixed-point float histograms with f64 gains and one host round trip per split.
 
 `e2e` is the same metric through the C ABI with host buffers: every step copies that step's
 gradients / hessians from pinned host memory to the device inside the timed region and reads
@@ -295,9 +295,7 @@ def run_gpu(args, rank, world):
     ms, value = aggregate_ranks(main["ms_per_step"], world)
     hist_gbs = roof["hist_bytes"] / (roof["hist_ms"] * 1e6) if roof["hist_ms"] > 0 else None
     hist_launches = (args.leaves - 1) * args.steps  # one histogram launch per split step of a tree
-    # per step: objective gradients, row init, discretization (4), root sums (2), tree begin, three
-    # kernels per split (histogram, search, partition), the last split's bookkeeping, score update
-    launches_per_step = 1 + 1 + 4 + 2 + 1 + 3 * (args.leaves - 1) + 1 + 1
+    launches_per_step = _launches_per_step(args.leaves)
     line = {
         "metric": METRIC, "value": round(value, 4), "unit": "iters/s", "n_gpus": world, "steps": args.steps,
         "warmup": args.warmup, "ms_per_step": round(ms, 3), "higher_is_better": True, "scaling": "weak",
@@ -689,6 +687,19 @@ def run_hist_traffic(args):
     tm = learner.last_timing()
     learner.close()
     return {"rows": n, "hist_launches": args.leaves - 1, "hist_alg_bytes": tm["hist_bytes"]}
+
+
+def _launches_per_step(leaves):
+    """Kernels a step launches at least: objective gradients, job states, row init, discretization (4),
+    root sums (2), pool zeroing, tree begin, three kernels (histogram, search, partition) for each grow
+    round captured with the tree, the tree's records, score update. A tree that takes more rounds, or
+    (launch shapes with clusters) one split at a time, launches more."""
+    w = min(16, max(4, (leaves + 7) // 8))
+    rounds = (leaves - 1 + w - 1) // w + 3 + (w - 1).bit_length()
+    rounds = min(rounds + rounds % 2, leaves + leaves % 2)
+    if leaves > 512:  # one split at a time
+        rounds = leaves - 1
+    return 1 + 1 + 1 + 4 + 2 + 1 + 1 + 3 * rounds + 1 + 1
 
 
 def _shape_dict(shape, tuned):

@@ -172,7 +172,9 @@ int bk_learner_add_prediction_to_score(bk_learner* learner, const double* leaf_v
 int bk_learner_row_leaf(bk_learner* learner, int32_t* out);
 
 /* Grow-loop execution: 0 = one host round trip per split (the plain form); 1 = the whole
- * grow loop of an iteration captured once as a CUDA graph and replayed (default). */
+ * grow loop of an iteration captured once as a CUDA graph and replayed (default). The graph form
+ * grows up to 16 leaves a round, with the same result; phase timing, by-node sampling, interaction
+ * constraints, histogram clusters and trees above 512 leaves make it grow one split at a time. */
 int bk_learner_set_loop_mode(bk_learner* learner, int32_t mode);
 
 /* Grow-loop kernel launches: 1 (default) = each kernel is launched with programmatic dependent
@@ -217,7 +219,7 @@ int bk_learner_set_interaction_constraints(bk_learner* learner, const int32_t* f
  * tile, partition CTAs, and (quantized) the most rows a histogram CTA adds straight to the pool
  * slot with global atomics instead of through a shared histogram, and the histogram CTAs of a tile
  * per thread-block cluster (1, 2 or 4; a cluster adds up its CTAs' shared histograms in distributed
- * shared memory before one flush) — and keeps the fastest. Choices are cached per shape class (device,
+ * shared memory before one flush, and makes the learner grow one split at a time) — and keeps the fastest. Choices are cached per shape class (device,
  * log2 rows, feature tiles, bins per feature, quantized, num_leaves, num_jobs): a later learner of
  * the same class takes the cached shape without timing. The learner's state across trees (the
  * stochastic-rounding engine) is restored afterwards; the trial trees replace the "last tree"
@@ -242,8 +244,9 @@ int bk_learner_set_launch_shape(bk_learner* learner, const int32_t* shape);
 int bk_learner_reset_constant_hessian(bk_learner* learner, int32_t value);
 
 /* Threads per split-search CTA (one CTA per leaf side and feature) of the learner's next train call
- * (GB300-only): 64 when every feature is numerical with at most 63 searched bins and the grow
- * loop runs the single-pass form without L1 / max_delta_step / path_smooth, else 256. */
+ * (GB300-only) where it searches with a CTA per feature: 64 when every feature is numerical with at
+ * most 63 searched bins and the grow loop runs the single-pass form without L1 / max_delta_step /
+ * path_smooth, else 256. Large quantized rounds search eight features per 256-thread CTA. */
 int bk_learner_search_threads(bk_learner* learner, int32_t* threads);
 
 /* Replaces SerialTreeLearner::histogram_cache_capacity (serial.rs:250-252): the histogram slots
@@ -262,7 +265,8 @@ int bk_learner_reset_histogram_pool_config(bk_learner* learner);
  * and the histogram kernels' time (ms), plus the algorithmic bytes the histogram kernels moved. */
 int bk_learner_last_timing(bk_learner* learner, double* total_ms, double* hist_ms, double* hist_bytes);
 
-/* With timing on: the split-search and partition phases of the last train call (ms). */
+/* With timing on (trees then grow one split at a time): the split-search and partition phases of the
+ * last train call (ms). */
 int bk_learner_last_phase_timing(bk_learner* learner, double* search_ms, double* partition_ms);
 
 /* With timing on: the phases of every grow-loop step of the last train call, out[3 * i + k] (ms)
