@@ -29,7 +29,7 @@ namespace {
 // The gradients end as fp32, so they are computed as fp32 pairs and, where a pair's error could move
 // the rounding, in f64 (bk_pair.cuh): the same fp32 numbers without the f64 pipe. `rel` is the bound on
 // a pair's relative error, plus what the f64 evaluation itself rounds away. Measured, 10M rows: L2 60
-// -> 48 us (HBM), binary 637 -> 89 us; softmax of ten classes on 2M rows 1277 -> 282 us (issue).
+// -> 48 us (HBM), binary 637 -> 89 us; softmax of ten classes on 2M rows 1277 -> 262 us (issue).
 __host__ __device__ constexpr float kTwo(int e) { return e >= 0 ? (float)(1ull << e) : 1.0f / (float)(1ull << -e); }
 
 __global__ void __launch_bounds__(256) k_grad_l2(const double* __restrict__ score, const float* __restrict__ label,
@@ -181,24 +181,31 @@ __global__ void __launch_bounds__(kSoftmaxThreads)
       mine[k * kSoftmaxThreads] = make_float2(x.hi, x.lo);
       if (x.hi > top.hi || (x.hi == top.hi && x.lo > top.lo)) top = x;
     }
+    // two classes at a time: the chains of a class alone leave the schedulers idle
     Pair sum{0.f, 0.f}, others{0.f, 0.f};
     top = pair_neg(top);
-    for (int k = 0; ok && k < K; ++k) {
+#pragma unroll 2
+    for (int k = 0; k < K; ++k) {
       const float2 x = mine[k * kSoftmaxThreads];
-      const Pair z = pair_add(Pair{x.x, x.y}, top);
-      ok = z.hi >= -60.0f;
-      const Pair e = ok ? pair_exp(z, st) : Pair{0.f, 0.f};
+      Pair z = pair_add(Pair{x.x, x.y}, top);
+      if (!(z.hi >= -60.0f)) {
+        ok = false;
+        z = Pair{0.f, 0.f};
+      }
+      const Pair e = pair_exp(z, st);
       sum = pair_add(sum, e);
       if (k != lab) others = pair_add(others, e);
       mine[k * kSoftmaxThreads] = make_float2(e.hi, e.lo);
     }
     const Pair wi{w ? w[i] : 1.0f, 0.f};
-    for (int k = 0; ok && k < K; ++k) {
+    const Pair per = pair_div(Pair{1.f, 0.f}, sum);
+#pragma unroll 2
+    for (int k = 0; k < K; ++k) {
       const float2 x = mine[k * kSoftmaxThreads];
       const Pair e{x.x, x.y};
-      const Pair p = pair_div(e, sum);
+      const Pair p = pair_mul(e, per);
       const Pair rest = k == lab ? others : pair_add(sum, pair_neg(e));
-      const Pair np = pair_div(rest, sum);  // 1 - p
+      const Pair np = pair_mul(rest, per);  // 1 - p
       const float inv = __fdividef(1.0f, np.hi);
       Pair gp = k == lab ? np : p, hp = pair_mul(pair_mul(factor, p), np);
       const float rel_g = kTwo(-38) + (k == lab ? __fmul_rn(kTwo(-51), inv) : 0.f);
@@ -209,12 +216,9 @@ __global__ void __launch_bounds__(kSoftmaxThreads)
       }
       float gv, hv;
       const bool a = pair_round(gp, rel_g, &gv), b = pair_round(hp, rel_h, &hv);
-      ok = a && b;
-      if (k == lab) gv = -gv;
-      if (ok) {
-        g[(size_t)k * n + i] = gv;
-        h[(size_t)k * n + i] = hv;
-      }
+      ok = ok && a && b;
+      g[(size_t)k * n + i] = k == lab ? -gv : gv;
+      h[(size_t)k * n + i] = hv;
     }
     if (!ok) softmax_row(score, n, i, K, lab, w, g, h);
   }
