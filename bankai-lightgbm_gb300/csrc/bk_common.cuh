@@ -318,6 +318,7 @@ void launch_zero_pool(void* pool, size_t bytes_per_job, size_t bytes, int num_jo
 // need_stop: only finished jobs' rows
 void launch_row_leaf(const Job* d_jobs, int num_jobs, const Params& p, int32_t* out, int need_stop, cudaStream_t s);
 void launch_mt_seed(const Job* d_jobs, int num_jobs, uint32_t seed, cudaStream_t s);
+constexpr int kFloatRootGrid = 256;  // CTAs of the float path's root sums (their number is part of the sum's order)
 constexpr int kRootGrid = 1216;  // CTAs of the root sums and the discretization: eight per SM
 
 // bk_renew.cu

@@ -104,7 +104,7 @@ __device__ __forceinline__ void compute_leaf_const_ls(const Job& J, const Params
     const double d = p.l2 == 0.0 ? p.min_gain : c.mgs - s0;
     c.hs2 = (float)h2;
     c.r2 = p.quant ? 0.0 : c.sum_g / h2;
-    const float ymin = (float)(p.min_hess + p.l2), s0f = (float)s0, arel = 4e-15f + 1.01e-15f / ymin;
+    const float ymin = (float)(p.min_hess + p.l2), s0f = (float)s0, arel = (p.quant ? 4e-15f : 4e-14f) + 1.01e-15f / ymin;  // float: its sums round too
     c.bk1 = 44.0f * 5.9604645e-08f + arel;
     c.bk0 = s0f * arel + 1e-24f;
     if (!(ymin >= 1e-6f) || !(c.hs2 <= 1e10f) || !(s0f < 1e30f) ||

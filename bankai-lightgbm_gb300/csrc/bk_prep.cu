@@ -278,18 +278,37 @@ __global__ void __launch_bounds__(256) k_root_partial(const Job* __restrict__ jo
     hi = max(hi, a);
     if (a) lo = min(lo, a);
   };
-  for (int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; k < cnt; k += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t i = bagged ? J.idx0[k] : k;
-    if (p.quant) {
-      int32_t pk = J.packed[i];
+  const int64_t step = (int64_t)gridDim.x * blockDim.x;
+  int64_t k = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (p.quant) {
+    for (; k < cnt; k += step) {
+      int32_t pk = J.packed[bagged ? J.idx0[k] : k];
       ig += (int8_t)(pk >> 8);
       ih += pk & 0xff;
-    } else {
-      const float g = J.g[i], h = J.h[i];
-      sg += (double)g;
-      sh += (double)h;
-      range(g, max_g, min_g);
-      range(h, max_h, min_h);
+    }
+  } else {
+    // four rows' values on their way at a time, added in order
+    for (; k < cnt; k += 4 * step) {
+      float g[4], h[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int64_t at = k + u * step;
+        g[u] = h[u] = 0.f;
+        if (at < cnt) {
+          const int64_t i = bagged ? J.idx0[at] : at;
+          g[u] = J.g[i];
+          h[u] = J.h[i];
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (k + u * step < cnt) {
+          sg += (double)g[u];
+          sh += (double)h[u];
+        }
+        range(g[u], max_g, min_g);
+        range(h[u], max_h, min_h);
+      }
     }
   }
 #pragma unroll
@@ -338,8 +357,8 @@ __global__ void __launch_bounds__(256) k_root_partial(const Job* __restrict__ jo
   }
 }
 
-// One warp: the partials, lane l taking CTAs l, l + 32, ... and a tree over the lanes (one lane over
-// all of them took 45 us: a chain of f64 additions).
+// One warp: the partials, on the quantized path lane l taking CTAs l, l + 32, ... and a tree over the
+// lanes (one lane over all of them took 45 us).
 __global__ void __launch_bounds__(32) k_root_finish(const Job* __restrict__ jobs, Params p, int exact_quant_root) {
   const Job& J = jobs[blockIdx.z];
   JobState* s = J.st;
@@ -359,17 +378,28 @@ __global__ void __launch_bounds__(32) k_root_finish(const Job* __restrict__ jobs
       ih += __shfl_xor_sync(FULL, ih, o);
     }
   } else {
-#pragma unroll 4
-    for (int b = 0; b < kRootGrid; b += 32) {
-      sg += J.red[2 * (b + lane)];
-      sh += J.red[2 * (b + lane) + 1];
-      ig = join_range(b ? ig : J.ired[2 * lane], J.ired[2 * (b + lane)]);
-      ih = join_range(b ? ih : J.ired[2 * lane + 1], J.ired[2 * (b + lane) + 1]);
+    // CTA after CTA, as a column whose most frequent bin holds no rows (the bin of zero) gets this sum's
+    // rounding for that bin, which decides between the two equal thresholds around it: the order is part
+    // of the result. Even lanes add the gradients, odd lanes the hessians.
+    double pg[kFloatRootGrid / 32], ph[kFloatRootGrid / 32], sum = 0.0;
+#pragma unroll
+    for (int r = 0; r < kFloatRootGrid / 32; ++r) {
+      pg[r] = J.red[2 * (32 * r + lane)];
+      ph[r] = J.red[2 * (32 * r + lane) + 1];
+      ig = join_range(r ? ig : J.ired[2 * lane], J.ired[2 * (32 * r + lane)]);
+      ih = join_range(r ? ih : J.ired[2 * lane + 1], J.ired[2 * (32 * r + lane) + 1]);
     }
 #pragma unroll
+    for (int r = 0; r < kFloatRootGrid / 32; ++r)
+#pragma unroll 4
+      for (int l = 0; l < 32; ++l) {
+        const double a = __shfl_sync(FULL, pg[r], l), b = __shfl_sync(FULL, ph[r], l);
+        sum += (lane & 1) ? b : a;
+      }
+    sg = __shfl_sync(FULL, sum, 0);
+    sh = __shfl_sync(FULL, sum, 1);
+#pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
-      sg += __shfl_xor_sync(FULL, sg, o);
-      sh += __shfl_xor_sync(FULL, sh, o);
       ig = join_range(ig, __shfl_xor_sync(FULL, ig, o));
       ih = join_range(ih, __shfl_xor_sync(FULL, ih, o));
     }
@@ -549,7 +579,7 @@ void launch_discretize(const Job* d_jobs, int num_jobs, const Params& p, const d
 }
 
 void launch_root_sums(const Job* d_jobs, int num_jobs, const Params& p, int exact_quant_root, cudaStream_t s) {
-  k_root_partial<<<dim3(kRootGrid, 1, num_jobs), 256, 0, s>>>(d_jobs, p);
+  k_root_partial<<<dim3(p.quant ? kRootGrid : kFloatRootGrid, 1, num_jobs), 256, 0, s>>>(d_jobs, p);
   k_root_finish<<<dim3(1, 1, num_jobs), 32, 0, s>>>(d_jobs, p, exact_quant_root);
 }
 

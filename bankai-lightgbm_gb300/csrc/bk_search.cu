@@ -222,9 +222,7 @@ struct SearchSmemT {
   int32_t wc[3][NW];
   WarpFilt wf[2][NW];
   WarpFilt xf;  // the forward scan's position -1 (last thread)
-  // search_float_fixed: the warps' sums of gradients, hessians and counts, those that FixHistogram takes,
-  // the top bin's
-  Fixed fx[3][NW], ff[2][NW], top[3];
+  Fixed fx[3][NW], top[3];  // search_float_fixed: the warps' sums of gradients, hessians, counts; the top bin's
   int32_t spl[2][NW];
   DirBest wb[2][NW];
 };
@@ -966,13 +964,14 @@ __device__ __forceinline__ Filt filt_of_d(bool cand, const Approx& a, const Leaf
   return f;
 }
 
-// search_float for plain gains of a tree with fixed-point histograms (JobState::fix_ok): the same
-// candidate from exact sums. The bins' doubles are multiples of the tree's units, so one prefix scan of
-// 96-bit integers gives the sums of both directions (the reverse side is the total minus a prefix), the
-// validity tests compare integers, and only the queued positions' sums become doubles again. That leaves
-// two f64 instructions a bin for the larger child's difference, two for the count estimate and one a
-// threshold; with f64 scans, sums and fp32 conversions there were about 110 (32 leaves x 100 features
-// of 255 bins: 100 -> 37 us a round).
+// search_float for plain gains of a tree with fixed-point histograms (JobState::fix_ok). The bins' doubles
+// are multiples of the tree's units, so one prefix scan of 96-bit integers gives the exact sums of both
+// directions (the reverse side is the total minus a prefix); the validity tests compare integers, and the
+// bounds come from them. The queued positions' gains are taken from f64 sums added in search_float's
+// order: around an empty bin whose sum is rounding (the most frequent bin of a column without zeros gets
+// the leaf's total minus the others) two thresholds are equal but for those roundings, and the choice
+// should not depend on the form of the search. That leaves about 45 f64 instructions a bin, where there were
+// about 110 (32 leaves x 100 features of 255 bins: 100 -> 45 us a round; 37 with exact sums throughout).
 template <int NW>
 __device__ void search_float_fixed(const Job& J, const Params& p, const SearchIn& si, const DevFeature& m, int side,
                                    int32_t f, int32_t leaf, SearchSmemT<NW>& sm) {
@@ -999,26 +998,20 @@ __device__ void search_float_fixed(const Job& J, const Params& p, const SearchIn
   if (t < 2) sm.qn[t] = 0;
   const double sum_g = C.sum_g, sum_h = C.sum_h;
   if (fix) {  // FixHistogram: the smaller leaf's most frequent bin is its total minus every other bin
-    Fixed a = double_to_fixed(sv.x, K.g_exp), b = double_to_fixed(sv.y, K.h_exp);
-#pragma unroll 1
-    for (int o = 16; o > 0; o >>= 1) {
-      a = a + shfl_xor_fixed(a, o);
-      b = b + shfl_xor_fixed(b, o);
-    }
+    const double ag = warp_sum(sv.x), ah = warp_sum(sv.y);
     if (lane == 0) {
-      sm.ff[0][warp] = a;
-      sm.ff[1][warp] = b;
+      sm.wd[0][warp] = ag;
+      sm.wd[1][warp] = ah;
     }
     __syncthreads();
     if (t == m.mfb) {
-      a = double_to_fixed(S0.sg, K.g_exp);
-      b = double_to_fixed(S0.sh, K.h_exp);
+      double a = 0.0, b = 0.0;
 #pragma unroll 1
       for (int i = 0; i < NW; ++i) {
-        a = a - sm.ff[0][i];
-        b = b - sm.ff[1][i];
+        a += sm.wd[0][i];
+        b += sm.wd[1][i];
       }
-      sv = make_double2(fixed_to_double(a.lo, a.mid, a.hi, K.g_exp), fixed_to_double(b.lo, b.mid, b.hi, K.h_exp));
+      sv = make_double2(S0.sg - a, S0.sh - b);
       if (side == 0) hs[(size_t)(t + 1) * TILE] = sv;
     }
   }
@@ -1042,6 +1035,29 @@ __device__ void search_float_fixed(const Job& J, const Params& p, const SearchIn
       ph = ph + b;
       pc += c;
     }
+  }
+  // the f64 sums that a queued position's gain is taken from, as search_float adds them
+  double qg[2] = {acc ? v.x : 0.0, 0.0}, qh[2] = {acc ? v.y : 0.0, 0.0};
+  if (G.two) {  // uniform
+    qg[1] = warp_incl_scan(skip_t ? 0.0 : v.x, lane);
+    qh[1] = warp_incl_scan(skip_t ? 0.0 : v.y, lane);
+    if (lane == 31) {
+      sm.wd[2][warp] = qg[1];
+      sm.wd[3][warp] = qh[1];
+    }
+    if (G.fwd_rest) {
+      const double ug = warp_sum(v.x), uh = warp_sum(v.y);
+      if (lane == 0) {
+        sm.wd[6][warp] = ug;
+        sm.wd[7][warp] = uh;
+      }
+    }
+  }
+  qg[0] = warp_incl_scan_down(qg[0], lane);
+  qh[0] = warp_incl_scan_down(qh[0], lane);
+  if (lane == 0) {
+    sm.wd[4][warp] = qg[0];
+    sm.wd[5][warp] = qh[0];
   }
   if (lane == 31) {
     sm.fx[0][warp] = pg;
@@ -1137,10 +1153,38 @@ __device__ void search_float_fixed(const Job& J, const Params& p, const SearchIn
   for (int d = 0; d < 2; ++d) {
     const bool exact = valid[d] && !rep[d] && (fl[d].unc || (fl[d].mp && fl[d].up >= M[d]));
     QEnt e{0, 0, 0, 0, 0};
-    if (exact) {  // the accumulated side (reverse: right, forward: left) in doubles
-      const Fixed ag = d == 0 ? rg : fg, ah = d == 0 ? rh : fh;
-      e.a = __double_as_longlong(fixed_to_double(ag.lo, ag.mid, ag.hi, K.g_exp));
-      e.b = __double_as_longlong(BK_EPS + fixed_to_double(ah.lo, ah.mid, ah.hi, K.h_exp));
+    if (exact) {  // the accumulated side (reverse: right, forward: left): the other warps' part
+      double ag = 0.0, ah = 0.0;
+      if (d == 0) {
+#pragma unroll 1
+        for (int i = NW - 1; i > warp; --i) {
+          ag += sm.wd[4][i];
+          ah += sm.wd[5][i];
+        }
+        ag = qg[0] + ag;
+        ah = BK_EPS + (qh[0] + ah);
+      } else {
+#pragma unroll 1
+        for (int i = 0; i < warp; ++i) {
+          ag += sm.wd[2][i];
+          ah += sm.wd[3][i];
+        }
+        double bg = 0.0, bhd = BK_EPS;
+        if (G.fwd_rest) {
+          double ug = 0.0, uh = 0.0;
+#pragma unroll 1
+          for (int i = 0; i < NW; ++i) {
+            ug += sm.wd[6][i];
+            uh += sm.wd[7][i];
+          }
+          bg = sum_g - ug;
+          bhd = (sum_h - BK_EPS) - uh;
+        }
+        ag = xpos ? bg : bg + (qg[1] + ag);
+        ah = xpos ? bhd : bhd + (qh[1] + ah);
+      }
+      e.a = __double_as_longlong(ag);
+      e.b = __double_as_longlong(ah);
       e.c = d == 0 ? rc : fc;
       e.t = (int16_t)(d == 0 || !xpos ? t : -1);
       e.d = (int16_t)d;
@@ -2115,8 +2159,8 @@ int rounds_groups(const Params& p) {
 }
 
 // The float search's registers allow three CTAs per SM. From two waves of those on, four with some spilled
-// are faster: the rounds of 255 leaves x 100 features (3200 CTAs) 50 -> 37 us, of 63 leaves x 28
-// features (448 CTAs) 8 -> 11 us.
+// are faster (before the f64 sums of the queued positions: rounds of 255 leaves x 100 features, 3200 CTAs, 50 -> 37 us, of 31 leaves x 28
+// features, 224 CTAs, 8 -> 11 us).
 constexpr int64_t kManySearches = 2 * 3 * 152;
 
 void launch_search_round(const Job* h_jobs, int num_jobs, const Params& p, const DevFeature* feats, int q,
