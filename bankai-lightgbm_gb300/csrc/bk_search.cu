@@ -2158,9 +2158,9 @@ int rounds_groups(const Params& p) {
   return (p.n_numeric + kWarpFeatures - 1) / kWarpFeatures + (p.F - p.n_numeric);
 }
 
-// The float search's registers allow three CTAs per SM. From two waves of those on, four with some spilled
-// are faster (before the f64 sums of the queued positions: rounds of 255 leaves x 100 features, 3200 CTAs, 50 -> 37 us, of 31 leaves x 28
-// features, 224 CTAs, 8 -> 11 us).
+// The float search's registers allow two CTAs per SM. From 912 CTAs on, four with some spilled are faster
+// (before the f64 sums of the queued positions: rounds of 255 leaves x 100 features, 3200 CTAs, 50 -> 37
+// us; of 31 leaves x 28 features, 224 CTAs, 8 -> 11 us).
 constexpr int64_t kManySearches = 2 * 3 * 152;
 
 void launch_search_round(const Job* h_jobs, int num_jobs, const Params& p, const DevFeature* feats, int q,
