@@ -146,10 +146,6 @@ __device__ __forceinline__ Fixed shfl_up_fixed(const Fixed& x, int o, int width)
   return Fixed{__shfl_up_sync(0xffffffffu, x.lo, o, width), __shfl_up_sync(0xffffffffu, x.mid, o, width),
                __shfl_up_sync(0xffffffffu, x.hi, o, width)};
 }
-__device__ __forceinline__ Fixed shfl_xor_fixed(const Fixed& x, int o) {
-  return Fixed{__shfl_xor_sync(0xffffffffu, x.lo, o), __shfl_xor_sync(0xffffffffu, x.mid, o),
-               __shfl_xor_sync(0xffffffffu, x.hi, o)};
-}
 
 }  // namespace
 
