@@ -86,7 +86,7 @@ __global__ void __launch_bounds__(256) k_grad_binary(const double* __restrict__ 
     const double s = score[i];
     const bool pos = label[i] > 0.0f;
     bool ok;
-    Pair z = pair_of(one ? s : sigmoid * s, &ok);
+    Pair z = pair_of<true>(one ? s : sigmoid * s, &ok);  // exp(z) and 1 + exp(z): absolute errors count
     if (!pos) z = pair_neg(z);
     ok = ok && ok_c && fabsf(z.hi) <= 60.0f;
     float gv = 0.f, hv = 0.f;
@@ -171,12 +171,13 @@ __global__ void __launch_bounds__(kSoftmaxThreads)
   float2* mine = s_e + threadIdx.x;
   for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     const int lab = class_of(label[i], K, bad_label);
-    // the scores as pairs; their maximum (pairs compare like the scores up to 2^-53, which the bound allows)
+    // the scores as pairs, whose differences' absolute errors count; their maximum (pairs compare like the
+    // scores up to 2^-53, which the bound allows)
     bool ok = ok_f;
     Pair top{-CUDART_INF_F, 0.f};
     for (int k = 0; k < K; ++k) {
       bool o;
-      const Pair x = pair_of(score[(size_t)k * n + i], &o);
+      const Pair x = pair_of<true>(score[(size_t)k * n + i], &o);
       ok = ok && o && fabsf(x.hi) <= 64.0f;
       mine[k * kSoftmaxThreads] = make_float2(x.hi, x.lo);
       if (x.hi > top.hi || (x.hi == top.hi && x.lo > top.lo)) top = x;

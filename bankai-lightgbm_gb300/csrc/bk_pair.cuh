@@ -42,12 +42,14 @@ __device__ __forceinline__ Pair pair_div(Pair a, Pair b) {  // relative error at
 __device__ __forceinline__ Pair pair_neg(Pair a) { return Pair{-a.hi, -a.lo}; }
 
 // An f64 value as a pair, by integer operations: the high 24 bits of its significand, then the other
-// 29 rounded to 24 (error 2^-53 of the value). Magnitudes below 2^-60 become 0; ok = false above 2^60
-// and for NaN.
+// 29 rounded to 24 (error 2^-53 of the value). ok = false above 2^60 and for NaN, and for magnitudes
+// below 2^-60 but zero, whose parts an fp32 pair cannot hold. ABSOLUTE: the caller needs an error below
+// 2^-60 only, not one relative to the value, so those become 0 with ok true.
+template <bool ABSOLUTE = false>
 __device__ __forceinline__ Pair pair_of(double x, bool* ok) {
   const uint32_t h = (uint32_t)__double2hiint(x), l = (uint32_t)__double2loint(x);
   const int e = (int)((h >> 20) & 0x7ffu) - 1023;
-  *ok = e < 60;
+  *ok = e < 60 && (ABSOLUTE || e >= -60 || ((h << 1) | l) == 0u);
   if (e < -60 || e >= 60) return Pair{0.f, 0.f};
   const uint32_t sign = h & 0x80000000u;
   const float hi = __uint_as_float(sign | ((uint32_t)(e + 127) << 23) | ((h & 0xfffffu) << 3) | (l >> 29));
