@@ -109,7 +109,7 @@ __global__ void __launch_bounds__(256) k_grad_binary(const double* __restrict__ 
         q = pair_mul(q, wi);
       }
       const bool a = pair_round(r, kTwo(-40), &gv), b = pair_round(q, rel_h, &hv);
-      ok = a && b;
+      ok = (a && b) || (w && w[i] == 0.f);  // a row of no weight: zeros
       if (pos) gv = -gv;
     }
     if (!ok) {
@@ -217,7 +217,7 @@ __global__ void __launch_bounds__(kSoftmaxThreads)
       }
       float gv, hv;
       const bool a = pair_round(gp, rel_g, &gv), b = pair_round(hp, rel_h, &hv);
-      ok = ok && a && b;
+      ok = ok && ((a && b) || wi.hi == 0.f);  // a row of no weight: zeros
       g[(size_t)k * n + i] = k == lab ? -gv : gv;
       h[(size_t)k * n + i] = hv;
     }

@@ -91,12 +91,14 @@ __device__ __forceinline__ Pair pair_exp(Pair z, const ExpTable& T) {
   return Pair{__fmul_rn(e.hi, s), __fmul_rn(e.lo, s)};
 }
 
-// Rounds a (normalized) pair to fp32: false when a relative error `rel` of it could change the result.
+// Rounds a (normalized) pair to fp32: false when a relative error `rel` of it could change the result,
+// or when the pair is so small that its low part, or the result itself, is not held in full.
 __device__ __forceinline__ bool pair_round(Pair a, float rel, float* out) {
   *out = a.hi;
-  if (a.lo == 0.f && rel < 1e-9f) return true;
   const uint32_t b = __float_as_uint(a.hi) & 0x7fffffffu;
-  if (b < (40u << 23) || b >= (250u << 23) || (b & 0x7fffffu) == 0u) return false;  // tiny, huge, a power of two
+  if (b < (40u << 23) || b >= (250u << 23)) return false;  // tiny (zero too), huge
+  if (a.lo == 0.f && rel < 1e-9f) return true;
+  if ((b & 0x7fffffu) == 0u) return false;  // a power of two
   const float half = __uint_as_float((b & 0x7f800000u) - (24u << 23));  // half a unit in the last place
   return fabsf(__fsub_rn(half, fabsf(a.lo))) > __fmul_rn(rel, fabsf(a.hi));
 }

@@ -65,3 +65,35 @@ def test_binary_gradients_of_small_values(sigmoid, lw, scale):
     ar = resp.abs()
     _equal(g, (resp * lwr).float())
     _equal(h, ((ar * (sigmoid - ar)) * lwr).float())
+
+
+@pytest.mark.parametrize("K", [1, 3])
+@pytest.mark.parametrize("scale", [1.0, 1e-25, 1e-36, 1e-38, 1e-41])
+def test_gradients_of_small_row_weights(K, scale):
+    """Products down to the subnormal fp32 numbers, and rows of no weight."""
+    import torch
+    n = 100003
+    L = _learner(n, K)
+    rng = np.random.default_rng(7)
+    s = torch.from_numpy(rng.standard_normal((K, n)) * 4.0).cuda()
+    label = torch.from_numpy(rng.integers(0, max(K, 2), n)).float().cuda()
+    w = (torch.rand(n, device="cuda") + 0.5) * scale
+    w[::7] = 0.0
+    L.set_objective_weights(w.data_ptr())
+    torch.cuda.synchronize()
+    wd = w.double()
+    if K == 1:
+        g, h = _gradients(L, 1, s, label)
+        lab = torch.where(label > 0, 1.0, -1.0).double()
+        resp = -lab / (1.0 + torch.exp(lab * s[0]))
+        ar = resp.abs()
+        _equal(g, (resp * wd).float())
+        _equal(h, ((ar * (1.0 - ar)) * wd).float())
+        return
+    g, h = (x.view(K, n) for x in _gradients(L, 2, s, label))
+    rec = torch.exp(s - s.max(0).values)
+    wsum = rec[0] + rec[1] + rec[2]
+    for k in range(K):
+        p = rec[k] / wsum
+        _equal(g[k], (torch.where(label == k, p - 1.0, p) * wd).float())
+        _equal(h[k], ((K / (K - 1.0) * p) * (1.0 - p) * wd).float())
