@@ -321,7 +321,8 @@ __device__ __forceinline__ void add_own_row(const IntHist<WIDE>& H, const RoundL
 }
 
 // Folds the hot counters into the cold ones and clears them. Every thread of the CTA calls it
-// between barriers.
+// between barriers. A leaf's hessians fit 32 unsigned bits (checked when the learner is created), so the
+// cold hessian counters are read as such.
 __device__ __forceinline__ void fold_hot(const IntHist<false>& H, int shift) {
   uint4* row4 = reinterpret_cast<uint4*>(H.base);   // 16 per bin: 8 hot, then 8 cold gradient
   int4* h4 = reinterpret_cast<int4*>(H.cold_h());  // 8 per bin
@@ -472,7 +473,7 @@ __device__ __forceinline__ void hist_int_rows(const Job& J, const Params& p, con
       hh += __shfl_xor_sync(0xffffffffu, hh, o);
     }
     if ((gg | hh) && col < nf) {
-      int64_t pk = (int64_t)gg * 4294967296LL + (int64_t)hh;
+      int64_t pk = (int64_t)gg * 4294967296LL + (int64_t)(uint32_t)hh;
       atomicAdd(slot + e, (unsigned long long)pk);
     }
   }
@@ -517,7 +518,7 @@ __device__ __forceinline__ void hist_cluster_flush(const Params& p, const TileGe
     for (int k = 0; k < 4; ++k) {
       const int f = (4 * (e & 7) + k) & (steps - 1);  // a column holds a copy of feature column mod steps
       if ((gg[k] | hh[k]) && f < nf)
-        atomicAdd(slot + (e >> 3) * TILE + f, (unsigned long long)((int64_t)gg[k] * 4294967296LL + (int64_t)hh[k]));
+        atomicAdd(slot + (e >> 3) * TILE + f, (unsigned long long)((int64_t)gg[k] * 4294967296LL + (int64_t)(uint32_t)hh[k]));
     }
   }
   cluster_sync_all();
