@@ -1,7 +1,10 @@
-"""Integer histograms at the end of their counters: a histogram CTA whose hessian sum needs all 32 bits.
+"""Integer histograms at the ends of their counters: the wide form with every bin of a tile in use,
+and a histogram CTA whose hessian sum needs all 32 bits.
 """
 import numpy as np
 import pytest
+
+from test_gpu_hist_tiles import _learner
 
 pytestmark = pytest.mark.gpu
 
@@ -11,6 +14,22 @@ def _gpu():
     import torch
     if not torch.cuda.is_available():
         pytest.skip("no CUDA device")
+
+
+@pytest.mark.parametrize("F", [1, 5, 9, 17, 33, 49])
+def test_wide_counters_of_255_bins_match_oracle(F):
+    """127 gradient levels fill a packed counter in 511 rows, fewer than a round of the CTA's."""
+    import harness
+    n = 20000 + F
+    ds, L, g, h = _learner(n, F, 255, 127, K=2, leaves=7)
+    tree = L.train_raw(g, h)
+    for j in range(2):
+        rec, values = harness.OracleLearner(ds, L.cfg).train(g[j], h[j])[:2]
+        k = int(tree[3][j])
+        assert k == len(rec) + 1 and np.any(tree[0][j, 0]["left_int_sum"] != 0)
+        for name in ("leaf", "inner_feature", "threshold", "left_count", "left_int_sum", "gain"):
+            assert np.array_equal(tree[0][j, :k - 1][name], rec[name]), name
+        assert np.array_equal(tree[1][j, :k], values)
 
 
 @pytest.mark.parametrize("loop_mode", [1, 0])
