@@ -130,6 +130,7 @@ struct LeafConst {
   // and constant (bk1 < 0: the leaf is outside its range), min_gain_shift - s0 rounded up / down
   float hs2, bk1, bk0, d_up, d_dn;
   double r2;               // float path: g / (h + 2 lambda_l2)
+  float off_g, off_h;      // float path: bounds on the f64 sums' errors (search_float_fixed)
   int32_t go;              // 0: the leaf is not searched (grow rounds: 1 the left child, 2 the right child)
   double gs, hs;           // quantized path: the gradient / hessian scales
   LeafSum ls;              // the leaf's sums (its LeafSplits), as leaf_sum[leaf] holds them

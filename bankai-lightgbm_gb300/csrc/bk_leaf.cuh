@@ -104,7 +104,15 @@ __device__ __forceinline__ void compute_leaf_const_ls(const Job& J, const Params
     const double d = p.l2 == 0.0 ? p.min_gain : c.mgs - s0;
     c.hs2 = (float)h2;
     c.r2 = p.quant ? 0.0 : c.sum_g / h2;
-    const float ymin = (float)(p.min_hess + p.l2), s0f = (float)s0, arel = (p.quant ? 4e-15f : 4e-14f) + 1.01e-15f / ymin;  // float: its sums round too
+    const float ymin = (float)(p.min_hess + p.l2), s0f = (float)s0, arel = (p.quant ? 4e-15f : 4e-14f) + 1.01e-15f / ymin;
+    // what the f64 sums of a side can be off by: 32 additions of partial sums up to the rows' total magnitude,
+    // at most their number times the largest one's bound, the power of two above it; doubled
+    c.off_g = c.off_h = 0.f;
+    if (!p.quant) {
+      const double rows = (double)ls.num_data * 7.1054273576010019e-15;  // 2^-47
+      c.off_g = __double2float_ru(rows * __longlong_as_double((long long)(st->red_maxg + 897u) << 52));
+      c.off_h = __double2float_ru(rows * __longlong_as_double((long long)(st->red_maxh + 897u) << 52));
+    }
     c.bk1 = 44.0f * 5.9604645e-08f + arel;
     c.bk0 = s0f * arel + 1e-24f;
     if (!(ymin >= 1e-6f) || !(c.hs2 <= 1e10f) || !(s0f < 1e30f) ||

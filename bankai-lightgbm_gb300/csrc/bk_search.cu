@@ -935,7 +935,11 @@ __device__ void search_float(const Job& J, const Params& p, const SearchIn& si, 
 // threshold. With H2 = h + 2 l2 and yl, yr = hl + l2, hr + l2, d = t^2 H2 / (yl yr) where
 // t = gl - (g / H2) yl, the left gradients centred on the leaf's mean: one f64 multiply-add keeps what
 // cancels. Its f64 error is below 2^-50 (|gl| + |g / H2| yl); the fp32 rest, truncations of 2^-23
-// included, errs less than the 44 u of LeafConst::bk1.
+// included, errs less than the 44 u of LeafConst::bk1. The gain itself is taken from f64 sums, which
+// round: by up to off_g, off_h (LeafConst), whatever the sums come to, so where large bins of both signs
+// cancel that is far more than 2^-50 of them. One side's sum is the leaf's minus the other's, so t moves
+// by at most off_g + |g / H2| off_h, and 1 / (yl yr) by a factor of up to 1 + 2 (off_h / yl + off_h / yr)
+// = 1 + 2 off_h q while off_h q <= 1/4.
 struct FloatLeaf {
   float r2f;  // g / H2
   int g_exp, h_exp;
@@ -948,11 +952,13 @@ __device__ __forceinline__ Approx bound_float(const Params& p, const Fixed& gl, 
   const float t = double_to_float(fma(-C.r2, yl, g)), ylf = double_to_float(yl);
   const float yrf = __fadd_rn(fixed_to_float(hr, K.h_exp), C.l2f);
   const float q = __fdividef(C.hs2, __fmul_rn(ylf, yrf));
-  const float off = __fmul_rn(fmaf(fabsf(K.r2f), ylf, fabsf(double_to_float(g))), 1.7763568e-15f);  // 2^-49
+  const float hq = __fmul_rn(C.off_h, q);
+  float off = __fmul_rn(fmaf(fabsf(K.r2f), ylf, fabsf(double_to_float(g))), 1.7763568e-15f);  // 2^-49
+  off = __fadd_rn(off, fmaf(fabsf(K.r2f), C.off_h, C.off_g));
   Approx a;
   a.g = __fmul_rn(__fmul_rn(t, t), q);
-  a.e = fmaf(__fmul_rn(off, fmaf(2.0f, fabsf(t), off)), q, fmaf(a.g, C.bk1, C.bk0));
-  a.uncertain = !(__fadd_rn(a.g, a.e) < 1e30f) || C.bk1 < 0.f;
+  a.e = fmaf(__fmul_rn(off, fmaf(2.0f, fabsf(t), off)), q, fmaf(a.g, fmaf(2.0f, hq, C.bk1), C.bk0));
+  a.uncertain = !(__fadd_rn(a.g, a.e) < 1e30f) || C.bk1 < 0.f || !(hq <= 0.25f);
   return a;
 }
 __device__ __forceinline__ Filt filt_of_d(bool cand, const Approx& a, const LeafConst& C) {
