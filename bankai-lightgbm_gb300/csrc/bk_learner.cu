@@ -261,6 +261,7 @@ struct bk_learner {
   }
 
   int spare_rounds = 0;  // rounds captured beyond first_rounds()
+  bool one_split = false;  // the graph form grows one split at a time (the autotuner, for a learner in the plain form)
   bool capturing = false;
   void record_hist_event(int i) {
     if (!timing || (size_t)i >= hist_events.size()) return;
@@ -296,7 +297,7 @@ struct bk_learner {
   // by-node sampler's stream, per-split phase timing) or by one leaf at a
   // time (thread-block clusters over a leaf's histogram CTAs), or the leaves do not fit the decision.
   bool rounds() const {
-    return loop_mode == 1 && !timing && !p.bynode && hl.cluster == 1 && p.max_exp > 0;
+    return loop_mode == 1 && !one_split && !timing && !p.bynode && hl.cluster == 1 && p.max_exp > 0;
   }
   // Rounds captured with the tree: doubling up to round_w leaves, then round_w splits a round, and a
   // few more for the trees whose best leaves come one after the other; even, as the rounds' two
@@ -938,14 +939,16 @@ int bk_learner_train(bk_learner* L, const float* gradients, const float* hessian
 namespace {
 
 // Autotuned launch shapes by shape class: (device, log2 rows, feature tiles, bins per feature
-// slot, quantized, num_leaves, jobs) -> (hist_min_rows, hist CTAs per tile, partition CTAs).
+// slot, quantized, num_leaves, jobs, grown in rounds) -> the shape. Rounds and single splits run
+// different kernels, so a shape of the one says nothing about the other.
 std::mutex g_tune_mutex;
-std::map<std::array<int, 7>, std::array<int, 5>> g_tune_cache;
+std::map<std::array<int, 8>, std::array<int, 5>> g_tune_cache;
 
-std::array<int, 7> tune_key(const bk_learner* L) {
+std::array<int, 8> tune_key(const bk_learner* L) {
   int lg = 0;
   while ((int64_t(1) << (lg + 1)) <= L->p.n) ++lg;
-  return {L->device, lg, L->p.T, L->p.B, L->p.quant, L->p.num_leaves, L->K};
+  const bool rounds = L->loop_mode == 1 && !L->timing && !L->p.bynode && L->p.max_exp > 0;
+  return {L->device, lg, L->p.T, L->p.B, L->p.quant, L->p.num_leaves, L->K, rounds ? 1 : 0};
 }
 
 }  // namespace
@@ -979,6 +982,7 @@ int bk_learner_autotune(bk_learner* L, const float* gradients, const float* hess
     if (gradients != L->d_g) CK(cudaMemcpyAsync(L->d_g, gradients, n * sizeof(float), kind, L->stream));
     if (hessians != L->d_h) CK(cudaMemcpyAsync(L->d_h, hessians, n * sizeof(float), kind, L->stream));
     L->loop_mode = 1;
+    L->one_split = saved_mode == 0;
     std::map<std::array<int, 5>, double> seen;
     // one tree per trial (graph form) after one untimed tree of each shape; the median device time
     auto measure = [&](const std::array<int, 5>& c) -> std::pair<std::array<int, 5>, double> {
@@ -1021,14 +1025,17 @@ int bk_learner_autotune(bk_learner* L, const float* gradients, const float* hess
     if (L->p.quant) {
       // the global-atomic variant of the quantized histogram for CTAs with few rows
       for (int dr : {128, 256, 512, 1024, 2048}) consider({best[0], best[1], best[2], dr, best[4]});
-      // clusters of a tile's CTAs that add up their histograms in distributed shared memory
-      for (int cl : {2, 4}) consider({best[0], best[1], best[2], best[3], cl});
+      // clusters of a tile's CTAs that add up their histograms in distributed shared memory: they make a
+      // learner grow one split at a time, so only where it can do nothing else
+      if (L->p.max_exp == 0)
+        for (int cl : {2, 4}) consider({best[0], best[1], best[2], best[3], cl});
     }
     CK(cudaMemcpyAsync(L->jobs[0].st, saved, state_bytes, cudaMemcpyDeviceToDevice, L->stream));
     CK(cudaFreeAsync(saved, L->stream));
     saved = nullptr;
     CK(cudaStreamSynchronize(L->stream));
     L->loop_mode = saved_mode;
+    L->one_split = false;
     L->set_launch_shape(best[0], best[1], best[2], best[3], best[4]);
     {
       std::lock_guard<std::mutex> g(g_tune_mutex);
@@ -1042,6 +1049,8 @@ int bk_learner_autotune(bk_learner* L, const float* gradients, const float* hess
       cudaStreamSynchronize(L->stream);
     }
     L->loop_mode = saved_mode;
+    L->one_split = false;
+    L->drop_graph();
     set_error("bk_learner_autotune: %s", e.msg.c_str());
     return -1;
   }

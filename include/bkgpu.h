@@ -217,11 +217,14 @@ int bk_learner_set_interaction_constraints(bk_learner* learner, const int32_t* f
  * the given gradients (as bk_learner_train takes them, all rows) over a coordinate descent of
  * five launch parameters — the fewest rows a histogram CTA takes, histogram CTAs per 32-feature
  * tile, partition CTAs, and (quantized) the most rows a histogram CTA adds straight to the pool
- * slot with global atomics instead of through a shared histogram, and the histogram CTAs of a tile
- * per thread-block cluster (1, 2 or 4; a cluster adds up its CTAs' shared histograms in distributed
- * shared memory before one flush, and makes the learner grow one split at a time) — and keeps the fastest. Choices are cached per shape class (device,
- * log2 rows, feature tiles, bins per feature, quantized, num_leaves, num_jobs): a later learner of
- * the same class takes the cached shape without timing. The learner's state across trees (the
+ * slot with global atomics instead of through a shared histogram, and (quantized, more than 512
+ * leaves) the histogram CTAs of a tile per thread-block cluster (1, 2 or 4; a cluster adds up its
+ * CTAs' shared histograms in distributed shared memory before one flush, and makes the learner grow
+ * one split at a time) — and keeps the fastest. The trees grow as the learner's own would: in
+ * rounds, or (loop mode 0, phase timing, by-node sampling, interaction constraints, more than 512
+ * leaves) one split at a time. Choices are cached per shape class (device, log2 rows, feature
+ * tiles, bins per feature, quantized, num_leaves, num_jobs, rounds or single splits): a later
+ * learner of the same class takes the cached shape without timing. The learner's state across trees (the
  * stochastic-rounding engine) is restored afterwards; the trial trees replace the "last tree"
  * outputs (bk_learner_row_leaf), so call it before the first bk_learner_train. shape_out (host,
  * 5 ints, may be NULL) receives the chosen shape. */
