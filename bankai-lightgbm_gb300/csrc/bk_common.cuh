@@ -180,7 +180,8 @@ struct Job {
   int64_t* leaf_count;
   int32_t* leaf_buf;
   int32_t* leaf_depth;
-  int32_t* leaf_slot;
+  int32_t* leaf_slot;  // [3][L] each leaf's pool slot; after grow rounds, the slot that holds the rest of its
+                       //        histogram (-1: none; bk_learner_leaf_histogram), and its node
   LeafSum* leaf_sum;
   double* bgain;       // [L]   gain of each leaf's best split (the arg-max reads these)
   int32_t* bfeat;      // [L]   real feature of each leaf's best split

@@ -673,9 +673,9 @@ int learner_create(const bk_feature* features, int32_t num_features, const uint8
     L->d_g = L->dalloc<float>(n * K);
     L->d_h = L->dalloc<float>(n * K);
     L->d_rows = L->dalloc<int32_t>(n);
-    // one histogram slot per leaf; in grow rounds one for the root and two for every expansion
+    // one histogram slot per leaf; in grow rounds one for the root and one for every expansion
     L->slot_bytes = (size_t)p.T * p.B * TILE * (quant ? sizeof(int64_t) : sizeof(double2));
-    L->pool_bytes_per_job = (size_t)std::max(Lv, 1 + 2 * p.max_exp) * L->slot_bytes;
+    L->pool_bytes_per_job = (size_t)std::max(Lv, 1 + p.max_exp) * L->slot_bytes;
     L->d_pool = L->dalloc<uint8_t>(L->pool_bytes_per_job * K);
     static_assert(sizeof(bk_split) % sizeof(double) == 0, "the leaf values follow the records");
     L->results_bytes = (sizeof(bk_split) + sizeof(double)) * (size_t)Lv * K + 16;
@@ -703,7 +703,7 @@ int learner_create(const bk_feature* features, int32_t num_features, const uint8
       J.leaf_count = L->dalloc<int64_t>(Lv);
       J.leaf_buf = L->dalloc<int32_t>(Lv);
       J.leaf_depth = L->dalloc<int32_t>(Lv);
-      J.leaf_slot = L->dalloc<int32_t>(Lv);
+      J.leaf_slot = L->dalloc<int32_t>(3 * (size_t)Lv);
       J.leaf_sum = L->dalloc<LeafSum>(Lv);
       J.bgain = L->dalloc<double>(Lv);
       J.bfeat = L->dalloc<int32_t>(Lv);
@@ -1869,24 +1869,48 @@ int bk_learner_leaf_histogram(bk_learner* L, int32_t job, int32_t leaf, void* ou
     // the slot [T][B][32]: tile f / 32, group bin b, lane f % 32
     const size_t cells = (size_t)p.T * p.B * TILE;
     const size_t elem = p.quant ? sizeof(int64_t) : sizeof(double2);
-    std::vector<unsigned char> raw(cells * elem);
+    std::vector<unsigned char> raw(cells * elem), more;
     CK(cudaMemcpyAsync(raw.data(), reinterpret_cast<const unsigned char*>(J.pool) + (size_t)slot * cells * elem,
                        cells * elem, cudaMemcpyDeviceToHost, L->stream));
+    // a leaf that grow rounds expanded but did not split: its larger child has its slot; the searched
+    // features' bins past the first get the smaller child's back
+    int32_t rest = -1, node = 0;
+    std::vector<uint8_t> split(p.F, 0);
+    CK(cudaMemcpyAsync(&rest, J.leaf_slot + p.num_leaves + leaf, sizeof(int32_t), cudaMemcpyDeviceToHost, L->stream));
+    CK(cudaMemcpyAsync(&node, J.leaf_slot + 2 * p.num_leaves + leaf, sizeof(int32_t), cudaMemcpyDeviceToHost, L->stream));
     CK(cudaStreamSynchronize(L->stream));
+    if (rest >= 0) {
+      more.resize(cells * elem);
+      CK(cudaMemcpyAsync(more.data(), reinterpret_cast<const unsigned char*>(J.pool) + (size_t)rest * cells * elem,
+                         cells * elem, cudaMemcpyDeviceToHost, L->stream));
+      CK(cudaMemcpyAsync(split.data(), J.splittable + (size_t)node * p.F, (size_t)p.F, cudaMemcpyDeviceToHost, L->stream));
+      CK(cudaStreamSynchronize(L->stream));
+    }
     size_t o = 0;
     for (int f = 0; f < p.F; ++f) {
       const DevFeature& d = L->h_feat[f];
       for (int b = 0; b < d.gbins; ++b, ++o) {
         const size_t c = ((size_t)(f / TILE) * p.B + b) * TILE + (f % TILE);
+        const bool both = rest >= 0 && split[f] && b > 0;
         if (p.quant) {
-          int64_t pk;
+          int64_t pk, other;
           std::memcpy(&pk, raw.data() + c * elem, sizeof(pk));
+          if (both) {
+            std::memcpy(&other, more.data() + c * elem, sizeof(other));
+            pk += other;
+          }
           const int64_t h = pk & 0xffffffffLL;
           reinterpret_cast<int64_t*>(out)[2 * o] = (pk - h) / 4294967296LL;
           reinterpret_cast<int64_t*>(out)[2 * o + 1] = h;
         } else {
           double2 v;
           std::memcpy(&v, raw.data() + c * elem, sizeof(v));
+          if (both) {
+            double2 other;
+            std::memcpy(&other, more.data() + c * elem, sizeof(other));
+            v.x += other.x;
+            v.y += other.y;
+          }
           reinterpret_cast<double*>(out)[2 * o] = v.x;
           reinterpret_cast<double*>(out)[2 * o + 1] = v.y;
         }

@@ -19,9 +19,11 @@
 // categories 2.49 -> 0.95 ms; 100k x 28 float, 31 leaves 1.64 -> 0.75 ms; 5k x 20, 31 leaves 0.72 ->
 // 0.60 ms; 12 jobs in one graph 2.90 -> 2.01 ms.
 //
-// An expanded leaf that is not split yet keeps everything it had: its rows stay in its own index
-// buffer (the children are written to the other one, and are expanded only after the commit), its
-// histogram in its own pool slot (the children get two new ones).
+// An expanded leaf that is not split yet keeps its rows: they stay in its own index buffer (the
+// children are written to the other one, and are expanded only after the commit). Its pool slot goes
+// to its larger child, whose histogram is the leaf's minus the smaller child's, as when one leaf is
+// split at a time; its own is both children's together, should anyone ask for it. So a tree of L
+// leaves has 1 + max_exp slots, 287 of 255 leaves (573 with two new ones for every expansion).
 //
 // Every partition CTA takes the round's decision from the same records (decide_round), CTA 0
 // writes it down. The state it reads and the state it writes are two copies that swap roles every
@@ -57,8 +59,8 @@ struct alignas(16) RoundExp {
   int32_t out, node, inner;
   uint32_t thr;          // threshold | default_left << 31
   int32_t begin, count, depth_buf;
-  int32_t slot, sslot, lslot;  // pool slots of the leaf, its smaller and its larger child
-  int32_t _pad;
+  int32_t slot, sslot;   // pool slots: the leaf's, which its larger child gets, and its smaller child's
+  int32_t leaf, _pad;
 };
 
 // The best candidate of one group of features (or of one feature) of a searched leaf.
@@ -122,9 +124,8 @@ __device__ __forceinline__ RoundView round_view(const Job& J, const Params& p) {
 }
 
 // Pool slots: the root's is 0; expansion x's smaller child gets 1 + x (zeroed when the tree starts,
-// as histograms are added up in it), its larger child 1 + max_exp + x (written by the search).
+// as histograms are added up in it).
 __host__ __device__ __forceinline__ int32_t round_sslot(int32_t x) { return 1 + x; }
-__host__ __device__ __forceinline__ int32_t round_lslot(const Params& p, int32_t x) { return 1 + p.max_exp + x; }
 
 // Whether the children of an expansion are searched (serial.rs:779-825: not at max_depth, not when
 // both have fewer than 2 min_data_in_leaf rows).
@@ -397,8 +398,8 @@ __device__ __forceinline__ void decide_round_commit(const Job& J, const Params& 
       o.pay[1] = s.fpay[ir];
       o.feat[1] = s.ffeat[ir];
       // children that are not searched: the left one keeps the leaf's slot, the right one has none
-      o.slot[0] = !h.go ? c.slot : (h.left_smaller ? c.sslot : c.lslot);
-      o.slot[1] = !h.go ? -1 : (h.left_smaller ? c.lslot : c.sslot);
+      o.slot[0] = !h.go ? c.slot : (h.left_smaller ? c.sslot : c.slot);
+      o.slot[1] = !h.go ? -1 : (h.left_smaller ? c.slot : c.sslot);
       o.x = c.x;
       o.L = L;
     }
@@ -526,8 +527,8 @@ __device__ __forceinline__ void decide_round_choose(const Job& J, const Params& 
       c.depth_buf = s.depth_buf[i];
       c.slot = s.slot[i];
       c.sslot = round_sslot(x);
-      c.lslot = round_lslot(p, x);
-      c._pad = i;
+      c.leaf = i;
+      c._pad = 0;
       s.nxt[rank] = c;
       s.ot[slot].leaf = i;
       s.out[i] = slot;
@@ -551,7 +552,7 @@ __device__ __forceinline__ void decide_round_choose(const Job& J, const Params& 
       // the tree's last split: nothing about its children is searched, so it is taken now; its row
       // counts come from the partition that follows
       const RoundExp c = s.nxt[0];
-      const int at = c._pad;
+      const int at = c.leaf;
       if (record) v.commit[leaves - 1] = Commit{c.x, at, -1, c.count};
       const int32_t db = ((c.depth_buf >> 1) + 1) * 2 + (1 - (c.depth_buf & 1));
       s.node[at] = 1 + 2 * c.x;

@@ -98,9 +98,7 @@ __device__ __forceinline__ double int_split_gain(const Params& p, int64_t lg, in
 struct SearchIn {
   LeafConst C;
   LeafSum S0;
-  // pool slots: the smaller leaf's, the one the larger leaf's histogram goes to, and its parent's
-  // (the same slot when one leaf is split at a time)
-  int32_t sslot, lslot, pslot;
+  int32_t sslot, lslot;  // pool slots: the smaller leaf's, and the larger one's, which holds its parent's
   int32_t group; // a grow round's search: the feature group of the candidate, else -1
   int32_t crow;  // row of the compact candidate copies: the side, or 2 e + side in a grow round
   // the integer search's two pool entries of this thread (IntPool), loaded from the slots known
@@ -115,7 +113,7 @@ struct IntPool {
   int64_t sv, lv;
 };
 __device__ __forceinline__ IntPool int_pool(const Job& J, const Params& p, const DevFeature& m, int side, int32_t f,
-                                            int32_t sslot, int32_t pslot) {
+                                            int32_t sslot, int32_t lslot) {
   const int t = threadIdx.x;
   const size_t slot_stride = (size_t)p.T * p.B * TILE;
   const size_t feat_off = (size_t)(f / TILE) * p.B * TILE + (f % TILE) + (size_t)(t + 1) * TILE;
@@ -124,7 +122,7 @@ __device__ __forceinline__ IntPool int_pool(const Job& J, const Params& p, const
   const bool in = t < m.len;
   IntPool r;
   r.sv = (in && !(fix && t == m.mfb)) ? pool[(size_t)sslot * slot_stride + feat_off] : 0;
-  r.lv = (side && in) ? pool[(size_t)pslot * slot_stride + feat_off] : 0;
+  r.lv = (side && in) ? pool[(size_t)lslot * slot_stride + feat_off] : 0;
   return r;
 }
 
@@ -573,7 +571,7 @@ __device__ void search_int(const Job& J, const Params& p, const SearchIn& si, co
   const bool fix = m.mfb > 0;  // offset 0: the slice holds every bin and the most frequent one is empty
   const bool in = t < m.len;
   // the smaller leaf's most-frequent entry is rewritten by its side-0 CTA; side 1 never reads it
-  const IntPool pv = si.pre ? IntPool{si.sv, si.lv} : int_pool(J, p, m, side, f, si.sslot, si.pslot);
+  const IntPool pv = si.pre ? IntPool{si.sv, si.lv} : int_pool(J, p, m, side, f, si.sslot, si.lslot);
   const int64_t sv = pv.sv, lv = pv.lv;
   const ScanGeom G = scan_geom(m);
   if (t < 2) sm.qn[t] = 0;
@@ -731,7 +729,7 @@ __device__ void search_float(const Job& J, const Params& p, const SearchIn& si, 
   const bool fix = m.mfb > 0;
   const bool in = t < m.len;
   double2 sv = (in && !(fix && t == m.mfb)) ? hs[(size_t)(t + 1) * TILE] : zero;
-  const double2 lv = (side && in) ? pool[(size_t)si.pslot * slot_stride + feat_off + (size_t)(t + 1) * TILE] : zero;
+  const double2 lv = (side && in) ? pool[(size_t)si.lslot * slot_stride + feat_off + (size_t)(t + 1) * TILE] : zero;
   const ScanGeom G = scan_geom(m);
   if (t < 2) sm.qn[t] = 0;
   const double sum_g = C.sum_g, sum_h = C.sum_h;
@@ -995,7 +993,7 @@ __device__ void search_float_fixed(const Job& J, const Params& p, const SearchIn
   const bool fix = m.mfb > 0;
   const bool in = t < m.len;
   double2 sv = (in && !(fix && t == m.mfb)) ? hs[(size_t)(t + 1) * TILE] : zero;
-  const double2 lv = (side && in) ? pool[(size_t)si.pslot * slot_stride + feat_off + (size_t)(t + 1) * TILE] : zero;
+  const double2 lv = (side && in) ? pool[(size_t)si.lslot * slot_stride + feat_off + (size_t)(t + 1) * TILE] : zero;
   const ScanGeom G = scan_geom(m);
   FloatLeaf K;
   K.g_exp = fixed_unit(p, J.st->red_maxg);
@@ -1373,7 +1371,7 @@ __device__ void search_cat(const Job& J, const Params& p, const SearchIn& si, co
     int64_t* hs = pool + (size_t)si.sslot * slot_stride + feat_off;
     int64_t* hl = pool + (size_t)(side ? si.lslot : si.sslot) * slot_stride + feat_off;
     const int64_t sv = (in && !(fix && t == m.mfb)) ? hs[(size_t)(t + 1) * TILE] : 0;
-    const int64_t lv = (side && in) ? pool[(size_t)si.pslot * slot_stride + feat_off + (size_t)(t + 1) * TILE] : 0;
+    const int64_t lv = (side && in) ? pool[(size_t)si.lslot * slot_stride + feat_off + (size_t)(t + 1) * TILE] : 0;
     int64_t v = side ? lv - sv : sv;
     if (fix) {
       const int64_t a = warp_sum(sv);
@@ -1398,7 +1396,7 @@ __device__ void search_cat(const Job& J, const Params& p, const SearchIn& si, co
     double2* hl = pool + (size_t)(side ? si.lslot : si.sslot) * slot_stride + feat_off;
     const double2 zero = make_double2(0.0, 0.0);
     double2 sv = (in && !(fix && t == m.mfb)) ? hs[(size_t)(t + 1) * TILE] : zero;
-    const double2 lv = (side && in) ? pool[(size_t)si.pslot * slot_stride + feat_off + (size_t)(t + 1) * TILE] : zero;
+    const double2 lv = (side && in) ? pool[(size_t)si.lslot * slot_stride + feat_off + (size_t)(t + 1) * TILE] : zero;
     if (fix) {
       const double ag = warp_sum(sv.x), ah = warp_sum(sv.y);
       if (lane == 0) {
@@ -1692,7 +1690,7 @@ __global__ void __launch_bounds__(32 * NW) k_search(const JobTable jobs, Params 
   const uint8_t used = J.used[f];
   SearchIn si;
   si.sslot = st->smaller_slot;
-  si.lslot = si.pslot = st->larger_slot;
+  si.lslot = st->larger_slot;
   si.group = -1;
   si.crow = side;
   si.C = J.lconst[side];
@@ -1736,10 +1734,8 @@ __global__ void __launch_bounds__(32 * NW) k_search(const JobTable jobs, Params 
 }
 
 // The search of a grow round (bk_rounds.cuh): blockIdx.x = 2 * feature group + side, blockIdx.y = the
-// expansion. The larger child's histogram goes to a slot of its own, with everything of the
-// parent's that the search does not derive (bin 0, features that are not searched) copied. The
-// expansion and, on the quantized path, the parent's bins are read while the histogram launch
-// finishes: both were written before it.
+// expansion. The expansion and, on the quantized path, the parent's bins are read while the histogram
+// launch finishes: both were written before it.
 // WARP: groups of kWarpFeatures numerical features, a warp each (bk_search_warp.cuh), then one
 // categorical feature per CTA; otherwise one feature per CTA in the form of k_search.
 struct RoundSearch {
@@ -1757,7 +1753,7 @@ __device__ __forceinline__ RoundSearch round_search_load(const Job& J, const Par
   r.stop = __ldcg(&r.hdr->stop);
   r.active = e < n_cur;
   r.c.x = -1;
-  r.c.node = r.c.slot = r.c.sslot = r.c.lslot = 0;
+  r.c.node = r.c.slot = r.c.sslot = 0;
   if (r.active) r.c = v.cur[q * kMaxRoundW + e];
   return r;
 }
@@ -1778,8 +1774,6 @@ __device__ __forceinline__ void round_clear_counters(const Job& J, const Params&
 template <bool PLAIN, bool QUANT, int NW>
 __device__ __forceinline__ void round_search_cta(const Job& J, const Params& p, const RoundExp& c, const DevFeature& m,
                                                  int f, int g, int e, int side, bool used, SearchSmemT<NW>& sm) {
-  using V = typename std::conditional<QUANT, int64_t, double2>::type;
-  const int t = (int)threadIdx.x;
   SearchIn si;
   si.group = g;
   si.crow = 2 * e + side;
@@ -1788,22 +1782,11 @@ __device__ __forceinline__ void round_search_cta(const Job& J, const Params& p, 
   if (!si.C.go) return;  // not searched (uniform over the expansion's side): no candidates
   const int32_t node = c.x < 0 ? 0 : 2 * c.x + si.C.go;
   si.sslot = c.x < 0 ? c.slot : c.sslot;
-  si.lslot = c.lslot;
-  si.pslot = c.slot;
+  si.lslot = c.slot;
   si.pre = false;
   si.sv = si.lv = 0;
-  const size_t slot_stride = (size_t)p.T * p.B * TILE;
-  const size_t feat_off = (size_t)(f / TILE) * p.B * TILE + (f % TILE);
-  V* pool = reinterpret_cast<V*>(J.pool);
-  if (side) {  // the slot entries the search does not write
-    const V* parent = pool + (size_t)c.slot * slot_stride + feat_off;
-    V* larger = pool + (size_t)c.lslot * slot_stride + feat_off;
-    if (t == 0) larger[0] = parent[0];
-    if (!used)
-      for (int b = t + 1; b < m.gbins; b += 32 * NW) larger[(size_t)b * TILE] = parent[(size_t)b * TILE];
-  }
   if (!used) {  // uniform over the CTA
-    if (t == 0) {
+    if (threadIdx.x == 0) {
       round_view(J, p).cand[(size_t)si.crow * p.n_groups + g] = RoundCand{kNoKey, 0u, 0x7fffffff};
       J.splittable[(size_t)node * p.F + f] = 0;
     }
@@ -1871,7 +1854,7 @@ __global__ void __launch_bounds__(32 * kWarpFeatures, 3)
   const size_t slot_stride = (size_t)p.T * p.B * TILE;
   int64_t* pool = reinterpret_cast<int64_t*>(J.pool);
   const size_t offj = fj >= 0 ? (size_t)(fj / TILE) * p.B * TILE + (fj % TILE) + TILE : 0;  // its bin 1
-  int64_t lv[8], lv0 = 0;
+  int64_t lv[8];
   bool usedj = false;
   if (r.active && side && c.x >= 0 && fj >= 0) {
     const int64_t* parent = pool + (size_t)c.slot * slot_stride + offj;
@@ -1881,7 +1864,6 @@ __global__ void __launch_bounds__(32 * kWarpFeatures, 3)
       const int t = t0 + 32 * i;
       lv[i] = t < lenj ? parent[(size_t)t * TILE] : 0;
     }
-    if (t0 == 0) lv0 = parent[-TILE];
   }
   griddep_wait();
   // the partition may be scheduled now: its CTAs read the round's state while this search runs
@@ -1899,31 +1881,25 @@ __global__ void __launch_bounds__(32 * kWarpFeatures, 3)
   if (!C.go) return;  // uniform over the CTA
   const int32_t node = c.x < 0 ? 0 : 2 * c.x + C.go;
   if (fj >= 0) {
-    // the larger leaf: parent minus smaller, bin 0 and the features that are not searched copied
-    // (their most frequent bin is fixed below)
+    // the larger leaf: parent minus smaller, in place (its most frequent bin is fixed below)
     const int64_t* hs = pool + (size_t)(c.x < 0 ? c.slot : c.sslot) * slot_stride + offj;
-    int64_t* hl = pool + (size_t)c.lslot * slot_stride + offj;
-    if (side && t0 == 0) hl[-TILE] = lv0;
+    int64_t* hl = pool + (size_t)c.slot * slot_stride + offj;
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int t = t0 + 32 * i;
       int64_t v = 0;
-      if (t < lenj) {
-        if (side && !usedj) {
-          hl[(size_t)t * TILE] = lv[i];
-        } else if (t != mfbj) {
-          v = hs[(size_t)t * TILE];
-          if (side) {
-            v = lv[i] - v;
-            hl[(size_t)t * TILE] = v;
-          }
+      if (t < lenj && t != mfbj && (!side || usedj)) {
+        v = hs[(size_t)t * TILE];
+        if (side) {
+          v = lv[i] - v;
+          hl[(size_t)t * TILE] = v;
         }
       }
       sm.w.w[j].e[slice_at(t)] = v;
     }
   }
   __syncthreads();
-  int64_t* own = pool + (size_t)(side ? c.lslot : (c.x < 0 ? c.slot : c.sslot)) * slot_stride +
+  int64_t* own = pool + (size_t)(side || c.x < 0 ? c.slot : c.sslot) * slot_stride +
                  (f >= 0 ? (size_t)(f / TILE) * p.B * TILE + (f % TILE) : 0);
   const ScanGeom G = scan_geom(m);
   WarpSlice& ws = sm.w.w[warp];
@@ -2023,7 +1999,7 @@ __global__ void __launch_bounds__(256) k_rounds_finish(const JobTable jobs, Para
   const int32_t last_L = h.last_x >= 0 ? (int32_t)(v.pcnt[(size_t)h.last_par * 2 * kMaxRoundW] & 0xffffffffLL) : 0;
   if (i < leaves) {
     const LeafEnt e = ent[i];
-    int32_t begin = e.begin, count = e.count, slot = e.slot;
+    int32_t begin = e.begin, count = e.count, slot = e.slot, rest = -1;
     if (h.last_x >= 0 && e.node > 2 * h.last_x) {  // one of its children (no later nodes exist)
       const bool left = e.node == 1 + 2 * h.last_x;
       const int32_t R = count - last_L, pslot = ent[v.commit[leaves - 2].leaf].slot;
@@ -2032,11 +2008,16 @@ __global__ void __launch_bounds__(256) k_rounds_finish(const JobTable jobs, Para
       slot = !go ? (left ? pslot : -1) : (left == (last_L < R) ? round_sslot(h.last_x) : pslot);
       begin = left ? begin : begin + last_L;
       count = left ? last_L : R;
+    } else if (e.out >= 0) {  // expanded, not split: its slot holds its larger child's histogram by now
+      const OutEnt o = v.out[st->fin_q * kMaxRoundOut + e.out];
+      if (o.slot[1] >= 0) rest = round_sslot(o.x);
     }
     J.leaf_begin[i] = begin;
     J.leaf_count[i] = count;
     J.leaf_buf[i] = e.depth_buf & 1;
     J.leaf_slot[i] = slot;
+    J.leaf_slot[p.num_leaves + i] = rest;
+    J.leaf_slot[2 * p.num_leaves + i] = e.node;
     J.leaf_depth[i] = e.depth_buf >> 1;
     if (e.node > 0) {  // a tree of one leaf keeps the root's output
       const int2 xi = v.xinfo[(e.node - 1) >> 1];
@@ -2086,7 +2067,7 @@ __global__ void __launch_bounds__(256) k_tree_begin(const Job* __restrict__ jobs
     J.leaf_count[i] = i == 0 ? st->root_count : 0;
     J.leaf_buf[i] = 0;
     J.leaf_depth[i] = 0;
-    J.leaf_slot[i] = -1;
+    J.leaf_slot[i] = J.leaf_slot[p.num_leaves + i] = -1;
     J.leaf_value[i] = 0.0;
     J.bgain[i] = -CUDART_INF;
     J.bfeat[i] = -1;
