@@ -710,9 +710,9 @@ int learner_create(const bk_feature* features, int32_t num_features, const uint8
       // the candidates, then the categorical candidates' bin bitsets
       J.cand = L->dalloc<Cand>((size_t)p.cand_rows * F +
                                (cand_cat_words(p.cand_rows, F) * sizeof(uint32_t) + sizeof(Cand) - 1) / sizeof(Cand));
-      J.cgain = L->dalloc<double>(2 * (size_t)p.round_w * F);
+      J.cgain = L->dalloc<double>(2 * (size_t)F);
       J.csplit = L->dalloc<uint8_t>(2 * (size_t)F);
-      J.cthr = L->dalloc<uint32_t>(2 * (size_t)p.round_w * F);
+      J.cthr = L->dalloc<uint32_t>(2 * (size_t)F);
       J.bsplit = L->dalloc<int64_t>(Lv);
       J.lconst = L->dalloc<LeafConst>(2 * (size_t)p.round_w);
       J.splittable = L->dalloc<uint8_t>((size_t)p.cand_rows * F);
