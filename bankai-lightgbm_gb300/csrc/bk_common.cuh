@@ -305,7 +305,7 @@ void launch_job_begin(const Job* d_jobs, int num_jobs, bool use_rows, int64_t ro
 // bagged_only: the identity of an unbagged root is not written
 void launch_init_rows(const Job* d_jobs, int num_jobs, const Params& p, const int32_t* rows, bool bagged_only,
                       cudaStream_t s);
-// noise_gf / noise_hf: the noise rounded to fp32 (launch_noise_f32)
+// noise_gf / noise_hf: the noise rounded to fp32 (launch_noise_f32), or null
 void launch_discretize(const Job* d_jobs, int num_jobs, const Params& p, const double* noise_g, const double* noise_h,
                        const float* noise_gf, const float* noise_hf, cudaStream_t s);
 void launch_noise_f32(const double* a, float* b, int64_t n, cudaStream_t s);

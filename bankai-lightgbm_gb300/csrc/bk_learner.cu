@@ -48,12 +48,13 @@ void set_error(const char* fmt, ...) {
 
 struct CudaError {
   std::string msg;
+  cudaError_t code = cudaErrorUnknown;
 };
 
 #define CK(call)                                                                                  \
   do {                                                                                            \
     cudaError_t e_ = (call);                                                                      \
-    if (e_ != cudaSuccess) throw CudaError{std::string(#call) + ": " + cudaGetErrorString(e_)}; \
+    if (e_ != cudaSuccess) throw CudaError{std::string(#call) + ": " + cudaGetErrorString(e_), e_}; \
   } while (0)
 
 // ---- host std::mt19937 for the per-row stochastic-rounding noise (mt19937.rs:32-101) ----
@@ -152,7 +153,7 @@ struct bk_learner {
   std::vector<TileGeom> h_tiles;
   double* d_noise_g = nullptr;
   double* d_noise_h = nullptr;
-  float *d_noise_gf = nullptr, *d_noise_hf = nullptr;  // the same in fp32
+  float *d_noise_gf = nullptr, *d_noise_hf = nullptr;  // the same in fp32 (null: rounded from f64 when read)
   // jobs
   std::vector<Job> jobs;
   Job* d_jobs = nullptr;
@@ -429,15 +430,18 @@ namespace {
 // a 255-leaf tree of the L2 workload, one split at a time 254: 4 leaves 66, 8 36, 16 22; on its
 // 63-leaf tree 4 18, 8 12, 16 12; on its 31-leaf tree 2 16, 4 10, 8 9. More leaves a round than that
 // only add expansions that are never split.
-void rounds_shape(Params& p) {
+void rounds_shape(Params& p, bool rounds) {
   p.round_w = std::min(kMaxRoundW, std::max(4, (p.num_leaves + 7) / 8));
   p.round_out = std::min(kMaxRoundOut, 2 * p.round_w);
-  p.max_exp = p.num_leaves <= kMaxRoundLeaves ? p.num_leaves - 1 + p.round_out : 0;
+  p.max_exp = rounds && p.num_leaves <= kMaxRoundLeaves ? p.num_leaves - 1 + p.round_out : 0;
   p.cand_rows = std::max(p.num_leaves, 1 + 2 * p.max_exp);
 }
 
+// rounds: with what grow rounds need beyond single splits (an eighth more histogram slots, twice the
+// candidates, the grouping of leaf renewal, the noise in fp32 as well). A learner that does not fit the
+// device's free memory with it is created without, and grows one split at a time.
 int learner_create(const bk_feature* features, int32_t num_features, const uint8_t* bins, int64_t num_data,
-                   const bk_config* c, int32_t num_jobs, bk_learner** out, bool device_bins) {
+                   const bk_config* c, int32_t num_jobs, bk_learner** out, bool device_bins, bool rounds = true) {
   if (!features || !bins || !c || !out || num_features <= 0 || num_data <= 0 || num_jobs <= 0) {
     set_error("bk_learner_create: invalid arguments");
     return -1;
@@ -498,7 +502,7 @@ int learner_create(const bk_feature* features, int32_t num_features, const uint8
     p.bynode = 0;
     p.n_icons = 0;
     p.path_words = (num_features + 31) / 32;
-    rounds_shape(p);
+    rounds_shape(p, rounds);
     p.icons = nullptr;
     L->K = num_jobs;
     int maxb = 0;
@@ -664,10 +668,12 @@ int learner_create(const bk_feature* features, int32_t num_features, const uint8
       L->d_noise_h = L->dalloc<double>(n);
       CK(cudaMemcpy(L->d_noise_g, ng.data(), n * sizeof(double), cudaMemcpyHostToDevice));
       CK(cudaMemcpy(L->d_noise_h, nh.data(), n * sizeof(double), cudaMemcpyHostToDevice));
-      L->d_noise_gf = L->dalloc<float>(n);
-      L->d_noise_hf = L->dalloc<float>(n);
-      launch_noise_f32(L->d_noise_g, L->d_noise_gf, num_data, L->stream);
-      launch_noise_f32(L->d_noise_h, L->d_noise_hf, num_data, L->stream);
+      if (rounds) {
+        L->d_noise_gf = L->dalloc<float>(n);
+        L->d_noise_hf = L->dalloc<float>(n);
+        launch_noise_f32(L->d_noise_g, L->d_noise_gf, num_data, L->stream);
+        launch_noise_f32(L->d_noise_h, L->d_noise_hf, num_data, L->stream);
+      }
     }
     const int Lv = p.num_leaves, F = num_features, K = num_jobs;
     L->d_g = L->dalloc<float>(n * K);
@@ -764,6 +770,10 @@ int learner_create(const bk_feature* features, int32_t num_features, const uint8
     CK(cudaGetLastError());
   } catch (const CudaError& e) {
     delete L;
+    if (e.code == cudaErrorMemoryAllocation && rounds) {
+      (void)cudaGetLastError();
+      return learner_create(features, num_features, bins, num_data, c, num_jobs, out, device_bins, false);
+    }
     return fail_cuda(e);
   }
   *out = L;

@@ -193,8 +193,9 @@ __global__ void __launch_bounds__(256) k_discretize(const Job* __restrict__ jobs
     if (pos >= n) pos -= n;
     int32_t gi, hi = 1;
     if (p.stochastic) {
-      gi = disc_value(g, igf, noise_gf[pos], ig, noise_g + pos, 0.0, fused);
-      if (!p.const_hess) hi = disc_value(h, ihf, noise_hf[pos], ih, noise_h + pos, 0.0, fused);
+      gi = disc_value(g, igf, noise_gf ? noise_gf[pos] : (float)noise_g[pos], ig, noise_g + pos, 0.0, fused);
+      if (!p.const_hess)
+        hi = disc_value(h, ihf, noise_hf ? noise_hf[pos] : (float)noise_h[pos], ih, noise_h + pos, 0.0, fused);
     } else {
       gi = disc_value(g, igf, 0.5f, ig, nullptr, 0.5, fused);
       if (!p.const_hess) hi = disc_value(h, ihf, 0.5f, ih, nullptr, 0.5, fused);

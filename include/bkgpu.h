@@ -74,7 +74,9 @@ typedef struct bk_learner_group bk_learner_group;
 
 /* Replaces SerialTreeLearner::new (serial.rs:284-565). `bins` is column-major uint8
  * [num_features][num_data] of stored bins. `num_jobs` trees are grown per train call over the
- * same dataset (all K class trees of one multiclass iteration, objective/multiclass.rs). */
+ * same dataset (all K class trees of one multiclass iteration, objective/multiclass.rs). A learner
+ * that only fits the device's free memory without what grow rounds need (bk_learner_set_loop_mode)
+ * is created without it and grows one split at a time. */
 int bk_learner_create(const bk_feature* features, int32_t num_features, const uint8_t* bins, int64_t num_data,
                       const bk_config* config, int32_t num_jobs, bk_learner** out);
 
@@ -174,7 +176,8 @@ int bk_learner_row_leaf(bk_learner* learner, int32_t* out);
 /* Grow-loop execution: 0 = one host round trip per split (the plain form); 1 = the whole
  * grow loop of an iteration captured once as a CUDA graph and replayed (default). The graph form
  * grows up to 16 leaves a round, with the same result; phase timing, by-node sampling, interaction
- * constraints, histogram clusters and trees above 512 leaves make it grow one split at a time. */
+ * constraints, histogram clusters, trees above 512 leaves and too little device memory make it grow
+ * one split at a time. */
 int bk_learner_set_loop_mode(bk_learner* learner, int32_t mode);
 
 /* Grow-loop kernel launches: 1 (default) = each kernel is launched with programmatic dependent

@@ -66,3 +66,34 @@ def test_device_memory_is_near_one_slot_a_leaf():
     used = before - torch.cuda.mem_get_info()[0]
     assert used <= 1.35 * 255 * slot, (used, 255 * slot)
     L.close()
+
+
+@pytest.mark.parametrize("quant", [1, 0])
+def test_learner_without_room_for_rounds_grows_one_split_at_a_time(quant):
+    """With less free memory than a learner with grow rounds takes, but enough for one without, creation
+    succeeds and the trees are the same."""
+    import torch
+    from lgbm_gb300 import GpuTreeLearner, LearnerConfig
+    ds, g, h = _data(4000, 2000, 6, nan=0.0)
+    cfg = LearnerConfig(num_leaves=255, use_quantized_grad=quant, seed=2, num_threads=2)
+    GpuTreeLearner(ds, cfg).train(g, h)  # the library's own startup
+    torch.cuda.empty_cache()
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    a = GpuTreeLearner(ds, cfg)
+    used = before - torch.cuda.mem_get_info()[0]
+    want = a.train(g, h)
+    a.close()
+    held = torch.empty(torch.cuda.mem_get_info()[0] - used + (96 << 20), dtype=torch.uint8, device="cuda")
+    b = GpuTreeLearner(ds, cfg)
+    left = torch.cuda.mem_get_info()[0]
+    del held
+    torch.cuda.empty_cache()
+    assert left < used
+    got = b.train(g, h)
+    assert len(got[0]) == len(want[0])
+    if quant:
+        assert got[0].tobytes() == want[0].tobytes() and np.array_equal(got[1], want[1])
+    else:
+        np.testing.assert_allclose(got[0]["gain"], want[0]["gain"], rtol=1e-6)
+    b.close()
