@@ -1391,6 +1391,8 @@ int bk_learner_group_autotune(bk_learner_group* G, const float* const* gradients
           restore();
           CK(cudaEventRecord(e0, G->stream));
           CK(cudaGraphLaunch(G->exec, G->stream));
+          CK(cudaStreamSynchronize(G->stream));
+          finish_trees(G->learners.data(), count, 0.0, nullptr);  // trees that need more rounds, as a call's
           CK(cudaEventRecord(e1, G->stream));
           CK(cudaEventSynchronize(e1));
           float ms = 0.f;
