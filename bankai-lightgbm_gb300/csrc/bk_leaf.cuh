@@ -104,7 +104,12 @@ __device__ __forceinline__ void compute_leaf_const_ls(const Job& J, const Params
     const double d = p.l2 == 0.0 ? p.min_gain : c.mgs - s0;
     c.hs2 = (float)h2;
     c.r2 = p.quant ? 0.0 : c.sum_g / h2;
-    const float ymin = (float)(p.min_hess + p.l2), s0f = (float)s0, arel = (p.quant ? 4e-15f : 4e-14f) + 1.01e-15f / ymin;
+    // the smallest denominator of a valid position; on the quantized path both its sides' hessians are known
+    // to a unit (first_x units at least on the one, th - brk_x + 1 on the other; bound_int takes sides of no
+    // unit apart), so a leaf without min_sum_hessian_in_leaf has bounds too
+    const double units = (double)max(min(c.first_x, (int64_t)((ls.int_sum & 0xffffffffLL) - c.brk_x + 1)), (int64_t)1);
+    const double hmin = p.quant ? fmax(p.min_hess, units * st->hscale) : p.min_hess;
+    const float ymin = (float)(hmin + p.l2), s0f = (float)s0, arel = (p.quant ? 4e-15f : 4e-14f) + 1.01e-15f / ymin;
     // what the f64 sums of a side can be off by: 32 additions of partial sums up to the rows' total magnitude,
     // at most their number times the largest one's bound, the power of two above it; doubled
     c.off_g = c.off_h = 0.f;

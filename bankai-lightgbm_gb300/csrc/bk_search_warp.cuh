@@ -54,8 +54,8 @@ struct WarpSearchSmem {
   int32_t real[kWarpFeatures];
 };
 
-// fp32 bounds on d (see above). Leaves outside the range where they hold (LeafConst::bk1 < 0) and
-// results that overflow give lo / up = -inf / +inf. Sums fit in 32 signed bits there.
+// fp32 bounds on d (see above). Leaves outside the range where they hold (LeafConst::bk1 < 0), sides
+// without hessian and results that overflow give lo / up = -inf / +inf. Sums fit in 32 signed bits there.
 struct Bound {
   float lo, up;
 };
@@ -73,7 +73,7 @@ __device__ __forceinline__ Bound bound_int(int64_t left, int32_t tg, int32_t th,
   const float d = __fmul_rn(__fmul_rn(t, t), q), dm = __fmul_rn(__fmul_rn(tm, tm), q);
   const float e = fmaf(dm, C.bk1, C.bk0);
   Bound r{__fsub_rn(d, e), __fadd_rn(d, e)};
-  if (!(r.up < 1e30f) || C.bk1 < 0.f) r = Bound{-CUDART_INF_F, CUDART_INF_F};
+  if (!(r.up < 1e30f) || C.bk1 < 0.f || lh == 0 || rh == 0) r = Bound{-CUDART_INF_F, CUDART_INF_F};
   return r;
 }
 
