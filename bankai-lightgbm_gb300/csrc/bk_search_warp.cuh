@@ -74,6 +74,7 @@ __device__ __forceinline__ Bound bound_int(int64_t left, int32_t tg, int32_t th,
   const float e = fmaf(dm, C.bk1, C.bk0);
   Bound r{__fsub_rn(d, e), __fadd_rn(d, e)};
   if (!(r.up < 1e30f) || C.bk1 < 0.f || lh == 0 || rh == 0) r = Bound{-CUDART_INF_F, CUDART_INF_F};
+  if ((lg | tg) == 0) r = Bound{0.f, 0.f};  // no gradient on either side: gain and s0 are exactly 0
   return r;
 }
 

@@ -53,3 +53,13 @@ def _tree(ds, g, h, **kw):
 def test_leaves_without_a_least_hessian(kw):
     ds, X, g, h = _data()
     assert _tree(ds, g, h, **kw) < 2.0 * _tree(ds, g, h)
+
+
+@pytest.mark.parametrize("min_gain", [0.0, 1e-3])
+def test_leaves_without_gradients(min_gain):
+    """Only the rows of a corner have gradients; most leaves and features have none to split by."""
+    ds, X, g, h = _data()
+    g = np.where((X[:, 0] > 1.0) & (X[:, 1] > 0.0), g, 0.0).astype(np.float32)
+    g[:600] *= np.float32(0.1)
+    kw = dict(min_gain_to_split=min_gain, min_data_in_leaf=3)
+    assert _tree(ds, g, h, **kw) < 1.6 * _tree(*_data()[:1], *_data()[2:], **kw)
