@@ -125,8 +125,8 @@ struct LeafConst {
   double sum_g, sum_h, parent, mgs, cnt_factor;  // mgs = min_gain_shift
   int64_t first_x, brk_x;  // quantized path: validity thresholds on the accumulated hessian
   float mgs_up, mgs_dn;    // min_gain_shift rounded up / down to fp32
-  float gsf, hsf, l2f;     // fp32 copies of the gradient / hessian scales and lambda_l2
-  // the warp search's bounds (bk_search_warp.cuh): hs2 = h + 2 lambda_l2, the error bound's factor
+  float gsf, hsf, l2f;     // the gradient scale brought to [1, 2), the hessian scale and lambda_l2
+  // the warp search's bounds (bk_search_warp.cuh), gains in units of gsf: hs2 = h + 2 lambda_l2, the error bound's factor
   // and constant (bk1 < 0: the leaf is outside its range), min_gain_shift - s0 rounded up / down
   float hs2, bk1, bk0, d_up, d_dn;
   double r2;               // float path: g / (h + 2 lambda_l2)

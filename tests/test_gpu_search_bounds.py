@@ -63,3 +63,10 @@ def test_leaves_without_gradients(min_gain):
     g[:600] *= np.float32(0.1)
     kw = dict(min_gain_to_split=min_gain, min_data_in_leaf=3)
     assert _tree(ds, g, h, **kw) < 1.6 * _tree(*_data()[:1], *_data()[2:], **kw)
+
+
+@pytest.mark.parametrize("unit", [1e-30, 1e-20, 1e-13, 1e13, 1e16])
+@pytest.mark.parametrize("l2", [0.0, 3.0])
+def test_units_of_the_gradients(unit, l2):
+    ds, X, g, h = _data()
+    assert _tree(ds, (g * np.float32(unit)).astype(np.float32), h, lambda_l2=l2) < 2.0 * _tree(ds, g, h, lambda_l2=l2)
