@@ -75,10 +75,15 @@ __device__ __forceinline__ double parent_output_of(const Params& p, bool root, c
   return ls.weight;
 }
 
-// The power of two that brings a positive normal number to [1, 2); 1 for the others.
-__device__ __forceinline__ double pow2_inverse(double x) {
-  const int e = (int)((unsigned long long)__double_as_longlong(x) >> 52);
-  return e == 0 || e >= 2046 ? 1.0 : __longlong_as_double((long long)(2046 - e) << 52);
+// x 2^k by its exponent field (an f64 multiplication holds a scheduler for 64 cycles); what is or falls
+// below the normal range becomes 0.
+__device__ __forceinline__ double scale_pow2(double x, int k) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const int e = (int)((b >> 52) & 0x7ffu), r = e + k;
+  if (e == 0 || r <= 0) return 0.0;
+  if (e == 2047) return x;
+  return r >= 2047 ? copysign((double)CUDART_INF_F, x)
+                   : __longlong_as_double((long long)(b + ((unsigned long long)(long long)k << 52)));
 }
 
 // One warp: the constants of side `side` (0 = smaller leaf, 1 = larger leaf) of the coming search,
@@ -108,18 +113,24 @@ __device__ __forceinline__ void compute_leaf_const_ls(const Job& J, const Params
     const double h2 = c.sum_h + 2.0 * p.l2;
     const double s0 = p.l2 == 0.0 ? c.mgs - p.min_gain : c.sum_g * c.sum_g / h2;
     const double d = p.l2 == 0.0 ? p.min_gain : c.mgs - s0;
-    // quantized: the bounds are taken with the gradients' scale brought to [1, 2), gains times its square,
-    // so that fp32 holds them whatever the gradients' unit
-    const double unit = p.quant ? pow2_inverse(st->gscale) : 1.0, unit2 = unit * unit;
+    // quantized: the bounds are taken with the gradients' scale brought to [1, 2), gains times the square of
+    // the same power of two, so that fp32 holds them whatever the gradients' unit
+    c.gsf = (float)st->gscale;
+    const uint32_t ge = __float_as_uint(c.gsf) >> 23;
+    const int unit = p.quant && ge > 0u && ge < 255u ? 127 - (int)ge : 0;
+    if (unit) c.gsf = __uint_as_float(__float_as_uint(c.gsf) + ((uint32_t)unit << 23));
     c.hs2 = (float)h2;
-    c.gsf = (float)(st->gscale * unit);
     c.r2 = p.quant ? 0.0 : c.sum_g / h2;
     // the smallest denominator of a valid position; on the quantized path both its sides' hessians are known
     // to a unit (first_x units at least on the one, th - brk_x + 1 on the other; bound_int takes sides of no
     // unit apart), so a leaf without min_sum_hessian_in_leaf has bounds too
-    const double units = (double)max(min(c.first_x, (int64_t)((ls.int_sum & 0xffffffffLL) - c.brk_x + 1)), (int64_t)1);
-    const double hmin = p.quant ? fmax(p.min_hess, units * st->hscale) : p.min_hess;
-    const float ymin = (float)(hmin + p.l2), s0f = (float)(s0 * unit2), arel = (p.quant ? 4e-15f : 4e-14f) + 1.01e-15f / ymin;
+    float ymin = (float)p.min_hess;
+    if (p.quant) {
+      const int64_t units = min(c.first_x, (int64_t)((ls.int_sum & 0xffffffffLL) - c.brk_x + 1));
+      ymin = fmaxf(ymin, __fmul_rn((float)(uint32_t)max(units, (int64_t)1), (float)st->hscale));
+    }
+    ymin = __fadd_rn(ymin, (float)p.l2);
+    const float s0f = (float)scale_pow2(s0, 2 * unit), arel = (p.quant ? 4e-15f : 4e-14f) + 1.01e-15f / ymin;
     // what the f64 sums of a side can be off by: 32 additions of partial sums up to the rows' total magnitude,
     // at most their number times the largest one's bound, the power of two above it; doubled
     c.off_g = c.off_h = 0.f;
@@ -134,8 +145,8 @@ __device__ __forceinline__ void compute_leaf_const_ls(const Job& J, const Params
         (p.quant && (ls.int_sum & 0xffffffffLL) >= 0x80000000LL))
       c.bk1 = -1.f;
     const bool ok = !isnan(c.mgs) && !isnan(d);  // else every threshold is evaluated
-    c.d_up = ok ? __double2float_ru(d * unit2) : CUDART_INF_F;
-    c.d_dn = ok ? __double2float_rd(d * unit2) : -CUDART_INF_F;
+    c.d_up = ok ? __double2float_ru(scale_pow2(d, 2 * unit)) : CUDART_INF_F;
+    c.d_dn = ok ? __double2float_rd(scale_pow2(d, 2 * unit)) : -CUDART_INF_F;
   }
   c.hsf = (float)st->hscale;
   c.l2f = (float)p.l2;
