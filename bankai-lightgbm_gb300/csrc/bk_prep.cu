@@ -411,26 +411,30 @@ __global__ void __launch_bounds__(32) k_root_finish(const Job* __restrict__ jobs
     }
   }
   if (p.quant && !exact_quant_root) {
-    // sequential f64 sum of int * scale in root row order (serial.rs:717-739)
-    double a = 0.0, b = 0.0;
+    // sequential f64 sum of int * scale in root row order (serial.rs:717-739): even lanes the gradients, odd
+    // lanes the hessians, a batch of rows on its way while the one before is added
     const int64_t cnt = s->root_count;
+    const bool bagged = s->use_rows != 0;
+    const int16_t* packed = J.packed;
+    const int32_t* idx = J.idx0;
+    const double scale = (lane & 1) ? s->hscale : s->gscale;
+    auto load = [&](int64_t base) -> int32_t {
+      const int64_t k = base + lane;
+      return k < cnt ? packed[bagged ? idx[k] : (int32_t)k] : 0;
+    };
+    double sum = 0.0;
+    int32_t next = load(0);
     for (int64_t base = 0; base < cnt; base += 32) {
-      int64_t k = base + lane;
-      int32_t gi = 0, hi = 0;
-      if (k < cnt) {
-        int32_t pk = J.packed[s->use_rows ? J.idx0[k] : (int32_t)k];
-        gi = (int8_t)(pk >> 8);
-        hi = pk & 0xff;
-      }
-      int jn = (int)min((int64_t)32, cnt - base);
+      const int32_t pk = next;
+      next = load(base + 32);
+      const int jn = (int)min((int64_t)32, cnt - base);
+#pragma unroll 4
       for (int j = 0; j < jn; ++j) {
-        int32_t g = __shfl_sync(FULL, gi, j), h = __shfl_sync(FULL, hi, j);
-        if (lane == 0) {
-          a += (double)g * s->gscale;
-          b += (double)h * s->hscale;
-        }
+        const int32_t x = __shfl_sync(FULL, pk, j);
+        sum += (double)((lane & 1) ? x & 0xff : (int32_t)(int8_t)(x >> 8)) * scale;
       }
     }
+    const double a = __shfl_sync(FULL, sum, 0), b = __shfl_sync(FULL, sum, 1);
     sg = a;
     sh = b;
   } else if (p.quant) {
