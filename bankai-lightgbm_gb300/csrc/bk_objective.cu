@@ -89,6 +89,8 @@ __global__ void __launch_bounds__(256) k_grad_binary(const double* __restrict__ 
     Pair z = pair_of<true>(one ? s : sigmoid * s, &ok);  // exp(z) and 1 + exp(z): absolute errors count
     if (!pos) z = pair_neg(z);
     ok = ok && ok_c && fabsf(z.hi) <= 60.0f;
+    // a warp with a row for f64 takes all of them there: the f64 instructions cost the same
+    ok = __all_sync(__activemask(), ok);
     float gv = 0.f, hv = 0.f;
     if (ok) {
       // response = -label s / (1 + e), hessian |response| (s - |response|) = s^2 e / (1 + e)^2
@@ -175,12 +177,20 @@ __global__ void __launch_bounds__(kSoftmaxThreads)
     // scores up to 2^-53, which the bound allows)
     bool ok = ok_f;
     Pair top{-CUDART_INF_F, 0.f};
+    float least = CUDART_INF_F;
     for (int k = 0; k < K; ++k) {
       bool o;
       const Pair x = pair_of<true>(score[(size_t)k * n + i], &o);
       ok = ok && o && fabsf(x.hi) <= 64.0f;
       mine[k * kSoftmaxThreads] = make_float2(x.hi, x.lo);
       if (x.hi > top.hi || (x.hi == top.hi && x.lo > top.lo)) top = x;
+      least = fminf(least, x.hi);
+    }
+    // as in k_grad_binary; the exponents reach down to the lowest score's
+    ok = ok && __fsub_rn(least, top.hi) >= -59.0f;
+    if (!__all_sync(__activemask(), ok)) {
+      softmax_row(score, n, i, K, lab, w, g, h);
+      continue;
     }
     // two classes at a time: the chains of a class alone leave the schedulers idle
     Pair sum{0.f, 0.f}, others{0.f, 0.f};
@@ -188,11 +198,7 @@ __global__ void __launch_bounds__(kSoftmaxThreads)
 #pragma unroll 2
     for (int k = 0; k < K; ++k) {
       const float2 x = mine[k * kSoftmaxThreads];
-      Pair z = pair_add(Pair{x.x, x.y}, top);
-      if (!(z.hi >= -60.0f)) {
-        ok = false;
-        z = Pair{0.f, 0.f};
-      }
+      const Pair z = pair_add(Pair{x.x, x.y}, top);
       const Pair e = pair_exp(z, st);
       sum = pair_add(sum, e);
       if (k != lab) others = pair_add(others, e);

@@ -98,8 +98,9 @@ __device__ __forceinline__ bool pair_round(Pair a, float rel, float* out) {
   const uint32_t b = __float_as_uint(a.hi) & 0x7fffffffu;
   if (b < (40u << 23) || b >= (250u << 23)) return false;  // tiny (zero too), huge
   if (a.lo == 0.f && rel < 1e-9f) return true;
-  if ((b & 0x7fffffu) == 0u) return false;  // a power of two
-  const float half = __uint_as_float((b & 0x7f800000u) - (24u << 23));  // half a unit in the last place
+  // half a unit in the last place; below a power of two the units are half as large
+  const bool below = (b & 0x7fffffu) == 0u && (__float_as_uint(a.hi) ^ __float_as_uint(a.lo)) >> 31 != 0u;
+  const float half = __uint_as_float((b & 0x7f800000u) - ((below ? 25u : 24u) << 23));
   return fabsf(__fsub_rn(half, fabsf(a.lo))) > __fmul_rn(rel, fabsf(a.hi));
 }
 
