@@ -2131,11 +2131,12 @@ void launch_apply_split(const Job* h_jobs, int num_jobs, const Params& p, int pa
 }
 
 // The warp form takes the quantized, plain searches of rounds that would not fit the chip at once with a
-// CTA per feature (by their registers two of 256 threads per SM); there the latter is faster, as it
-// spreads a feature's positions over eight warps: iterations with 20 features x 4 leaves a round (160
-// CTAs) take 467 us instead of 560, with 40 x 8 (640 CTAs) 926 instead of 908. With 64-thread CTAs
-// (narrow features) it gains up to 800 CTAs (50 x 8: 572 for 587 us), but costs learners that train
-// side by side more than that (twelve in a group: 2055 for 1960 us), so one line serves both.
+// CTA per feature (by their registers two of 256 threads per SM). Both forms on 20k and 300k rows, 6 to 200
+// features, 15 to 127 leaves, time of a tree with a CTA per feature over that with warps, by the round's
+// CTAs: 255 bins 0.83 at 304, 0.88 at 608, 1.0 at 912, 1.17 at 1600, 1.84 at 6400; 63 bins 0.94 at 304, 0.95
+// at 912, 1.0 at 1600, 1.17 at 6400. The line lies below the crossing for the sake of learners that train
+// side by side, whose warps share an SM better: twelve in a group took 1.6% longer with the line at 912,
+// and a learner with categorical features (300k x 40) 2%.
 static bool search_round_warp(const Params& p) {
   return p.quant && !p.use_l1 && !p.use_max && !p.use_smooth && 2 * p.F * p.round_w * p.search_jobs > 2 * 152;
 }
@@ -2145,10 +2146,11 @@ int rounds_groups(const Params& p) {
   return (p.n_numeric + kWarpFeatures - 1) / kWarpFeatures + (p.F - p.n_numeric);
 }
 
-// The float search's registers allow two CTAs per SM. From 912 CTAs on, four with some spilled are faster
-// (before the f64 sums of the queued positions: rounds of 255 leaves x 100 features, 3200 CTAs, 50 -> 37
-// us; of 31 leaves x 28 features, 224 CTAs, 8 -> 11 us).
-constexpr int64_t kManySearches = 2 * 3 * 152;
+// The float search's registers allow two CTAs per SM; four with some spilled are faster once there are
+// several waves of them. Time of a tree with two over that with four, the shapes above, by the round's CTAs:
+// 0.88 at 304, 0.92 at 608, 0.97 at 1024, 1.05 at 1280 (80 features; 0.99 at 1408 with 44), 1.09 at 1600,
+// 1.15 at 3200, 1.22 at 6400.
+constexpr int64_t kManySearches = 8 * 152;
 
 void launch_search_round(const Job* h_jobs, int num_jobs, const Params& p, const DevFeature* feats, int q,
                          cudaStream_t s) {
