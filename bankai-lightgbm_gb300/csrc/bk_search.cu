@@ -2012,6 +2012,8 @@ __global__ void __launch_bounds__(256) k_rounds_finish(const JobTable jobs, Para
       const OutEnt o = v.out[st->fin_q * kMaxRoundOut + e.out];
       if (o.slot[1] >= 0) rest = round_sslot(o.x);
     }
+    // a root that was not searched (round_go) has no histogram
+    if (leaves == 1 && ((p.max_depth > 0 && (e.depth_buf >> 1) >= p.max_depth) || count < p.min_data * 2)) slot = -1;
     J.leaf_begin[i] = begin;
     J.leaf_count[i] = count;
     J.leaf_buf[i] = e.depth_buf & 1;

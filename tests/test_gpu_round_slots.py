@@ -97,3 +97,15 @@ def test_learner_without_room_for_rounds_grows_one_split_at_a_time(quant):
     else:
         np.testing.assert_allclose(got[0]["gain"], want[0]["gain"], rtol=1e-6)
     b.close()
+
+
+@pytest.mark.parametrize("timed", [False, True])
+def test_root_that_is_not_searched_has_no_histogram(timed):
+    from lgbm_gb300 import GpuTreeLearner, LearnerConfig
+    ds, g, h = _data(500, 4, 8)
+    L = GpuTreeLearner(ds, LearnerConfig(num_leaves=31, use_quantized_grad=1, min_data_in_leaf=60))
+    L.set_timing(timed)
+    for rows, searched in ((None, True), (np.arange(0, 110, dtype=np.int32), False), (None, True)):
+        assert len(L.train(g, h, rows)[1]) == 1 or searched
+        assert (L.leaf_histogram(0) is not None) == searched
+    L.close()
