@@ -75,17 +75,6 @@ __device__ __forceinline__ double parent_output_of(const Params& p, bool root, c
   return ls.weight;
 }
 
-// x 2^k by its exponent field (an f64 multiplication holds a scheduler for 64 cycles); what is or falls
-// below the normal range becomes 0.
-__device__ __forceinline__ double scale_pow2(double x, int k) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const int e = (int)((b >> 52) & 0x7ffu), r = e + k;
-  if (e == 0 || r <= 0) return 0.0;
-  if (e == 2047) return x;
-  return r >= 2047 ? copysign((double)CUDART_INF_F, x)
-                   : __longlong_as_double((long long)(b + ((unsigned long long)(long long)k << 52)));
-}
-
 // One warp: the constants of side `side` (0 = smaller leaf, 1 = larger leaf) of the coming search,
 // for a leaf with sums `ls` (`root`: the tree's only leaf). In a grow round `side` is 2 e + side for
 // expansion e, and `go` says which child of the leaf it is.
@@ -112,13 +101,19 @@ __device__ __forceinline__ void compute_leaf_const_ls(const Job& J, const Params
     // without lambda_l2, s0 is the leaf's own gain (up to its rounding, which the bounds allow for)
     const double h2 = c.sum_h + 2.0 * p.l2;
     const double s0 = p.l2 == 0.0 ? c.mgs - p.min_gain : c.sum_g * c.sum_g / h2;
-    const double d = p.l2 == 0.0 ? p.min_gain : c.mgs - s0;
+    double d = p.l2 == 0.0 ? p.min_gain : c.mgs - s0;
     // quantized: the bounds are taken with the gradients' scale brought to [1, 2), gains times the square of
     // the same power of two, so that fp32 holds them whatever the gradients' unit
     c.gsf = (float)st->gscale;
     const uint32_t ge = __float_as_uint(c.gsf) >> 23;
     const int unit = p.quant && ge > 0u && ge < 255u ? 127 - (int)ge : 0;
-    if (unit) c.gsf = __uint_as_float(__float_as_uint(c.gsf) + ((uint32_t)unit << 23));
+    float s0f = (float)s0;
+    if (unit) {
+      c.gsf = __uint_as_float(__float_as_uint(c.gsf) + ((uint32_t)unit << 23));
+      const float g = __fmul_rn((float)(int32_t)(ls.int_sum >> 32), c.gsf);
+      s0f = __fdividef(__fmul_rn(g, g), (float)h2);  // good to 1e-6, of which bk0 has plenty
+      if (d != 0.0) d *= __longlong_as_double((long long)(1023 + 2 * unit) << 52);
+    }
     c.hs2 = (float)h2;
     c.r2 = p.quant ? 0.0 : c.sum_g / h2;
     // the smallest denominator of a valid position; on the quantized path both its sides' hessians are known
@@ -130,14 +125,14 @@ __device__ __forceinline__ void compute_leaf_const_ls(const Job& J, const Params
       ymin = fmaxf(ymin, __fmul_rn((float)(uint32_t)max(units, (int64_t)1), (float)st->hscale));
     }
     ymin = __fadd_rn(ymin, (float)p.l2);
-    const float s0f = (float)scale_pow2(s0, 2 * unit), arel = (p.quant ? 4e-15f : 4e-14f) + 1.01e-15f / ymin;
+    const float arel = (p.quant ? 4e-15f : 4e-14f) + 1.01e-15f / ymin;
     // what the f64 sums of a side can be off by: 32 additions of partial sums up to the rows' total magnitude,
     // at most their number times the largest one's bound, the power of two above it; doubled
     c.off_g = c.off_h = 0.f;
-    if (!p.quant) {
-      const double rows = (double)ls.num_data * 7.1054273576010019e-15;  // 2^-47
-      c.off_g = __double2float_ru(rows * __longlong_as_double((long long)(st->red_maxg + 897u) << 52));
-      c.off_h = __double2float_ru(rows * __longlong_as_double((long long)(st->red_maxh + 897u) << 52));
+    if (!p.quant) {  // 2^(exponent - 126) above the magnitudes, 2^-47
+      auto off = [&](uint32_t e) { return __fmul_ru(__int2float_ru(ls.num_data), __uint_as_float(max((int)e - 46, 1) << 23)); };
+      c.off_g = off(st->red_maxg);
+      c.off_h = off(st->red_maxh);
     }
     c.bk1 = 44.0f * 5.9604645e-08f + arel;
     c.bk0 = s0f * arel + 1e-24f;
@@ -145,8 +140,8 @@ __device__ __forceinline__ void compute_leaf_const_ls(const Job& J, const Params
         (p.quant && (ls.int_sum & 0xffffffffLL) >= 0x80000000LL))
       c.bk1 = -1.f;
     const bool ok = !isnan(c.mgs) && !isnan(d);  // else every threshold is evaluated
-    c.d_up = ok ? __double2float_ru(scale_pow2(d, 2 * unit)) : CUDART_INF_F;
-    c.d_dn = ok ? __double2float_rd(scale_pow2(d, 2 * unit)) : -CUDART_INF_F;
+    c.d_up = ok ? __double2float_ru(d) : CUDART_INF_F;
+    c.d_dn = ok ? __double2float_rd(d) : -CUDART_INF_F;
   }
   c.hsf = (float)st->hscale;
   c.l2f = (float)p.l2;
