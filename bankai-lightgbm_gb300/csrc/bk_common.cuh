@@ -301,6 +301,8 @@ void launch_partition(const Job* h_jobs, int num_jobs, const Params& p, const ui
 cudaError_t hist_set_smem_attrs(size_t smem);
 
 // bk_prep.cu
+void launch_results(const void* results, void* h_results, size_t bytes, const JobState* states, JobState* h_states,
+                    int num_jobs, cudaStream_t s);
 void launch_job_begin(const Job* d_jobs, int num_jobs, bool use_rows, int64_t root_count, cudaStream_t s);
 // bagged_only: the identity of an unbagged root is not written
 void launch_init_rows(const Job* d_jobs, int num_jobs, const Params& p, const int32_t* rows, bool bagged_only,

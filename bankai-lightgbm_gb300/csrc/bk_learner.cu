@@ -701,7 +701,7 @@ int learner_create(const bk_feature* features, int32_t num_features, const uint8
     L->pool_bytes_per_job = (size_t)std::max(Lv, 1 + p.max_exp) * L->slot_bytes;
     L->d_pool = L->dalloc<uint8_t>(L->pool_bytes_per_job * K);
     static_assert(sizeof(bk_split) % sizeof(double) == 0, "the leaf values follow the records");
-    L->results_bytes = (sizeof(bk_split) + sizeof(double)) * (size_t)Lv * K + 16;
+    L->results_bytes = ((sizeof(bk_split) + sizeof(double)) * (size_t)Lv * K + 15) / 16 * 16 + 16;
     L->d_results = L->dalloc<unsigned char>(L->results_bytes);
     CK(cudaMemset(L->d_results, 0, L->results_bytes));
     L->d_bad_label = reinterpret_cast<int32_t*>(L->d_results + L->results_bytes - 16);
@@ -774,7 +774,7 @@ int learner_create(const bk_feature* features, int32_t num_features, const uint8
     std::memset(L->h_results, 0, L->results_bytes);
     L->h_records = reinterpret_cast<bk_split*>(L->h_results);
     L->h_leaf_values = reinterpret_cast<double*>(L->h_records + (size_t)Lv * K);
-    L->h_bad_label = reinterpret_cast<int32_t*>(L->h_leaf_values + (size_t)Lv * K);
+    L->h_bad_label = reinterpret_cast<int32_t*>(L->h_results + L->results_bytes - 16);
     CK(cudaMallocHost(&L->h_state, sizeof(JobState) * K));
     L->d_leaf_vals_in = L->dalloc<double>((size_t)Lv * K);
     L->d_tree = L->dalloc<int32_t>(13 * (size_t)Lv + 4);
@@ -857,13 +857,12 @@ void enqueue_results(bk_learner* L, double shrinkage, double* score) {
     launch_add_score_own(L->d_jobs, L->K, p, shrinkage, score, L->rounds() ? 1 : 0, L->stream);
     CK(cudaGetLastError());
   }
-  // every job's records and leaf values and the rejected labels in one copy, the states in another
-  CK(cudaMemcpyAsync(L->h_results, L->d_results, L->results_bytes, cudaMemcpyDeviceToHost, L->stream));
-  CK(cudaMemcpy2DAsync(L->h_state, sizeof(JobState), L->jobs[0].st, sizeof(JobState), offsetof(JobState, mt),
-                       (size_t)L->K, cudaMemcpyDeviceToHost, L->stream));
+  // every job's records and leaf values, the rejected labels and the states, written by a kernel
+  launch_results(L->d_results, L->h_results, L->results_bytes, L->jobs[0].st, L->h_state, L->K, L->stream);
+  CK(cudaGetLastError());
 }
 
-// With the learners' streams waited for: the further rounds of those whose trees are not finished,
+// With the learners' calls waited for: the further rounds of those whose trees are not finished,
 // all of them queued before any is waited for. scores: per learner, or null.
 void finish_trees(bk_learner* const* learners, size_t count, double shrinkage, double* const* scores) {
   std::vector<bk_learner*> open;
@@ -879,7 +878,7 @@ void finish_trees(bk_learner* const* learners, size_t count, double shrinkage, d
       open.push_back(L);
     }
     if (open.empty()) return;
-    for (bk_learner* L : open) CK(cudaStreamSynchronize(L->stream));
+    for (bk_learner* L : open) CK(cudaEventSynchronize(L->ev_end));
   }
 }
 
@@ -952,7 +951,7 @@ int bk_learner_train(bk_learner* L, const float* gradients, const float* hessian
   }
   try {
     if (!train_enqueue(L, gradients, hessians, on_device, rows, num_rows, 0.0, nullptr)) return -1;
-    CK(cudaStreamSynchronize(L->stream));
+    CK(cudaEventSynchronize(L->ev_end));
     CK(cudaGetLastError());
     finish_trees(&L, 1, 0.0, nullptr);
     train_finish(L, splits, leaf_values, root_outputs, num_leaves_out);
@@ -1134,7 +1133,7 @@ int bk_learners_train_batch(bk_learner* const* learners, int32_t count, const fl
         set_error("bk_learners_train_batch: %s", msg.c_str());
         return -1;
       }
-    for (int32_t k = 0; k < count; ++k) CK(cudaStreamSynchronize(learners[k]->stream));
+    for (int32_t k = 0; k < count; ++k) CK(cudaEventSynchronize(learners[k]->ev_end));
     CK(cudaGetLastError());
     finish_trees(learners, (size_t)count, shrinkage, scores);
     for (i = 0; i < count; ++i)

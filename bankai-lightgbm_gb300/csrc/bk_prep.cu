@@ -8,6 +8,7 @@
 #include <math_constants.h>
 
 #include <algorithm>
+#include <cstddef>
 
 #include "bk_math.cuh"
 
@@ -25,6 +26,23 @@ __global__ void __launch_bounds__(32) k_job_begin(const Job* __restrict__ jobs, 
     s->use_rows = use_rows;
     s->root_count = root_count;
     s->hist_rows_direct = s->hist_rows_gather = s->hist_builds = 0;
+  }
+}
+
+// What a train call returns, written to the host's pinned memory: the results (a multiple of 16 bytes) and
+// each job's state without its random engine. Two copies took longer, and a stream that ends in a copy
+// shares half as many of the device's queues in the next calls: 32 learners of 2000 x 10 in one batch call
+// 2290 us with copies, 1488 with this.
+__global__ void __launch_bounds__(256) k_results(const uint4* __restrict__ results, uint4* __restrict__ h_results, int n16,
+                                                 const JobState* __restrict__ states, JobState* __restrict__ h_states,
+                                                 int num_jobs) {
+  static_assert(offsetof(JobState, mt) % 4 == 0, "the state is written in words");
+  constexpr int kWords = (int)(offsetof(JobState, mt) / 4);
+  const int step = gridDim.x * blockDim.x, t = blockIdx.x * blockDim.x + threadIdx.x;
+  for (int i = t; i < n16; i += step) h_results[i] = results[i];
+  for (int i = t; i < num_jobs * kWords; i += step) {
+    const int j = i / kWords, w = i % kWords;
+    reinterpret_cast<uint32_t*>(h_states + j)[w] = reinterpret_cast<const uint32_t*>(states + j)[w];
   }
 }
 
@@ -560,6 +578,13 @@ __global__ void k_zero_pool(uint4* __restrict__ pool, size_t per_job, size_t n) 
 
 void launch_job_begin(const Job* d_jobs, int num_jobs, bool use_rows, int64_t root_count, cudaStream_t s) {
   k_job_begin<<<1, 32, 0, s>>>(d_jobs, num_jobs, use_rows ? 1 : 0, root_count);
+}
+
+void launch_results(const void* results, void* h_results, size_t bytes, const JobState* states, JobState* h_states,
+                    int num_jobs, cudaStream_t s) {
+  const int n16 = (int)(bytes / 16), grid = std::min(32, 1 + n16 / 256);
+  k_results<<<grid, 256, 0, s>>>(static_cast<const uint4*>(results), static_cast<uint4*>(h_results), n16, states, h_states,
+                                 num_jobs);
 }
 
 void launch_init_rows(const Job* d_jobs, int num_jobs, const Params& p, const int32_t* rows, bool bagged_only,

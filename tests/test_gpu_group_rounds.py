@@ -31,3 +31,35 @@ def test_group_autotune_finishes_its_trial_trees():
     group.close()
     for L in members:
         L.close()
+
+
+def test_batch_calls_run_side_by_side():
+    """The learners of a batch call share all of the device's queues: sixteen small ones take less than three
+    times as long as four (3.4 times when only half of the queues are in use)."""
+    import time
+
+    import numpy as np
+    import torch
+    from lgbm_gb300 import BinnedDataset, GpuTreeLearner, LearnerConfig, train_batch
+    n = 2000
+    rng = np.random.default_rng(1)
+    X = rng.standard_normal((n, 10))
+    ds = BinnedDataset.from_dense(X)
+    g = torch.from_numpy((X[:, 0] + 0.3 * rng.standard_normal(n)).astype(np.float32)).cuda()
+    h = torch.from_numpy((0.1 + rng.random(n)).astype(np.float32)).cuda()
+    members = [GpuTreeLearner(ds, LearnerConfig(num_leaves=15, use_quantized_grad=1, seed=1)) for _ in range(32)]
+    torch.cuda.synchronize()
+
+    def run(count):
+        t = []
+        for _ in range(25):
+            a = time.perf_counter()
+            outs = train_batch(members[:count], [g.data_ptr()] * count, [h.data_ptr()] * count, on_device=True)
+            t.append(time.perf_counter() - a)
+        assert all(int(o[3][0]) == 15 for o in outs)
+        return float(np.median(t))
+
+    run(32)  # every learner's graph, and its place in the queues
+    assert run(16) < 2.9 * run(4)
+    for L in members:
+        L.close()
