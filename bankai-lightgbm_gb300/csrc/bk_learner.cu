@@ -880,7 +880,7 @@ void finish_trees(bk_learner* const* learners, size_t count, double shrinkage, d
       open.push_back(L);
     }
     if (open.empty()) return;
-    for (bk_learner* L : open) CK(cudaEventSynchronize(L->ev_end));
+    for (bk_learner* L : open) CK(cudaStreamSynchronize(L->stream));
   }
 }
 
@@ -953,7 +953,7 @@ int bk_learner_train(bk_learner* L, const float* gradients, const float* hessian
   }
   try {
     if (!train_enqueue(L, gradients, hessians, on_device, rows, num_rows, 0.0, nullptr)) return -1;
-    CK(cudaEventSynchronize(L->ev_end));
+    CK(cudaStreamSynchronize(L->stream));
     CK(cudaGetLastError());
     finish_trees(&L, 1, 0.0, nullptr);
     train_finish(L, splits, leaf_values, root_outputs, num_leaves_out);
@@ -1135,7 +1135,8 @@ int bk_learners_train_batch(bk_learner* const* learners, int32_t count, const fl
         set_error("bk_learners_train_batch: %s", msg.c_str());
         return -1;
       }
-    for (int32_t k = 0; k < count; ++k) CK(cudaEventSynchronize(learners[k]->ev_end));
+    for (i = 0; i < count; ++i) CK(cudaStreamSynchronize(learners[i]->stream));
+    i = 0;
     CK(cudaGetLastError());
     finish_trees(learners, (size_t)count, shrinkage, scores);
     for (i = 0; i < count; ++i)
