@@ -12,9 +12,10 @@
 //   bins_tm   [T] x uint8 [n][w_t]   the same runs tile-major: the root and dense leaves (a
 //                                quarter of the rows or more) stream each tile contiguously;
 //   bins_cm   uint8 [F][n]       column-major stored bins, read by the partition (one byte/row);
-//   pool      [L][T][B][32]      histogram pool, one slot per leaf (serial.rs:80-162 with a full
-//                                pool): double2 (grad, hess) on the float path, int64
-//                                (grad << 32) + hess on the quantized path;
+//   pool      [S][T][B][32]      histogram pool (serial.rs:80-162 with a full pool), S = one slot per
+//                                leaf, or 1 + max_exp for grow rounds (bk_rounds.cuh): double2
+//                                (grad, hess) on the float path, int64 (grad << 32) + hess on the
+//                                quantized path;
 // and per job (one tree of the K trees grown together): gradients, packed int8 gradients,
 // two row-index buffers (ping-pong between a leaf and its children) and, on the quantized path,
 // the packed values in the same leaf order beside them (the partition moves them with the row
@@ -124,7 +125,7 @@ struct Params {
 struct LeafConst {
   double sum_g, sum_h, parent, mgs, cnt_factor;  // mgs = min_gain_shift
   int64_t first_x, brk_x;  // quantized path: validity thresholds on the accumulated hessian
-  float mgs_up, mgs_dn;    // min_gain_shift rounded up / down to fp32
+  float mgs_dn;            // min_gain_shift rounded down to fp32
   float gsf, hsf, l2f;     // the gradient scale brought to [1, 2), the hessian scale and lambda_l2
   // the warp search's bounds (bk_search_warp.cuh), gains in units of gsf: hs2 = h + 2 lambda_l2, the error bound's factor
   // and constant (bk1 < 0: the leaf is outside its range), min_gain_shift - s0 rounded up / down
@@ -185,21 +186,23 @@ struct Job {
   LeafSum* leaf_sum;
   double* bgain;       // [L]   gain of each leaf's best split (the arg-max reads these)
   int32_t* bfeat;      // [L]   real feature of each leaf's best split
-  Cand* cand;          // [L][F] the candidate of every searched (leaf, feature); a leaf's best split is
-                       //        cand[leaf][inner feature of bsplit[leaf]]
+  Cand* cand;          // [cand_rows][F] the candidate of every searched (leaf, feature), rows by leaf, or by
+                       //        node in grow rounds; a leaf's best split is cand[leaf][inner feature of
+                       //        bsplit[leaf]]
   double* cgain;       // [2][F] gains of the current search's candidates (compact copy for the fold)
   uint8_t* csplit;     // [2][F] splittable flags of the current search's candidates
   uint32_t* cthr;      // [2][F] threshold | default_left << 31 of cand[]
   int64_t* bsplit;     // [L]   inner feature << 32 | threshold | default_left << 31 of each leaf's best split
-  LeafConst* lconst;   // [2]   constants of the smaller / larger leaf of the current search
-  uint8_t* splittable; // [L][F]
+  LeafConst* lconst;   // [2 round_w] constants of the smaller / larger leaf of the current search (of every
+                       //        expansion's, in grow rounds)
+  uint8_t* splittable; // [cand_rows][F] rows by pool slot, or by node in grow rounds
   uint8_t* used;       // [4][F] features searched in the current step; the by-node masks of the
                        //        smaller / larger leaf; the sample's scratch; then [L][path_words]
                        //        uint32 bitsets of the features on the path to each leaf
   uint8_t* tree_mask;  // [F]   features the tree may split on (by-tree column sample), 1 by default
   bk_split* records;   // [L-1]
   double* leaf_value;  // [L]
-  void* pool;          // [L][T][B][32]
+  void* pool;          // [slots][T][B][32]
   int64_t* part_cnt;   // [part_grid] partition block counts (scratch)
   double* red;         // reduction partials (scratch)
   int64_t* ired;       // integer reduction partials (scratch)

@@ -3,9 +3,11 @@
 // finishes. It runs its independent prologue (shared-memory setup, static metadata), then waits in
 // griddep_wait() until the previous grid has completed and its writes are visible. The histogram,
 // search and single-pass partition kernels call griddep_launch() right after that wait, so the
-// next kernel's CTAs are resident and through their own prologue by the time this one completes
-// (every grid of the chain is small enough to be resident beside the one before it); the stable
-// partition's kernels call it when only their last-CTA bookkeeping is left. Without the launch
+// next kernel's CTAs come in as this one's leave room and are through their own prologue by the time it
+// completes. Searches and partitions of small rounds fit beside the kernel before them; a histogram CTA
+// (1024 threads of 64 registers) takes an SM's whole register file, so on large rounds the next kernel's
+// CTAs start as the histogram's end. The stable partition's kernels call it when only their last-CTA
+// bookkeeping is left. Without the launch
 // attribute (or when the previous stream operation is not a kernel) both are no-ops.
 #pragma once
 #include <cuda_runtime.h>

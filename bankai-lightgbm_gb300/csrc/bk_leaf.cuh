@@ -95,7 +95,6 @@ __device__ __forceinline__ void compute_leaf_const_ls(const Job& J, const Params
   }
   c.parent = parent_output_of(p, root, ls);
   c.mgs = leaf_gain(p, c.sum_g, c.sum_h, ls.num_data, c.parent) + p.min_gain;
-  c.mgs_up = __double2float_ru(c.mgs);
   c.mgs_dn = __double2float_rd(c.mgs);
   {
     // without lambda_l2, s0 is the leaf's own gain (up to its rounding, which the bounds allow for)

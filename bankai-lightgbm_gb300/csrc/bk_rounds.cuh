@@ -12,12 +12,11 @@
 // round_w 16 a tree of 255 leaves takes about 22 rounds and, in practice, no work that the
 // one-by-one loop does not do; the records, leaf numbers, values and partitions are the same.
 // What bounds the one-by-one loop is its chain of 3 dependent launches per split (25 us, most of it
-// latency); a round is the same three launches (40 us for 4 small leaves, 90 us for 16 of 40,000
+// latency); a round is the same three launches (25 us for 4 small leaves, 80 us for 16 of 40,000
 // rows) for up to 16 splits, and its launches have enough rows and slices to fill the chip. A boosting
-// iteration, one split at a time -> in rounds (quantized unless said otherwise): 10M x 100, 255 leaves
-// 10.2 -> 4.39 ms; 10M x 200 12.1 -> 7.48 ms; 4M x 100 float 17.6 -> 9.44 ms; 300k x 40 with
-// categories 2.49 -> 0.95 ms; 100k x 28 float, 31 leaves 1.64 -> 0.75 ms; 5k x 20, 31 leaves 0.72 ->
-// 0.60 ms; 12 jobs in one graph 2.90 -> 2.01 ms.
+// iteration before rounds and now, other changes included: 10M x 100, 255 leaves 9.58 -> 3.75 ms; 10M x
+// 200 12.1 -> 6.06 ms; 4M x 100 float 16.9 -> 4.21 ms; 300k x 40 with categories 2.51 -> 0.77 ms; 100k x 28
+// float, 31 leaves 1.64 -> 0.50 ms; 5k x 20, 31 leaves 0.71 -> 0.44 ms; 12 jobs in one graph 2.90 -> 1.84 ms.
 //
 // An expanded leaf that is not split yet keeps its rows: they stay in its own index buffer (the
 // children are written to the other one, and are expanded only after the commit). Its pool slot goes

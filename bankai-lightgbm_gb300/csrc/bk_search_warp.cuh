@@ -17,8 +17,8 @@
 // Error bound (u = 2^-24), with t = a + b the numerator's root, a the integer part times the scales
 // (4u) and b the l2 part (5u): |d - exact| <= 44 u (|a| + |b|)^2 / denominator, plus the f64
 // rounding of the reference's own evaluation and its +kEpsilon on the hessians, together below
-// (4e-15 + 1.01e-15 / ymin) (s0 + d), where ymin = min_sum_hessian_in_leaf + l2 is the smallest
-// denominator of a valid position, plus 1e-24 where products underflow. So only the thresholds whose
+// (4e-15 + 1.01e-15 / ymin) (s0 + d), where ymin is the smallest denominator of a valid position
+// (bk_leaf.cuh), plus 1e-24 where products underflow; all of it with the gradients' scale brought to [1, 2). So only the thresholds whose
 // upper bound reaches the best lower bound of the CTA's features (when no feature is penalized) can
 // be the leaf's best split among them, and a feature is splittable if a lower bound passes
 // min_gain_shift; a feature with no certain answer evaluates every threshold that may pass. The

@@ -330,6 +330,8 @@ def run_gpu(args, rank, world):
                                        "algorithmic byte, %.3f) x this run's algorithmic bytes per launch"
                                        % HIST_TRAFFIC_PER_BYTE,
                      "kernel": "k_hist_int (quantized histogram)", "peak_kind": peak_kind,
+                     "form": "one split at a time, with phase timing on; the timed form builds up to 16 leaves' "
+                             "histograms in a launch",
                      "by_leaf_size": _roofline_by_leaf_size(roof["launches"], ds, n, peak)},
         "gpu_launches": launches_per_step * args.steps,
         "clocks": clk,
@@ -692,14 +694,14 @@ def run_hist_traffic(args):
 def _launches_per_step(leaves):
     """Kernels a step launches at least: objective gradients, job states, row init, discretization (4),
     root sums (2), pool zeroing, tree begin, three kernels (histogram, search, partition) for each grow
-    round captured with the tree, the tree's records, score update. A tree that takes more rounds, or
+    round captured with the tree, the tree's records, the results, score update. A tree that takes more rounds, or
     (launch shapes with clusters) one split at a time, launches more."""
     w = min(16, max(4, (leaves + 7) // 8))
     rounds = (leaves - 1 + w - 1) // w + 3 + (w - 1).bit_length()
     rounds = min(rounds + rounds % 2, leaves + leaves % 2)
     if leaves > 512:  # one split at a time
         rounds = leaves - 1
-    return 1 + 1 + 1 + 4 + 2 + 1 + 1 + 3 * rounds + 1 + 1
+    return 1 + 1 + 1 + 4 + 2 + 1 + 1 + 3 * rounds + 1 + 1 + 1
 
 
 def _shape_dict(shape, tuned):

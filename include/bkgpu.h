@@ -252,12 +252,14 @@ int bk_learner_reset_constant_hessian(bk_learner* learner, int32_t value);
 /* Threads per split-search CTA (one CTA per leaf side and feature) of the learner's next train call
  * (GB300-only) where it searches with a CTA per feature: 64 when every feature is numerical with at
  * most 63 searched bins and the grow loop runs the single-pass form without L1 / max_delta_step /
- * path_smooth, else 256. Large quantized rounds search eight features per 256-thread CTA. */
+ * path_smooth, else 256. Large quantized rounds do not: they search eight features per 256-thread CTA,
+ * which this call does not report. */
 int bk_learner_search_threads(bk_learner* learner, int32_t* threads);
 
 /* Replaces SerialTreeLearner::histogram_cache_capacity (serial.rs:250-252): the histogram slots
- * the learner keeps, into *capacity (host). This learner always keeps a full pool, one slot per
- * leaf (num_leaves), whatever histogram_pool_size says; the pool size never changes a result. */
+ * the learner keeps, into *capacity (host): num_leaves, as every leaf's histogram stays available
+ * whatever histogram_pool_size says (grow rounds hold up to 32 more for leaves that they expand ahead);
+ * the pool size never changes a result. */
 int bk_learner_histogram_cache_capacity(bk_learner* learner, int64_t* capacity);
 
 /* Replaces SerialTreeLearner::reset_histogram_pool_config (serial.rs:254-264), the Trainer's
