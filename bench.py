@@ -321,7 +321,8 @@ def run_gpu(args, rank, world):
                   "multiclass_k10": multiclass, "batched_jobs": batched_jobs, "binary_quantized_200": binary},
         "e2e": {"value": round(world * 1000.0 / e2e["ms_per_step"], 4), "unit": "iters/s",
                 "h2d_bytes_per_step": 2 * 4 * ds.num_data,
-                "d2h_bytes_per_step": 112 * (args.leaves - 1) + 8 * args.leaves + 8 + 8},
+                # a split record (152 bytes) and a leaf value for every leaf, and the rejected labels
+                "d2h_bytes_per_step": (152 + 8) * args.leaves + 16},
         "roofline": {"bound": "hbm", "achieved": round(hist_gbs, 1) if hist_gbs else None, "peak": peak,
                      "unit": "GB/s", "frac": round(hist_gbs / peak, 4) if hist_gbs else None,
                      "traffic": round(HIST_TRAFFIC_PER_BYTE * roof["hist_bytes"] / hist_launches, 0),
