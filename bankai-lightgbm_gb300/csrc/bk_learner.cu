@@ -198,12 +198,29 @@ struct bk_learner {
   std::vector<cudaEvent_t> hist_events;
   double last_total_ms = 0, last_hist_ms = 0, last_hist_bytes = 0, last_search_ms = 0, last_part_ms = 0;
 
+  // Small arrays share blocks: with a cudaMalloc each, a quantized learner of 1000 x 5 takes 583 us to
+  // create and 360 to destroy, with blocks 400 and 234 (ten class trees of 50k x 30: 2106 -> 1601).
+  static constexpr size_t kBlock = 512 << 10, kSmall = 64 << 10;
+  unsigned char* block = nullptr;
+  size_t block_left = 0;
+  void* device_alloc(size_t bytes) {
+    void* ptr = nullptr;
+    CK(cudaMalloc(&ptr, bytes));
+    allocs.push_back(ptr);
+    return ptr;
+  }
   template <typename T>
   T* dalloc(size_t count) {
-    void* ptr = nullptr;
-    CK(cudaMalloc(&ptr, std::max<size_t>(count * sizeof(T), 16)));
-    allocs.push_back(ptr);
-    return reinterpret_cast<T*>(ptr);
+    const size_t bytes = (std::max<size_t>(count * sizeof(T), 16) + 255) / 256 * 256;
+    if (bytes > kSmall) return reinterpret_cast<T*>(device_alloc(bytes));
+    if (bytes > block_left) {
+      block = static_cast<unsigned char*>(device_alloc(kBlock));
+      block_left = kBlock;
+    }
+    T* ptr = reinterpret_cast<T*>(block);
+    block += bytes;
+    block_left -= bytes;
+    return ptr;
   }
 
   ~bk_learner() {
