@@ -705,7 +705,9 @@ int learner_create(const bk_feature* features, int32_t num_features, const uint8
     L->d_results = L->dalloc<unsigned char>(L->results_bytes);
     CK(cudaMemset(L->d_results, 0, L->results_bytes));
     L->d_bad_label = reinterpret_cast<int32_t*>(L->d_results + L->results_bytes - 16);
-    JobState* d_states = L->dalloc<JobState>(K);
+    // the states apart from the small arrays: the plain form copies one back every split (62 splits of 1M x 67
+    // 4194 us, 4250 beside them)
+    JobState* d_states = static_cast<JobState*>(L->device_alloc(sizeof(JobState) * K));
     CK(cudaMemset(d_states, 0, sizeof(JobState) * K));
     for (int j = 0; j < K; ++j) {  // no by-node sampling until bk_learner_set_bynode
       const double one = 1.0;
