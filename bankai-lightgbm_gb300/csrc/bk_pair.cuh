@@ -92,16 +92,15 @@ __device__ __forceinline__ Pair pair_exp(Pair z, const ExpTable& T) {
 }
 
 // Rounds a (normalized) pair to fp32: false when a relative error `rel` of it could change the result,
-// or when the pair is so small that its low part, or the result itself, is not held in full.
+// or when the pair is so small that its low part, or the result itself, is not held in full (zero too).
 __device__ __forceinline__ bool pair_round(Pair a, float rel, float* out) {
   *out = a.hi;
-  const uint32_t b = __float_as_uint(a.hi) & 0x7fffffffu;
-  if (b < (40u << 23) || b >= (250u << 23)) return false;  // tiny (zero too), huge
-  if (a.lo == 0.f && rel < 1e-9f) return true;
-  // half a unit in the last place; below a power of two the units are half as large
-  const bool below = (b & 0x7fffffu) == 0u && (__float_as_uint(a.hi) ^ __float_as_uint(a.lo)) >> 31 != 0u;
-  const float half = __uint_as_float((b & 0x7f800000u) - ((below ? 25u : 24u) << 23));
-  return fabsf(__fsub_rn(half, fabsf(a.lo))) > __fmul_rn(rel, fabsf(a.hi));
+  const uint32_t u = __float_as_uint(a.hi), b = u & 0x7fffffffu;
+  uint32_t half = (b & 0x7f800000u) - (24u << 23);  // half a unit in the last place
+  // below a power of two the units are half as large
+  if ((b & 0x7fffffu) == 0u && (a.lo == 0.f || ((u ^ __float_as_uint(a.lo)) >> 31) != 0u)) half -= 1u << 23;
+  return b - (40u << 23) < (210u << 23) &&
+         fabsf(__fsub_rn(__uint_as_float(half), fabsf(a.lo))) > __fmul_rn(rel, fabsf(a.hi));
 }
 
 }  // namespace bk
