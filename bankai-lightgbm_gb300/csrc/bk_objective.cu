@@ -56,16 +56,15 @@ __global__ void __launch_bounds__(256) k_grad_l2(const double* __restrict__ scor
   }
 }
 
-// The reference's arithmetic of one binary row in f64.
-__device__ __noinline__ float2 binary_row(double score, bool pos, double sigmoid, double lw, const float* wi) {
-  const double lab = pos ? 1.0 : -1.0;
-  const double t = -lab * sigmoid;
-  const double e = exp(lab * sigmoid * score);
-  const double response = t / (1.0 + e);
-  const double ar = fabs(response);
-  const double q = ar * (sigmoid - ar);
-  if (wi) return make_float2((float)(response * lw * (double)*wi), (float)(q * lw * (double)*wi));
-  return make_float2((float)(response * lw), (float)(q * lw));
+// The reference's arithmetic of one binary row in f64 (zs = sigmoid * score; the factors with the label's sign
+// and label weights of 1 change nothing but signs).
+__device__ __noinline__ float2 binary_row(double zs, bool pos, double sigmoid, double lw, bool unit, const float* wi) {
+  const double e = exp(pos ? zs : -zs);
+  const double ar = sigmoid / (1.0 + e);
+  double r = ar, q = ar * (sigmoid - ar);
+  if (!unit) r *= lw, q *= lw;
+  if (wi) r *= (double)*wi, q *= (double)*wi;
+  return make_float2((float)(pos ? -r : r), (float)q);
 }
 
 __global__ void __launch_bounds__(256) k_grad_binary(const double* __restrict__ score, const float* __restrict__ label,
@@ -86,7 +85,8 @@ __global__ void __launch_bounds__(256) k_grad_binary(const double* __restrict__ 
     const double s = score[i];
     const bool pos = label[i] > 0.0f;
     bool ok;
-    Pair z = pair_of<true>(one ? s : sigmoid * s, &ok);  // exp(z) and 1 + exp(z): absolute errors count
+    const double zs = one ? s : sigmoid * s;
+    Pair z = pair_of<true>(zs, &ok);  // exp(z) and 1 + exp(z): absolute errors count
     if (!pos) z = pair_neg(z);
     ok = ok && ok_c && fabsf(z.hi) <= 60.0f;
     // a warp with a row for f64 takes all of them there: the f64 instructions cost the same
@@ -115,7 +115,7 @@ __global__ void __launch_bounds__(256) k_grad_binary(const double* __restrict__ 
       if (pos) gv = -gv;
     }
     if (!ok) {
-      const float2 v = binary_row(s, pos, sigmoid, pos ? lw_pos : lw_neg, w ? w + i : nullptr);
+      const float2 v = binary_row(zs, pos, sigmoid, pos ? lw_pos : lw_neg, unit, w ? w + i : nullptr);
       gv = v.x;
       hv = v.y;
     }
